@@ -213,7 +213,7 @@ int  ep_diffusion_half_step(ep_handle *h, int32_t *iters, double *relres);
  * Bval = B, dinv = 1/diag(A); values FP64 or FP32 per `precision`) and x,
  * which holds V on entry and A^-1 B V on return; stream may be NULL.  The
  * working vectors live in one static device array of this library sized for
- * at most 262144 rows (about 8.2 MB, held by every GPU that loads the
+ * at most 262144 rows (about 17 MB, held by every GPU that loads the
  * library until exit); larger n returns EP_ERR_ARG.  Every call shares that
  * array, so calls that overlap on the GPU race: serialise them.  Each call
  * looks up the array's address on the current device.  The call waits on
@@ -328,7 +328,9 @@ int  ep_assemble_operators(const ep_mesh_desc *mesh, const ep_cables_desc *cable
 
 /* Launch shape of ep_step (no reference counterpart).  cg_block: threads
  * per CTA of the persistent CG launch (128, 256, 512 or 768); cg_per_sm: its CTAs per
- * SM (0 = as many as are co-resident); ionic_block: threads per CTA of the
+ * SM (0 = by the size of the mesh: no more CTAs than it has slices for, and for
+ * cg_block 256 with cg_batch 4 one CTA of up to 1024 threads per SM on large
+ * meshes, since every CTA takes part in each iteration's reduction); ionic_block: threads per CTA of the
  * ionic kernel (64 or 128); graph_steps: 0 launches every kernel from the
  * host, k > 0 replays the steps from an instantiated CUDA graph of k steps
  * (rounded up to a multiple of the ECG interval); ionic_min_ctas: FP32
@@ -341,10 +343,10 @@ int  ep_assemble_operators(const ep_mesh_desc *mesh, const ep_cables_desc *cable
  * indices and values) into a ring of shared memory with asynchronous copies
  * while it gathers the current one, cg_prefetch units ahead (1..4; 0 = 2),
  * 256 threads per CTA, cg_variant 0 only);
- * cg_variant: 0 the CG recurrences of the reference (two reductions per
- * iteration), 1 the Chronopoulos-Gear recurrences (one reduction per
- * iteration; same iterates in exact arithmetic, rounding-level differences;
- * five more vectors on the device). */
+ * cg_variant: 0 the CG recurrences of the reference, both of an iteration's
+ * scalars taken from one reduction; 1 the Chronopoulos-Gear recurrences (same
+ * iterates in exact arithmetic, rounding-level differences; seven more
+ * vectors on the device). */
 typedef struct ep_launch_config {
     int32_t cg_block, cg_per_sm, ionic_block, graph_steps, ionic_min_ctas, cg_batch, cg_variant;
     int32_t cg_predict;   /* 1: each CG solve starts from V + the previous solve's

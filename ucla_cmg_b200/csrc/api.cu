@@ -71,6 +71,7 @@ struct ep_handle {
     DBuf cl;                             // explicit scheme: lumped capacitance C_L
     int cg_maxit = 1000;
     int cg_grid = 0, cg_block = 256;
+    int cg_threads = 256;                // threads per CTA of the planned launch (cg_block, or the library's choice)
     int ecg_every = 0;
     double act_thr = -40.0;
     TTOpts tt{};
@@ -78,11 +79,12 @@ struct ep_handle {
     long long step = 0;
     int nslices = 0;
     // device memory
-    DBuf V, S, Aval, Bval, dinv, r, q, p0, zv, consts, gks, lr_table, type, slice_ptr, col;
-    DBuf r1, w0, w1, s0, s1;             // single-reduction CG only (allocated on first use)
-    DBuf pd0, pd1, pvin;                 // CG predictor: x - V of the first / second half step, scratch
+    DBuf V, S, Aval, Bval, dinv, qd0, qd1, consts, gks, lr_table, type, slice_ptr, col;
+    DBuf r, r1, w0, w1, s0, s1, p0;      // Chronopoulos-Gear CG only (allocated on first use)
+    DBuf ex_tmp;                         // explicit scheme: scratch vector
+    DBuf pd0, pd1;                       // CG predictor: x - V of the first / second half step
     DBuf pq0, pq1;                       // linear CG predictor: each half step's next start, 2 delta - delta_prev
-    DBuf partial, bar, status, cg_stats, cg_last, d_step, track;
+    DBuf slots, partial, bar, status, cg_stats, cg_last, d_step, track;
     DBuf stim_head, stim_next, stim_on, stim_off, stim_amp;
     int nstim = 0;
     DBuf W, ecg_buf, ecg_partial, ecg_counter;
@@ -226,9 +228,9 @@ void fill_cg_args(ep_handle *h, CGArgs<R> &a) {
     a.n = h->n; a.nslices = h->nslices;
     a.slice_ptr = h->slice_ptr.as<int>(); a.col = h->col.as<int>();
     a.Aval = h->Aval.as<R>(); a.Bval = h->Bval.as<R>(); a.dinv = h->dinv.as<R>();
-    a.x = h->V.as<R>(); a.r = h->r.as<R>(); a.q = h->q.as<R>(); a.zp = h->zv.as<R>();
-    a.p0 = h->p0.as<R>();
-    a.partial = h->partial.as<double>();
+    a.x = h->V.as<R>();
+    a.q0 = h->qd0.as<R>(); a.q1 = h->qd1.as<R>();
+    a.slots = h->slots.as<CgSlot>();
     a.bar = h->bar.as<GridBarrier>();
     a.tol = h->cg_tol; a.maxit = h->cg_maxit;
     a.floor_rel = sizeof(R) == 4 ? 1.2e-7 : 2.2e-16;   // unit roundoff of R
@@ -240,9 +242,11 @@ void fill_cg_args(ep_handle *h, CGArgs<R> &a) {
     a.ninst = h->ninst;
     a.inst_row = h->d_inst_row.as<int>();
     a.inst_blk = h->d_inst_blk.as<int>();
+    a.r = h->r.as<R>(); a.p0 = h->p0.as<R>();
     a.r1 = h->r1.as<R>(); a.w0 = h->w0.as<R>(); a.w1 = h->w1.as<R>();
     a.s0 = h->s0.as<R>(); a.s1 = h->s1.as<R>();
-    a.delta = nullptr; a.dext = nullptr; a.vin = nullptr;   // the time step sets the predictor
+    a.partial = h->partial.as<double>();
+    a.delta = nullptr; a.dext = nullptr;   // the time step sets the predictor
     a.prefetch = h->cg_batch == kStagedBatch ? 0 : h->cg_prefetch;   // the staged kernel's is its ring depth
     a.bar_extra = h->bar_extra;
     a.depth = stage_depth(h);
@@ -277,10 +281,15 @@ int create_typed(ep_handle *h, const HostCSR &csr, const std::vector<double> &st
     }
     if ((rc = upload<R>(h->dinv, dinv))) return rc;
     const size_t vb = (size_t)h->pitch * sizeof(R);
-    if ((rc = h->r.alloc(vb)) || (rc = h->q.alloc(vb)) || (rc = h->p0.alloc(vb)) || (rc = h->zv.alloc(2 * vb)))
-        return rc;
-    EP_CUDA(cudaMemset(h->r.p, 0, vb)); EP_CUDA(cudaMemset(h->q.p, 0, vb)); EP_CUDA(cudaMemset(h->zv.p, 0, 2 * vb));
-    EP_CUDA(cudaMemset(h->p0.p, 0, vb));
+    if (h->scheme == EP_SCHEME_EXPLICIT) {
+        if ((rc = h->ex_tmp.alloc(vb))) return rc;
+    } else {
+        // rows past n are gathered by nobody; zero all the same
+        for (DBuf *b : {&h->qd0, &h->qd1}) {
+            if ((rc = b->alloc(4 * vb))) return rc;
+            EP_CUDA(cudaMemset(b->p, 0, 4 * vb));
+        }
+    }
     // cell states (SoA) and voltage
     std::vector<double> V(h->pitch, 0.0), S((size_t)h->ns * h->pitch, 0.0);
     const int off = is_lr(h->model) ? 0 : 1;       // LR keeps V in slot 7
@@ -433,25 +442,35 @@ extern "C" int ep_batch_plan(int32_t ninst, const int32_t *inst_row, int32_t gri
 
 // (re)size the CG launch for the handle's launch shape: grid, CTA groups,
 // partials, barriers and per-instance results
-// every instance's grid barrier back to its initial state (count, generation
-// and error word 0) with the handle's poll limit: at creation, and after a
-// wait gave up (the blocks that left early leave count and err behind)
+// every instance's grid barrier back to its initial state (count, generation,
+// error word and tags 0) with the handle's poll limit: at creation, and after
+// a wait gave up (the blocks that left early leave count and err behind, and
+// tags that the next solve would take for its own)
 static int reset_barriers(ep_handle *h) {
     std::vector<GridBarrier> b(h->ninst);
-    for (GridBarrier &x : b) x = GridBarrier{0u, 0u, 0u, h->wait_grid};
+    for (GridBarrier &x : b) x = GridBarrier{0u, 0u, 0u, h->wait_grid, 0ull, 0ull};
+    EP_CUDA(cudaMemsetAsync(h->slots.p, 0, h->slots.bytes, h->stream));
+    EP_CUDA(cudaStreamSynchronize(h->stream));
     EP_CUDA(cudaMemcpy(h->bar.p, b.data(), sizeof(GridBarrier) * b.size(), cudaMemcpyHostToDevice));
     return EP_OK;
 }
 
 static int plan_cg(ep_handle *h) {
     const int ws = stage_depth(h);
-    int rc = h->precision == EP_FP64
+    int rc;
+    h->cg_threads = h->cg_block;
+    if (h->cg_per_sm == 0)
+        rc = h->precision == EP_FP64
+                 ? cg_auto_shape<double>(h->nslices, h->ninst, h->cg_batch, h->cg_variant, ws, &h->cg_threads, &h->cg_grid)
+                 : cg_auto_shape<float>(h->nslices, h->ninst, h->cg_batch, h->cg_variant, ws, &h->cg_threads, &h->cg_grid);
+    else
+        rc = h->precision == EP_FP64
                  ? cg_grid_size<double>(h->cg_block, &h->cg_grid, h->cg_per_sm, h->cg_batch, h->cg_variant, ws)
                  : cg_grid_size<float>(h->cg_block, &h->cg_grid, h->cg_per_sm, h->cg_batch, h->cg_variant, ws);
     if (rc) return rc;
     if (h->cg_variant == 1 && !h->w0.p) {
         const size_t vb = (size_t)h->pitch * h->rsize;
-        for (DBuf *b : {&h->r1, &h->w0, &h->w1, &h->s0, &h->s1}) {
+        for (DBuf *b : {&h->r, &h->r1, &h->w0, &h->w1, &h->s0, &h->s1, &h->p0}) {
             if ((rc = b->alloc(vb))) return rc;
             EP_CUDA(cudaMemset(b->p, 0, vb));
         }
@@ -467,7 +486,9 @@ static int plan_cg(ep_handle *h) {
     }
     if ((rc = upload_raw(h->d_inst_row, h->inst_row.data(), h->inst_row.size()))) return rc;
     if ((rc = upload_raw(h->d_inst_blk, h->inst_blk.data(), h->inst_blk.size()))) return rc;
-    if ((rc = h->partial.alloc(sizeof(double) * 12 * (size_t)h->cg_grid))) return rc;
+    if (h->cg_variant == 1 && (rc = h->partial.alloc(sizeof(double) * 12 * (size_t)h->cg_grid))) return rc;
+    if ((rc = h->slots.alloc(sizeof(CgSlot) * 16 * (size_t)h->cg_grid))) return rc;
+    EP_CUDA(cudaMemsetAsync(h->slots.p, 0, h->slots.bytes, h->stream));
     if (h->bar.bytes != sizeof(GridBarrier) * (size_t)h->ninst) {
         if ((rc = h->bar.alloc(sizeof(GridBarrier) * (size_t)h->ninst))) return rc;
         if ((rc = reset_barriers(h))) return rc;
@@ -577,13 +598,13 @@ static int half_diffusion(ep_handle *h, const CGArgs<R> &ca) {
     if (h->scheme == EP_SCHEME_EXPLICIT) {
         for (double hh : h->ex_h) {
             int rc = launch_explicit<R>(h->n, h->nslices, h->slice_ptr.as<int>(), h->col.as<int>(), h->Aval.as<R>(),
-                                        h->cl.as<R>(), h->V.as<R>(), h->q.as<R>(), hh, h->stream);
+                                        h->cl.as<R>(), h->V.as<R>(), h->ex_tmp.as<R>(), hh, h->stream);
             if (rc) return rc;
         }
         h->launches += (long long)h->ex_h.size() - 1;
         return EP_OK;
     }
-    return launch_cg<R>(ca, h->cg_grid, h->cg_block, h->stream, h->cg_batch, h->cg_variant);
+    return launch_cg<R>(ca, h->cg_grid, h->cg_threads, h->stream, h->cg_batch, h->cg_variant);
 }
 
 // The plain ionic phase: the tissue model over every node, and in a mixed
@@ -621,7 +642,6 @@ static int step_typed(ep_handle *h, int nsteps, size_t &ne) {
     ca2 = ca;
     if (h->cg_predict) {
         ca.delta = h->pd0.as<R>(); ca2.delta = h->pd1.as<R>();
-        ca.vin = ca2.vin = h->pvin.as<R>();
         if (h->cg_predict == 2) { ca.dext = h->pq0.as<R>(); ca2.dext = h->pq1.as<R>(); }
     }
     int rc;
@@ -1646,7 +1666,7 @@ int ep_get_launch_config(const ep_handle *h, ep_launch_config *cfg) {
     int dev = 0, nsm = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    cfg->cg_per_sm = h->cg_grid / std::max(1, nsm);
+    cfg->cg_per_sm = h->cg_per_sm ? h->cg_grid / std::max(1, nsm) : 0;
     cfg->ionic_block = h->ionic_block;
     cfg->ionic_min_ctas = h->ionic_min;
     cfg->graph_steps = h->graph_steps;
@@ -1708,7 +1728,7 @@ int ep_set_launch_config(ep_handle *h, const ep_launch_config *cfg) {
     }
     const size_t vb = (size_t)h->pitch * h->rsize;
     if (cfg->cg_predict && !h->pd0.p) {
-        for (DBuf *b : {&h->pd0, &h->pd1, &h->pvin}) {
+        for (DBuf *b : {&h->pd0, &h->pd1}) {
             if ((rc = b->alloc(vb))) return rc;
             EP_CUDA(cudaMemset(b->p, 0, vb));
         }
@@ -1796,7 +1816,7 @@ int ep_autotune(ep_handle *h, int32_t trial_steps, ep_launch_config *best, doubl
     cur.cg_predict = h->cg_predict;
     cur.cg_prefetch = h->cg_prefetch;
     cur.sg_variant = h->sg_variant;
-    cur.cg_per_sm = h->cg_grid / std::max(1, nsm);
+    cur.cg_per_sm = h->cg_per_sm ? h->cg_grid / std::max(1, nsm) : 0;
     cur.ionic_block = h->ionic_block;
     cur.ionic_min_ctas = h->ionic_min;
     cur.graph_steps = h->graph_steps;

@@ -10,20 +10,27 @@
 // slice, one warp per slice, one lane per row) so every value/column load is
 // a coalesced 128-byte transaction.  A and B share the column array.
 //
-// Per iteration two grid barriers:
-//   phase A  p' = z + beta p (recomputed on the fly for each column, z =
-//            dinv r), q = A p', partial p'.q          -> barrier
-//   phase B  x += alpha p', r -= alpha q, partial r.z, r.r -> barrier
-// The same thread owns a row in every phase, so x, r, q need no cross-block
-// visibility; z and p are read across blocks, interleaved as (z_i, p_i) pairs
-// so that one load brings a neighbour's both (phase B writes the pair: the
-// new z and the p' it used).  Phase A gathers them with
-// plain (L1-allocating) loads: neither changes during the phase, and the grid
-// barrier before it (a gpu-scope fence after the arrival wait, then the CTA
-// barrier, as a cooperative grid sync) orders every block's writes of the
-// previous phase before them, so the neighbouring rows of a slice, which
-// gather many of the same nodes, hit L1 (2 % faster than L2-only loads on
-// the 2M-node shell, same bits).
+// One grid barrier per iteration.  Each node keeps (z, p, w, d) together, z =
+// dinv r, p the direction, w = dinv A p, d = x - V, double-buffered.  One sweep of an
+// iteration rebuilds, for every column it gathers, the neighbour's new
+//   z' = z - alpha w,  p' = z' + beta p
+// from its old triple (explicit fma, so the owner and every neighbour round
+// alike), forms q = A p' and writes the own row's (z', p', dinv q, d + alpha
+// p) to the other buffer; nothing of the old buffer changes during the sweep.
+// alpha and beta come from one reduction at the end of the sweep: besides
+// (p', q) and the residual's own (r, z), (r, r) it sums the products that
+// give the next residual's,
+//   (r, z)_next = (r, z) - 2 alpha d(z, w) + alpha^2 d(w, w)   (d = diag A)
+// and (r, r)_next likewise.  Both start from sums of the vectors themselves
+// in every sweep, so the differences (one iteration's reduction, a factor of
+// ten or so, out of FP64's sixteen digits) do not accumulate: the iterates
+// and the stop test are those of the two-reduction recurrences to rounding.
+// The second sweep and second barrier of those (x, r, z updated after alpha
+// is known) cost 12 us a phase with 888 CTAs polling one counter, which was
+// most of a solve's time on every mesh under a million nodes.
+// Gathers are plain (L1-allocating) loads: the barrier's acquire orders every
+// block's writes of the previous sweep before them, and the rows of a slice
+// share many neighbours.
 // Dot products accumulate in FP64 whatever the vector type.  Reductions
 // sum the per-block partials in block order, so results are deterministic.
 #include <algorithm>
@@ -35,20 +42,164 @@ namespace ep {
 __device__ __forceinline__ float ldcg(const float *p) { return __ldcg(p); }
 __device__ __forceinline__ double ldcg(const double *p) { return __ldcg(p); }
 
-// p' = z + beta p with z = dinv r, written as one explicit fma so the owner
-// row and every neighbour that recomputes it round identically
+// A node's vectors, (z, p, w, d), d the correction x - V so far (added to V
+// once, at the end, so V is rounded once a solve): one 16-byte (FP64: 32-byte) record, so a
+// neighbour's z, p and w come from one sector.
+template <typename R> struct Quad { R z, p, w, d; };
+__device__ __forceinline__ Quad<float> quad_load(const float *q, int i) {
+    const float4 t = reinterpret_cast<const float4 *>(q)[i];
+    return {t.x, t.y, t.z, t.w};
+}
+__device__ __forceinline__ Quad<double> quad_load(const double *q, int i) {
+    const double2 *t = reinterpret_cast<const double2 *>(q) + 2 * (size_t)i;
+    const double2 u = t[0], v = t[1];
+    return {u.x, u.y, v.x, v.y};
+}
+__device__ __forceinline__ void quad_store(float *q, int i, float z, float p, float w, float d) {
+    reinterpret_cast<float4 *>(q)[i] = make_float4(z, p, w, d);
+}
+__device__ __forceinline__ void quad_store(double *q, int i, double z, double p, double w, double d) {
+    double2 *t = reinterpret_cast<double2 *>(q) + 2 * (size_t)i;
+    t[0] = make_double2(z, p);
+    t[1] = make_double2(w, d);
+}
+// the new direction p' = (z - alpha w) + beta p of a gathered node
 template <typename R>
-__device__ __forceinline__ R pdir(R dinv, R r, R beta, R p) { return fma(beta, p, dinv * r); }
-// the same with z = dinv r already rounded and stored
-template <typename R>
-__device__ __forceinline__ R pdir_z(R z, R beta, R p) { return fma(beta, p, z); }
+__device__ __forceinline__ R quad_dir(const R *q, int c, R alpha, R beta);
+template <>
+__device__ __forceinline__ float quad_dir(const float *q, int c, float alpha, float beta) {
+    const float4 t = reinterpret_cast<const float4 *>(q)[c];
+    return fmaf(beta, t.y, fmaf(-alpha, t.z, t.x));
+}
+template <>
+__device__ __forceinline__ double quad_dir(const double *q, int c, double alpha, double beta) {
+    const double2 u = reinterpret_cast<const double2 *>(q)[2 * (size_t)c];
+    const double w = q[4 * (size_t)c + 2];
+    return fma(beta, u.y, fma(-alpha, w, u.x));
+}
 
-// the gathered pair (z_i, p_i) of the two-reduction kernels, interleaved so a
-// neighbour's two values come in one load (zp[2i] = z_i, zp[2i+1] = p_i)
-template <typename R> struct ZP;
-template <> struct ZP<float> { using T = float2; };
-template <> struct ZP<double> { using T = double2; };
-template <typename R> using zp_t = typename ZP<R>::T;
+// ---- grid barrier and reduction in one ----
+// Every CTA of a group publishes its partial sums as 16-byte {value, tag}
+// units (one 128-byte line per CTA) and then reads every other CTA's line
+// until the tags are this phase's: one store and one load round trip, where
+// a counter barrier followed by a read of the partials takes an atomic, a
+// generation poll and a read.  A unit is one 128-bit access, so a value
+// never comes with another phase's tag.  Two sets of lines alternate: a CTA
+// writes set s again only after the next phase's tags of everybody, which
+// nobody publishes before it has read set s.  Tags go on from launch to
+// launch (GridBarrier::seq), so a line never holds a tag of the future.
+// Waits are bounded as in grid_sync.  A group of one CTA needs no global
+// memory at all.
+constexpr int kRedMax = 8;                    // values of one reduction, at most
+__device__ __forceinline__ void slot_store(CgSlot *p, double v, unsigned long long tag) {
+    asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(p),
+                 "l"((unsigned long long)__double_as_longlong(v)), "l"(tag)
+                 : "memory");
+}
+__device__ __forceinline__ void slot_load(const CgSlot *p, double &v, unsigned long long &tag) {
+    unsigned long long u;
+    asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+                 : "=l"(u), "=l"(tag)
+                 : "l"(p)
+                 : "memory");
+    v = __longlong_as_double((long long)u);
+}
+__device__ __forceinline__ void fence_acq_rel_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+
+// NV <= 8 sums over the CTAs [b0, b0 + nb) of a group, the same bits in every
+// thread of every CTA, and a barrier between what the group wrote before and
+// what it reads after.  false: a wait gave up.
+template <int NV>
+__device__ __forceinline__ bool group_reduce(CgSlot *slots, int G, unsigned long long tag, int b0, int nb,
+                                             unsigned int hold, GridBarrier *bar, const double (&vin)[NV],
+                                             double (&tot)[NV]) {
+    static_assert(NV <= kRedMax, "too many values");
+    __shared__ double sh_a[32][kRedMax], sh_b[32][kRedMax];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+    // a warp's sums: each step halves the values a lane carries, so lane l
+    // ends with value l / 4 (18 shuffles for 8 FP64 sums instead of 80)
+    double v[kRedMax];
+#pragma unroll
+    for (int k = 0; k < kRedMax; k++) v[k] = k < NV ? vin[k < NV ? k : 0] : 0.0;
+#pragma unroll
+    for (int st = 0; st < 3; st++) {
+        const int half = 4 >> st, o = 16 >> st;
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int i = 0; i < half; i++) {
+            const double send = up ? v[i] : v[i + half], keep = up ? v[i + half] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+    if ((lane & 3) == 0) sh_a[warp][lane >> 2] = v[0];
+    __syncthreads();
+    // value lane & 7 summed over the rows of a [rows][8] array, on every lane
+    auto column_sum = [&](const double (*sh)[kRedMax], int rows) {
+        double t = 0.0;
+        for (int r = lane >> 3; r < rows; r += 4) t += sh[r][lane & 7];
+        t += __shfl_xor_sync(0xffffffffu, t, 8);
+        t += __shfl_xor_sync(0xffffffffu, t, 16);
+        return t;
+    };
+    double t;
+    if (nb == 1 && !hold) {
+        t = column_sum(sh_a, nw);
+        __syncthreads();                      // sh_a is free again
+    } else {
+        CgSlot *set = slots + (size_t)(tag & 1) * G * kRedMax;
+        if (warp == 0) {
+            const double mine = column_sum(sh_a, nw);
+            fence_acq_rel_gpu();              // the CTA's writes (ordered here by the CTA barrier) before the tag
+            if (lane < NV) slot_store(set + (size_t)blockIdx.x * kRedMax + lane, mine, tag);
+        }
+        const unsigned int lim = bar->limit ? bar->limit : kGridPolls;
+        const CgSlot *grp = set + (size_t)b0 * kRedMax;
+        const int units = nb * kRedMax;
+        const bool mine = (tid & (kRedMax - 1)) < NV;
+        unsigned int polls = 0;
+        int bad = 0;
+        double acc = 0.0;
+        for (int u0 = tid; u0 < units && mine && !bad; u0 += 4 * (int)blockDim.x) {
+            double x[4];
+            unsigned int pend = 0;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                x[i] = 0.0;
+                if (u0 + i * (int)blockDim.x < units) pend |= 1u << i;
+            }
+            if (hold) pend |= 16u;            // arrivals that never come (ep_test_hold_barrier)
+            while (pend) {
+                unsigned long long tg[4];
+                double xv[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+                    if (pend >> i & 1u) slot_load(grp + u0 + i * (int)blockDim.x, xv[i], tg[i]);
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+                    if ((pend >> i & 1u) && tg[i] == tag) { x[i] = xv[i]; pend &= ~(1u << i); }
+                if (pend) {
+                    if (++polls > lim) { atomicExch(&bar->err, 1u); bad = 1; break; }
+                    if ((polls & 15u) == 0) {
+                        if (*(volatile unsigned int *)&bar->err) { bad = 1; break; }
+                        __nanosleep(64);
+                    }
+                }
+            }
+            acc += (x[0] + x[1]) + (x[2] + x[3]);
+        }
+        fence_acq_rel_gpu();
+        acc += __shfl_xor_sync(0xffffffffu, acc, 8);
+        acc += __shfl_xor_sync(0xffffffffu, acc, 16);
+        if (lane < kRedMax) sh_b[warp][lane] = acc;
+        if (__syncthreads_or(bad)) return false;
+        t = column_sum(sh_b, nw);
+    }
+#pragma unroll
+    for (int k = 0; k < NV; k++) tot[k] = __shfl_sync(0xffffffffu, t, k);
+    return true;
+}
 
 template <int NV>
 __device__ __forceinline__ void block_reduce_store(double (&v)[NV], double *out, int stride) {
@@ -254,13 +405,179 @@ __device__ __forceinline__ R slice_row_sum_pipe(const int *__restrict__ col, con
     return acc;
 }
 
-// register budget: NB = 4 takes 42 (six 256-thread CTAs, or two of 768, per
-// SM); NB = 8 takes 64 (four 256-thread CTAs) for twice the loads in flight;
-// NB = 16 is NB = 8 software-pipelined (64 registers)
+constexpr int kUnitCols = 8;
+
+__host__ __device__ inline size_t unit_bytes(int rsize) { return (size_t)kUnitCols * kSlice * (4 + (size_t)rsize); }
+// dynamic shared memory of a CTA of `block` threads, `depth` units in flight per warp
+__host__ __device__ inline size_t stage_smem_bytes(int block, int depth, int rsize) {
+    return (size_t)(block / 32) * (size_t)(depth + 1) * unit_bytes(rsize);
+}
+
+__device__ __forceinline__ uint32_t cg_smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ uint64_t l2_evict_first_policy() {
+    uint64_t pol;
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
+    return pol;
+}
+
+// one 16-byte global -> shared copy, cached in L2 only (both addresses
+// 16-byte aligned: every unit starts on a 128-byte boundary of the SELL
+// arrays and of the ring)
+__device__ __forceinline__ void cp16(void *dst, const void *src, uint64_t pol) {
+    asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(cg_smem_u32(dst)), "l"(src),
+                 "l"(pol)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+// this thread's copies of every unit but the newest depth - 1 have landed
+__device__ __forceinline__ void unit_wait(int depth) {
+    switch (depth) {
+        case 1: cp_wait<0>(); break;
+        case 2: cp_wait<1>(); break;
+        case 3: cp_wait<2>(); break;
+        default: cp_wait<3>(); break;
+    }
+}
+
+template <typename R>
+struct UnitRing {
+    int *idx;          // slot k's indices at idx + k * kUnitCols * kSlice
+    R *val;            // slot k's values at val + k * kUnitCols * kSlice
+    int slots, depth;  // slots = depth + 1
+    int L;             // this warp's slices per sweep (0: nothing to stage)
+    int j, k, beg, w;  // producer cursor: slice j of the warp, its column k, start, width
+    int issued;        // units issued so far
+    uint64_t pol;
+};
+
+// issue the unit under the cursor into the ring slot of its position and
+// advance the cursor (the next unit of the slice, or the next slice,
+// wrapping to the warp's first slice: the next sweep).  Every lane commits
+// one copy group per call, empty or not, so the group counts stay uniform.
+template <typename R>
+__device__ __forceinline__ void unit_issue(UnitRing<R> &q, const CGArgs<R> &a, int gwarp, int nwarps, int lane) {
+    if (q.L > 0) {
+        const int slot = q.issued % q.slots;
+        const int nc = min(kUnitCols, q.w - q.k);
+        int *di = q.idx + slot * (kUnitCols * kSlice);
+        R *dv = q.val + slot * (kUnitCols * kSlice);
+        const int *si = a.col + q.beg + q.k * kSlice;
+        const R *sv = a.Aval + q.beg + q.k * kSlice;
+        // indices: column u, 16-byte piece p is chunk c = 8 u + p
+#pragma unroll
+        for (int t = 0; t < 2; t++) {
+            const int c = lane + 32 * t;
+            if ((c >> 3) < nc) cp16(di + 4 * c, si + 4 * c, q.pol);
+        }
+        // values: VPC chunks of VE values per column
+        constexpr int VPC = kSlice * (int)sizeof(R) / 16, VE = 16 / (int)sizeof(R);
+#pragma unroll
+        for (int t = 0; t < VPC * kUnitCols / 32; t++) {
+            const int c = lane + 32 * t;
+            if (c / VPC < nc) cp16(dv + VE * c, sv + VE * c, q.pol);
+        }
+        q.k += kUnitCols;
+        while (q.k >= q.w) {               // ends: some slice of the warp has columns (q.L > 0)
+            q.j = q.j + 1 == q.L ? 0 : q.j + 1;
+            const int s = gwarp + q.j * nwarps;
+            q.beg = __ldg(a.slice_ptr + s);
+            q.w = (__ldg(a.slice_ptr + s + 1) - q.beg) / kSlice;
+            q.k = 0;
+        }
+    }
+    q.issued++;
+    cp_commit();
+}
+
+// the warp's ring and its cursor at the first unit
+template <typename R>
+__device__ __forceinline__ void ring_start(UnitRing<R> &q, const CGArgs<R> &a, unsigned char *sm, int gwarp, int nwarps,
+                                           int s_hi) {
+    q.depth = a.depth;
+    q.slots = a.depth + 1;
+    // slots x unit of indices, then slots x unit of values
+    unsigned char *base = sm + (size_t)(threadIdx.x >> 5) * q.slots * unit_bytes((int)sizeof(R));
+    q.idx = reinterpret_cast<int *>(base);
+    q.val = reinterpret_cast<R *>(base + (size_t)q.slots * kUnitCols * kSlice * 4);
+    q.L = gwarp < s_hi ? (s_hi - gwarp + nwarps - 1) / nwarps : 0;
+    int cols = 0;
+    for (int j = 0; j < q.L; j++) {
+        const int s = gwarp + j * nwarps;
+        cols += __ldg(a.slice_ptr + s + 1) - __ldg(a.slice_ptr + s);
+    }
+    if (cols == 0) q.L = 0;
+    q.j = 0;
+    q.k = 0;
+    q.beg = q.L > 0 ? __ldg(a.slice_ptr + gwarp) : 0;
+    q.w = q.L > 0 ? (__ldg(a.slice_ptr + gwarp + 1) - q.beg) / kSlice : 0;
+    while (q.L > 0 && q.w == 0) {      // ends: some slice has columns
+        q.j++;
+        const int s = gwarp + q.j * nwarps;
+        q.beg = __ldg(a.slice_ptr + s);
+        q.w = (__ldg(a.slice_ptr + s + 1) - q.beg) / kSlice;
+    }
+    q.issued = 0;
+    q.pol = l2_evict_first_policy();
+}
+
+// the row sum of a slice of w columns out of the ring
+template <typename R, typename F>
+__device__ __forceinline__ R ring_row_sum(UnitRing<R> &q, const CGArgs<R> &a, int gwarp, int nwarps, int lane, int w,
+                                          int &cons, F gather) {
+    R acc = R(0);
+    for (int k = 0; k < w; k += kUnitCols, cons++) {
+        unit_wait(q.depth);
+        __syncwarp();                 // the unit is visible to every lane, and every
+                                      // lane is done with the slot refilled next
+        unit_issue(q, a, gwarp, nwarps, lane);
+        const int off = (cons % q.slots) * (kUnitCols * kSlice) + lane;
+        const int *ci = q.idx + off;
+        const R *cv = q.val + off;
+        const int nc = min(kUnitCols, w - k);
+        int c[kUnitCols];
+        R g[kUnitCols];
+#pragma unroll
+        for (int u = 0; u < kUnitCols; u++)
+            if (u < nc) c[u] = ci[u * kSlice];
+#pragma unroll
+        for (int u = 0; u < kUnitCols; u++)
+            if (u < nc) g[u] = gather(c[u]);
+#pragma unroll
+        for (int u = 0; u < kUnitCols; u++)
+            if (u < nc) acc += cv[u * kSlice] * g[u];
+    }
+    return acc;
+}
+
+// The solve.  NB: slice columns gathered together (4, 8; 16: 8 with the next
+// group's indices and values loaded ahead; kStagedBatch: 8 out of a shared-
+// memory ring, below).  64 registers in all of them, so one CTA of up to 1024
+// threads (NB = 4) or four of 256 per SM.
+//
+// The staged form takes the matrix stream of the sweeps off the warps'
+// critical path.  A warp's slices are cut into units of kUnitCols slice
+// columns: the column indices and A values of one slice's columns k .. k+7 (8
+// x 128 bytes of indices, 8 x 32 x sizeof(R) bytes of values).  The warp
+// copies the units into a ring of shared memory with per-thread asynchronous
+// copies (cp.async.cg: 16 bytes each, L2 only, evict-first, so the matrix
+// streams through L2 while the gathered records stay there), `depth` units
+// ahead of the one it gathers for; the loads in flight occupy ring slots
+// instead of registers.  The stream runs on past the end of a sweep into the
+// next iteration's first units (the matrix does not change), under the
+// reduction.  No wait on it spins: cp.async.wait_group is the hardware's wait
+// for the thread's own copies, and every exit path waits for all of them.
+// Same order of additions in every form, so the same bits on the same grid.
 template <typename R, int NB>
-__global__ void __launch_bounds__(NB == 4 ? 768 : 256, NB == 4 ? 2 : 4) k_cn_half(const CGArgs<R> a) {
+__global__ void __launch_bounds__(NB == 4 ? 1024 : 256, NB == 4 ? 1 : (NB == kStagedBatch && sizeof(R) == 8) ? 3 : 4)
+k_cn_half(const CGArgs<R> a) {
+    constexpr bool STAGED = NB == kStagedBatch;
+    extern __shared__ __align__(128) unsigned char cg_sm[];
     const int lane = threadIdx.x & 31;
-    const int G = gridDim.x;                 // partial-array stride
+    const int G = gridDim.x;
     // this CTA's instance: its rows, its CTA group and its barrier
     int inst = 0, b0 = 0, nb = G, rb = 0, re = a.n;
     if (a.ninst > 1) {
@@ -274,24 +591,34 @@ __global__ void __launch_bounds__(NB == 4 ? 768 : 256, NB == 4 ? 2 : 4) k_cn_hal
         rb = a.inst_row[inst]; re = a.inst_row[inst + 1];
     }
     GridBarrier *bar = a.bar + inst;
-    const unsigned int nblk = nb + a.bar_extra;
+    unsigned long long tag = *(volatile unsigned long long *)&bar->seq;
     const int s_lo = rb / kSlice, s_hi = (re + kSlice - 1) / kSlice;
     const int gwarp = s_lo + (((int)blockIdx.x - b0) * (int)blockDim.x + (int)threadIdx.x) / 32;
     const int nwarps = (nb * (int)blockDim.x) >> 5;
 
-    // ---- prologue: r = B x - A x, z = dinv r, p = 0 ----
+    UnitRing<R> ring;                         // this warp's ring (staged form)
+    if constexpr (STAGED) {
+        ring_start(ring, a, cg_sm, gwarp, nwarps, s_hi);
+        for (int d = 0; d < ring.depth; d++) unit_issue(ring, a, gwarp, nwarps, lane);
+    }
+
+    // ---- prologue: r = B x - A x, z = dinv r, p = w = 0 ----
     // With a predictor (delta: the previous solve's correction x - V of
     // this half step; with dext its linear extrapolation 2 delta - delta_prev,
     // stored by the previous solve) the iteration starts from x + pred
     // instead, r = B x - A (x + pred), while the stop test keeps the
-    // reference's r0 = B x - A x; x itself is not touched before the barrier
+    // reference's r0 = B x - A x.  a.x itself is written only at the end
     // (neighbours read it here).
     const bool pred = a.delta != nullptr;
     const bool lin = a.dext != nullptr;
+    R *cur = a.q0, *nxt = a.q1;
+    double rr0, stop2, rr_last;
+    bool converged;
     {
-        double v[4] = {0.0, 0.0, 0.0, 0.0};
+        double v[3] = {0.0, 0.0, 0.0};
         for (int s = gwarp; s < s_hi; s += nwarps) {
-            if (a.prefetch) prefetch_slice(a.slice_ptr, a.col, a.Aval, a.Bval, s + a.prefetch * nwarps, s_hi, lane);
+            if (!STAGED && a.prefetch)
+                prefetch_slice(a.slice_ptr, a.col, a.Aval, a.Bval, s + a.prefetch * nwarps, s_hi, lane);
             const int row = s * kSlice + lane;
             const int beg = a.slice_ptr[s], w = (a.slice_ptr[s + 1] - beg) / kSlice;
             R ax = R(0), bx = R(0), ad = R(0);
@@ -301,140 +628,102 @@ __global__ void __launch_bounds__(NB == 4 ? 768 : 256, NB == 4 ? 2 : 4) k_cn_hal
             if (row >= rb && row < re) {
                 const R rref = bx - ax;
                 const R r = pred ? rref - ad : rref;
-                const R z = __ldg(a.dinv + row) * r;
-                a.r[row] = r;
-                reinterpret_cast<zp_t<R> *>(a.zp)[row] = zp_t<R>{z, R(0)};
-                if (pred) a.vin[row] = a.x[row];
-                v[0] += (double)r * (double)z;
-                v[1] += (double)r * (double)r;
-                v[2] += (double)bx * (double)bx;
-                v[3] += (double)rref * (double)rref;
+                quad_store(cur, row, __ldg(a.dinv + row) * r, R(0), R(0),
+                           pred ? (lin ? a.dext[row] : a.delta[row]) : R(0));
+                v[0] += (double)r * (double)r;
+                v[1] += (double)bx * (double)bx;
+                v[2] += (double)rref * (double)rref;
             }
         }
-        block_reduce_store<4>(v, a.partial + 6 * G, G);      // slots [6G, 10G): the iterations use [0, 4G)
+        double t[3];
+        if (!group_reduce(a.slots, G, ++tag, b0, nb, a.bar_extra, bar, v, t)) {
+            if constexpr (STAGED) cp_wait_all();
+            return;
+        }
+        // ||r|| <= tol ||r0||, or the residual is at the resolution of b in the
+        // vector type (FP32 cannot resolve a 1e-7 reduction of an r0 that is
+        // itself rounding noise of B x - A x; in FP64 the floor is ~1e-16 ||b||)
+        rr0 = t[2];
+        stop2 = fmax(a.tol * a.tol * rr0, a.floor_rel * a.floor_rel * t[1]);
+        rr_last = t[0];
+        converged = t[0] <= stop2;
     }
-    if (!grid_sync(bar, nblk)) return;
-    double rz, rr_start, bb, rr0;
-    {
-        double t[4];
-        grid_total<4>(a.partial + 6 * G, G, b0, nb, t);
-        rz = t[0]; rr_start = t[1]; bb = t[2]; rr0 = t[3];
-    }
-    // ||r|| <= tol ||r0||, or the residual is at the resolution of b in the
-    // vector type (FP32 cannot resolve a 1e-7 reduction of an r0 that is
-    // itself rounding noise of B x - A x; in FP64 the floor is ~1e-16 ||b||)
-    const double floor2 = a.floor_rel * a.floor_rel * bb;
-    const double stop2 = fmax(a.tol * a.tol * rr0, floor2);
-    double beta = 0.0;
-    int it = 0;
-    bool converged = (rr_start <= stop2);
-    double rr_last = rr_start;
-    zp_t<R> *zp = reinterpret_cast<zp_t<R> *>(a.zp);
-    R *pn = a.p0;                             // p' of the own rows, phase A -> phase B
+    int it = 0, cons = 0;                     // cons: ring units consumed so far
+    R al = R(0), be = R(0);
     while (!converged && it < a.maxit) {
-        // ---- phase A: p' = z + beta p; q = A p' ----
-        {
-            double v[1] = {0.0};
-            const R bR = (R)beta;
-            for (int s = gwarp; s < s_hi; s += nwarps) {
-                if (a.prefetch)
-                    prefetch_slice<R>(a.slice_ptr, a.col, a.Aval, nullptr, s + a.prefetch * nwarps, s_hi, lane);
-                const int row = s * kSlice + lane;
-                const int beg = a.slice_ptr[s], w = (a.slice_ptr[s + 1] - beg) / kSlice;
-                auto gat = [&](int c) { const zp_t<R> t = zp[c]; return pdir_z(t.x, bR, t.y); };
-                R q;
-                if constexpr (NB == 16) q = slice_row_sum_pipe<8>(a.col, a.Aval, beg, w, lane, gat);
-                else q = slice_row_sum<NB>(a.col, a.Aval, beg, w, lane, gat);
-                if (row >= rb && row < re) {
-                    const zp_t<R> t = zp[row];
-                    const R pi = pdir_z(t.x, bR, t.y);
-                    pn[row] = pi;
-                    a.q[row] = q;
-                    v[0] += (double)pi * (double)q;
-                }
+        double v[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        for (int s = gwarp; s < s_hi; s += nwarps) {
+            if (!STAGED && a.prefetch)
+                prefetch_slice<R>(a.slice_ptr, a.col, a.Aval, nullptr, s + a.prefetch * nwarps, s_hi, lane);
+            const int row = s * kSlice + lane;
+            const int beg = __ldg(a.slice_ptr + s), w = (__ldg(a.slice_ptr + s + 1) - beg) / kSlice;
+            auto gat = [&](int c) { return quad_dir(cur, c, al, be); };
+            R q;
+            if constexpr (STAGED) q = ring_row_sum(ring, a, gwarp, nwarps, lane, w, cons, gat);
+            else if constexpr (NB == 16) q = slice_row_sum_pipe<8>(a.col, a.Aval, beg, w, lane, gat);
+            else q = slice_row_sum<NB>(a.col, a.Aval, beg, w, lane, gat);
+            if (row >= rb && row < re) {
+                const Quad<R> o = quad_load(cur, row);
+                const R di = __ldg(a.dinv + row);
+                const R z = fma(-al, o.w, o.z), p = fma(be, o.p, z), wv = di * q;
+                quad_store(nxt, row, z, p, wv, fma(al, o.p, o.d));
+                const double d = (double)(R(1) / di), dz = d * (double)z, dw = d * (double)wv;
+                v[0] += (double)p * (double)q;
+                v[1] += dz * (double)z;
+                v[2] += dz * (double)wv;
+                v[3] += dw * (double)wv;
+                v[4] += dz * dz;
+                v[5] += dz * dw;
+                v[6] += dw * dw;
             }
-            block_reduce_store<1>(v, a.partial + 3 * G, G);   // disjoint from the neighbours' slots
         }
-        if (!grid_sync(bar, nblk)) return;
-        double pq;
-        {
-            double t[1];
-            grid_total<1>(a.partial + 3 * G, G, b0, nb, t);
-            pq = t[0];
+        double t[7];
+        if (!group_reduce(a.slots, G, ++tag, b0, nb, a.bar_extra, bar, v, t)) {
+            if constexpr (STAGED) cp_wait_all();
+            return;
         }
-        const double alpha = rz / pq;
-        // ---- phase B: x += alpha p', r -= alpha q, z = dinv r ----
-        // two of the warp's slices a pass: both slices' loads are issued
-        // before either is updated (the rows are added to the dots in the
-        // same order as one slice at a time)
-        {
-            double v[2] = {0.0, 0.0};
-            const R aR = (R)alpha;
-            for (int s = gwarp; s < s_hi; s += 2 * nwarps) {
-                const int row = s * kSlice + lane, row2 = row + nwarps * kSlice;
-                const bool on = row >= rb && row < re;
-                const bool on2 = s + nwarps < s_hi && row2 >= rb && row2 < re;
-                R pi = R(0), xi = R(0), ri = R(0), qi = R(0), di = R(0);
-                R pi2 = R(0), xi2 = R(0), ri2 = R(0), qi2 = R(0), di2 = R(0);
-                if (on) { pi = pn[row]; xi = a.x[row]; ri = a.r[row]; qi = a.q[row]; di = __ldg(a.dinv + row); }
-                if (on2) { pi2 = pn[row2]; xi2 = a.x[row2]; ri2 = a.r[row2]; qi2 = a.q[row2]; di2 = __ldg(a.dinv + row2); }
-                if (on) {
-                    a.x[row] = xi + aR * pi;
-                    const R r = ri - aR * qi;
-                    a.r[row] = r;
-                    const R z = di * r;
-                    zp[row] = zp_t<R>{z, pi};
-                    v[0] += (double)r * (double)z;
-                    v[1] += (double)r * (double)r;
-                }
-                if (on2) {
-                    a.x[row2] = xi2 + aR * pi2;
-                    const R r = ri2 - aR * qi2;
-                    a.r[row2] = r;
-                    const R z = di2 * r;
-                    zp[row2] = zp_t<R>{z, pi2};
-                    v[0] += (double)r * (double)z;
-                    v[1] += (double)r * (double)r;
-                }
-            }
-            block_reduce_store<2>(v, a.partial, G);
-        }
-        if (!grid_sync(bar, nblk)) return;
-        double t[2];
-        grid_total<2>(a.partial, G, b0, nb, t);
+        { R *sw = cur; cur = nxt; nxt = sw; }
+        // the residual this sweep started from is small enough already (the
+        // test at the end of the last one could not tell): its step is not taken
+        if (t[4] <= stop2) { rr_last = t[4]; converged = true; al = R(0); break; }
+        const double alpha = t[1] / t[0];
+        const double rz = t[1] - 2.0 * alpha * t[2] + alpha * alpha * t[3];
+        const double rr = t[4] - 2.0 * alpha * t[5] + alpha * alpha * t[6];
         it++;
-        rr_last = t[1];
-        converged = (t[1] <= stop2);
+        al = (R)alpha;
+        be = (R)(rz / t[1]);
+        rr_last = rr;
         // a non-finite residual (a NaN or inf voltage upstream) cannot
         // recover: stop now, counted as a failed solve (every block sees the
         // same total and leaves at the same iteration)
-        if (!isfinite(t[1])) break;
-        beta = t[0] / rz;
-        rz = t[0];
+        if (!isfinite(rr)) break;
+        // rr is a difference: below 1e-12 of what it came from only the next
+        // sweep's own sum can tell
+        converged = rr <= stop2 && stop2 >= 1e-12 * t[4];
     }
-    if (pred) {
-        // the solution x + delta, and the correction this solve made, for the
-        // next solve of this half step (own rows; every block is past the
-        // prologue's reads of delta)
-        for (int s = gwarp; s < s_hi; s += nwarps) {
-            const int row = s * kSlice + lane;
-            if (row >= rb && row < re) {
-                const R d = a.delta[row];
-                const R xf = a.x[row] + (lin ? a.dext[row] : d);
-                a.x[row] = xf;
-                const R dn = xf - a.vin[row];
+    if constexpr (STAGED) cp_wait_all();      // the units that ran ahead into the next sweep
+    // V + the solve's correction (alpha p of the last step added), which is also
+    // the next solve's predictor (own rows)
+    for (int s = gwarp; s < s_hi; s += nwarps) {
+        const int row = s * kSlice + lane;
+        if (row >= rb && row < re) {
+            const Quad<R> o = quad_load(cur, row);
+            const R dn = fma(al, o.p, o.d);
+            a.x[row] += dn;
+            if (pred) {
+                if (lin) a.dext[row] = R(2) * dn - a.delta[row];     // the next solve's start: 2 delta - delta_prev
                 a.delta[row] = dn;
-                if (lin) a.dext[row] = R(2) * dn - d;     // the next solve's start: 2 delta - delta_prev
             }
         }
     }
     if ((int)blockIdx.x == b0 && threadIdx.x == 0) {
+        bar->seq = tag;                       // every CTA of the group has read the old one
         atomicAdd(a.iters_total, (unsigned long long)it);
         atomicMax(a.iters_max, (unsigned int)it);
         if (!converged) atomicAdd(a.fails, 1u);
         if (a.last) {
             a.last[2 * inst] = (double)it;
-            a.last[2 * inst + 1] = rr0 > 0.0 ? sqrt(rr_last / rr0) : 0.0;
+            a.last[2 * inst + 1] = rr0 > 0.0 ? sqrt(fmax(rr_last, 0.0) / rr0) : 0.0;
         }
     }
 }
@@ -594,326 +883,6 @@ __global__ void __launch_bounds__(NB == 4 ? 768 : 256, NB == 4 ? 2 : 4) k_cn_hal
     }
 }
 
-// ---------------------------------------------------------------------------
-// k_cn_half_staged: the two-reduction solve of k_cn_half (same recurrences,
-// same order of additions, so the same bits on the same grid) with the matrix
-// stream of phase A taken off the warps' critical path.  A warp's slices are
-// cut into units of kUnitCols slice columns: the column indices and A values
-// of one slice's columns k .. k+7 (8 x 128 bytes of indices, 8 x 32 x
-// sizeof(R) bytes of values).  The warp copies the units into a ring of
-// shared memory with per-thread asynchronous copies (cp.async.cg: 16 bytes
-// each, L2 only, evict-first, so the matrix streams through L2 while the
-// gathered vectors stay there), `depth` units ahead of the one it gathers
-// for.  The DRAM latency of the index -> gather chain is then hidden behind
-// the gathers of the units before it, and the loads in flight occupy ring
-// slots instead of registers.  The stream runs on past the end of a sweep
-// into the next iteration's first units (the matrix does not change), under
-// phase B and the grid barriers.  No wait in this kernel spins:
-// cp.async.wait_group is the hardware's wait for the thread's own copies, and
-// every exit path waits for all of them before the CTA leaves.
-constexpr int kUnitCols = 8;
-
-__host__ __device__ inline size_t unit_bytes(int rsize) { return (size_t)kUnitCols * kSlice * (4 + (size_t)rsize); }
-// dynamic shared memory of a CTA of `block` threads, `depth` units in flight per warp
-__host__ __device__ inline size_t stage_smem_bytes(int block, int depth, int rsize) {
-    return (size_t)(block / 32) * (size_t)(depth + 1) * unit_bytes(rsize);
-}
-
-__device__ __forceinline__ uint32_t cg_smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ uint64_t l2_evict_first_policy() {
-    uint64_t pol;
-    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
-    return pol;
-}
-
-// one 16-byte global -> shared copy, cached in L2 only (both addresses
-// 16-byte aligned: every unit starts on a 128-byte boundary of the SELL
-// arrays and of the ring)
-__device__ __forceinline__ void cp16(void *dst, const void *src, uint64_t pol) {
-    asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(cg_smem_u32(dst)), "l"(src),
-                 "l"(pol)
-                 : "memory");
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-__device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-// this thread's copies of every unit but the newest depth - 1 have landed
-__device__ __forceinline__ void unit_wait(int depth) {
-    switch (depth) {
-        case 1: cp_wait<0>(); break;
-        case 2: cp_wait<1>(); break;
-        case 3: cp_wait<2>(); break;
-        default: cp_wait<3>(); break;
-    }
-}
-
-template <typename R>
-struct UnitRing {
-    int *idx;          // slot k's indices at idx + k * kUnitCols * kSlice
-    R *val;            // slot k's values at val + k * kUnitCols * kSlice
-    int slots, depth;  // slots = depth + 1
-    int L;             // this warp's slices per sweep (0: nothing to stage)
-    int j, k, beg, w;  // producer cursor: slice j of the warp, its column k, start, width
-    int issued;        // units issued so far
-    uint64_t pol;
-};
-
-// issue the unit under the cursor into the ring slot of its position and
-// advance the cursor (the next unit of the slice, or the next slice,
-// wrapping to the warp's first slice: the next sweep).  Every lane commits
-// one copy group per call, empty or not, so the group counts stay uniform.
-template <typename R>
-__device__ __forceinline__ void unit_issue(UnitRing<R> &q, const CGArgs<R> &a, int gwarp, int nwarps, int lane) {
-    if (q.L > 0) {
-        const int slot = q.issued % q.slots;
-        const int nc = min(kUnitCols, q.w - q.k);
-        int *di = q.idx + slot * (kUnitCols * kSlice);
-        R *dv = q.val + slot * (kUnitCols * kSlice);
-        const int *si = a.col + q.beg + q.k * kSlice;
-        const R *sv = a.Aval + q.beg + q.k * kSlice;
-        // indices: column u, 16-byte piece p is chunk c = 8 u + p
-#pragma unroll
-        for (int t = 0; t < 2; t++) {
-            const int c = lane + 32 * t;
-            if ((c >> 3) < nc) cp16(di + 4 * c, si + 4 * c, q.pol);
-        }
-        // values: VPC chunks of VE values per column
-        constexpr int VPC = kSlice * (int)sizeof(R) / 16, VE = 16 / (int)sizeof(R);
-#pragma unroll
-        for (int t = 0; t < VPC * kUnitCols / 32; t++) {
-            const int c = lane + 32 * t;
-            if (c / VPC < nc) cp16(dv + VE * c, sv + VE * c, q.pol);
-        }
-        q.k += kUnitCols;
-        while (q.k >= q.w) {               // ends: some slice of the warp has columns (q.L > 0)
-            q.j = q.j + 1 == q.L ? 0 : q.j + 1;
-            const int s = gwarp + q.j * nwarps;
-            q.beg = __ldg(a.slice_ptr + s);
-            q.w = (__ldg(a.slice_ptr + s + 1) - q.beg) / kSlice;
-            q.k = 0;
-        }
-    }
-    q.issued++;
-    cp_commit();
-}
-
-template <typename R>
-__global__ void __launch_bounds__(256, sizeof(R) == 8 ? 3 : 4) k_cn_half_staged(const CGArgs<R> a) {
-    extern __shared__ __align__(128) unsigned char cg_sm[];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int G = gridDim.x;
-    int inst = 0, b0 = 0, nb = G, rb = 0, re = a.n;
-    if (a.ninst > 1) {
-        int lo = 0, hi = a.ninst - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (a.inst_blk[mid] <= (int)blockIdx.x) lo = mid; else hi = mid - 1;
-        }
-        inst = lo;
-        b0 = a.inst_blk[inst]; nb = a.inst_blk[inst + 1] - b0;
-        rb = a.inst_row[inst]; re = a.inst_row[inst + 1];
-    }
-    GridBarrier *bar = a.bar + inst;
-    const unsigned int nblk = nb + a.bar_extra;
-    const int s_lo = rb / kSlice, s_hi = (re + kSlice - 1) / kSlice;
-    const int gwarp = s_lo + (((int)blockIdx.x - b0) * (int)blockDim.x + (int)threadIdx.x) / 32;
-    const int nwarps = (nb * (int)blockDim.x) >> 5;
-
-    // this warp's ring: slots x unit of indices, then slots x unit of values
-    UnitRing<R> q;
-    {
-        q.depth = a.depth;
-        q.slots = a.depth + 1;
-        unsigned char *base = cg_sm + (size_t)wib * q.slots * unit_bytes((int)sizeof(R));
-        q.idx = reinterpret_cast<int *>(base);
-        q.val = reinterpret_cast<R *>(base + (size_t)q.slots * kUnitCols * kSlice * 4);
-        q.L = gwarp < s_hi ? (s_hi - gwarp + nwarps - 1) / nwarps : 0;
-        int cols = 0;
-        for (int j = 0; j < q.L; j++) {
-            const int s = gwarp + j * nwarps;
-            cols += __ldg(a.slice_ptr + s + 1) - __ldg(a.slice_ptr + s);
-        }
-        if (cols == 0) q.L = 0;
-        q.j = 0;
-        q.k = 0;
-        q.beg = q.L > 0 ? __ldg(a.slice_ptr + gwarp) : 0;
-        q.w = q.L > 0 ? (__ldg(a.slice_ptr + gwarp + 1) - q.beg) / kSlice : 0;
-        while (q.L > 0 && q.w == 0) {      // ends: some slice has columns
-            q.j++;
-            const int s = gwarp + q.j * nwarps;
-            q.beg = __ldg(a.slice_ptr + s);
-            q.w = (__ldg(a.slice_ptr + s + 1) - q.beg) / kSlice;
-        }
-        q.issued = 0;
-        q.pol = l2_evict_first_policy();
-    }
-    // the first units start streaming under the prologue
-    for (int d = 0; d < q.depth; d++) unit_issue(q, a, gwarp, nwarps, lane);
-    int cons = 0;                             // units consumed so far
-
-    // ---- prologue: as k_cn_half ----
-    const bool pred = a.delta != nullptr;
-    const bool lin = a.dext != nullptr;
-    {
-        double v[4] = {0.0, 0.0, 0.0, 0.0};
-        for (int s = gwarp; s < s_hi; s += nwarps) {
-            const int row = s * kSlice + lane;
-            const int beg = a.slice_ptr[s], w = (a.slice_ptr[s + 1] - beg) / kSlice;
-            R ax = R(0), bx = R(0), ad = R(0);
-            slice_ab_sums<4>(a.col, a.Aval, a.Bval, a.x, beg, w, lane, pred, [&](int c) {
-                return lin ? a.dext[c] : a.delta[c];
-            }, ax, bx, ad);
-            if (row >= rb && row < re) {
-                const R rref = bx - ax;
-                const R r = pred ? rref - ad : rref;
-                const R z = __ldg(a.dinv + row) * r;
-                a.r[row] = r;
-                reinterpret_cast<zp_t<R> *>(a.zp)[row] = zp_t<R>{z, R(0)};
-                if (pred) a.vin[row] = a.x[row];
-                v[0] += (double)r * (double)z;
-                v[1] += (double)r * (double)r;
-                v[2] += (double)bx * (double)bx;
-                v[3] += (double)rref * (double)rref;
-            }
-        }
-        block_reduce_store<4>(v, a.partial + 6 * G, G);
-    }
-    if (!grid_sync(bar, nblk)) { cp_wait_all(); return; }
-    double rz, rr_start, bb, rr0;
-    {
-        double t[4];
-        grid_total<4>(a.partial + 6 * G, G, b0, nb, t);
-        rz = t[0]; rr_start = t[1]; bb = t[2]; rr0 = t[3];
-    }
-    const double floor2 = a.floor_rel * a.floor_rel * bb;
-    const double stop2 = fmax(a.tol * a.tol * rr0, floor2);
-    double beta = 0.0;
-    int it = 0;
-    bool converged = (rr_start <= stop2);
-    double rr_last = rr_start;
-    zp_t<R> *zp = reinterpret_cast<zp_t<R> *>(a.zp);
-    R *pn = a.p0;                             // p' of the own rows, phase A -> phase B
-    while (!converged && it < a.maxit) {
-        // ---- phase A: q = A p', p' = z + beta p, the units from the ring ----
-        {
-            double v[1] = {0.0};
-            const R bR = (R)beta;
-            for (int s = gwarp; s < s_hi; s += nwarps) {
-                const int row = s * kSlice + lane;
-                const int beg = __ldg(a.slice_ptr + s), w = (__ldg(a.slice_ptr + s + 1) - beg) / kSlice;
-                R qv = R(0);
-                for (int k = 0; k < w; k += kUnitCols, cons++) {
-                    unit_wait(q.depth);
-                    __syncwarp();                 // the unit is visible to every lane, and every
-                                                  // lane is done with the slot refilled next
-                    unit_issue(q, a, gwarp, nwarps, lane);
-                    const int off = (cons % q.slots) * (kUnitCols * kSlice) + lane;
-                    const int *ci = q.idx + off;
-                    const R *cv = q.val + off;
-                    const int nc = min(kUnitCols, w - k);
-                    int c[kUnitCols];
-                    R g[kUnitCols];
-#pragma unroll
-                    for (int u = 0; u < kUnitCols; u++)
-                        if (u < nc) c[u] = ci[u * kSlice];
-#pragma unroll
-                    for (int u = 0; u < kUnitCols; u++)
-                        if (u < nc) {
-                            const zp_t<R> t = zp[c[u]];
-                            g[u] = pdir_z(t.x, bR, t.y);
-                        }
-#pragma unroll
-                    for (int u = 0; u < kUnitCols; u++)
-                        if (u < nc) qv += cv[u * kSlice] * g[u];
-                }
-                if (row >= rb && row < re) {
-                    const zp_t<R> t = zp[row];
-                    const R pi = pdir_z(t.x, bR, t.y);
-                    pn[row] = pi;
-                    a.q[row] = qv;
-                    v[0] += (double)pi * (double)qv;
-                }
-            }
-            block_reduce_store<1>(v, a.partial + 3 * G, G);
-        }
-        if (!grid_sync(bar, nblk)) { cp_wait_all(); return; }
-        double pq;
-        {
-            double t[1];
-            grid_total<1>(a.partial + 3 * G, G, b0, nb, t);
-            pq = t[0];
-        }
-        const double alpha = rz / pq;
-        // ---- phase B: as k_cn_half ----
-        {
-            double v[2] = {0.0, 0.0};
-            const R aR = (R)alpha;
-            for (int s = gwarp; s < s_hi; s += 2 * nwarps) {
-                const int row = s * kSlice + lane, row2 = row + nwarps * kSlice;
-                const bool on = row >= rb && row < re;
-                const bool on2 = s + nwarps < s_hi && row2 >= rb && row2 < re;
-                R pi = R(0), xi = R(0), ri = R(0), qi = R(0), di = R(0);
-                R pi2 = R(0), xi2 = R(0), ri2 = R(0), qi2 = R(0), di2 = R(0);
-                if (on) { pi = pn[row]; xi = a.x[row]; ri = a.r[row]; qi = a.q[row]; di = __ldg(a.dinv + row); }
-                if (on2) { pi2 = pn[row2]; xi2 = a.x[row2]; ri2 = a.r[row2]; qi2 = a.q[row2]; di2 = __ldg(a.dinv + row2); }
-                if (on) {
-                    a.x[row] = xi + aR * pi;
-                    const R r = ri - aR * qi;
-                    a.r[row] = r;
-                    const R z = di * r;
-                    zp[row] = zp_t<R>{z, pi};
-                    v[0] += (double)r * (double)z;
-                    v[1] += (double)r * (double)r;
-                }
-                if (on2) {
-                    a.x[row2] = xi2 + aR * pi2;
-                    const R r = ri2 - aR * qi2;
-                    a.r[row2] = r;
-                    const R z = di2 * r;
-                    zp[row2] = zp_t<R>{z, pi2};
-                    v[0] += (double)r * (double)z;
-                    v[1] += (double)r * (double)r;
-                }
-            }
-            block_reduce_store<2>(v, a.partial, G);
-        }
-        if (!grid_sync(bar, nblk)) { cp_wait_all(); return; }
-        double t[2];
-        grid_total<2>(a.partial, G, b0, nb, t);
-        it++;
-        rr_last = t[1];
-        converged = (t[1] <= stop2);
-        if (!isfinite(t[1])) break;
-        beta = t[0] / rz;
-        rz = t[0];
-    }
-    cp_wait_all();                            // the units that ran ahead into the next sweep
-    if (pred) {
-        for (int s = gwarp; s < s_hi; s += nwarps) {
-            const int row = s * kSlice + lane;
-            if (row >= rb && row < re) {
-                const R d = a.delta[row];
-                const R xf = a.x[row] + (lin ? a.dext[row] : d);
-                a.x[row] = xf;
-                const R dn = xf - a.vin[row];
-                a.delta[row] = dn;
-                if (lin) a.dext[row] = R(2) * dn - d;     // the next solve's start: 2 delta - delta_prev
-            }
-        }
-    }
-    if ((int)blockIdx.x == b0 && threadIdx.x == 0) {
-        atomicAdd(a.iters_total, (unsigned long long)it);
-        atomicMax(a.iters_max, (unsigned int)it);
-        if (!converged) atomicAdd(a.fails, 1u);
-        if (a.last) {
-            a.last[2 * inst] = (double)it;
-            a.last[2 * inst + 1] = rr0 > 0.0 ? sqrt(rr_last / rr0) : 0.0;
-        }
-    }
-}
-
 // the kernel of a (gather width, variant) choice and its dynamic shared
 // memory; cg_batch kStagedBatch selects k_cn_half_staged with `depth` units
 // in flight per warp (1 .. kStageMaxDepth)
@@ -930,7 +899,7 @@ static int cg_kernel(int block, int batch, int variant, int depth, const void **
             set_error("staged CG: %d units in flight, not 1..%d", depth, kStageMaxDepth);
             return EP_ERR_ARG;
         }
-        *fn = (const void *)k_cn_half_staged<R>;
+        *fn = (const void *)k_cn_half<R, kStagedBatch>;
         *smem = stage_smem_bytes(block, depth, (int)sizeof(R));
         if (set_attr)
             EP_CUDA(cudaFuncSetAttribute(*fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -958,6 +927,39 @@ int cg_max_per_sm(int block, int *per, int batch, int variant, int depth) {
     }
     EP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per, fn, block, smem));
     if (*per < 1) { set_error("CG kernel cannot be resident with %d threads per CTA", block); return EP_ERR_CUDA; }
+    return EP_OK;
+}
+
+// The launch of a handle that leaves cg_per_sm to the library (0), and of
+// ep_cn_half_step_noalloc: no more CTAs than there are slices for, since
+// every CTA takes part in each iteration's reduction, and one CTA per SM once
+// the slices fill the GPU.
+//   up to 32 slices: one CTA, whose reductions need no global memory;
+//   up to 8 warps per SM: 256 threads, one slice per warp;
+//   beyond: one CTA per SM, of 512 threads up to 16 slices per SM and of 1024
+//   above (with the 64 registers a thread has, a full SM either way).
+// Batches keep CTAs of `block` threads, as many as fit: each instance's group
+// is small already and more CTAs split the GPU more evenly between them.
+template <typename R>
+int cg_auto_shape(int nslices, int ninst, int batch, int variant, int depth, int *block, int *grid) {
+    int dev = 0, nsm = 0, per = 0;
+    EP_CUDA(cudaGetDevice(&dev));
+    EP_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    int rc = cg_max_per_sm<R>(*block, &per, batch, variant, depth);
+    if (rc) return rc;
+    if (variant == 0 && batch == 4 && *block == 256 && ninst == 1) {
+        if (nslices <= 32) *block = std::max(256, nslices * 32);
+        else if (nslices > 16 * nsm) *block = 1024;
+        else if (nslices > 8 * nsm) *block = 512;
+        if (*block != 256) per = 1;
+    }
+    if (ninst > nsm * per && *block > 128) {
+        // more instances than CTAs of this size fit: a warp group each
+        *block = 128;
+        if ((rc = cg_max_per_sm<R>(*block, &per, batch, variant, depth))) return rc;
+    }
+    // an instance's share of the slices is rounded up to whole CTAs
+    *grid = std::min(nsm * per, div_up(nslices, *block / 32) + (ninst > 1 ? ninst : 0));
     return EP_OK;
 }
 
@@ -991,7 +993,7 @@ int launch_cg(const CGArgs<R> &a, int grid, int block, cudaStream_t s, int batch
         int rc = cg_kernel<R>(block, batch, variant, a.depth, &fn, &smem, false);
         if (rc) return rc;
         cfg.dynamicSmemBytes = smem;
-        EP_CUDA(cudaLaunchKernelEx(&cfg, k_cn_half_staged<R>, a));
+        EP_CUDA(cudaLaunchKernelEx(&cfg, k_cn_half<R, kStagedBatch>, a));
     } else if (variant == 1) {
         if (!a.r1 || !a.w0 || !a.w1 || !a.s0 || !a.s1) { set_error("single-reduction CG needs its vectors"); return EP_ERR_ARG; }
         if (batch >= 8) EP_CUDA(cudaLaunchKernelEx(&cfg, k_cn_half_cg1<R, 8>, a));
@@ -1008,6 +1010,8 @@ int launch_cg(const CGArgs<R> &a, int grid, int block, cudaStream_t s, int batch
 
 template int launch_cg<float>(const CGArgs<float> &, int, int, cudaStream_t, int, int);
 template int launch_cg<double>(const CGArgs<double> &, int, int, cudaStream_t, int, int);
+template int cg_auto_shape<float>(int, int, int, int, int, int *, int *);
+template int cg_auto_shape<double>(int, int, int, int, int, int *, int *);
 template int cg_grid_size<float>(int, int *, int, int, int, int);
 template int cg_grid_size<double>(int, int *, int, int, int, int);
 template int cg_max_per_sm<float>(int, int *, int, int, int);

@@ -58,6 +58,8 @@ struct GridBarrier {
     unsigned int gen;
     unsigned int err;
     unsigned int limit;
+    unsigned long long seq;      // last tag of the solves so far (cg.cu group_reduce)
+    unsigned long long pad;
 };
 
 __device__ __forceinline__ bool grid_sync(GridBarrier *b, unsigned int nblocks) {

@@ -97,6 +97,9 @@ template <typename R> struct IonicArgs {
 template <typename R>
 int launch_ionic(int model, const IonicArgs<R> &a, cudaStream_t s, int block = 128, int min_ctas = 0);
 
+// One value of a CTA's partial sums and the phase it belongs to (cg.cu)
+struct __align__(16) CgSlot { double v; unsigned long long tag; };
+
 // Crank-Nicolson half diffusion step: x <- A^-1 (B x) by Jacobi-PCG in one
 // persistent cooperative launch (Solvers/EP_CrankNicholson.cc:99-104).
 template <typename R> struct CGArgs {
@@ -104,10 +107,9 @@ template <typename R> struct CGArgs {
     const int *slice_ptr;        // nslices + 1
     const int *col;
     const R *Aval, *Bval, *dinv;
-    R *x, *r, *q, *p0;           // p0: the direction p (two-reduction: p' of the own rows)
-    R *zp;                       // two-reduction variant: 2 * pitch, (z_i, p_i) pairs with
-                                 // z = dinv r, gathered by the neighbours (16-byte aligned)
-    double *partial;             // 12 * grid: consecutive phases use disjoint slots
+    R *x;
+    R *q0, *q1;                  // two buffers of 4 * pitch: (z, p, w, d) per node (16-byte aligned)
+    CgSlot *slots;               // 2 sets x grid x 8 reduction units (zeroed before the first launch)
     GridBarrier *bar;
     double tol;
     double floor_rel;            // stop also when ||r|| <= floor_rel ||B x||
@@ -121,16 +123,17 @@ template <typename R> struct CGArgs {
     // one instance owning every row and CTA.
     int ninst;
     const int *inst_row, *inst_blk;
-    // single-reduction variant only: second r buffer, w = A z and s = A p
-    // (two buffers each); p lives in p0
-    R *r1, *w0, *w1, *s0, *s1;
-    // predictor (two-reduction variant only; nullable): delta = the previous
-    // solve's x - V for this half step, updated in place; dext (nullable) the
-    // linear extrapolation 2 delta - delta_prev of the last two, which the
-    // previous solve stores for the next one's start (one vector gathered in
-    // the prologue, not two); vin scratch of n
-    R *delta, *dext, *vin;
-    // two-reduction variant: each warp asks L2 for the indices and values of
+    // Chronopoulos-Gear variant only: r and w = A z, s = A p (two buffers
+    // each), the direction p0 and 12 * grid partial sums
+    R *r, *r1, *w0, *w1, *s0, *s1, *p0;
+    double *partial;
+    // predictor (cg_variant 0 only; nullable): delta = the previous solve's
+    // x - V for this half step, updated in place; dext (nullable) the linear
+    // extrapolation 2 delta - delta_prev of the last two, which the previous
+    // solve stores for the next one's start (one vector gathered in the
+    // prologue, not two)
+    R *delta, *dext;
+    // cg_variant 0: each warp asks L2 for the indices and values of
     // the slice it reads `prefetch` slices ahead (0: no prefetch)
     int prefetch;
     // arrivals the grid barrier waits for beyond the CTAs that exist (0;
@@ -153,10 +156,14 @@ constexpr int kStageMaxDepth = 4;
 constexpr int kStageDepthDefault = 2;
 
 // batch: SELL columns gathered per group (4 or 8; two register budgets);
-// variant 0: the two-reduction CG of the reference, 1: Chronopoulos-Gear
-// (one reduction per iteration; needs r1, w0, w1, s0, s1)
+// variant 0: the CG recurrences of the reference, 1: Chronopoulos-Gear
+// (needs r, r1, w0, w1, s0, s1, p0)
 template <typename R>
 int launch_cg(const CGArgs<R> &a, int grid, int block, cudaStream_t s, int batch = 4, int variant = 0);
+// block and grid of a launch whose shape is left to the library (*block: the
+// asked block size in, the launch's out)
+template <typename R>
+int cg_auto_shape(int nslices, int ninst, int batch, int variant, int depth, int *block, int *grid);
 // CTAs of the persistent launch: per_sm (0 = as many as fit) x SM count
 template <typename R>
 int cg_grid_size(int block, int *grid, int per_sm = 0, int batch = 4, int variant = 0, int depth = 0);

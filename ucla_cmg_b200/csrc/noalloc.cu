@@ -6,8 +6,8 @@
 // call cudaMalloc once its time loop has started (allocation synchronises the
 // device and can fail late in a long run), or a C/Fortran caller that only
 // hands over buffers it manages.  ep_cn_half_step_noalloc gives them the
-// persistent Jacobi-PCG kernel with its working vectors (r, q and the two
-// search-direction buffers), the reduction partials and the grid barrier
+// persistent Jacobi-PCG kernel with its working vectors (two buffers of the
+// nodes' (z, p, w, d) records), the reduction slots and the grid barrier
 // placed in one statically sized device array defined in this file, so a
 // call performs no device allocation at all.  The caller passes the matrix
 // (SELL-32 layout) and the voltage vector, both in its own device memory.
@@ -15,7 +15,7 @@
 // Limits and rules (repeated in include/ep_gpu.h):
 // * at most kNoAllocMaxRows rows; larger systems are rejected with
 //   EP_ERR_ARG;
-// * the array (about 8.2 MB) is part of the module: every GPU that loads the
+// * the array (about 17 MB) is part of the module: every GPU that loads the
 //   library holds it until the process exits;
 // * every call shares the one array, so calls that overlap on the GPU (two
 //   streams, two host threads) race -- serialise them;
@@ -26,6 +26,8 @@
 // * the call waits on `stream` for its own results before it returns; on a
 //   stream in capture mode it returns EP_ERR_ARG before touching the stream,
 //   so the caller's capture stays intact.
+#include <cstring>
+
 #include "kernels.cuh"
 
 namespace ep {
@@ -33,8 +35,8 @@ namespace ep {
 constexpr int kNoAllocMaxRows = 262144;                 // 2^18 rows
 constexpr int kNoAllocMaxGrid = 2048;                   // >= 148 SMs x 8 blocks
 constexpr size_t kVecBytes = sizeof(double) * (size_t)kNoAllocMaxRows;   // one vector, FP64
-constexpr size_t kScratchBytes = 5 * kVecBytes                            // r, q, p0, (z, p) pairs (2)
-                               + sizeof(double) * 12 * kNoAllocMaxGrid    // reduction partials (12 slots)
+constexpr size_t kScratchBytes = 8 * kVecBytes                            // the (z, p, w, d) records, two buffers
+                               + sizeof(CgSlot) * 16 * kNoAllocMaxGrid    // reduction slots
                                + 256;                                     // barrier, stats, result
 
 // the only storage a call uses beyond the caller's buffers
@@ -66,13 +68,11 @@ int run(unsigned char *base, int n, int nslices, const int *slice_ptr, const int
     a.n = n; a.nslices = nslices;
     a.slice_ptr = slice_ptr; a.col = col;
     a.Aval = A; a.Bval = B; a.dinv = dinv; a.x = x;
-    a.r = (R *)(base + 0 * kVecBytes);
-    a.q = (R *)(base + 1 * kVecBytes);
-    a.p0 = (R *)(base + 2 * kVecBytes);
-    a.zp = (R *)(base + 3 * kVecBytes);                            // two vectors: (z, p) pairs
-    a.partial = (double *)(base + 5 * kVecBytes);
-    unsigned char *tail = base + 5 * kVecBytes + sizeof(double) * 12 * kNoAllocMaxGrid;
-    a.bar = (GridBarrier *)tail;                                   // 16 B
+    a.q0 = (R *)(base + 0 * kVecBytes);
+    a.q1 = (R *)(base + 4 * kVecBytes);
+    a.slots = (CgSlot *)(base + 8 * kVecBytes);
+    unsigned char *tail = base + 8 * kVecBytes + sizeof(CgSlot) * 16 * kNoAllocMaxGrid;
+    a.bar = (GridBarrier *)tail;                                   // 32 B
     unsigned long long *st = (unsigned long long *)(tail + 64);   // 32 B of counters
     a.iters_total = st;
     a.iters_max = (unsigned int *)(st + 1);
@@ -81,22 +81,29 @@ int run(unsigned char *base, int n, int nslices, const int *slice_ptr, const int
     a.tol = tol > 0 ? tol : 1e-7;
     a.floor_rel = sizeof(R) == 4 ? 1.2e-7 : 2.2e-16;
     a.maxit = maxit > 0 ? maxit : 1000;
-    // the barrier and the counters must start at zero; the kernel writes the
-    // vectors and partials before it reads them
-    EP_CUDA(cudaMemsetAsync(tail, 0, 256, s));
-    int grid = 0;
-    int rc = cg_grid_size<R>(256, &grid);
+    // the barrier's tags go on from call to call (the array starts zeroed),
+    // and the kernel writes the records before it reads them
+    int grid = 0, block = 256;
+    int rc = cg_auto_shape<R>(nslices, 1, 4, 0, 0, &block, &grid);
     if (rc) return rc;
-    grid = grid < kNoAllocMaxGrid ? grid : kNoAllocMaxGrid;
-    if ((rc = launch_cg<R>(a, grid, 256, s))) return rc;
-    double last[2] = {0.0, 0.0};
-    GridBarrier bar{};
-    EP_CUDA(cudaMemcpyAsync(last, a.last, sizeof last, cudaMemcpyDeviceToHost, s));
-    EP_CUDA(cudaMemcpyAsync(&bar, a.bar, sizeof bar, cudaMemcpyDeviceToHost, s));
+    if ((rc = launch_cg<R>(a, grid, block, s))) return rc;
+    // barrier and result in one copy
+    unsigned char back[160];
+    EP_CUDA(cudaMemcpyAsync(back, tail, sizeof back, cudaMemcpyDeviceToHost, s));
     EP_CUDA(cudaStreamSynchronize(s));
+    double last[2];
+    GridBarrier bar;
+    std::memcpy(last, back + 128, sizeof last);
+    std::memcpy(&bar, back, sizeof bar);
     if (iters) *iters = (int)last[0];
     if (relres) *relres = last[1];
-    if (bar.err) { set_error("a grid barrier wait gave up"); return EP_ERR_TIMEOUT; }
+    if (bar.err) {
+        // tags of the blocks that left early must not meet the next call
+        EP_CUDA(cudaMemsetAsync(a.slots, 0, sizeof(CgSlot) * 16 * kNoAllocMaxGrid + 256, s));
+        EP_CUDA(cudaStreamSynchronize(s));
+        set_error("a grid barrier wait gave up");
+        return EP_ERR_TIMEOUT;
+    }
     return EP_OK;
 }
 
