@@ -71,7 +71,7 @@ struct ep_handle {
     DBuf cl;                             // explicit scheme: lumped capacitance C_L
     int cg_maxit = 1000;
     int cg_grid = 0, cg_block = 256;
-    int cg_threads = 256;                // threads per CTA of the planned launch (cg_block, or the library's choice)
+    CgShape cg{4, 256, 0, 0, 0, 0};      // the planned CG launch: the launch config's, or the library's choice
     int ecg_every = 0;
     double act_thr = -40.0;
     TTOpts tt{};
@@ -250,6 +250,8 @@ void fill_cg_args(ep_handle *h, CGArgs<R> &a) {
     a.prefetch = h->cg_batch == kStagedBatch ? 0 : h->cg_prefetch;   // the staged kernel's is its ring depth
     a.bar_extra = h->bar_extra;
     a.depth = stage_depth(h);
+    a.ring_cols = h->cg.ring_cols;
+    a.smem = h->cg.smem;
 }
 
 // start the CG predictor from x0 = V again (after a state upload or when it
@@ -458,15 +460,17 @@ static int reset_barriers(ep_handle *h) {
 static int plan_cg(ep_handle *h) {
     const int ws = stage_depth(h);
     int rc;
-    h->cg_threads = h->cg_block;
-    if (h->cg_per_sm == 0)
+    h->cg = CgShape{h->cg_batch, h->cg_block, 0, 0, 0, 0};
+    if (h->cg_per_sm == 0) {
         rc = h->precision == EP_FP64
-                 ? cg_auto_shape<double>(h->nslices, h->ninst, h->cg_batch, h->cg_variant, ws, &h->cg_threads, &h->cg_grid)
-                 : cg_auto_shape<float>(h->nslices, h->ninst, h->cg_batch, h->cg_variant, ws, &h->cg_threads, &h->cg_grid);
-    else
+                 ? cg_auto_shape<double>(h->nslices, h->ninst, h->cg_batch, h->cg_variant, ws, &h->cg)
+                 : cg_auto_shape<float>(h->nslices, h->ninst, h->cg_batch, h->cg_variant, ws, &h->cg);
+        h->cg_grid = h->cg.grid;
+    } else {
         rc = h->precision == EP_FP64
                  ? cg_grid_size<double>(h->cg_block, &h->cg_grid, h->cg_per_sm, h->cg_batch, h->cg_variant, ws)
                  : cg_grid_size<float>(h->cg_block, &h->cg_grid, h->cg_per_sm, h->cg_batch, h->cg_variant, ws);
+    }
     if (rc) return rc;
     if (h->cg_variant == 1 && !h->w0.p) {
         const size_t vb = (size_t)h->pitch * h->rsize;
@@ -483,6 +487,16 @@ static int plan_cg(ep_handle *h) {
     if ((rc = ep_batch_plan(h->ninst, h->inst_row.data(), h->cg_grid, h->inst_blk.data()))) {
         set_error("bad instance layout");
         return rc;
+    }
+    if (h->cg.batch == kSmemBatch) {
+        int ns = 0;                       // slices of a CTA, at most
+        for (int k = 0; k < h->ninst; k++) {
+            const int all = div_up(h->inst_row[k + 1], kSlice) - h->inst_row[k] / kSlice;
+            ns = std::max(ns, div_up(all, h->inst_blk[k + 1] - h->inst_blk[k]));
+        }
+        const int cols = div_up((long long)(h->col.bytes / sizeof(int)), (long long)kSlice * h->nslices);
+        rc = h->precision == EP_FP64 ? cg_fit_smem<double>(ns, cols, &h->cg) : cg_fit_smem<float>(ns, cols, &h->cg);
+        if (rc) return rc;
     }
     if ((rc = upload_raw(h->d_inst_row, h->inst_row.data(), h->inst_row.size()))) return rc;
     if ((rc = upload_raw(h->d_inst_blk, h->inst_blk.data(), h->inst_blk.size()))) return rc;
@@ -604,7 +618,7 @@ static int half_diffusion(ep_handle *h, const CGArgs<R> &ca) {
         h->launches += (long long)h->ex_h.size() - 1;
         return EP_OK;
     }
-    return launch_cg<R>(ca, h->cg_grid, h->cg_threads, h->stream, h->cg_batch, h->cg_variant);
+    return launch_cg<R>(ca, h->cg_grid, h->cg.block, h->stream, h->cg.batch, h->cg_variant);
 }
 
 // The plain ionic phase: the tissue model over every node, and in a mixed

@@ -98,7 +98,7 @@ __device__ __forceinline__ void slot_store(CgSlot *p, double v, unsigned long lo
 }
 __device__ __forceinline__ void slot_load(const CgSlot *p, double &v, unsigned long long &tag) {
     unsigned long long u;
-    asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+    asm volatile("{\n\t.reg .b128 t;\n\tld.acquire.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
                  : "=l"(u), "=l"(tag)
                  : "l"(p)
                  : "memory");
@@ -108,11 +108,11 @@ __device__ __forceinline__ void fence_acq_rel_gpu() { asm volatile("fence.acq_re
 
 // NV <= 8 sums over the CTAs [b0, b0 + nb) of a group, the same bits in every
 // thread of every CTA, and a barrier between what the group wrote before and
-// what it reads after.  false: a wait gave up.
+// what it reads after.  false: a wait gave up, here or (ok false) before.
 template <int NV>
 __device__ __forceinline__ bool group_reduce(CgSlot *slots, int G, unsigned long long tag, int b0, int nb,
                                              unsigned int hold, GridBarrier *bar, const double (&vin)[NV],
-                                             double (&tot)[NV]) {
+                                             double (&tot)[NV], bool ok = true) {
     static_assert(NV <= kRedMax, "too many values");
     __shared__ double sh_a[32][kRedMax], sh_b[32][kRedMax];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
@@ -146,7 +146,10 @@ __device__ __forceinline__ bool group_reduce(CgSlot *slots, int G, unsigned long
     double t;
     if (nb == 1 && !hold) {
         t = column_sum(sh_a, nw);
-        __syncthreads();                      // sh_a is free again
+        if (__syncthreads_or(!ok)) {          // sh_a is free again
+            if (tid == 0) atomicExch(&bar->err, 1u);
+            return false;
+        }
     } else {
         CgSlot *set = slots + (size_t)(tag & 1) * G * kRedMax;
         if (warp == 0) {
@@ -159,7 +162,8 @@ __device__ __forceinline__ bool group_reduce(CgSlot *slots, int G, unsigned long
         const int units = nb * kRedMax;
         const bool mine = (tid & (kRedMax - 1)) < NV;
         unsigned int polls = 0;
-        int bad = 0;
+        int bad = ok ? 0 : 1;
+        if (bad) atomicExch(&bar->err, 1u);
         double acc = 0.0;
         for (int u0 = tid; u0 < units && mine && !bad; u0 += 4 * (int)blockDim.x) {
             double x[4];
@@ -189,7 +193,6 @@ __device__ __forceinline__ bool group_reduce(CgSlot *slots, int G, unsigned long
             }
             acc += (x[0] + x[1]) + (x[2] + x[3]);
         }
-        fence_acq_rel_gpu();
         acc += __shfl_xor_sync(0xffffffffu, acc, 8);
         acc += __shfl_xor_sync(0xffffffffu, acc, 16);
         if (lane < kRedMax) sh_b[warp][lane] = acc;
@@ -553,6 +556,66 @@ __device__ __forceinline__ R ring_row_sum(UnitRing<R> &q, const CGArgs<R> &a, in
     return acc;
 }
 
+// A CTA's instance (its rows [rb, re), its CTA group [b0, b0 + nb) and its
+// barrier) and its slices [s0, s1): a contiguous share of the instance's, so
+// that neighbouring rows share gathered values in L1; its warps take them in
+// turn.
+struct CgShare { int inst, b0, nb, rb, re, s0, s1; };
+template <typename R>
+__device__ __forceinline__ CgShare cg_share(const CGArgs<R> &a) {
+    CgShare h{0, 0, (int)gridDim.x, 0, a.n, 0, 0};
+    if (a.ninst > 1) {
+        int lo = 0, hi = a.ninst - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (a.inst_blk[mid] <= (int)blockIdx.x) lo = mid; else hi = mid - 1;
+        }
+        h.inst = lo;
+        h.b0 = a.inst_blk[lo]; h.nb = a.inst_blk[lo + 1] - h.b0;
+        h.rb = a.inst_row[lo]; h.re = a.inst_row[lo + 1];
+    }
+    const int lo = h.rb / kSlice, all = (h.re + kSlice - 1) / kSlice - lo, ci = (int)blockIdx.x - h.b0;
+    h.s0 = lo + (int)((long long)all * ci / h.nb);
+    h.s1 = lo + (int)((long long)all * (ci + 1) / h.nb);
+    return h;
+}
+
+// The end of a solve: V + its correction (alpha p of the last step added),
+// which is also the next solve's predictor (own rows), and the statistics.
+template <typename R>
+__device__ __forceinline__ void cg_finish(const CGArgs<R> &a, const CgShare &sh, int warp, int nw, int lane,
+                                          const R *cur, R al, R be, bool converged, unsigned long long tag, int it,
+                                          double rr, double rr0) {
+    for (int s = sh.s0 + warp; s < sh.s1; s += nw) {
+        const int row = s * kSlice + lane;
+        if (row >= sh.rb && row < sh.re) {
+            const Quad<R> o = quad_load(cur, row);
+            R dn = fma(al, o.p, o.d);
+            // FP32, which stops at the resolution of b: one more step for
+            // free, the next iteration's direction taken with this iteration's
+            // length (successive lengths differ by a few percent on these
+            // mass-dominated systems, so it lowers the error 2-3 fold, as the
+            // iteration itself would).  FP64 keeps the reference's iterate.
+            if (sizeof(R) == 4 && converged) dn = fma(al, fma(be, o.p, fma(-al, o.w, o.z)), dn);
+            a.x[row] += dn;
+            if (a.delta) {
+                if (a.dext) a.dext[row] = R(2) * dn - a.delta[row];     // the next solve's start: 2 delta - delta_prev
+                a.delta[row] = dn;
+            }
+        }
+    }
+    if ((int)blockIdx.x == sh.b0 && threadIdx.x == 0) {
+        a.bar[sh.inst].seq = tag;             // every CTA of the group has read the old one
+        atomicAdd(a.iters_total, (unsigned long long)it);
+        atomicMax(a.iters_max, (unsigned int)it);
+        if (!converged) atomicAdd(a.fails, 1u);
+        if (a.last) {
+            a.last[2 * sh.inst] = (double)it;
+            a.last[2 * sh.inst + 1] = rr0 > 0.0 ? sqrt(fmax(rr, 0.0) / rr0) : 0.0;
+        }
+    }
+}
+
 // The solve.  NB: slice columns gathered together (4, 8; 16: 8 with the next
 // group's indices and values loaded ahead; kStagedBatch: 8 out of a shared-
 // memory ring, below).  64 registers in all of them, so one CTA of up to 1024
@@ -578,23 +641,12 @@ k_cn_half(const CGArgs<R> a) {
     extern __shared__ __align__(128) unsigned char cg_sm[];
     const int lane = threadIdx.x & 31;
     const int G = gridDim.x;
-    // this CTA's instance: its rows, its CTA group and its barrier
-    int inst = 0, b0 = 0, nb = G, rb = 0, re = a.n;
-    if (a.ninst > 1) {
-        int lo = 0, hi = a.ninst - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (a.inst_blk[mid] <= (int)blockIdx.x) lo = mid; else hi = mid - 1;
-        }
-        inst = lo;
-        b0 = a.inst_blk[inst]; nb = a.inst_blk[inst + 1] - b0;
-        rb = a.inst_row[inst]; re = a.inst_row[inst + 1];
-    }
+    const CgShare sh = cg_share(a);
+    const int inst = sh.inst, b0 = sh.b0, nb = sh.nb, rb = sh.rb, re = sh.re;
     GridBarrier *bar = a.bar + inst;
     unsigned long long tag = *(volatile unsigned long long *)&bar->seq;
-    const int s_lo = rb / kSlice, s_hi = (re + kSlice - 1) / kSlice;
-    const int gwarp = s_lo + (((int)blockIdx.x - b0) * (int)blockDim.x + (int)threadIdx.x) / 32;
-    const int nwarps = (nb * (int)blockDim.x) >> 5;
+    const int gwarp = sh.s0 + (int)(threadIdx.x >> 5), s_hi = sh.s1;
+    const int nwarps = (int)blockDim.x >> 5;
 
     UnitRing<R> ring;                         // this warp's ring (staged form)
     if constexpr (STAGED) {
@@ -702,30 +754,303 @@ k_cn_half(const CGArgs<R> a) {
         converged = rr <= stop2 && stop2 >= 1e-12 * t[4];
     }
     if constexpr (STAGED) cp_wait_all();      // the units that ran ahead into the next sweep
-    // V + the solve's correction (alpha p of the last step added), which is also
-    // the next solve's predictor (own rows)
-    for (int s = gwarp; s < s_hi; s += nwarps) {
-        const int row = s * kSlice + lane;
-        if (row >= rb && row < re) {
-            const Quad<R> o = quad_load(cur, row);
-            const R dn = fma(al, o.p, o.d);
-            a.x[row] += dn;
-            if (pred) {
-                if (lin) a.dext[row] = R(2) * dn - a.delta[row];     // the next solve's start: 2 delta - delta_prev
-                a.delta[row] = dn;
+    cg_finish(a, sh, (int)(threadIdx.x >> 5), nwarps, lane, cur, al, be, converged, tag, it, rr_last, rr0);
+}
+
+// ---------------------------------------------------------------------------
+// k_cn_smem: the solve of k_cn_half with the matrix in shared memory, what a
+// handle runs unless its launch shape is set.  An iteration of k_cn_half is a
+// chain of exposed memory latencies (0.5-0.6 us each under load): the slice's
+// bounds, then for every four columns their indices and values and then the
+// gathers, then the own record, some eleven a slice, so a warp took 9.5 us a
+// slice on the 765K-node shell and one 23-warp CTA 6.5 us an iteration on 715
+// nodes.  Here the gathers are the only one: the slice bounds and the matrix
+// wait in shared memory, the own record is loaded beside the gathers, and a
+// slice's gathers go out 16 (FP64: 8) at a time.
+// Where a CTA's share of the matrix fits (about 250K nodes in FP32, 165K in
+// FP64 over 148 SMs) it is copied in once and stays for the whole solve; else
+// each warp's region is a ring of units of 8 slice columns that bulk copies
+// (cp.async.bulk, one lane issuing, an mbarrier per unit) refill as units are
+// consumed, running on into the next sweep under the reduction.
+constexpr int kUnit = 8, kUnitMax = 9;        // slice columns of a unit; a single left-over column joins the last
+constexpr int kMaxUnits = 64;                 // units in a warp's ring, at most
+constexpr unsigned int kCopyPolls = 1u << 18; // tries of one unit's wait
+
+__device__ __forceinline__ void cg_mbar_init(unsigned long long *b) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(cg_smem_u32(b)) : "memory");
+}
+__device__ __forceinline__ void cg_mbar_expect(unsigned long long *b, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(cg_smem_u32(b)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool cg_mbar_wait(unsigned long long *b, uint32_t parity) {
+    for (unsigned int k = 0; k < kCopyPolls; k++) {
+        uint32_t ok;
+        asm volatile("{\n\t.reg .pred p;\n\t"
+                     "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                     "selp.b32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok)
+                     : "r"(cg_smem_u32(b)), "r"(parity)
+                     : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+// both addresses 16-byte aligned, bytes a multiple of 16: units start on
+// 128-byte boundaries of the SELL arrays and of the region
+__device__ __forceinline__ void cg_bulk(void *dst, const void *src, uint32_t bytes, unsigned long long *bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     cg_smem_u32(dst)),
+                 "l"(src), "r"(bytes), "r"(cg_smem_u32(bar))
+                 : "memory");
+}
+
+// columns of the next unit of a slice with `rem` columns left
+__device__ __forceinline__ int unit_cols(int rem) { return rem == kUnitMax ? kUnitMax : min(kUnit, rem); }
+
+// A warp's share of the matrix in shared memory.
+template <typename R>
+struct MatRing {
+    static constexpr int kColBytes = kSlice * (4 + (int)sizeof(R));   // one slice column
+    unsigned char *base;          // the warp's region
+    unsigned long long *bars;     // an mbarrier per unit slot
+    const int *sp;                // slice bounds, sp[j * nw], sp[j * nw + 1]: the warp's j-th slice
+    int nw, L;                    // warps of the CTA; the warp's slices
+    int slots;                    // unit slots (resident: the units of the share)
+    bool resident;
+    int pj, pk, pslot, pcol;      // producer (lane 0): slice, column, slot and running column of the next unit
+    int slot, ccol;               // consumer: slot and running column of the next unit
+    uint32_t phase;               // and its mbarrier's parity
+
+    // where a unit lies: packed by columns when resident, in its slot else
+    __device__ __forceinline__ unsigned char *unit(int s, int col) const {
+        return base + (size_t)(resident ? col : s * kUnitMax) * kColBytes;
+    }
+    // lane 0: copy the next unit of the share (a ring goes round and round)
+    __device__ __forceinline__ void issue(const int *cols, const R *vals) {
+        while (sp[pj * nw + 1] == sp[pj * nw]) next_slice();      // empty slices; the share has others
+        const int beg = sp[pj * nw], w = (sp[pj * nw + 1] - beg) / kSlice;
+        const int nc = unit_cols(w - pk), n = nc * kSlice;
+        unsigned char *d = unit(pslot, pcol);
+        unsigned long long *b = bars + pslot;
+        const int *ci = cols + beg + pk * kSlice;
+        const R *av = vals + beg + pk * kSlice;
+        if ((((uintptr_t)ci | (uintptr_t)av) & 15u) == 0) {
+            cg_mbar_expect(b, (uint32_t)nc * kColBytes);
+            cg_bulk(d, ci, (uint32_t)n * 4u, b);
+            cg_bulk(d + n * 4, av, (uint32_t)n * (uint32_t)sizeof(R), b);
+        } else {
+            // a caller's arrays that bulk copies cannot read (ep_cn_half_step_noalloc)
+            for (int e = 0; e < n; e++) {
+                reinterpret_cast<int *>(d)[e] = ci[e];
+                reinterpret_cast<R *>(d + n * 4)[e] = av[e];
+            }
+            cg_mbar_expect(b, 0u);
+        }
+        pcol += nc;
+        pk += nc;
+        if (pk >= w) next_slice();
+        if (++pslot == slots) pslot = 0;
+    }
+    __device__ __forceinline__ void next_slice() {
+        pk = 0;
+        if (++pj == L) { pj = 0; pcol = 0; }
+    }
+    // the next unit: wait for it where it has just been copied.  A wait that
+    // gives up clears ok for good; the caller then reads no unit any more (its
+    // indices are not there)
+    __device__ __forceinline__ const unsigned char *take(int nc, bool first, bool &ok) {
+        if (first || !resident) ok = ok && cg_mbar_wait(bars + slot, phase);
+        const unsigned char *d = unit(slot, ccol);
+        ccol += nc;
+        if (++slot == slots) { slot = 0; phase ^= 1u; }
+        return d;
+    }
+};
+
+// Set up the warp's region and issue its first units.  sp: the CTA's slice
+// bounds in shared memory; cols: columns a warp's region holds.
+template <typename R>
+__device__ __forceinline__ void mat_start(MatRing<R> &m, const CGArgs<R> &a, const int *sp, int nslices,
+                                          unsigned char *region, unsigned long long *bars, int lane, int warp, int nw) {
+    m.base = region + (size_t)warp * a.ring_cols * MatRing<R>::kColBytes;
+    m.bars = bars + warp * kMaxUnits;
+    m.sp = sp + warp;
+    m.nw = nw;
+    m.L = warp < nslices ? (nslices - warp + nw - 1) / nw : 0;
+    int cols = 0, units = 0;
+    for (int j = 0; j < m.L; j++) {
+        const int w = (m.sp[j * nw + 1] - m.sp[j * nw]) / kSlice;
+        cols += w;
+        for (int k = 0; k < w; k += unit_cols(w - k)) units++;
+    }
+    m.resident = cols <= a.ring_cols && units <= kMaxUnits;
+    m.slots = m.resident ? units : min(kMaxUnits, a.ring_cols / kUnitMax);
+    m.pj = m.pk = m.pslot = m.pcol = 0;
+    m.slot = m.ccol = 0;
+    m.phase = 0;
+    if (lane == 0) {
+        for (int k = 0; k < m.slots; k++) cg_mbar_init(m.bars + k);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        for (int k = 0; k < m.slots; k++) m.issue(a.col, a.Aval);
+    }
+    __syncwarp();
+}
+
+// The row sum sum_k val_k gather(col_k) of the warp's next slice (w columns),
+// GU units' gathers in flight together; per(k, v, g) sees every product's
+// parts in column order.  Refills what it consumed.
+template <typename R, int GU, typename F, typename P>
+__device__ __forceinline__ void mat_slice(MatRing<R> &m, const CGArgs<R> &a, int w, bool first, int lane, bool &ok,
+                                          F gather, P per) {
+    using G = decltype(gather(0, 0));
+    int used = 0;
+    for (int k = 0; k < w;) {
+        G g[GU][kUnitMax];
+        const R *vp[GU];
+        int nc[GU];
+        int kk = k;
+#pragma unroll
+        for (int u = 0; u < GU; u++) {
+            nc[u] = kk < w ? unit_cols(w - kk) : 0;
+            if (nc[u] == 0) continue;
+            const unsigned char *d = m.take(nc[u], first, ok);
+            kk += nc[u];
+            used++;
+            if (!ok) { nc[u] = 0; continue; }
+            const int *ci = reinterpret_cast<const int *>(d) + lane;
+            vp[u] = reinterpret_cast<const R *>(d + nc[u] * kSlice * 4) + lane;
+#pragma unroll
+            for (int j = 0; j < kUnitMax; j++)
+                if (j < nc[u]) g[u][j] = gather(ci[j * kSlice], kk - nc[u] + j);
+        }
+#pragma unroll
+        for (int u = 0; u < GU; u++) {
+#pragma unroll
+            for (int j = 0; j < kUnitMax; j++)
+                if (j < nc[u]) per(vp[u][j * kSlice], g[u][j]);
+        }
+        k = kk;
+        if (!m.resident) {
+            __syncwarp();                     // every lane is done with the units refilled now
+            if (lane == 0 && ok)
+                for (int u = 0; u < used; u++) m.issue(a.col, a.Aval);
+            used = 0;
+        }
+    }
+}
+
+template <typename R>
+__global__ void __launch_bounds__(512, 1) k_cn_smem(const CGArgs<R> a) {
+    constexpr int GU = sizeof(R) == 4 ? 2 : 1;
+    extern __shared__ __align__(128) unsigned char cg_sm[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int G = gridDim.x;
+    const CgShare sh = cg_share(a);
+    const int b0 = sh.b0, nb = sh.nb, rb = sh.rb, re = sh.re, ns = sh.s1 - sh.s0;
+    GridBarrier *bar = a.bar + sh.inst;
+    unsigned long long tag = *(volatile unsigned long long *)&bar->seq;
+    // dynamic shared memory: the warps' regions, their mbarriers, the slice bounds
+    unsigned long long *bars =
+        reinterpret_cast<unsigned long long *>(cg_sm + (size_t)nw * a.ring_cols * MatRing<R>::kColBytes);
+    int *sp = reinterpret_cast<int *>(bars + nw * kMaxUnits);
+    for (int k = threadIdx.x; k <= ns; k += blockDim.x) sp[k] = __ldg(a.slice_ptr + sh.s0 + k);
+    __syncthreads();
+    MatRing<R> m;
+    mat_start(m, a, sp, ns, cg_sm, bars, lane, warp, nw);
+    bool ok = true;                           // no copy's wait has given up
+    auto leave = [&]() {
+        // the copies in flight land before the CTA's memory goes: a ring has
+        // all its slots issued, a resident share none after the first sweep
+        if (!m.resident && lane == 0) {
+            for (int k = 0; k < m.slots; k++) {
+                bool landed = true;
+                m.take(0, true, landed);
             }
         }
-    }
-    if ((int)blockIdx.x == b0 && threadIdx.x == 0) {
-        bar->seq = tag;                       // every CTA of the group has read the old one
-        atomicAdd(a.iters_total, (unsigned long long)it);
-        atomicMax(a.iters_max, (unsigned int)it);
-        if (!converged) atomicAdd(a.fails, 1u);
-        if (a.last) {
-            a.last[2 * inst] = (double)it;
-            a.last[2 * inst + 1] = rr0 > 0.0 ? sqrt(fmax(rr_last, 0.0) / rr0) : 0.0;
+        __syncwarp();
+    };
+
+    // ---- prologue, as k_cn_half's ----
+    const bool pred = a.delta != nullptr;
+    const bool lin = a.dext != nullptr;
+    R *cur = a.q0, *nxt = a.q1;
+    double rr0, stop2, rr_last;
+    bool converged;
+    {
+        double v[3] = {0.0, 0.0, 0.0};
+        const R *dv0 = lin ? a.dext : a.delta;
+        for (int j = warp; j < ns; j += nw) {
+            const int row = (sh.s0 + j) * kSlice + lane, beg = sp[j], w = (sp[j + 1] - beg) / kSlice;
+            const bool on = row >= rb && row < re;
+            const R di = on ? __ldg(a.dinv + row) : R(1), d0 = on && pred ? dv0[row] : R(0);
+            R ax = R(0), bx = R(0), ad = R(0);
+            mat_slice<R, 1>(m, a, w, true, lane, ok, [&](int c, int k) {
+                return Quad<R>{a.x[c], __ldg(a.Bval + beg + k * kSlice + lane), pred ? dv0[c] : R(0), R(0)};
+            }, [&](R av, const Quad<R> &t) {
+                ax += av * t.z;
+                bx += t.p * t.z;
+                ad += av * t.w;
+            });
+            if (on) {
+                const R rref = bx - ax;
+                const R r = pred ? rref - ad : rref;
+                quad_store(cur, row, di * r, R(0), R(0), d0);
+                v[0] += (double)r * (double)r;
+                v[1] += (double)bx * (double)bx;
+                v[2] += (double)rref * (double)rref;
+            }
         }
+        double t[3];
+        if (!group_reduce(a.slots, G, ++tag, b0, nb, a.bar_extra, bar, v, t, ok)) { leave(); return; }
+        rr0 = t[2];
+        stop2 = fmax(a.tol * a.tol * rr0, a.floor_rel * a.floor_rel * t[1]);
+        rr_last = t[0];
+        converged = t[0] <= stop2;
     }
+    int it = 0;
+    R al = R(0), be = R(0);
+    while (!converged && it < a.maxit) {
+        double v[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        if (m.resident) m.ccol = 0;
+        for (int j = warp; j < ns; j += nw) {
+            const int row = (sh.s0 + j) * kSlice + lane, w = (sp[j + 1] - sp[j]) / kSlice;
+            const bool on = row >= rb && row < re;
+            Quad<R> o{R(0), R(0), R(0), R(0)};
+            R di = R(1);
+            if (on) { o = quad_load(cur, row); di = __ldg(a.dinv + row); }
+            R q = R(0);
+            mat_slice<R, GU>(m, a, w, false, lane, ok, [&](int c, int) { return quad_dir(cur, c, al, be); },
+                             [&](R av, R g) { q += av * g; });
+            if (on) {
+                const R z = fma(-al, o.w, o.z), p = fma(be, o.p, z), wv = di * q;
+                quad_store(nxt, row, z, p, wv, fma(al, o.p, o.d));
+                const double d = (double)(R(1) / di), dz = d * (double)z, dw = d * (double)wv;
+                v[0] += (double)p * (double)q;
+                v[1] += dz * (double)z;
+                v[2] += dz * (double)wv;
+                v[3] += dw * (double)wv;
+                v[4] += dz * dz;
+                v[5] += dz * dw;
+                v[6] += dw * dw;
+            }
+        }
+        double t[7];
+        if (!group_reduce(a.slots, G, ++tag, b0, nb, a.bar_extra, bar, v, t, ok)) { leave(); return; }
+        { R *sw = cur; cur = nxt; nxt = sw; }
+        // the scalars and tests of k_cn_half
+        if (t[4] <= stop2) { rr_last = t[4]; converged = true; al = R(0); break; }
+        const double alpha = t[1] / t[0];
+        const double rz = t[1] - 2.0 * alpha * t[2] + alpha * alpha * t[3];
+        rr_last = t[4] - 2.0 * alpha * t[5] + alpha * alpha * t[6];
+        it++;
+        al = (R)alpha;
+        be = (R)(rz / t[1]);
+        if (!isfinite(rr_last)) break;
+        converged = rr_last <= stop2 && stop2 >= 1e-12 * t[4];
+    }
+    leave();
+    cg_finish(a, sh, warp, nw, lane, cur, al, be, converged, tag, it, rr_last, rr0);
 }
 
 // ---------------------------------------------------------------------------
@@ -883,6 +1208,12 @@ __global__ void __launch_bounds__(NB == 4 ? 768 : 256, NB == 4 ? 2 : 4) k_cn_hal
     }
 }
 
+// k_cn_smem: shared memory of a CTA with `cols` matrix columns per warp and ns
+// slices at most
+static size_t smem_bytes(int block, int cols, int ns, int rsize) {
+    return (size_t)(block / 32) * ((size_t)cols * kSlice * (4 + rsize) + kMaxUnits * 8) + ((size_t)ns + 1) * 4;
+}
+
 // the kernel of a (gather width, variant) choice and its dynamic shared
 // memory; cg_batch kStagedBatch selects k_cn_half_staged with `depth` units
 // in flight per warp (1 .. kStageMaxDepth)
@@ -892,7 +1223,7 @@ __global__ void __launch_bounds__(NB == 4 ? 768 : 256, NB == 4 ? 2 : 4) k_cn_hal
 template <typename R>
 static int cg_kernel(int block, int batch, int variant, int depth, const void **fn, size_t *smem,
                      bool set_attr) {
-    *smem = 0;
+    *smem = 0;                 // (k_cn_smem: `depth` is its bytes)
     if (batch == kStagedBatch) {
         if (variant != 0) { set_error("the staged CG runs the two-reduction recurrences only"); return EP_ERR_ARG; }
         if (depth < 1 || depth > kStageMaxDepth) {
@@ -904,6 +1235,13 @@ static int cg_kernel(int block, int batch, int variant, int depth, const void **
         if (set_attr)
             EP_CUDA(cudaFuncSetAttribute(*fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)stage_smem_bytes(256, kStageMaxDepth, (int)sizeof(R))));
+        return EP_OK;
+    }
+    if (batch == kSmemBatch) {
+        *fn = (const void *)k_cn_smem<R>;
+        *smem = (size_t)depth;
+        if (set_attr)
+            EP_CUDA(cudaFuncSetAttribute(*fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
         return EP_OK;
     }
     *fn = variant == 1 ? (batch >= 8 ? (const void *)k_cn_half_cg1<R, 8> : (const void *)k_cn_half_cg1<R, 4>)
@@ -930,37 +1268,83 @@ int cg_max_per_sm(int block, int *per, int batch, int variant, int depth) {
     return EP_OK;
 }
 
-// The launch of a handle that leaves cg_per_sm to the library (0), and of
-// ep_cn_half_step_noalloc: no more CTAs than there are slices for, since
-// every CTA takes part in each iteration's reduction, and one CTA per SM once
-// the slices fill the GPU.
-//   up to 32 slices: one CTA, whose reductions need no global memory;
-//   up to 8 warps per SM: 256 threads, one slice per warp;
-//   beyond: one CTA per SM, of 512 threads up to 16 slices per SM and of 1024
-//   above (with the 64 registers a thread has, a full SM either way).
-// Batches keep CTAs of `block` threads, as many as fit: each instance's group
-// is small already and more CTAs split the GPU more evenly between them.
+// The launch of a handle that leaves cg_per_sm to the library (0) and keeps
+// cg_block 256, cg_batch 4 and cg_variant 0, and of ep_cn_half_step_noalloc.
+// No more CTAs than there are slices for, since every CTA takes part in each
+// iteration's reduction (measured: CG us a step, two solves, 16-30 iterations):
+//   up to 32 slices: k_cn_half on one CTA, whose reductions need no global
+//     memory (FP32, 715 nodes: 86 us against 87; FP64 takes k_cn_smem, 158
+//     against 205);
+//   up to 8 slices per SM: k_cn_smem with 256 threads, one slice per warp
+//     (28.6K nodes, FP32 / FP64: 105 / 192 us; 512 threads 111 / 223; k_cn_half
+//     149 / 257);
+//   beyond: k_cn_smem with 512 threads, one CTA per SM (143K nodes: 144 / 337
+//     us, k_cn_half 171 / 384), with 200 KB of shared memory where the matrix
+//     then stays in it, else 120 KB, which leaves the gathers more L1 (765K
+//     nodes, FP32: 735 us, 784 with 200 KB, 1131 with k_cn_half);
+//   except FP32 just past that (its matrix still in L2, up to 64 slices per
+//     SM): k_cn_half with 1024 threads, whose twice as many warps hide the
+//     latency as well (263K nodes: 270 us against 284).
+// Batches run k_cn_smem in two CTAs of 256 threads per SM (24 slabs, 446K
+// nodes: 397 us; k_cn_half 416): more CTAs split the GPU more evenly between
+// the instances, whose groups are small already.
+// Any other launch config, and more instances than those CTAs, run k_cn_half
+// with CTAs of `block` threads, as many as fit.
 template <typename R>
-int cg_auto_shape(int nslices, int ninst, int batch, int variant, int depth, int *block, int *grid) {
+int cg_auto_shape(int nslices, int ninst, int batch, int variant, int depth, CgShape *out) {
     int dev = 0, nsm = 0, per = 0;
     EP_CUDA(cudaGetDevice(&dev));
     EP_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    int rc = cg_max_per_sm<R>(*block, &per, batch, variant, depth);
-    if (rc) return rc;
-    if (variant == 0 && batch == 4 && *block == 256 && ninst == 1) {
-        if (nslices <= 32) *block = std::max(256, nslices * 32);
-        else if (nslices > 16 * nsm) *block = 1024;
-        else if (nslices > 8 * nsm) *block = 512;
-        if (*block != 256) per = 1;
+    out->batch = batch;
+    out->ring_cols = out->smem = 0;
+    if (variant == 0 && batch == 4 && out->block == 256 && ninst <= 2 * nsm) {
+        if (ninst == 1 && sizeof(R) == 4 && nslices <= 32) {
+            out->block = std::max(256, nslices * 32);
+            out->grid = 1;
+            return EP_OK;
+        }
+        out->batch = kSmemBatch;
+        out->per_sm = ninst > 1 ? 2 : 1;
+        out->block = ninst > 1 || nslices <= 8 * nsm ? 256 : 512;
+        out->grid = std::min(out->per_sm * nsm, div_up(nslices, out->block / 32) + (ninst > 1 ? ninst : 0));
+        return EP_OK;
     }
-    if (ninst > nsm * per && *block > 128) {
+    int rc = cg_max_per_sm<R>(out->block, &per, batch, variant, depth);
+    if (rc) return rc;
+    if (ninst > nsm * per && out->block > 128) {
         // more instances than CTAs of this size fit: a warp group each
-        *block = 128;
-        if ((rc = cg_max_per_sm<R>(*block, &per, batch, variant, depth))) return rc;
+        out->block = 128;
+        if ((rc = cg_max_per_sm<R>(out->block, &per, batch, variant, depth))) return rc;
     }
     // an instance's share of the slices is rounded up to whole CTAs
-    *grid = std::min(nsm * per, div_up(nslices, *block / 32) + (ninst > 1 ? ninst : 0));
+    out->grid = std::min(nsm * per, div_up(nslices, out->block / 32) + (ninst > 1 ? ninst : 0));
     return EP_OK;
+}
+
+// k_cn_smem's sizes for CTAs of at most ns slices of about `cols` columns (and
+// the one range of sizes that goes back to k_cn_half)
+template <typename R>
+int cg_fit_smem(int ns, int cols, CgShape *out) {
+    const int warps = out->block / 32, spw = div_up(ns, warps);
+    auto fit = [&](int kb) {
+        const long long budget = (long long)kb * 1024 / out->per_sm - ((long long)ns + 1) * 4;
+        return (int)((budget / warps - kMaxUnits * 8) / (kSlice * (4 + (int)sizeof(R))));
+    };
+    const bool stays = out->per_sm == 1 && spw * (cols + 1) <= fit(200);
+    if (!stays && out->per_sm == 1 && sizeof(R) == 4 && ns <= 64) {
+        out->batch = 4;
+        out->block = 1024;
+        return EP_OK;
+    }
+    // a share that stays gets room for slices half as wide again
+    out->ring_cols = std::min(std::max(spw * (cols + cols / 2), 2 * kUnitMax), fit(stays ? 200 : 120));
+    // a slice's gathers take up to two units of the ring at once
+    if (out->ring_cols < 2 * kUnitMax) { set_error("CG kernel: %d matrix columns per warp are too few", out->ring_cols); return EP_ERR_ARG; }
+    out->smem = (int)smem_bytes(out->block, out->ring_cols, ns, (int)sizeof(R));
+    int per = 0;
+    int rc = cg_max_per_sm<R>(out->block, &per, kSmemBatch, 0, out->smem);
+    if (!rc && per < out->per_sm) { set_error("CG kernel: %d CTAs per SM instead of %d", per, out->per_sm); rc = EP_ERR_CUDA; }
+    return rc;
 }
 
 template <typename R>
@@ -987,7 +1371,10 @@ int launch_cg(const CGArgs<R> &a, int grid, int block, cudaStream_t s, int batch
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (batch == kStagedBatch) {
+    if (batch == kSmemBatch) {
+        cfg.dynamicSmemBytes = a.smem;
+        EP_CUDA(cudaLaunchKernelEx(&cfg, k_cn_smem<R>, a));
+    } else if (batch == kStagedBatch) {
         const void *fn = nullptr;
         size_t smem = 0;
         int rc = cg_kernel<R>(block, batch, variant, a.depth, &fn, &smem, false);
@@ -1010,8 +1397,10 @@ int launch_cg(const CGArgs<R> &a, int grid, int block, cudaStream_t s, int batch
 
 template int launch_cg<float>(const CGArgs<float> &, int, int, cudaStream_t, int, int);
 template int launch_cg<double>(const CGArgs<double> &, int, int, cudaStream_t, int, int);
-template int cg_auto_shape<float>(int, int, int, int, int, int *, int *);
-template int cg_auto_shape<double>(int, int, int, int, int, int *, int *);
+template int cg_auto_shape<float>(int, int, int, int, int, CgShape *);
+template int cg_auto_shape<double>(int, int, int, int, int, CgShape *);
+template int cg_fit_smem<float>(int, int, CgShape *);
+template int cg_fit_smem<double>(int, int, CgShape *);
 template int cg_grid_size<float>(int, int *, int, int, int, int);
 template int cg_grid_size<double>(int, int *, int, int, int, int);
 template int cg_max_per_sm<float>(int, int *, int, int, int);

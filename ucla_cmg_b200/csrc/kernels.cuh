@@ -142,12 +142,17 @@ template <typename R> struct CGArgs {
     // staged variant (cg_batch kStagedBatch): units of 8 slice columns each
     // warp keeps in flight in its shared-memory ring (1 .. kStageMaxDepth)
     int depth;
+    // k_cn_smem: matrix columns of a warp's region and the CTA's dynamic shared memory
+    int ring_cols, smem;
 };
 
 // cg_batch value of the staged kernel (asynchronous copies of each warp's
 // next units of SELL columns into shared memory), its deepest ring and the
 // depth it runs at when none is asked for
 constexpr int kStagedBatch = 32;
+// the library's own choice (k_cn_smem; not a cg_batch value) and its shared memory at most
+constexpr int kSmemBatch = 64;
+constexpr int kSmemMax = 216 * 1024;
 // the learned step's fallback list runs one warp per node up to this many
 // nodes (its time is then one node's serial Newton chain), one thread per
 // node beyond (throughput)
@@ -160,10 +165,13 @@ constexpr int kStageDepthDefault = 2;
 // (needs r, r1, w0, w1, s0, s1, p0)
 template <typename R>
 int launch_cg(const CGArgs<R> &a, int grid, int block, cudaStream_t s, int batch = 4, int variant = 0);
-// block and grid of a launch whose shape is left to the library (*block: the
-// asked block size in, the launch's out)
+// a launch whose shape is left to the library: kernel (batch), threads, CTAs
+// and k_cn_smem's sizes (block: the asked size in, the launch's out)
+struct CgShape { int batch, block, grid, per_sm, ring_cols, smem; };
 template <typename R>
-int cg_auto_shape(int nslices, int ninst, int batch, int variant, int depth, int *block, int *grid);
+int cg_auto_shape(int nslices, int ninst, int batch, int variant, int depth, CgShape *out);
+template <typename R>
+int cg_fit_smem(int ns, int cols, CgShape *out);
 // CTAs of the persistent launch: per_sm (0 = as many as fit) x SM count
 template <typename R>
 int cg_grid_size(int block, int *grid, int per_sm = 0, int batch = 4, int variant = 0, int depth = 0);

@@ -83,10 +83,15 @@ int run(unsigned char *base, int n, int nslices, const int *slice_ptr, const int
     a.maxit = maxit > 0 ? maxit : 1000;
     // the barrier's tags go on from call to call (the array starts zeroed),
     // and the kernel writes the records before it reads them
-    int grid = 0, block = 256;
-    int rc = cg_auto_shape<R>(nslices, 1, 4, 0, 0, &block, &grid);
+    CgShape cg{4, 256, 0, 0, 0, 0};
+    int rc = cg_auto_shape<R>(nslices, 1, 4, 0, 0, &cg);
+    // the rows' widths are on the device; 16 columns are a linear-tet mesh's
+    // (wider slices only make a share that would stay a ring)
+    if (!rc && cg.batch == kSmemBatch) rc = cg_fit_smem<R>(div_up(nslices, cg.grid), 16, &cg);
     if (rc) return rc;
-    if ((rc = launch_cg<R>(a, grid, block, s))) return rc;
+    a.ring_cols = cg.ring_cols;
+    a.smem = cg.smem;
+    if ((rc = launch_cg<R>(a, cg.grid, cg.block, s, cg.batch))) return rc;
     // barrier and result in one copy
     unsigned char back[160];
     EP_CUDA(cudaMemcpyAsync(back, tail, sizeof back, cudaMemcpyDeviceToHost, s));
