@@ -335,7 +335,7 @@ int  ep_assemble_operators(const ep_mesh_desc *mesh, const ep_cables_desc *cable
  * host, k > 0 replays the steps from an instantiated CUDA graph of k steps
  * (rounded up to a multiple of the ECG interval); ionic_min_ctas: FP32
  * ionic kernel compiled for at least 3 or 4 resident 128-thread CTAs per SM
- * (fewer registers per thread), 0 = the compiler's register choice;
+ * (fewer registers per thread), 0 = the library's choice by cell model;
  * cg_batch: SELL columns whose gathers the CG kernel issues together (4 or
  * 8; 8 keeps more loads in flight at a larger register budget; 16: groups of
  * 8 with the next group's index loads issued before the current gathers;

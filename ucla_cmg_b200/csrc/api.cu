@@ -579,7 +579,6 @@ static int launch_learned_phase(ep_handle *h, const IonicArgs<float> &ia) {
     IonicArgs<float> fb = ia;
     fb.node_list = h->sg_list.as<int>();
     fb.list_count = h->sg_count.as<int>();
-    fb.list_warp_max = kFallbackWarpMax;    // a short list: one warp per node
     EP_CUDA(cudaEventRecord(h->ev_fork, h->stream));
     EP_CUDA(cudaStreamWaitEvent(h->side, h->ev_fork, 0));
     if ((rc = launch_ionic<float>(EP_TUSSCHER, fb, h->side, h->ionic_block, h->ionic_min))) return rc;
@@ -666,7 +665,7 @@ static int step_typed(ep_handle *h, int nsteps, size_t &ne) {
         if constexpr (sizeof(R) == 4) {
             if (h->precision == EP_SURROGATE) {
                 if ((rc = launch_learned_phase(h, ia))) return rc;
-                h->launches += h->sg_vupdate == 2 ? 4 : 3;   // network, [physics,] fallback by warps and by threads
+                h->launches += h->sg_vupdate == 2 ? 3 : 2;   // network, [physics,] fallback list
             } else if ((rc = ionic_phase<R>(h, ia))) {
                 return rc;
             }
@@ -2233,6 +2232,7 @@ static int ionic_batch(const ep_model_desc *md, int32_t precision, int32_t n, do
         fill_ionic_args<R>(&h, a);
         a.track = nullptr;
         a.dvdt_out = dvdt ? dvd.as<R>() : nullptr;
+        a.ref_order = sizeof(R) == 4;        // FP32 plugin results keep their bits
         if ((r2 = launch_ionic<R>(h.model, a, h.stream))) return r2;
         EP_CUDA(cudaStreamSynchronize(h.stream));
         std::vector<double> o, so;

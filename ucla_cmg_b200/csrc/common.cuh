@@ -99,6 +99,40 @@ __device__ __forceinline__ bool grid_sync(GridBarrier *b, unsigned int nblocks) 
     return s_ok != 0;
 }
 
+// ---- arithmetic of the cell models ----
+// a / b.  FP32 on the device: the hardware reciprocal estimate (1 ulp) and one
+// correction of the quotient by its exact remainder (P. Markstein, IBM J.
+// Res. Dev. 34 (1990) 111), four instructions without the special-case branch
+// of the / operator, which the models' wide-ranging denominators take often
+// enough to cost more than the arithmetic around them (Mahajan's FP32 kernel
+// ran with 9 of 32 lanes active).  Within 0.51 ulp where b and the quotient
+// are normal and |b| < 2^126; the callers keep their denominators there.
+EP_HD double dv(double a, double b) { return a / b; }
+EP_HD float dv(float a, float b) {
+#ifdef __CUDA_ARCH__
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
+    const float q = a * r;
+    return fmaf(fmaf(-b, q, a), r, q);
+#else
+    return a / b;
+#endif
+}
+// x / d for a constant d: the reciprocal in two parts, the quotient rounded
+// as a division's to within half an ulp more
+template <typename R> EP_HD R over(R x, double d) {
+    const R hi = (R)(1.0 / d);
+    const R lo = sizeof(R) == 4 ? (R)(1.0 / d - (double)hi) : (R)(fma(-(double)hi, d, 1.0) / d);
+    return fma(x, hi, x * lo);
+}
+// exp(x), the argument capped where 1 + exp(x) is exp(x) to every digit and
+// products of three such factors still fit the type
+EP_HD float cexp(float x) { return expf(fminf(x, 28.f)); }
+EP_HD double cexp(double x) { return exp(fmin(x, 200.0)); }
+// exp(x) - 1, the argument capped as the reach of the type asks
+EP_HD float cexpm1(float x) { return expm1f(fminf(x, 80.f)); }
+EP_HD double cexpm1(double x) { return expm1(fmin(x, 600.0)); }
+
 template <typename T> struct RealName;
 template <> struct RealName<float> { static constexpr const char *s = "f32"; };
 template <> struct RealName<double> { static constexpr const char *s = "f64"; };

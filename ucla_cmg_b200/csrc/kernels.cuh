@@ -2,6 +2,7 @@
 #pragma once
 #include "common.cuh"
 #include "tt.cuh"
+#include "tt_step.cuh"
 #include "mahajan.cuh"
 #include "lr.cuh"
 #include "purkinje.cuh"
@@ -78,13 +79,11 @@ template <typename R> struct IonicArgs {
                                  // dV/dt, leave V unchanged (one sub-step)
     const int *node_list;        // non-null: run only these nodes (count on the device)
     const int *list_count;
-    int list_warp_max;           // > 0 (ten Tusscher lists): a list of at most this many
-                                 // nodes runs one warp per node (k_ionic_warp), a longer
-                                 // one one thread per node
     const uint8_t *skip;         // non-null: nodes with skip[i] != 0 are left alone (mixed
                                  // tissues: the Purkinje nodes in the tissue model's launch)
     // model options
     TTOpts tt;
+    int ref_order;               // ten Tusscher: the reference's order of operations (tt.cuh) with either Jacobian
     int mh_abs;
     const R *lr_table;           // nullable
     // stride: the per-node adaptive sub-steps of the backward-Euler and
@@ -153,10 +152,6 @@ constexpr int kStagedBatch = 32;
 // the library's own choice (k_cn_smem; not a cg_batch value) and its shared memory at most
 constexpr int kSmemBatch = 64;
 constexpr int kSmemMax = 216 * 1024;
-// the learned step's fallback list runs one warp per node up to this many
-// nodes (its time is then one node's serial Newton chain), one thread per
-// node beyond (throughput)
-constexpr int kFallbackWarpMax = 4096;
 constexpr int kStageMaxDepth = 4;
 constexpr int kStageDepthDefault = 2;
 

@@ -15,90 +15,95 @@ constexpr int MH_NS = 25;   // stored states besides V: reference State[1..25]
 constexpr int MH_NC = 35;
 
 // r[k] receives the rate of reference state k (k = 0..25); s[k] holds
-// reference state k (s[0] = V).
+// reference state k (s[0] = V).  The reference's expressions with their
+// fractions brought over one denominator (some 110 divisions of one call
+// become 40), 1 - x as the complementary fraction, exp(x) - 1 as expm1, and
+// factors that cancel left out (fca in k4 and s2).
 template <typename R>
 EP_HD void mh_rhs(const R s[26], const R *__restrict__ c, R h, R istim, R r[26]) {
-    const R V = s[0], frt = c[24];
-    const R inv_frt = R(1) / frt;
+    const R one = R(1);
+    const R V = s[0], frt = c[24], vf = V * frt;
+    const R rtf = dv(one, frt), inv_h = dv(one, h);
+    // a gate's rate over the step, (inf - s)(1 - exp(-h k)) / h with k = 1 / tau
+    auto relax = [&](R inf, R sk, R hk) { return (sk - inf) * expm1(-hk) * inv_h; };
     // I_K1
-    const R ek1 = inv_frt * log((R(100) * c[2] + R(1) * c[0]) / (R(100) * c[1] + R(1) * s[19]));
-    const R gki = sqrt(c[2] / R(5.4));
-    const R aki = R(1.02) / (R(1) + exp(R(0.2385) * (V - ek1 - R(59.215))));
-    const R bki = (R(0.49124) * exp(R(0.08032) * (V - ek1 + R(5.476))) + exp(R(0.061750) * (V - ek1 - R(594.31))))
-                / (R(1) + exp(R(-0.5143) * (V - ek1 + R(4.753))));
-    const R xik1 = c[11] * gki * (aki / (aki + bki)) * (V - ek1);
+    R xik1;
+    {
+        const R w = V - rtf * log(dv(R(100) * c[2] + c[0], R(100) * c[1] + s[19]));
+        const R e1 = one + cexp(R(0.2385) * (w - R(59.215)));
+        const R n = R(0.49124) * cexp(R(0.08032) * (w + R(5.476))) + exp(R(0.061750) * (w - R(594.31)));
+        const R d = R(1.02) * (one + cexp(R(-0.5143) * (w + R(4.753))));
+        xik1 = c[11] * sqrt(over(c[2], 5.4)) * dv(d, d + n * e1) * w;
+    }
     // I_to (slow + fast)
-    const R ek = inv_frt * log(c[2] / c[1]);
-    const R rt1 = -(V + R(3)) / R(15), rt2 = (V + R(33.5)) / R(10), rt3 = (V + R(60)) / R(10);
-    const R xtos_inf = R(1) / (R(1) + exp(rt1));
-    const R ytos_inf = R(1) / (R(1) + exp(rt2));
-    const R txs = R(9) / (R(1) + exp(-rt1)) + R(0.5);
-    const R tys = R(3000) / (R(1) + exp(rt3)) + R(30);
-    const R xitos = c[6] * s[22] * (s[23] + R(0.5) * ytos_inf) * (V - ek);
-    r[22] = (xtos_inf - (xtos_inf - s[22]) * exp(-h / txs) - s[22]) / h;
-    r[23] = (ytos_inf - (ytos_inf - s[23]) * exp(-h / tys) - s[23]) / h;
-    const R rt4 = -(V / R(30)) * (V / R(30));
-    const R txf = R(3.5) * exp(rt4) + R(1.5);
-    const R tyf = R(20) / (R(1) + exp(rt2)) + R(20);
-    const R xitof = c[7] * s[20] * s[21] * (V - ek);
-    r[20] = (xtos_inf - (xtos_inf - s[20]) * exp(-h / txf) - s[20]) / h;
-    r[21] = (ytos_inf - (ytos_inf - s[21]) * exp(-h / tyf) - s[21]) / h;
-    const R xito = xitos + xitof;
+    const R vk = V - rtf * log(dv(c[2], c[1]));
+    R xito;
+    {
+        const R e1 = cexp(over(-(V + R(3)), 15));
+        const R xi = dv(one, one + e1);
+        const R yi = dv(one, one + cexp(over(V + R(33.5), 10)));
+        const R e3 = one + cexp(over(V + R(60), 10));
+        xito = (c[6] * s[22] * (s[23] + R(0.5) * yi) + c[7] * s[20] * s[21]) * vk;
+        r[22] = relax(xi, s[22], dv(h, R(9) * (e1 * xi) + R(0.5)));
+        r[23] = relax(yi, s[23], dv(h * e3, R(3000) + R(30) * e3));
+        const R v30 = over(V, 30);
+        r[20] = relax(xi, s[20], dv(h, R(3.5) * exp(-(v30 * v30)) + R(1.5)));
+        r[21] = relax(yi, s[21], dv(h, R(20) * yi + R(20)));
+    }
     // I_NaK
-    const R sigma = (exp(c[0] / R(67.3)) - R(1)) / R(7);
-    const R fnak = R(1) / (R(1) + R(0.1245) * exp(R(-0.1) * V * frt) + R(0.0365) * sigma * exp(-V * frt));
-    const R xinak = c[12] * fnak * (R(1) / (R(1) + (R(12) / s[19]))) * c[2] / (c[2] + R(1.5));
+    const R sigma = over(exp(over(c[0], 67.3)) - one, 7);
+    const R xinak = dv(c[12] * c[2] * s[19], (c[2] + R(1.5)) * (s[19] + R(12)) *
+                       (one + R(0.1245) * cexp(R(-0.1) * vf) + R(0.0365) * sigma * cexp(-vf)));
     // Na-Ca exchange flux
-    const R csm = s[8] / R(1000);
+    const R csm = over(s[8], 1000);
     const R na3 = s[19] * s[19] * s[19], nao3 = c[0] * c[0] * c[0];
-    const R ez = exp(V * (R(0.35) - R(1)) * frt);
     R jnaca;
     {
-        const R zw3 = na3 * c[3] * exp(V * R(0.35) * frt) - nao3 * csm * ez;
-        const R zw4 = R(1) + R(0.2) * ez;
-        const R q = R(0.3) / s[8];
-        const R aloss = R(1) / (R(1) + q * q * q);
-        const R yz1 = R(1.3) * na3 + R(669921.875) * csm;               // 87.5^3
-        const R yz2 = R(1860.867) * c[3] * (R(1) + csm / R(0.0036));    // 12.3^3
-        const R qn = s[19] / R(12.3);
-        const R yz3 = R(0.0036) * nao3 * (R(1) + qn * qn * qn);
-        const R yz4 = na3 * c[3] + nao3 * csm;
-        jnaca = c[8] * aloss * zw3 / (zw4 * (yz1 + yz2 + yz3 + yz4));
+        const R ez = cexp(R(-0.65) * vf);
+        const R zw3 = na3 * c[3] * cexp(R(0.35) * vf) - nao3 * csm * ez;
+        const R c3 = s[8] * s[8] * s[8];
+        const R qn = over(s[19], 12.3);
+        const R yz = R(1.3) * na3 + R(669921.875) * csm                                  // 87.5^3
+                   + R(1860.867) * c[3] * (one + over(csm, 0.0036))                      // 12.3^3
+                   + R(0.0036) * nao3 * (one + qn * qn * qn) + na3 * c[3] + nao3 * csm;
+        jnaca = dv(c[8] * c3 * zw3, (c3 + R(0.027)) * (one + R(0.2) * ez) * yz);
     }
     // Ca cycling
-    const R jd = c[28] * (s[8] - s[9]) / c[14];
+    const R jd = dv(c[28] * (s[8] - s[9]), c[14]);
     r[24] = c[29] * (R(0.0327) * s[9] * (R(70) - s[24]) - R(0.0196) * s[24]);
     r[25] = R(0.0327) * s[8] * (R(70) - s[25]) - R(0.0196) * s[25];
-    const R jup = c[30] * (c[13] * s[9] * s[9] / (s[9] * s[9] + R(0.25)));
-    const R jleak = c[27] * (R(0.00002069) * s[10] * s[10] / (s[10] * s[10] + R(2500)) * (s[10] * R(16.667) - s[9]));
+    const R jup = dv(c[30] * c[13] * (s[9] * s[9]), s[9] * s[9] + R(0.25));
+    const R jleak = c[27] * dv(R(0.00002069) * (s[10] * s[10]), s[10] * s[10] + R(2500)) * (s[10] * R(16.667) - s[9]);
     // Markov L-type Ca channel
     R po;
     {
-        const R poinf = R(1) / (R(1) + exp(-V / R(8)));
-        const R alpha = poinf, beta = R(1) - poinf;
+        const R e8 = cexp(over(-V, 8));
+        const R alpha = dv(one, one + e8), beta = e8 * alpha;
         const R r1 = R(0.30), r2 = R(3);
-        const R q = R(3) / s[7];
-        const R fca = R(1) / (R(1) + q * q * q);
+        const R cp3 = s[7] * s[7] * s[7], fca = dv(cp3, cp3 + R(27));
         const R s1 = R(0.0182688) * fca, s1t = R(0.00195);
         const R k1 = R(0.024168) * fca;
         const R k2 = R(1.03615e-4), k1t = R(0.00413), k2t = R(0.00224);
-        const R s2 = s1 * (r1 / r2) * (k2 / k1);
-        const R s2t = s1t * (r1 / r2) * (k2t / k1t);
-        const R poi = R(1) / (R(1) + exp(-(V + R(40)) / R(3)));
-        const R k3 = (R(1) - poi) / R(3), k3t = k3;
-        const R Pr = R(1) - R(1) / (R(1) + exp(-(V + R(40)) / R(4)));
-        const R recov = R(10) + R(4954) * exp(V / R(15.6));
-        const R qc = s[7] / R(6.09365);
+        const R s2 = R(0.0182688 * (0.30 / 3.0) * (1.03615e-4 / 0.024168)), s2t = R(0.00195 * (0.30 / 3.0) * (0.00224 / 0.00413));
+        const R e3 = cexp(over(-(V + R(40)), 3));
+        const R k3 = dv(e3, R(3) + R(3) * e3), k3t = k3;
+        const R e4 = cexp(over(-(V + R(40)), 4));
+        const R Pr = dv(e4, one + e4);
+        const R recov = R(10) + R(4954) * cexp(over(V, 15.6));
+        const R qc = over(s[7], 6.09365);
         const R qc2 = qc * qc;
-        const R tau_ca = R(78.0329) / (R(1) + qc2 * qc2) + R(0.1);
-        const R tauca = (recov - tau_ca) * Pr + tau_ca;
-        const R tauba = (recov - R(450)) * Pr + R(450);
-        const R Ps = R(1) / (R(1) + exp(-(V + R(40)) / R(11.32)));
-        const R k6 = fca * Ps / tauca, k5 = (R(1) - Ps) / tauca;
-        const R k6t = Ps / tauba, k5t = (R(1) - Ps) / tauba;
-        const R k4 = k3 * (alpha / beta) * (k1 / k2) * (k5 / k6);
-        const R k4t = k3t * (alpha / beta) * (k1t / k2t) * (k5t / k6t);
-        po = R(1) - s[15] - s[17] - s[16] - s[18] - s[13] - s[14];
+        const R tau_ca = dv(R(78.0329), one + qc2 * qc2) + R(0.1);
+        const R e11 = cexp(over(-(V + R(40)), 11.32));
+        const R Ps = dv(one, one + e11), Qs = e11 * Ps;
+        const R ica = dv(one, (recov - tau_ca) * Pr + tau_ca);
+        const R iba = dv(one, (recov - R(450)) * Pr + R(450));
+        const R k6 = fca * Ps * ica, k5 = Qs * ica;
+        const R k6t = Ps * iba, k5t = Qs * iba;
+        // alpha / beta = 1 / e8; k5 / k6 = e11 / fca, k5t / k6t = e11
+        const R kab = k3 * dv(e11, e8);
+        const R k4 = kab * R(0.024168 / 1.03615e-4);
+        const R k4t = kab * R(0.00413 / 0.00224);
+        po = one - s[15] - s[17] - s[16] - s[18] - s[13] - s[14];
         r[14] = beta * s[13] + k5 * s[17] + k5t * s[18] - (k6 + k6t + alpha) * s[14];
         r[13] = alpha * s[14] + k2 * s[15] + k2t * s[16] + r2 * po - (beta + r1 + k1t + k1) * s[13];
         r[15] = k1 * s[13] + k4 * s[17] + s1 * po - (k3 + k2 + s2) * s[15];
@@ -109,23 +114,25 @@ EP_HD void mh_rhs(const R s[26], const R *__restrict__ c, R h, R istim, R r[26])
     // driving force of I_Ca
     R rxa;
     {
-        const R za = V * R(2) * frt;
-        const R factor1 = R(4) * R(0.00054) * c[23] * c[23] / (c[22] * c[20]);
-        const R ez2 = exp(za);
-        if (fabs(za) < R(0.001))
-            rxa = factor1 * (csm * ez2 - R(0.341) * c[3]) / (R(2) * frt);
-        else
-            rxa = V * factor1 * (csm * ez2 - R(0.341) * c[3]) / (ez2 - R(1));
+        const R za = R(2) * vf;
+        const R factor1 = dv(R(4) * R(0.00054) * c[23] * c[23], c[22] * c[20]);
+        const R em = cexpm1(za);
+        const R num = factor1 * (csm * (em + one) - R(0.341) * c[3]);
+        if (fabs(za) < R(0.001)) rxa = dv(num, R(2) * frt);
+        else rxa = dv(V * num, em);
     }
     const R jca = c[4] * po * rxa;
+    // 1 / (1 + 168 / (7 + c)^2 + 28.2 / (0.6 + c)^2 + 4.5 / (0.3 + c)^2 + 546 / (13 + c)^2)
     auto buf = [](R cv) {
-        return R(1) / (R(1) + R(168) / ((R(7) + cv) * (R(7) + cv)) + R(28.2) / ((R(0.6) + cv) * (R(0.6) + cv))
-                       + R(4.5) / ((R(0.3) + cv) * (R(0.3) + cv)) + R(546) / ((R(13) + cv) * (R(13) + cv)));
+        const R a = (R(7) + cv) * (R(7) + cv), b = (R(0.6) + cv) * (R(0.6) + cv);
+        const R d = (R(0.3) + cv) * (R(0.3) + cv), e = (R(13) + cv) * (R(13) + cv);
+        const R bd = b * d, ae = a * e;
+        return dv(ae * bd, ae * bd + R(168) * e * bd + R(546) * a * bd + ae * (R(28.2) * d + R(4.5) * b));
     };
     r[8] = buf(s[8]) * (R(50) * (s[12] - jd - jca + jnaca) - r[25]);
     r[9] = buf(s[9]) * (jd - jup + jleak - r[24]);
     r[10] = -s[12] + jup - jleak;
-    r[11] = (s[10] - s[11]) / c[17];
+    r[11] = dv(s[10] - s[11], c[17]);
     R Qr;
     {
         const R bv = (c[19] - c[26]) - c[18] * c[19];
@@ -133,78 +140,76 @@ EP_HD void mh_rhs(const R s[26], const R *__restrict__ c, R h, R istim, R r[26])
         if (s[11] > c[26] && s[11] < c[19]) q = s[11] - c[26];
         else if (s[11] >= c[19]) q = c[18] * s[11] + bv;
         if (q >= c[25]) q = c[25];
-        Qr = s[10] * q / c[19];
+        Qr = dv(s[10] * q, c[19]);
     }
     const R arxa = fabs(rxa);
     {
-        const R e = exp(R(-0.05) * (V + R(30)));
-        const R sparkV = e / (R(1) + e);
-        const R spark_rate = R(2.58079) * po * arxa * sparkV;
-        r[12] = spark_rate * Qr - s[12] * (R(1) - c[16] * r[10] / s[10]) / c[16];
+        const R e = cexp(R(-0.05) * (V + R(30)));
+        r[12] = R(2.58079) * po * arxa * dv(e, one + e) * Qr - s[12] * (dv(one, c[16]) - dv(r[10], s[10]));
     }
     {
-        const R e = exp(R(-0.3576) * (V + R(30)));
-        const R gsr = R(26841.8) * e / (R(1) + e);
-        r[7] = po * Qr * arxa * gsr + po * R(9000) * arxa - (s[7] - s[8]) / R(0.5);
+        const R e = cexp(R(-0.3576) * (V + R(30)));
+        r[7] = po * arxa * (Qr * R(26841.8) * dv(e, one + e) + R(9000)) - R(2) * (s[7] - s[8]);
     }
-    // I_Na
+    // I_Na; a = e / (1 + e) switches the h and j rates at -40 mV (over 4 mV):
+    // each side's terms only where the other's weight does not leave them
+    // under the type's last digit
     R xina;
     {
-        const R ena = inv_frt * log(c[0] / s[19]);
+        const R x = V + R(47.13);
         R am = R(3.2);
-        if (fabs(V + R(47.13)) > R(0.001)) am = R(0.32) * (V + R(47.13)) / (R(1) - exp(R(-0.1) * (V + R(47.13))));
-        const R bm = R(0.08) * exp(-V / R(11));
-        const R a = R(1) - R(1) / (R(1) + exp(-(V + R(40)) / R(0.24)));
-        const R ah = a * R(0.135) * exp((R(80) + V) / R(-6.8));
-        const R bh = (R(1) - a) / (R(0.13) * (R(1) + exp((V + R(10.66)) / R(-11.1))))
-                   + a * (R(3.56) * exp(R(0.079) * V) + R(3.1e5) * exp(R(0.35) * V));
-        const R aj = a * (R(-1.2714e5) * exp(R(0.2444) * V) - R(3.474e-5) * exp(R(-0.04391) * V)) * (V + R(37.78))
-                   / (R(1) + exp(R(0.311) * (V + R(79.23))));
-        const R bj = (R(1) - a) * (R(0.3) * exp(R(-2.535e-7) * V) / (R(1) + exp(R(-0.1) * (V + R(32)))))
-                   + a * (R(0.1212) * exp(R(-0.01052) * V) / (R(1) + exp(R(-0.1378) * (V + R(40.14)))));
-        const R tauh = R(1) / (ah + bh);
-        const R tauj = c[34] * (R(1) / (aj + bj));
-        const R taum = R(1) / (am + bm);
-        const R gm = (s[1] + c[31]) / (R(1) + c[31]);
-        xina = c[15] * ((s[2] + c[32]) / (R(1) + c[32])) * ((s[3] + c[33]) / (R(1) + c[33])) * (gm * gm * gm) * (V - ena);
-        r[2] = (ah * tauh - (ah * tauh - s[2]) * exp(-h / tauh) - s[2]) / h;
-        r[3] = (aj * tauj - (aj * tauj - s[3]) * exp(-h / tauj) - s[3]) / h;
-        r[1] = (am * taum - (am * taum - s[1]) * exp(-h / taum) - s[1]) / h;
+        if (fabs(x) > R(0.001)) am = dv(R(-0.32) * x, cexpm1(R(-0.1) * x));
+        const R bm = R(0.08) * cexp(over(-V, 11));
+        const R u = over(V + R(40), 0.24), reach = sizeof(R) == 4 ? R(23) : R(46);
+        R ah = R(0), bh = R(0), aj = R(0), bj = R(0);
+        const R eu = exp(-fmin(fmax(u, -reach), reach));
+        const R al = dv(eu, one + eu), ar = dv(one, one + eu);       // a and 1 - a
+        if (u < reach) {
+            ah = al * R(0.135) * cexp(over(R(80) + V, -6.8));
+            bh = al * (R(3.56) * cexp(R(0.079) * V) + R(3.1e5) * cexp(R(0.35) * V));
+            aj = al * dv((R(-1.2714e5) * cexp(R(0.2444) * V) - R(3.474e-5) * cexp(R(-0.04391) * V)) * (V + R(37.78)),
+                         one + cexp(R(0.311) * (V + R(79.23))));
+            bj = al * dv(R(0.1212) * cexp(R(-0.01052) * V), one + cexp(R(-0.1378) * (V + R(40.14))));
+        }
+        if (u > -reach) {
+            bh += ar * dv(one, R(0.13) + R(0.13) * cexp(over(V + R(10.66), -11.1)));
+            bj += ar * dv(R(0.3) * exp(R(-2.535e-7) * V), one + cexp(R(-0.1) * (V + R(32))));
+        }
+        const R gm = dv(s[1] + c[31], one + c[31]);
+        const R gh = dv(s[2] + c[32], one + c[32]), gj = dv(s[3] + c[33], one + c[33]);
+        xina = c[15] * gh * gj * (gm * gm * gm) * (V - rtf * log(dv(c[0], s[19])));
+        r[2] = relax(dv(ah, ah + bh), s[2], h * (ah + bh));
+        const R ij = dv(one, aj + bj);
+        r[3] = relax(aj * (c[34] * ij), s[3], dv(h * (aj + bj), c[34]));
+        r[1] = relax(dv(am, am + bm), s[1], h * (am + bm));
     }
     // I_Kr
     R xikr;
     {
-        const R gss = sqrt(c[2] / R(5.4));
-        R v1 = R(0.00138) / R(0.123);
-        if (fabs(V + R(7)) > R(0.001)) v1 = R(0.00138) * (V + R(7)) / (R(1) - exp(R(-0.123) * (V + R(7))));
-        R v2 = R(0.00061) / R(0.145);
-        if (fabs(V + R(10)) > R(0.001)) v2 = R(0.00061) * (V + R(10)) / (exp(R(0.145) * (V + R(10))) - R(1));
-        const R taukr = R(1) / (v1 + v2);
-        const R xkrinf = R(1) / (R(1) + exp(-(V + R(50)) / R(7.5)));
-        const R rg = R(1) / (R(1) + exp((V + R(33)) / R(22.4)));
-        xikr = c[9] * gss * s[4] * rg * (V - ek);
-        r[4] = (xkrinf - (xkrinf - s[4]) * exp(-h / taukr) - s[4]) / h;
+        const R x = V + R(7), y = V + R(10);
+        R v1 = R(0.00138 / 0.123);
+        if (fabs(x) > R(0.001)) v1 = dv(R(-0.00138) * x, cexpm1(R(-0.123) * x));
+        R v2 = R(0.00061 / 0.145);
+        if (fabs(y) > R(0.001)) v2 = dv(R(0.00061) * y, cexpm1(R(0.145) * y));
+        xikr = dv(c[9] * sqrt(over(c[2], 5.4)) * s[4] * vk, one + cexp(over(V + R(33), 22.4)));
+        r[4] = relax(dv(one, one + cexp(over(V + R(50), -7.5))), s[4], h * (v1 + v2));
     }
     // I_Ks
     R xiks;
     {
-        const R eks = inv_frt * log((c[2] + R(0.018330) * c[0]) / (c[1] + R(0.018330) * s[19]));
-        const R xs1ss = R(1) / (R(1) + exp(-(V - R(1.5)) / R(16.7)));
-        R tauxs1;
-        if (fabs(V + R(30)) < R(0.001) / R(0.0687))
-            tauxs1 = R(1) / (R(0.0000719) / R(0.148) + R(0.000131) / R(0.0687));
-        else
-            tauxs1 = R(1) / (R(0.0000719) * (V + R(30)) / (R(1) - exp(R(-0.148) * (V + R(30))))
-                             + R(0.000131) * (V + R(30)) / (exp(R(0.0687) * (V + R(30))) - R(1)));
-        const R tauxs2 = R(4) * tauxs1;
-        const R q = R(0.5) / s[9];
-        const R gksx = R(1) + R(0.8) / (R(1) + q * q * q);
-        xiks = c[10] * gksx * s[5] * s[6] * (V - eks);
-        r[5] = (xs1ss - (xs1ss - s[5]) * exp(-h / tauxs1) - s[5]) / h;
-        r[6] = (xs1ss - (xs1ss - s[6]) * exp(-h / tauxs2) - s[6]) / h;
+        const R eks = rtf * log(dv(c[2] + R(0.018330) * c[0], c[1] + R(0.018330) * s[19]));
+        const R x = V + R(30);
+        const R xs1ss = dv(one, one + cexp(over(V - R(1.5), -16.7)));
+        R k = R(0.0000719 / 0.148 + 0.000131 / 0.0687);
+        if (fabs(x) >= R(0.001 / 0.0687))
+            k = dv(R(-0.0000719) * x, cexpm1(R(-0.148) * x)) + dv(R(0.000131) * x, cexpm1(R(0.0687) * x));
+        const R c3 = s[9] * s[9] * s[9];
+        xiks = c[10] * (one + dv(R(0.8) * c3, c3 + R(0.125))) * s[5] * s[6] * (V - eks);
+        r[5] = relax(xs1ss, s[5], h * k);
+        r[6] = relax(xs1ss, s[6], R(0.25) * (h * k));
     }
     const R wca = R(8.0313);
-    r[19] = -(R(1) / wca / R(1000)) * (xina + R(3) * xinak + R(3) * wca * jnaca);
+    r[19] = -over(xina + R(3) * xinak + R(3) * wca * jnaca, 8.0313 * 1000.0);
     r[0] = -(xina + xik1 + xikr + xiks + xito + wca * jnaca + R(2) * wca * jca + xinak) + istim;
 }
 
@@ -222,7 +227,7 @@ EP_HD R mh_compute_ion(R s[26], R V, R istim_pApF, R dt, const R *__restrict__ c
         for (int k = 0; k < 10; k++) {
             mh_rhs(s, c, h, istim_pApF, r);
 #pragma unroll
-            for (int j = 0; j < 26; j++) s[j] += r[j] * dt / R(10);
+            for (int j = 0; j < 26; j++) s[j] += r[j] * h;
         }
         substepped = 1;
     } else {

@@ -22,7 +22,7 @@
 #include <cuda_bf16.h>
 
 #include "surrogate.cuh"
-#include "tt.cuh"
+#include "tt_step.cuh"
 
 namespace ep {
 
@@ -601,7 +601,7 @@ __global__ void __launch_bounds__(128, 4) k_hybrid(const SurrogateArgs a) {
         double tsub = t0;
         for (int k = 0; k < ns; k++) {
             const float h = aux->hyb_sub > 0 ? hu : a.sub_dt[k];
-            tt_gate_step(s, V, h, c);
+            tts::tt_gate_step(s, V, h, c);
             tsum += h;
             const float w = fminf(tsum * rdt, 1.f);
 #pragma unroll
@@ -609,7 +609,7 @@ __global__ void __launch_bounds__(128, 4) k_hybrid(const SurrogateArgs a) {
                 const int q = cslot[j];
                 s[q] = ((lm >> (q + 1)) & 1u) ? c0[j] * __powf(c1[j] / c0[j], w) : c0[j] + w * (c1[j] - c0[j]);
             }
-            const float v1 = V + h * tt_dvdt<float>(V, s, c, 0.f, gks_i);
+            const float v1 = V + h * tts::tt_dvdt<float>(V, s, c, 0.f, gks_i);
             if (trk && tr.t_rep < 0.f) track_interval(tr, dirty, V, v1, tsub, h, a.act_thr);
             V = v1;
             tsub += (double)h;
