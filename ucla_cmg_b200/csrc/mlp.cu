@@ -1,12 +1,14 @@
 // mlp.cu -- trainer for the learned ionic step: a tanh MLP with FP32 master
 // weights, trained on the GPU by the kernels in this file (tiled SGEMM for
-// the forward and backward products, fused bias/tanh epilogues, loss and
-// Adam kernels).  Inference in the time loop uses the BF16 tensor-core
+// the forward and backward products, with the bias, tanh, tanh gradient and
+// loss in their epilogues and the weight gradients split over the batch, and
+// Adam).  Inference in the time loop uses the BF16 tensor-core
 // kernel in surrogate.cu; these kernels are for training only.
 #include <cstring>
 #include <vector>
 #include <random>
 #include <cmath>
+#include <algorithm>
 
 #include "kernels.cuh"
 
@@ -14,97 +16,126 @@ namespace ep {
 
 constexpr int GT = 64, GK = 16;   // 64x64 output tile, 16-deep k slices, 4x4 per thread
 
-// C = op(A) op(B) (+ beta C) (+ bias) (tanh); A: M x K (TA: K x M), B: K x N (TB: N x K)
+// what the product's epilogue does
+enum { E_BIAS = 0, E_TANH = 1, E_DTANH = 2, E_MSE = 3, E_PART = 4 };
+
+// Arguments beyond the operands, by epilogue:
+//   E_BIAS, E_TANH  bias[n]
+//   E_DTANH         h: the layer's activations, C = (A B) (1 - h^2)
+//   E_MSE           bias[n]; C = 2 w (P - Y) / rows, loss += sum w (P - Y)^2 / rows
+//   E_PART          C += z * cz: this k chunk's partial product; bsum (+ z * cz):
+//                   the column sums of A over the chunk
+struct GemmEpi {
+    const float *bias, *h, *Y, *w;
+    double *loss;
+    float *bsum;
+    long long cz;
+    int kchunk;
+};
+
+// C = op(A) op(B); A: M x K (TA: K x M), B: K x N (TB: N x K).  The next k
+// slice is loaded into registers while the current one is multiplied; the
+// products of a network step are small (K 23 .. 128 for the activations), so
+// a slice's load latency, not the multiply rate, is what a CTA would wait on.
 template <bool TA, bool TB, int EPI>
 __global__ void __launch_bounds__(256) k_sgemm(int M, int N, int K, const float *__restrict__ A, int lda,
-                                               const float *__restrict__ B, int ldb, float *C, int ldc,
-                                               const float *__restrict__ bias, float beta) {
-    __shared__ float As[GK][GT + 4];
-    __shared__ float Bs[GK][GT + 4];
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+                                               const float *__restrict__ B, int ldb, float *C, int ldc, GemmEpi ep) {
+    __shared__ __align__(16) float As[2][GK][GT + 4];
+    __shared__ __align__(16) float Bs[2][GK][GT + 4];
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     const int m0 = blockIdx.y * GT, n0 = blockIdx.x * GT;
-    float acc[4][4] = {{0.f}};
-    for (int k0 = 0; k0 < K; k0 += GK) {
-        for (int e = threadIdx.x; e < GT * GK; e += 256) {
-            const int mm = e / GK, kk = e % GK;     // A tile element (m, k)
-            const int gm = m0 + mm, gk = k0 + kk;
-            float v = 0.f;
-            if (gm < M && gk < K) v = TA ? A[(size_t)gk * lda + gm] : A[(size_t)gm * lda + gk];
-            As[kk][mm] = v;
-            const int nn = e / GK, kb = e % GK;     // B tile element (k, n)
-            const int gn = n0 + nn, gkb = k0 + kb;
-            float w = 0.f;
-            if (gn < N && gkb < K) w = TB ? B[(size_t)gn * ldb + gkb] : B[(size_t)gkb * ldb + gn];
-            Bs[kb][nn] = w;
+    int k0 = 0, k1 = K;
+    if (EPI == E_PART) {
+        k0 = (int)blockIdx.z * ep.kchunk;
+        k1 = min(K, k0 + ep.kchunk);
+        C += (long long)blockIdx.z * ep.cz;
+    }
+    // a thread's four elements of a slice of either operand, neighbouring
+    // threads along the operand's rows
+    const int ka = TA ? tid >> 6 : tid & 15, ma = TA ? tid & 63 : tid >> 4;
+    const int kb = TB ? tid & 15 : tid >> 6, nb = TB ? tid >> 4 : tid & 63;
+    float ra[4], rb[4];
+    auto load = [&](int k) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int gk = k + ka + (TA ? 4 * i : 0), gm = m0 + ma + (TA ? 0 : 16 * i);
+            ra[i] = gm < M && gk < k1 ? __ldg(A + (TA ? (size_t)gk * lda + gm : (size_t)gm * lda + gk)) : 0.f;
+            const int hk = k + kb + (TB ? 0 : 4 * i), gn = n0 + nb + (TB ? 16 * i : 0);
+            rb[i] = gn < N && hk < k1 ? __ldg(B + (TB ? (size_t)gn * ldb + hk : (size_t)hk * ldb + gn)) : 0.f;
         }
-        __syncthreads();
+    };
+    auto put = [&](int buf) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            As[buf][ka + (TA ? 4 * i : 0)][ma + (TA ? 0 : 16 * i)] = ra[i];
+            Bs[buf][kb + (TB ? 0 : 4 * i)][nb + (TB ? 16 * i : 0)] = rb[i];
+        }
+    };
+    float acc[4][4] = {{0.f}}, col[4] = {0.f, 0.f, 0.f, 0.f};
+    load(k0);
+    int buf = 0;
+    for (int k = k0; k < k1; k += GK, buf ^= 1) {
+        put(buf);
+        __syncthreads();                      // the slice before last is no longer read
+        if (k + GK < k1) load(k + GK);
 #pragma unroll
         for (int kk = 0; kk < GK; kk++) {
-            float a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) a[i] = As[kk][ty * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; j++) b[j] = Bs[kk][tx * 4 + j];
+            const float4 a4 = *reinterpret_cast<const float4 *>(&As[buf][kk][ty * 4]);
+            const float4 b4 = *reinterpret_cast<const float4 *>(&Bs[buf][kk][tx * 4]);
+            const float a[4] = {a4.x, a4.y, a4.z, a4.w}, b[4] = {b4.x, b4.y, b4.z, b4.w};
 #pragma unroll
             for (int i = 0; i < 4; i++)
 #pragma unroll
                 for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+            if (EPI == E_PART && blockIdx.x == 0)
+#pragma unroll
+                for (int i = 0; i < 4; i++) col[i] += a[i];
         }
-        __syncthreads();
     }
+    double l = 0.0;
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         const int gm = m0 + ty * 4 + i;
         if (gm >= M) continue;
+        if (EPI == E_PART && blockIdx.x == 0 && tx == 0) ep.bsum[(long long)blockIdx.z * ep.cz + gm] = col[i];
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             const int gn = n0 + tx * 4 + j;
             if (gn >= N) continue;
+            const size_t at = (size_t)gm * ldc + gn;
             float v = acc[i][j];
-            if (beta != 0.f) v += beta * C[(size_t)gm * ldc + gn];
-            if (EPI >= 1) v += bias[gn];
-            if (EPI == 2) v = tanhf(v);
-            C[(size_t)gm * ldc + gn] = v;
+            if (EPI == E_BIAS || EPI == E_TANH || EPI == E_MSE) v += ep.bias[gn];
+            if (EPI == E_TANH) v = tanhf(v);
+            if (EPI == E_DTANH) { const float h = ep.h[at]; v *= 1.f - h * h; }
+            if (EPI == E_MSE) {
+                const float d = v - ep.Y[at], wj = ep.w ? ep.w[gn] : 1.f;
+                v = 2.f * wj * d / (float)M;
+                l += (double)wj * (double)d * (double)d / (double)M;
+            }
+            C[at] = v;
         }
+    }
+    if (EPI == E_MSE) {
+        for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+        if ((tid & 31) == 0 && l != 0.0) atomicAdd(ep.loss, l);
     }
 }
 
 template <bool TA, bool TB, int EPI>
 static void sgemm(int M, int N, int K, const float *A, int lda, const float *B, int ldb, float *C, int ldc,
-                  const float *bias, float beta, cudaStream_t s) {
-    dim3 grid((N + GT - 1) / GT, (M + GT - 1) / GT);
-    k_sgemm<TA, TB, EPI><<<grid, 256, 0, s>>>(M, N, K, A, lda, B, ldb, C, ldc, bias, beta);
+                  const GemmEpi &ep, cudaStream_t s) {
+    dim3 grid((N + GT - 1) / GT, (M + GT - 1) / GT, EPI == E_PART ? (K + ep.kchunk - 1) / ep.kchunk : 1);
+    k_sgemm<TA, TB, EPI><<<grid, 256, 0, s>>>(M, N, K, A, lda, B, ldb, C, ldc, ep);
 }
 
-// delta <- delta * (1 - h^2)
-__global__ void k_tanh_back(int n, float *d, const float *h) {
+// the weight gradients' partial products summed over the chunks, in order
+__global__ void k_sum_parts(int n, int parts, const float *__restrict__ p, float *out) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) d[i] *= (1.f - h[i] * h[i]);
-}
-
-// column sums: out[j] (+)= sum_i D[i, j]
-__global__ void k_colsum(int rows, int cols, const float *D, float *out) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= cols) return;
+    if (i >= n) return;
     float s = 0.f;
-    for (int i = 0; i < rows; i++) s += D[(size_t)i * cols + j];
-    out[j] = s;
-}
-
-// delta = 2 w (P - Y) / batch ; loss += sum w (P - Y)^2 / batch
-__global__ void k_mse(int rows, int cols, const float *P, const float *Y, const float *w, float *delta,
-                      double *loss) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double l = 0.0;
-    if (i < rows * cols) {
-        const int j = i % cols;
-        const float d = P[i] - Y[i];
-        const float wj = w ? w[j] : 1.f;
-        delta[i] = 2.f * wj * d / (float)rows;
-        l = (double)wj * (double)d * (double)d / (double)rows;
-    }
-    for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-    if ((threadIdx.x & 31) == 0 && l != 0.0) atomicAdd(loss, l);
+#pragma unroll 8
+    for (int z = 0; z < parts; z++) s += __ldg(p + (size_t)z * n + i);
+    out[i] = s;
 }
 
 __global__ void k_adam(int n, float *p, const float *g, float *m, float *v, float lr, float b1, float b2,
@@ -130,28 +161,42 @@ struct ep_mlp {
     std::vector<size_t> woff, boff;  // offsets into the flat parameter vector
     size_t np = 0;
     float *p = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;
-    float *act = nullptr;            // activations of the largest batch (layers 1..L)
+    float *act = nullptr;            // activations of the largest batch (layers 1..L); the workspace's start
     float *dlt = nullptr, *dlt2 = nullptr;
     float *w_out = nullptr;
+    float *part = nullptr;           // the gradients of each chunk of a batch's rows
     double *loss = nullptr;
     int cap = 0;                     // batch capacity of act/dlt
     long long t = 0;                 // Adam step
     int maxw = 0;
 };
 
+// Chunks that a batch's rows are cut into for the weight gradients, whose
+// products are small (128 x 128) and deep (the batch): with one CTA per 64 x 64
+// tile four CTAs walked all 8192 rows.  At least 32 rows a chunk, at most 64
+// chunks, and 16M floats of partial gradients.
+static int grad_parts(const ep_mlp *m, int B) {
+    const long long most = std::max<long long>(1, (16ll << 20) / (long long)m->np);
+    return (int)std::min<long long>(std::min<long long>(64, most), (B + 31) / 32);
+}
+
+// one allocation for the activations, the two deltas and the partial gradients
 static int mlp_reserve(ep_mlp *m, int batch) {
     if (batch <= m->cap) return EP_OK;
     size_t tot = 0;
     for (int l = 1; l <= m->L; l++) tot += (size_t)m->dims[l];
-    cudaFree(m->act); cudaFree(m->dlt); cudaFree(m->dlt2);
-    m->act = m->dlt = m->dlt2 = nullptr;
-    if (cudaMalloc(&m->act, sizeof(float) * tot * batch) != cudaSuccess ||
-        cudaMalloc(&m->dlt, sizeof(float) * (size_t)m->maxw * batch) != cudaSuccess ||
-        cudaMalloc(&m->dlt2, sizeof(float) * (size_t)m->maxw * batch) != cudaSuccess) {
+    const size_t act = tot * batch, dlt = (size_t)m->maxw * batch, part = m->np * (size_t)grad_parts(m, batch);
+    cudaFree(m->act);
+    m->act = m->dlt = m->dlt2 = m->part = nullptr;
+    m->cap = 0;
+    if (cudaMalloc(&m->act, sizeof(float) * (act + 2 * dlt + part)) != cudaSuccess) {
         cudaGetLastError();
         set_error("MLP workspace allocation failed (batch %d)", batch);
         return EP_ERR_NOMEM;
     }
+    m->dlt = m->act + act;
+    m->dlt2 = m->dlt + dlt;
+    m->part = m->dlt2 + dlt;
     m->cap = batch;
     return EP_OK;
 }
@@ -163,18 +208,19 @@ static float *act_of(ep_mlp *m, int l) {
     return m->act + off;
 }
 
-static void forward(ep_mlp *m, const float *X, int B, cudaStream_t s) {
+// hidden layers 1 .. L-1
+static void forward_hidden(ep_mlp *m, const float *X, int B, cudaStream_t s) {
     const float *h = X;
-    for (int l = 1; l <= m->L; l++) {
+    for (int l = 1; l < m->L; l++) {
         float *z = act_of(m, l);
-        const float *W = m->p + m->woff[l - 1], *b = m->p + m->boff[l - 1];
-        if (l < m->L) sgemm<false, true, 2>(B, m->dims[l], m->dims[l - 1], h, m->dims[l - 1], W, m->dims[l - 1], z,
-                                             m->dims[l], b, 0.f, s);
-        else sgemm<false, true, 1>(B, m->dims[l], m->dims[l - 1], h, m->dims[l - 1], W, m->dims[l - 1], z,
-                                    m->dims[l], b, 0.f, s);
+        GemmEpi ep{};
+        ep.bias = m->p + m->boff[l - 1];
+        sgemm<false, true, E_TANH>(B, m->dims[l], m->dims[l - 1], h, m->dims[l - 1], m->p + m->woff[l - 1],
+                                   m->dims[l - 1], z, m->dims[l], ep, s);
         h = z;
     }
 }
+static const float *last_hidden(ep_mlp *m, const float *X) { return m->L > 1 ? act_of(m, m->L - 1) : X; }
 
 extern "C" {
 
@@ -223,7 +269,7 @@ int ep_mlp_create(int32_t n_layers, const int32_t *dims, uint64_t seed, int devi
 void ep_mlp_destroy(ep_mlp *m) {
     if (!m) return;
     cudaFree(m->p); cudaFree(m->g); cudaFree(m->m); cudaFree(m->v);
-    cudaFree(m->act); cudaFree(m->dlt); cudaFree(m->dlt2); cudaFree(m->w_out); cudaFree(m->loss);
+    cudaFree(m->act); cudaFree(m->w_out); cudaFree(m->loss);
     delete m;
 }
 
@@ -249,9 +295,14 @@ int ep_mlp_forward(ep_mlp *m, const float *X, float *Y, int32_t B, void *stream)
     int rc = mlp_reserve(m, B);
     if (rc) return rc;
     cudaStream_t s = (cudaStream_t)stream;
-    forward(m, X, B, s);
-    EP_CUDA(cudaMemcpyAsync(Y, act_of(m, m->L), sizeof(float) * (size_t)B * m->dims[m->L],
-                            cudaMemcpyDeviceToDevice, s));
+    forward_hidden(m, X, B, s);
+    const int L = m->L, nin = m->dims[L - 1], nout = m->dims[L];
+    GemmEpi ep{};
+    ep.bias = m->p + m->boff[L - 1];
+    // a single layer goes through the workspace: Y may be X
+    float *out = L > 1 ? Y : act_of(m, 1);
+    sgemm<false, true, E_BIAS>(B, nout, nin, last_hidden(m, X), nin, m->p + m->woff[L - 1], nin, out, nout, ep, s);
+    if (L == 1) EP_CUDA(cudaMemcpyAsync(Y, out, sizeof(float) * (size_t)B * nout, cudaMemcpyDeviceToDevice, s));
     EP_CUDA(cudaGetLastError());
     return EP_OK;
 }
@@ -264,25 +315,39 @@ int ep_mlp_loss_grad(ep_mlp *m, const float *X, const float *Y, const float *w_o
     cudaStream_t s = (cudaStream_t)stream;
     const int L = m->L, dout = m->dims[L];
     if (w_out_host) EP_CUDA(cudaMemcpyAsync(m->w_out, w_out_host, sizeof(float) * dout, cudaMemcpyHostToDevice, s));
-    forward(m, X, B, s);
+    const int parts = grad_parts(m, B);
+    forward_hidden(m, X, B, s);
     EP_CUDA(cudaMemsetAsync(m->loss, 0, sizeof(double), s));
-    const int ne = B * dout;
-    k_mse<<<(ne + 255) / 256, 256, 0, s>>>(B, dout, act_of(m, L), Y, w_out_host ? m->w_out : nullptr, m->dlt,
-                                           m->loss);
     float *d = m->dlt, *d2 = m->dlt2;
+    {
+        // the output layer with the loss and its gradient
+        GemmEpi ep{};
+        ep.bias = m->p + m->boff[L - 1];
+        ep.Y = Y;
+        ep.w = w_out_host ? m->w_out : nullptr;
+        ep.loss = m->loss;
+        const int nin = m->dims[L - 1];
+        sgemm<false, true, E_MSE>(B, dout, nin, last_hidden(m, X), nin, m->p + m->woff[L - 1], nin, d, dout, ep, s);
+    }
     for (int l = L; l >= 1; l--) {
         const float *hprev = l > 1 ? act_of(m, l - 1) : X;
         const int nout = m->dims[l], nin = m->dims[l - 1];
-        // dW_l = delta^T hprev  (nout x nin), db_l = colsum(delta)
-        sgemm<true, false, 0>(nout, nin, B, d, nout, hprev, nin, m->g + m->woff[l - 1], nin, nullptr, 0.f, s);
-        k_colsum<<<(nout + 127) / 128, 128, 0, s>>>(B, nout, d, m->g + m->boff[l - 1]);
+        // dW_l = delta^T hprev  (nout x nin), db_l = colsum(delta), a part per chunk of rows
+        GemmEpi ep{};
+        ep.bsum = m->part + m->boff[l - 1];
+        ep.cz = (long long)m->np;
+        ep.kchunk = (B + parts - 1) / parts;
+        sgemm<true, false, E_PART>(nout, nin, B, d, nout, hprev, nin, m->part + m->woff[l - 1], nin, ep, s);
         if (l > 1) {
             // delta_{l-1} = (delta W_l) * (1 - h_{l-1}^2)
-            sgemm<false, false, 0>(B, nin, nout, d, nout, m->p + m->woff[l - 1], nin, d2, nin, nullptr, 0.f, s);
-            k_tanh_back<<<(B * nin + 255) / 256, 256, 0, s>>>(B * nin, d2, act_of(m, l - 1));
+            GemmEpi eb{};
+            eb.h = hprev;
+            sgemm<false, false, E_DTANH>(B, nin, nout, d, nout, m->p + m->woff[l - 1], nin, d2, nin, eb, s);
             std::swap(d, d2);
         }
     }
+    const int used = (B + (B + parts - 1) / parts - 1) / ((B + parts - 1) / parts);    // chunks that have rows
+    k_sum_parts<<<(int)((m->np + 255) / 256), 256, 0, s>>>((int)m->np, used, m->part, m->g);
     EP_CUDA(cudaGetLastError());
     if (loss) {
         EP_CUDA(cudaMemcpyAsync(loss, m->loss, sizeof(double), cudaMemcpyDeviceToHost, s));
