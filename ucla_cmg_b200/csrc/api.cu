@@ -680,7 +680,7 @@ static int step_typed(ep_handle *h, int nsteps, size_t &ne) {
         h->step++;
         if (h->ecg_every && h->ne > 0 && h->step % h->ecg_every == 0) {
             if ((rc = mark(h, ne, K_ECG))) return rc;
-            rc = launch_ecg<R>(h->n, h->ne, h->W.as<R>(), h->pitch, h->V.as<R>(), h->ecg_partial.as<double>(),
+            rc = launch_ecg<R>(h->n, h->ne, h->W.as<R>(), h->pitch, h->V.as<R>(), 1, h->ecg_partial.as<double>(),
                                h->ecg_counter.as<unsigned int>(), h->ecg_buf.as<double>(), h->ecg_grid, h->stream,
                                h->ecg_slot.as<unsigned int>(), h->ecg_cap);
             if (rc) return rc;
@@ -1390,10 +1390,7 @@ int ep_set_electrodes(ep_handle *h, int32_t ne, const double *xyz, const double 
     int rc = h->precision == EP_FP64 ? upload<double>(h->W, Wp) : upload<float>(h->W, Wp);
     if (rc) return rc;
     h->ne = ne;
-    int dev = 0, nsm = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    h->ecg_grid = std::max(1, std::min(nsm * 4, div_up(h->n, 256)));
+    h->ecg_grid = ecg_chunks(h->n, ne, 1);
     if ((rc = h->ecg_partial.alloc(sizeof(double) * 16 * (size_t)h->ecg_grid))) return rc;
     if ((rc = h->ecg_counter.alloc(sizeof(unsigned int)))) return rc;
     EP_CUDA(cudaMemset(h->ecg_counter.p, 0, sizeof(unsigned int)));
@@ -1974,11 +1971,11 @@ int ep_compute_ecg(ep_handle *h, double *out) {
     int rc = tmp.alloc(sizeof(double) * h->ne);
     if (rc) return rc;
     if (h->precision == EP_FP64)
-        rc = launch_ecg<double>(h->n, h->ne, h->W.as<double>(), h->pitch, h->V.as<double>(),
+        rc = launch_ecg<double>(h->n, h->ne, h->W.as<double>(), h->pitch, h->V.as<double>(), 1,
                                 h->ecg_partial.as<double>(), h->ecg_counter.as<unsigned int>(),
                                 tmp.as<double>(), h->ecg_grid, h->stream);
     else
-        rc = launch_ecg<float>(h->n, h->ne, h->W.as<float>(), h->pitch, h->V.as<float>(),
+        rc = launch_ecg<float>(h->n, h->ne, h->W.as<float>(), h->pitch, h->V.as<float>(), 1,
                                h->ecg_partial.as<double>(), h->ecg_counter.as<unsigned int>(),
                                tmp.as<double>(), h->ecg_grid, h->stream);
     if (rc) return rc;
@@ -1989,7 +1986,7 @@ int ep_compute_ecg(ep_handle *h, double *out) {
 
 // ---- offline pseudo-ECG (ComputeECG) ----
 struct ep_ecg {
-    int device = 0, n = 0, ne = 0, grid = 1;
+    int device = 0, n = 0, ne = 0;
     cudaStream_t stream = nullptr;
     DBuf W, V, out, partial, counter;
     int cap_frames = 0;
@@ -2027,12 +2024,6 @@ int ep_ecg_create(const ep_mesh_desc *mesh, const ep_cables_desc *cables, int32_
     e->ne = ne;
     if ((rc = e->W.alloc(sizeof(double) * Wh.size()))) return rc;
     EP_CUDA(cudaMemcpy(e->W.p, Wh.data(), sizeof(double) * Wh.size(), cudaMemcpyHostToDevice));
-    int nsm = 148;
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
-    e->grid = std::max(1, std::min(nsm * 4, div_up(n, 256)));
-    if ((rc = e->partial.alloc(sizeof(double) * 16 * (size_t)e->grid))) return rc;
-    if ((rc = e->counter.alloc(sizeof(unsigned int)))) return rc;
-    EP_CUDA(cudaMemset(e->counter.p, 0, sizeof(unsigned int)));
     *out = e.release();
     return EP_OK;
 }
@@ -2043,21 +2034,24 @@ int ep_ecg_eval(ep_ecg *e, int32_t n_frames, const double *V, double *out) {
     // frames go up in chunks of at most ~256 MB
     const int chunk = std::max(1, (int)std::min<long long>(n_frames, (256ll << 20) / (8ll * e->n)));
     int rc;
+    const int nodes = ecg_chunks(e->n, e->ne, chunk), groups = div_up(std::max(1, chunk), ecg_frames(e->ne));
     if (chunk > e->cap_frames) {
         if ((rc = e->V.alloc(sizeof(double) * (size_t)chunk * e->n))) return rc;
         if ((rc = e->out.alloc(sizeof(double) * (size_t)chunk * e->ne))) return rc;
+        if ((rc = e->counter.alloc(sizeof(unsigned int) * (size_t)groups))) return rc;
+        EP_CUDA(cudaMemsetAsync(e->counter.p, 0, e->counter.bytes, e->stream));
         e->cap_frames = chunk;
     }
+    if (e->partial.bytes < sizeof(double) * (size_t)chunk * e->ne * nodes &&
+        (rc = e->partial.alloc(sizeof(double) * (size_t)chunk * e->ne * nodes)))
+        return rc;
     for (int f0 = 0; f0 < n_frames; f0 += chunk) {
         const int nf = std::min(chunk, n_frames - f0);
         EP_CUDA(cudaMemcpyAsync(e->V.p, V + (size_t)f0 * e->n, sizeof(double) * (size_t)nf * e->n,
                                 cudaMemcpyHostToDevice, e->stream));
-        for (int f = 0; f < nf; f++) {
-            rc = launch_ecg<double>(e->n, e->ne, e->W.as<double>(), e->n, e->V.as<double>() + (size_t)f * e->n,
-                                    e->partial.as<double>(), e->counter.as<unsigned int>(),
-                                    e->out.as<double>() + (size_t)f * e->ne, e->grid, e->stream);
-            if (rc) return rc;
-        }
+        rc = launch_ecg<double>(e->n, e->ne, e->W.as<double>(), e->n, e->V.as<double>(), nf, e->partial.as<double>(),
+                                e->counter.as<unsigned int>(), e->out.as<double>(), nodes, e->stream);
+        if (rc) return rc;
         EP_CUDA(cudaMemcpyAsync(out + (size_t)f0 * e->ne, e->out.p, sizeof(double) * (size_t)nf * e->ne,
                                 cudaMemcpyDeviceToHost, e->stream));
         EP_CUDA(cudaStreamSynchronize(e->stream));

@@ -1444,73 +1444,110 @@ template int launch_explicit<double>(int, int, const int *, const int *, const d
                                       double *, double, cudaStream_t);
 
 // ---------------------------------------------------------------------------
-// pseudo-ECG: out[k] = sum_i W[k * wpitch + i] V[i], FP64 accumulation.
-// Block partials, then the last block to finish sums them in block order.
-template <typename R>
+// pseudo-ECG: out[f * ne + k] = sum_i W[k * wpitch + i] V[f * n + i] over
+// frames f, FP64 accumulation.  A CTA takes a chunk of nodes and FB frames, so
+// the weights are read once for FB frames (one launch a frame read them again
+// for each, and its 592 partials a lead were added by one thread in series).
+// Partials per chunk, added in order by the last CTA of the frame group.
+template <int NE> struct EcgFrames { static constexpr int N = NE <= 4 ? 8 : NE <= 8 ? 4 : 2; };
+
+template <typename R, int NE>
 __global__ void __launch_bounds__(256) k_ecg(int n, int ne, const R *__restrict__ W, int wpitch,
-                                             const R *__restrict__ V, double *partial,
+                                             const R *__restrict__ V, int frames, double *partial,
                                              unsigned int *counter, double *out, unsigned int *slot, int cap) {
-    constexpr int MAXE = 16;
-    double acc[MAXE];
+    constexpr int FB = EcgFrames<NE>::N;
+    const int f0 = blockIdx.y * FB, nf = min(FB, frames - f0);
+    double acc[FB][NE];
 #pragma unroll
-    for (int k = 0; k < MAXE; k++) acc[k] = 0.0;
+    for (int f = 0; f < FB; f++)
+#pragma unroll
+        for (int k = 0; k < NE; k++) acc[f][k] = 0.0;
+    const R *Vf = V + (size_t)f0 * n;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const double v = (double)V[i];
+        double w[NE], v[FB];
 #pragma unroll
-        for (int k = 0; k < MAXE; k++)
-            if (k < ne) acc[k] += (double)__ldg(W + (size_t)k * wpitch + i) * v;
+        for (int k = 0; k < NE; k++) w[k] = k < ne ? (double)__ldg(W + (size_t)k * wpitch + i) : 0.0;
+#pragma unroll
+        for (int f = 0; f < FB; f++) v[f] = f < nf ? (double)__ldg(Vf + (size_t)f * n + i) : 0.0;
+#pragma unroll
+        for (int f = 0; f < FB; f++)
+#pragma unroll
+            for (int k = 0; k < NE; k++) acc[f][k] += w[k] * v[f];
     }
-    __shared__ double sh[MAXE][8];
+    __shared__ double sh[FB * NE][8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-    for (int k = 0; k < MAXE; k++) {
-        double t = acc[k];
-        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-        if (lane == 0) sh[k][warp] = t;
-    }
+    for (int f = 0; f < FB; f++)
+#pragma unroll
+        for (int k = 0; k < NE; k++) {
+            if (f >= nf || k >= ne) continue;
+            double t = acc[f][k];
+            for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+            if (lane == 0) sh[f * NE + k][warp] = t;
+        }
     __syncthreads();
-    __shared__ bool last;
-    if (threadIdx.x < ne) {
+    // partial of (frame, lead) j at part[j * chunks + chunk]
+    const int outs = nf * ne, chunks = gridDim.x;
+    double *part = partial + (size_t)f0 * ne * chunks;
+    if ((int)threadIdx.x < outs) {
+        const int f = threadIdx.x / ne, k = threadIdx.x % ne;
         double t = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += sh[threadIdx.x][w];
-        partial[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = t;
+        for (int w = 0; w < 8; w++) t += sh[f * NE + k][w];
+        part[(size_t)threadIdx.x * chunks + blockIdx.x] = t;
     }
     __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) last = (atomicAdd(counter, 1u) == gridDim.x - 1);
+    __shared__ bool last;
+    if (threadIdx.x == 0) last = (atomicAdd(counter + blockIdx.y, 1u) == gridDim.x - 1);
     __syncthreads();
     if (last) {
         __threadfence();
         // with a slot counter the sample goes to row *slot of out (the
         // counter lives on the device so that replayed graphs advance it)
         const unsigned int row = slot ? *(volatile unsigned int *)slot : 0u;
-        if (threadIdx.x < ne && (int)row < cap) {
-            double t = 0.0;
-            for (int b = 0; b < (int)gridDim.x; b++) t += __ldcg(partial + (size_t)threadIdx.x * gridDim.x + b);
-            out[(size_t)row * ne + threadIdx.x] = t;
-        }
+        if ((int)row < cap)
+            for (int j = warp; j < outs; j += 8) {
+                double t = 0.0;
+                for (int b = lane; b < chunks; b += 32) t += __ldcg(part + (size_t)j * chunks + b);
+                for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+                if (lane == 0) out[((size_t)row + f0) * ne + j] = t;
+            }
         __syncthreads();
         if (threadIdx.x == 0) {
-            *counter = 0;
+            counter[blockIdx.y] = 0;
             if (slot) *slot = row + 1u;
         }
     }
 }
 
+// CTAs over the nodes: four per SM over all frame groups, or 16 nodes a thread
+int ecg_chunks(int n, int ne, int frames) {
+    int dev = 0, nsm = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    const int groups = div_up(frames, ecg_frames(ne));
+    return std::max(1, std::min(div_up(n, 256), std::max(div_up(4 * nsm, groups), div_up(n, 16 * 256))));
+}
+int ecg_frames(int ne) { return ne <= 4 ? 8 : ne <= 8 ? 4 : 2; }
+
 template <typename R>
-int launch_ecg(int n, int ne, const R *W, int wpitch, const R *V, double *partial,
-               unsigned int *counter, double *out, int grid, cudaStream_t s, unsigned int *slot, int cap) {
-    if (ne <= 0) return EP_OK;
+int launch_ecg(int n, int ne, const R *W, int wpitch, const R *V, int frames, double *partial, unsigned int *counter,
+               double *out, int chunks, cudaStream_t s, unsigned int *slot, int cap) {
+    if (ne <= 0 || frames <= 0) return EP_OK;
     if (ne > 16) { set_error("at most 16 electrodes"); return EP_ERR_ARG; }
-    k_ecg<R><<<grid, 256, 0, s>>>(n, ne, W, wpitch, V, partial, counter, out, slot, slot ? cap : 1);
+    const dim3 grid(chunks, div_up(frames, ecg_frames(ne)));
+    const int c = slot ? cap : 1;
+    if (ne <= 4) k_ecg<R, 4><<<grid, 256, 0, s>>>(n, ne, W, wpitch, V, frames, partial, counter, out, slot, c);
+    else if (ne <= 8) k_ecg<R, 8><<<grid, 256, 0, s>>>(n, ne, W, wpitch, V, frames, partial, counter, out, slot, c);
+    else k_ecg<R, 16><<<grid, 256, 0, s>>>(n, ne, W, wpitch, V, frames, partial, counter, out, slot, c);
     EP_CUDA(cudaGetLastError());
     return EP_OK;
 }
 
-template int launch_ecg<float>(int, int, const float *, int, const float *, double *, unsigned int *,
-                               double *, int, cudaStream_t, unsigned int *, int);
-template int launch_ecg<double>(int, int, const double *, int, const double *, double *,
-                                unsigned int *, double *, int, cudaStream_t, unsigned int *, int);
+template int launch_ecg<float>(int, int, const float *, int, const float *, int, double *, unsigned int *, double *, int,
+                               cudaStream_t, unsigned int *, int);
+template int launch_ecg<double>(int, int, const double *, int, const double *, int, double *, unsigned int *, double *,
+                                int, cudaStream_t, unsigned int *, int);
 
 __global__ void k_step_inc(long long *step) { *step += 1; }
 void launch_step_inc(long long *step, cudaStream_t s) { k_step_inc<<<1, 1, 0, s>>>(step); }

@@ -173,12 +173,15 @@ int cg_grid_size(int block, int *grid, int per_sm = 0, int batch = 4, int varian
 template <typename R>
 int cg_max_per_sm(int block, int *per, int batch = 4, int variant = 0, int depth = 0);
 
-// ECG_k = sum_i W[k n + i] V[i] (ComputeECG.h:172-189 in per-node form),
-// deterministic two-level reduction, written to out[k].
+// ECG_k = sum_i W[k n + i] V[i] (ComputeECG.h:172-189 in per-node form) of
+// `frames` voltage fields, n apart, deterministic two-level reduction, written
+// to out[f * ne + k] (slot: to that row of out, one frame).  partial: frames *
+// ne * chunks values; counter: one per ecg_frames(ne) frames, zero before and after.
+int ecg_frames(int ne);
+int ecg_chunks(int n, int ne, int frames);
 template <typename R>
-int launch_ecg(int n, int ne, const R *W, int wpitch, const R *V, double *partial,
-               unsigned int *counter, double *out, int grid, cudaStream_t s,
-               unsigned int *slot = nullptr, int cap = 0);
+int launch_ecg(int n, int ne, const R *W, int wpitch, const R *V, int frames, double *partial, unsigned int *counter,
+               double *out, int chunks, cudaStream_t s, unsigned int *slot = nullptr, int cap = 0);
 
 void launch_step_inc(long long *step, cudaStream_t s);
 // explicit scheme: V <- V + h (D V) / C_L over the SELL operator D = -K
