@@ -47,6 +47,98 @@ struct DBuf {
     template <typename T> T *as() const { return (T *)p; }
 };
 
+// What the calls without a handle of their own (the plugin-level cells) and the
+// offline ECG's uploads work in: a stream, two events, one device block and one
+// pinned block per host thread, so that concurrent calls share nothing.  Kept
+// from call to call up to kKeep bytes each (a dozen cudaMalloc / cudaFree pairs
+// a call took most of its time), a larger block goes back when its call
+// returns, all of it when the thread ends.  Every call has waited for its work
+// when it returns, so nothing here is in use between calls.
+struct CallBuffers {
+    static constexpr size_t kKeep = 64u << 20;
+    int device = -1;
+    cudaStream_t stream = nullptr;
+    cudaEvent_t ev[2] = {};
+    void *dev = nullptr, *pin = nullptr;
+    size_t dev_bytes = 0, pin_bytes = 0;
+
+    // blocks of at least d (device) and p (pinned) bytes on the current device
+    int reserve(size_t d, size_t p) {
+        int cur = 0;
+        EP_CUDA(cudaGetDevice(&cur));
+        if (stream && cur != device) drop();
+        // a cudaDeviceReset since the last call took everything with it
+        cudaPointerAttributes at{};
+        if ((dev || pin) && (cudaPointerGetAttributes(&at, dev ? dev : pin) != cudaSuccess ||
+                             at.type != (dev ? cudaMemoryTypeDevice : cudaMemoryTypeHost))) {
+            cudaGetLastError();
+            forget();
+        }
+        device = cur;
+        if (!stream) {
+            EP_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+            for (cudaEvent_t &e : ev) EP_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        }
+        if (d > dev_bytes) {
+            if (dev) cudaFree(dev);
+            dev = nullptr;
+            dev_bytes = 0;
+            if (cudaMalloc(&dev, d) != cudaSuccess) {
+                cudaGetLastError();
+                set_error("cudaMalloc(%zu) failed", d);
+                return EP_ERR_NOMEM;
+            }
+            dev_bytes = d;
+        }
+        if (p > pin_bytes) {
+            if (pin) cudaFreeHost(pin);
+            pin = nullptr;
+            pin_bytes = 0;
+            if (cudaMallocHost(&pin, p) != cudaSuccess) {
+                cudaGetLastError();
+                set_error("cudaMallocHost(%zu) failed", p);
+                return EP_ERR_NOMEM;
+            }
+            pin_bytes = p;
+        }
+        return EP_OK;
+    }
+    void trim() {
+        if (dev_bytes > kKeep) { cudaFree(dev); dev = nullptr; dev_bytes = 0; }
+        if (pin_bytes > kKeep) { cudaFreeHost(pin); pin = nullptr; pin_bytes = 0; }
+    }
+    void forget() { stream = nullptr; ev[0] = ev[1] = nullptr; dev = pin = nullptr; dev_bytes = pin_bytes = 0; }
+    void drop() {
+        int cur = 0;
+        if (cudaGetDevice(&cur) == cudaSuccess) {
+            if (device >= 0) cudaSetDevice(device);
+            if (dev) cudaFree(dev);
+            if (pin) cudaFreeHost(pin);
+            for (cudaEvent_t e : ev)
+                if (e) cudaEventDestroy(e);
+            if (stream) cudaStreamDestroy(stream);
+            cudaSetDevice(cur);
+        }
+        cudaGetLastError();
+        forget();
+    }
+    ~CallBuffers() { if (device >= 0) drop(); }
+};
+static thread_local CallBuffers t_buf;
+
+// host memory to host memory by the threads that convert transfers, from 256
+// KB up (one thread copies at a third of the copy engine's rate)
+static void host_copy(void *dst, const void *src, size_t bytes) {
+    constexpr size_t piece = 64u << 10;
+    if (bytes < 4 * piece) { std::memcpy(dst, src, bytes); return; }
+    const long long n = (long long)((bytes + piece - 1) / piece);
+#pragma omp parallel for schedule(static)
+    for (long long k = 0; k < n; k++) {
+        const size_t at = (size_t)k * piece;
+        std::memcpy((char *)dst + at, (const char *)src + at, std::min(piece, bytes - at));
+    }
+}
+
 }  // namespace ep
 
 using namespace ep;
@@ -84,7 +176,7 @@ struct ep_handle {
     DBuf ex_tmp;                         // explicit scheme: scratch vector
     DBuf pd0, pd1;                       // CG predictor: x - V of the first / second half step
     DBuf pq0, pq1;                       // linear CG predictor: each half step's next start, 2 delta - delta_prev
-    DBuf slots, partial, bar, status, cg_stats, cg_last, d_step, track;
+    DBuf slots, partial, bar, status, cg_last, d_step, track;    // status: DevStatus, then the CG counters
     DBuf stim_head, stim_next, stim_on, stim_off, stim_amp;
     int nstim = 0;
     DBuf W, ecg_buf, ecg_partial, ecg_counter;
@@ -136,6 +228,9 @@ struct ep_handle {
     std::vector<double> cab_orient, cab_fib;
     int cab_quad = 2, cab_sticky = 1;
 };
+
+// the status block: DevStatus and 32 bytes of CG counters
+constexpr size_t kStatusBytes = sizeof(DevStatus) + 32;
 
 // the radius ComputeECG gives cables (ComputeECG.cc:75), so an in-run ECG
 // of a mixed tissue is the one the reference's post-processor computes
@@ -234,7 +329,7 @@ void fill_cg_args(ep_handle *h, CGArgs<R> &a) {
     a.bar = h->bar.as<GridBarrier>();
     a.tol = h->cg_tol; a.maxit = h->cg_maxit;
     a.floor_rel = sizeof(R) == 4 ? 1.2e-7 : 2.2e-16;   // unit roundoff of R
-    unsigned long long *st = h->cg_stats.as<unsigned long long>();
+    unsigned long long *st = (unsigned long long *)(h->status.as<DevStatus>() + 1);
     a.iters_total = st;
     a.iters_max = (unsigned int *)(st + 1);
     a.fails = (unsigned int *)(st + 1) + 1;
@@ -1051,12 +1146,10 @@ static int create_multi(int ninst, const ep_mesh_desc *meshes, const ep_model_de
     }
     // solver scratch and status
     if ((rc = plan_cg(h.get()))) return rc;
-    if ((rc = h->status.alloc(sizeof(DevStatus)))) return rc;
-    if ((rc = h->cg_stats.alloc(32))) return rc;
+    if ((rc = h->status.alloc(kStatusBytes))) return rc;
     if ((rc = h->d_step.alloc(sizeof(long long)))) return rc;
     if ((rc = h->ecg_slot.alloc(sizeof(unsigned int)))) return rc;
-    EP_CUDA(cudaMemset(h->status.p, 0, sizeof(DevStatus)));
-    EP_CUDA(cudaMemset(h->cg_stats.p, 0, 32));
+    EP_CUDA(cudaMemset(h->status.p, 0, kStatusBytes));
     EP_CUDA(cudaMemset(h->d_step.p, 0, sizeof(long long)));
     EP_CUDA(cudaMemset(h->ecg_slot.p, 0, sizeof(unsigned int)));
     std::vector<Track> tr(n, Track{-1.f, -1.f, -1.f, 1e30f});
@@ -1163,7 +1256,7 @@ static int put_voltage(ep_handle *h, const double *V) {
         int b, e;
         io_range(h->n, k, K, b, e);
         if (e <= b) continue;
-#pragma omp parallel for schedule(static)
+#pragma omp parallel for schedule(static) if (e - b >= (1 << 14))
         for (int i = b; i < e; i++) st[i] = (R)V[i];
         EP_CUDA(cudaMemcpyAsync(h->V.as<R>() + b, st + b, sizeof(R) * (e - b), cudaMemcpyHostToDevice, h->stream));
     }
@@ -1182,7 +1275,7 @@ static int get_voltage(ep_handle *h, double *V) {
     if (K == 1) {
         EP_CUDA(cudaMemcpyAsync(st, h->V.p, sizeof(R) * h->n, cudaMemcpyDeviceToHost, h->stream));
         EP_CUDA(cudaStreamSynchronize(h->stream));
-#pragma omp parallel for schedule(static)
+#pragma omp parallel for schedule(static) if (h->n >= (1 << 14))
         for (int i = 0; i < h->n; i++) V[i] = (double)st[i];
         return EP_OK;
     }
@@ -1407,8 +1500,7 @@ int ep_step(ep_handle *h, int32_t nsteps, ep_step_stats *stats) {
         int rc = ensure_ecg_cap(h, h->ecg_count + nsteps / h->ecg_every + 1);
         if (rc) return rc;
     }
-    EP_CUDA(cudaMemsetAsync(h->status.p, 0, sizeof(DevStatus), h->stream));
-    EP_CUDA(cudaMemsetAsync(h->cg_stats.p, 0, 32, h->stream));
+    EP_CUDA(cudaMemsetAsync(h->status.p, 0, kStatusBytes, h->stream));
     EP_CUDA(cudaEventRecord(h->ev0, h->stream));
     // the clock at entry: a call whose waits gave up did not take its steps
     const long long step0 = h->step;
@@ -1433,7 +1525,16 @@ int ep_step(ep_handle *h, int32_t nsteps, ep_step_stats *stats) {
     rc = h->precision == EP_FP64 ? step_typed<double>(h, left, ne) : step_typed<float>(h, left, ne);
     if (rc) return rc;
     EP_CUDA(cudaEventRecord(h->ev1, h->stream));
-    EP_CUDA(cudaEventSynchronize(h->ev1));
+    // the call's results into pinned memory behind it, and one wait for all
+    const size_t bar_bytes = sizeof(GridBarrier) * (size_t)h->ninst;
+    char *back = (char *)stage(h, kStatusBytes + bar_bytes + sizeof(unsigned int));
+    if (!back) return EP_ERR_NOMEM;
+    EP_CUDA(cudaMemcpyAsync(back, h->status.p, kStatusBytes, cudaMemcpyDeviceToHost, h->stream));
+    EP_CUDA(cudaMemcpyAsync(back + kStatusBytes, h->bar.p, bar_bytes, cudaMemcpyDeviceToHost, h->stream));
+    if (h->has_surrogate)
+        EP_CUDA(cudaMemcpyAsync(back + kStatusBytes + bar_bytes, h->sg_err.p, sizeof(unsigned int),
+                                cudaMemcpyDeviceToHost, h->stream));
+    EP_CUDA(cudaStreamSynchronize(h->stream));
     double kms[4] = {0, 0, 0, 0};
     for (size_t k = 0; k + 1 < ne; k++) {
         float e = 0.f;
@@ -1442,15 +1543,16 @@ int ep_step(ep_handle *h, int32_t nsteps, ep_step_stats *stats) {
     }
     DevStatus st;
     unsigned long long cgs[4];
-    GridBarrier bar;
-    EP_CUDA(cudaMemcpy(&st, h->status.p, sizeof st, cudaMemcpyDeviceToHost));
-    EP_CUDA(cudaMemcpy(cgs, h->cg_stats.p, 32, cudaMemcpyDeviceToHost));
-    {
-        std::vector<GridBarrier> bars(h->ninst);
-        EP_CUDA(cudaMemcpy(bars.data(), h->bar.p, sizeof(GridBarrier) * bars.size(), cudaMemcpyDeviceToHost));
-        bar = bars[0];
-        for (const GridBarrier &b : bars) bar.err |= b.err;
+    std::memcpy(&st, back, sizeof st);
+    std::memcpy(cgs, back + sizeof st, sizeof cgs);
+    GridBarrier bar{};
+    for (int k = 0; k < h->ninst; k++) {
+        GridBarrier b;
+        std::memcpy(&b, back + kStatusBytes + sizeof(GridBarrier) * (size_t)k, sizeof b);
+        bar.err |= b.err;
     }
+    unsigned int sg_err = 0;
+    if (h->has_surrogate) std::memcpy(&sg_err, back + kStatusBytes + bar_bytes, sizeof sg_err);
     float ms = 0.f;
     EP_CUDA(cudaEventElapsedTime(&ms, h->ev0, h->ev1));
     if (stats) {
@@ -1470,8 +1572,6 @@ int ep_step(ep_handle *h, int32_t nsteps, ep_step_stats *stats) {
         stats->ecg_ms = kms[K_ECG];
         stats->launches = h->launches;
     }
-    unsigned int sg_err = 0;
-    if (h->has_surrogate) EP_CUDA(cudaMemcpy(&sg_err, h->sg_err.p, sizeof sg_err, cudaMemcpyDeviceToHost));
     if (stats) stats->timeouts += (int32_t)sg_err;
     if (bar.err || sg_err) {
         // the kernels left early; put the wait state back so the handle can
@@ -2028,6 +2128,27 @@ int ep_ecg_create(const ep_mesh_desc *mesh, const ep_cables_desc *cables, int32_
     return EP_OK;
 }
 
+// host data to the device through two pinned pieces, the copy into one under
+// the transfer of the other (the driver stages pageable memory with one thread)
+static int upload_pieces(void *dst, const void *src, size_t bytes, cudaStream_t s) {
+    constexpr size_t piece = 4u << 20;
+    if (bytes < (1u << 20)) {
+        EP_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s));
+        return EP_OK;
+    }
+    int rc = t_buf.reserve(0, 2 * piece);
+    if (rc) return rc;
+    for (size_t at = 0, k = 0; at < bytes; at += piece, k++) {
+        const size_t b = std::min(piece, bytes - at);
+        char *p = (char *)t_buf.pin + (k & 1) * piece;
+        if (k >= 2) EP_CUDA(cudaEventSynchronize(t_buf.ev[k & 1]));
+        host_copy(p, (const char *)src + at, b);
+        EP_CUDA(cudaMemcpyAsync((char *)dst + at, p, b, cudaMemcpyHostToDevice, s));
+        EP_CUDA(cudaEventRecord(t_buf.ev[k & 1], s));
+    }
+    return EP_OK;
+}
+
 int ep_ecg_eval(ep_ecg *e, int32_t n_frames, const double *V, double *out) {
     EP_CHECK_ARG(e && n_frames >= 0 && (n_frames == 0 || (V && out)), "bad arguments");
     EP_CUDA(cudaSetDevice(e->device));
@@ -2047,8 +2168,7 @@ int ep_ecg_eval(ep_ecg *e, int32_t n_frames, const double *V, double *out) {
         return rc;
     for (int f0 = 0; f0 < n_frames; f0 += chunk) {
         const int nf = std::min(chunk, n_frames - f0);
-        EP_CUDA(cudaMemcpyAsync(e->V.p, V + (size_t)f0 * e->n, sizeof(double) * (size_t)nf * e->n,
-                                cudaMemcpyHostToDevice, e->stream));
+        if ((rc = upload_pieces(e->V.p, V + (size_t)f0 * e->n, sizeof(double) * (size_t)nf * e->n, e->stream))) return rc;
         rc = launch_ecg<double>(e->n, e->ne, e->W.as<double>(), e->n, e->V.as<double>(), nf, e->partial.as<double>(),
                                 e->counter.as<unsigned int>(), e->out.as<double>(), nodes, e->stream);
         if (rc) return rc;
@@ -2149,9 +2269,40 @@ int ep_read_restart(ep_handle *h, double t, const char *dir) {
     return EP_OK;
 }
 
+// The cells [0, n) of a chunk, node-major FP64 as the caller has them, to and
+// from the layout of the ionic kernel.  back: V (phase) or dV/dt (one call,
+// V unchanged) to out, the new states to states.
+}  // extern "C"
+namespace {
+template <typename R>
+__global__ void __launch_bounds__(256) k_cells(int n, int pitch, int nst, int ns, int first, int vslot, bool back,
+                                               double *states, double *out, const double *ist, const double *gks,
+                                               R *S, R *V, R *Ist, R *Gks, const R *dvdt) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    double *s = states + (size_t)i * nst;
+    if (!back) {
+        for (int k = 0; k < ns; k++) S[(size_t)k * pitch + i] = (R)s[k + first];
+        V[i] = (R)out[i];
+        Ist[i] = (R)ist[i];
+        if (Gks) Gks[i] = (R)gks[i];
+        return;
+    }
+    for (int k = 0; k < ns; k++) s[k + first] = (double)S[(size_t)k * pitch + i];
+    if (dvdt) {
+        s[vslot] = out[i];
+        out[i] = (double)dvdt[i];
+    } else {
+        out[i] = s[vslot] = (double)V[i];
+    }
+}
+}  // namespace
+extern "C" {
+
 // Independent cells through the ionic kernel: one Compute_Ion call per cell
 // returning dV/dt (dvdt != NULL, V unchanged), or a whole ionic phase of
-// sub-steps with the V update (dvdt == NULL, V advanced in place).
+// sub-steps with the V update (dvdt == NULL, V advanced in place).  In chunks
+// that bound the buffers; a chunk is one copy each way.
 static int ionic_batch(const ep_model_desc *md, int32_t precision, int32_t n, double dt,
                        double ionic_dt, double Cm, double *V, const double *istim, double *states,
                        double *dvdt) {
@@ -2162,8 +2313,7 @@ static int ionic_batch(const ep_model_desc *md, int32_t precision, int32_t n, do
     const int ntypes = md->n_types > 0 ? md->n_types : 1;
     EP_CHECK_ARG(ntypes <= kMaxTypes, "too many parameter sets");
     ep_handle h;
-    cudaGetDevice(&h.device);
-    h.n = n; h.pitch = (n + 31) / 32 * 32; h.model = md->model; h.precision = precision;
+    h.model = md->model; h.precision = precision;
     h.nstate = nst; h.ns = is_lr(md->model) ? 7 : nst - 1; h.ntypes = ntypes;
     h.dt = dt; h.nsub = 1; h.sub_dt[0] = dt; h.Cm = Cm;
     if (!dvdt) {
@@ -2182,73 +2332,76 @@ static int ionic_batch(const ep_model_desc *md, int32_t precision, int32_t n, do
         if (md->type_consts) std::memcpy(&consts[(size_t)t * nc], md->type_consts + (size_t)t * nc, sizeof(double) * nc);
         else default_consts(md->model, t, &consts[(size_t)t * nc]);
     }
-    std::vector<double> S((size_t)h.ns * h.pitch, 0.0), Vv(h.pitch, 0.0), ist(h.pitch, 0.0);
-    for (int i = 0; i < n; i++) {
-        const double *s = states + (size_t)i * nst;
-        if (is_lr(md->model)) for (int k = 0; k < 7; k++) S[(size_t)k * h.pitch + i] = s[k];
-        else for (int k = 0; k < h.ns; k++) S[(size_t)k * h.pitch + i] = s[k + 1];
-        Vv[i] = V[i];
-        ist[i] = istim ? istim[i] : 0.0;
-    }
-    // the stimulus enters as one window per node covering step 0
-    std::vector<int> head(n), next(n, -1);
-    std::vector<long long> on(n, 0), off(n, 1);
-    for (int i = 0; i < n; i++) head[i] = i;
-    DBuf dvd;
-    int rc;
-    EP_CUDA(cudaStreamCreateWithFlags(&h.stream, cudaStreamNonBlocking));
     auto run = [&](auto tag) -> int {
         using R = decltype(tag);
         int r2;
-        if ((r2 = upload<R>(h.S, S)) || (r2 = upload<R>(h.V, Vv)) || (r2 = upload<R>(h.consts, consts)) ||
-            (r2 = upload<R>(h.stim_amp, ist)))
-            return r2;
-        if ((r2 = upload_raw(h.stim_head, head.data(), n)) || (r2 = upload_raw(h.stim_next, next.data(), n)) ||
-            (r2 = upload_raw(h.stim_on, on.data(), n)) || (r2 = upload_raw(h.stim_off, off.data(), n)))
-            return r2;
-        h.nstim = n;
-        if (md->node_type && (r2 = upload_raw(h.type, md->node_type, (size_t)n))) return r2;
-        if (md->node_gks_scale) {
-            std::vector<double> g(md->node_gks_scale, md->node_gks_scale + n);
-            if ((r2 = upload<R>(h.gks, g))) return r2;
-        }
         if (md->model == EP_LUORUDYWITHGATE) {
             std::vector<double> tab;
             lr_gate_table(tab);
             if ((r2 = upload<R>(h.lr_table, tab))) return r2;
         }
-        if ((r2 = h.status.alloc(sizeof(DevStatus))) || (r2 = h.d_step.alloc(sizeof(long long))) ||
-            (r2 = dvd.alloc(sizeof(R) * h.pitch)))
-            return r2;
-        EP_CUDA(cudaMemset(h.status.p, 0, sizeof(DevStatus)));
-        EP_CUDA(cudaMemset(h.d_step.p, 0, sizeof(long long)));
-        IonicArgs<R> a;
-        fill_ionic_args<R>(&h, a);
-        a.track = nullptr;
-        a.dvdt_out = dvdt ? dvd.as<R>() : nullptr;
-        a.ref_order = sizeof(R) == 4;        // FP32 plugin results keep their bits
-        if ((r2 = launch_ionic<R>(h.model, a, h.stream))) return r2;
-        EP_CUDA(cudaStreamSynchronize(h.stream));
-        std::vector<double> o, so;
-        if ((r2 = download<R>(dvdt ? dvd : h.V, o, n, h.stream))) return r2;
-        if ((r2 = download<R>(h.S, so, (size_t)h.ns * h.pitch, h.stream))) return r2;
-        for (int i = 0; i < n; i++) {
-            if (dvdt) dvdt[i] = o[i];
-            else V[i] = o[i];
-            double *s = states + (size_t)i * nst;
-            if (is_lr(md->model)) {
-                for (int k = 0; k < 7; k++) s[k] = so[(size_t)k * h.pitch + i];
-                s[7] = V[i];
-            } else {
-                s[0] = V[i];
-                for (int k = 0; k < h.ns; k++) s[k + 1] = so[(size_t)k * h.pitch + i];
-            }
+        const int most = std::min(n, 1 << 17);
+        const size_t pitch = ((size_t)most + 31) / 32 * 32;
+        // one block each way: states, V, stimulus, [G_Ks], constants (as R), [types]
+        const bool gks = md->node_gks_scale != nullptr, types = md->node_type != nullptr;
+        auto in_bytes = [&](size_t m) {
+            return sizeof(double) * (m * (nst + 2 + (gks ? 1 : 0)) + consts.size()) + (types ? m : 0);
+        };
+        const size_t in_cap = (in_bytes(most) + 255) / 256 * 256;
+        const size_t dev = in_cap + sizeof(R) * pitch * (h.ns + 4) + 256;
+        if ((r2 = t_buf.reserve(dev, in_cap))) return r2;
+        cudaStream_t s = t_buf.stream;
+        char *db = (char *)t_buf.dev, *hb = (char *)t_buf.pin;
+        R *S = (R *)(db + in_cap), *Vr = S + pitch * h.ns, *Ist = Vr + pitch, *Gks = Ist + pitch, *Dv = Gks + pitch;
+        DevStatus *status = (DevStatus *)(db + dev - 256);
+        for (int i0 = 0; i0 < n; i0 += most) {
+            const int m = std::min(most, n - i0);
+            const size_t oV = sizeof(double) * (size_t)m * nst, oI = oV + sizeof(double) * m, oG = oI + sizeof(double) * m;
+            const size_t oC = oG + (gks ? sizeof(double) * m : 0), oT = oC + sizeof(double) * consts.size();
+            host_copy(hb, states + (size_t)i0 * nst, oV);
+            host_copy(hb + oV, V + i0, sizeof(double) * m);
+            if (istim) host_copy(hb + oI, istim + i0, sizeof(double) * m);
+            else std::memset(hb + oI, 0, sizeof(double) * m);
+            if (gks) host_copy(hb + oG, md->node_gks_scale + i0, sizeof(double) * m);
+            for (size_t k = 0; k < consts.size(); k++) ((R *)(hb + oC))[k] = (R)consts[k];
+            if (types) host_copy(hb + oT, md->node_type + i0, m);
+            EP_CUDA(cudaMemcpyAsync(db, hb, in_bytes(m), cudaMemcpyHostToDevice, s));
+            EP_CUDA(cudaMemsetAsync(status, 0, 256, s));           // the status and, behind it, step 0
+            h.n = m;
+            h.pitch = (int)pitch;
+            IonicArgs<R> a;
+            fill_ionic_args<R>(&h, a);
+            a.V = Vr; a.S = S;
+            a.istim = Ist;
+            a.gks = gks ? Gks : nullptr;
+            a.type = types ? (const uint8_t *)(db + oT) : nullptr;
+            a.consts = (const R *)(db + oC);
+            a.status = status;
+            a.step_ptr = (const long long *)(status + 1);
+            a.track = nullptr;
+            a.dvdt_out = dvdt ? Dv : nullptr;
+            a.ref_order = sizeof(R) == 4;        // FP32 plugin results keep their bits
+            const int first = is_lr(md->model) ? 0 : 1, vslot = is_lr(md->model) ? 7 : 0;
+            auto cells = [&](bool back) {
+                k_cells<R><<<div_up(m, 256), 256, 0, s>>>(m, (int)pitch, nst, h.ns, first, vslot, back, (double *)db,
+                                                          (double *)(db + oV), (const double *)(db + oI),
+                                                          (const double *)(db + oG), S, Vr, Ist, gks ? Gks : nullptr,
+                                                          dvdt ? Dv : nullptr);
+                return cudaGetLastError();
+            };
+            EP_CUDA(cells(false));
+            if ((r2 = launch_ionic<R>(h.model, a, s))) return r2;
+            EP_CUDA(cells(true));
+            EP_CUDA(cudaMemcpyAsync(hb, db, oI, cudaMemcpyDeviceToHost, s));
+            EP_CUDA(cudaStreamSynchronize(s));
+            host_copy(states + (size_t)i0 * nst, hb, oV);
+            host_copy((dvdt ? dvdt : V) + i0, hb + oV, sizeof(double) * m);
         }
         return EP_OK;
     };
-    rc = precision == EP_FP64 ? run(double(0)) : run(float(0));
-    cudaStreamDestroy(h.stream);
-    h.stream = nullptr;
+    const int rc = precision == EP_FP64 ? run(double(0)) : run(float(0));
+    if (rc && t_buf.stream) cudaStreamSynchronize(t_buf.stream);
+    t_buf.trim();
     return rc;
 }
 

@@ -738,12 +738,12 @@ k_cn_half(const CGArgs<R> a) {
         // the residual this sweep started from is small enough already (the
         // test at the end of the last one could not tell): its step is not taken
         if (t[4] <= stop2) { rr_last = t[4]; converged = true; al = R(0); break; }
-        const double alpha = t[1] / t[0];
+        const double alpha = t[1] / t[0], irz = 1.0 / t[1];       // the two divisions side by side
         const double rz = t[1] - 2.0 * alpha * t[2] + alpha * alpha * t[3];
         const double rr = t[4] - 2.0 * alpha * t[5] + alpha * alpha * t[6];
         it++;
         al = (R)alpha;
-        be = (R)(rz / t[1]);
+        be = (R)(rz * irz);
         rr_last = rr;
         // a non-finite residual (a NaN or inf voltage upstream) cannot
         // recover: stop now, counted as a failed solve (every block sees the
@@ -773,7 +773,7 @@ k_cn_half(const CGArgs<R> a) {
 // (cp.async.bulk, one lane issuing, an mbarrier per unit) refill as units are
 // consumed, running on into the next sweep under the reduction.
 constexpr int kUnit = 8, kUnitMax = 9;        // slice columns of a unit; a single left-over column joins the last
-constexpr int kMaxUnits = 64;                 // units in a warp's ring, at most
+constexpr int kMaxUnits = 32;                 // units in a warp's ring, at most
 constexpr unsigned int kCopyPolls = 1u << 18; // tries of one unit's wait
 
 __device__ __forceinline__ void cg_mbar_init(unsigned long long *b) {
@@ -1040,12 +1040,12 @@ __global__ void __launch_bounds__(512, 1) k_cn_smem(const CGArgs<R> a) {
         { R *sw = cur; cur = nxt; nxt = sw; }
         // the scalars and tests of k_cn_half
         if (t[4] <= stop2) { rr_last = t[4]; converged = true; al = R(0); break; }
-        const double alpha = t[1] / t[0];
+        const double alpha = t[1] / t[0], irz = 1.0 / t[1];
         const double rz = t[1] - 2.0 * alpha * t[2] + alpha * alpha * t[3];
         rr_last = t[4] - 2.0 * alpha * t[5] + alpha * alpha * t[6];
         it++;
         al = (R)alpha;
-        be = (R)(rz / t[1]);
+        be = (R)(rz * irz);
         if (!isfinite(rr_last)) break;
         converged = rr_last <= stop2 && stop2 >= 1e-12 * t[4];
     }
@@ -1330,7 +1330,7 @@ int cg_fit_smem(int ns, int cols, CgShape *out) {
         const long long budget = (long long)kb * 1024 / out->per_sm - ((long long)ns + 1) * 4;
         return (int)((budget / warps - kMaxUnits * 8) / (kSlice * (4 + (int)sizeof(R))));
     };
-    const bool stays = out->per_sm == 1 && spw * (cols + 1) <= fit(200);
+    const bool stays = out->per_sm == 1 && spw * cols <= fit(200);
     if (!stays && out->per_sm == 1 && sizeof(R) == 4 && ns <= 64) {
         out->batch = 4;
         out->block = 1024;

@@ -13,6 +13,7 @@ namespace ep {
 
 template <typename R>
 __device__ __forceinline__ R node_istim(const IonicArgs<R> &a, int i, long long step) {
+    if (a.istim) return a.istim[i];
     if (a.stim_head == nullptr) return R(0);
     int k = a.stim_head[i];
     long long best_on = -1;

@@ -65,6 +65,7 @@ template <typename R> struct IonicArgs {
     const int *stim_head, *stim_next;
     const long long *stim_on, *stim_off;
     const R *stim_amp;
+    const R *istim;              // non-null: every node's stimulus, in place of the windows
     const long long *step_ptr;   // device step counter (read)
     double t_per_step;           // dt
     R Cm, Xi;                    // Xi: the model's or the user's
