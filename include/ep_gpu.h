@@ -213,7 +213,7 @@ int  ep_diffusion_half_step(ep_handle *h, int32_t *iters, double *relres);
  * Bval = B, dinv = 1/diag(A); values FP64 or FP32 per `precision`) and x,
  * which holds V on entry and A^-1 B V on return; stream may be NULL.  The
  * working vectors live in one static device array of this library sized for
- * at most 262144 rows (about 17 MB, held by every GPU that loads the
+ * at most 262144 rows (about 15 MB, held by every GPU that loads the
  * library until exit); larger n returns EP_ERR_ARG.  Every call shares that
  * array, so calls that overlap on the GPU race: serialise them.  Each call
  * looks up the array's address on the current device.  The call waits on

@@ -163,7 +163,7 @@ struct ep_handle {
     DBuf cl;                             // explicit scheme: lumped capacitance C_L
     int cg_maxit = 1000;
     int cg_grid = 0, cg_block = 256;
-    CgShape cg{4, 256, 0, 0, 0, 0};      // the planned CG launch: the launch config's, or the library's choice
+    CgShape cg{4, 256, 0, 0, 0, 0, 1.0f};      // the planned CG launch: the launch config's, or the library's choice
     int ecg_every = 0;
     double act_thr = -40.0;
     TTOpts tt{};
@@ -171,7 +171,7 @@ struct ep_handle {
     long long step = 0;
     int nslices = 0;
     // device memory
-    DBuf V, S, Aval, Bval, dinv, qd0, qd1, consts, gks, lr_table, type, slice_ptr, col;
+    DBuf V, S, Aval, Bval, dinv, qd, consts, gks, lr_table, type, slice_ptr, col;
     DBuf r, r1, w0, w1, s0, s1, p0;      // Chronopoulos-Gear CG only (allocated on first use)
     DBuf ex_tmp;                         // explicit scheme: scratch vector
     DBuf pd0, pd1;                       // CG predictor: x - V of the first / second half step
@@ -324,7 +324,9 @@ void fill_cg_args(ep_handle *h, CGArgs<R> &a) {
     a.slice_ptr = h->slice_ptr.as<int>(); a.col = h->col.as<int>();
     a.Aval = h->Aval.as<R>(); a.Bval = h->Bval.as<R>(); a.dinv = h->dinv.as<R>();
     a.x = h->V.as<R>();
-    a.q0 = h->qd0.as<R>(); a.q1 = h->qd1.as<R>();
+    R *qd = h->qd.as<R>();
+    a.q0 = qd; a.q1 = qd + 2 * (size_t)h->pitch;
+    a.po = qd + 4 * (size_t)h->pitch; a.qo = a.po + h->pitch; a.dc = a.qo + h->pitch;
     a.slots = h->slots.as<CgSlot>();
     a.bar = h->bar.as<GridBarrier>();
     a.tol = h->cg_tol; a.maxit = h->cg_maxit;
@@ -347,6 +349,7 @@ void fill_cg_args(ep_handle *h, CGArgs<R> &a) {
     a.depth = stage_depth(h);
     a.ring_cols = h->cg.ring_cols;
     a.smem = h->cg.smem;
+    a.keep = h->cg.keep;
 }
 
 // start the CG predictor from x0 = V again (after a state upload or when it
@@ -381,11 +384,10 @@ int create_typed(ep_handle *h, const HostCSR &csr, const std::vector<double> &st
     if (h->scheme == EP_SCHEME_EXPLICIT) {
         if ((rc = h->ex_tmp.alloc(vb))) return rc;
     } else {
-        // rows past n are gathered by nobody; zero all the same
-        for (DBuf *b : {&h->qd0, &h->qd1}) {
-            if ((rc = b->alloc(4 * vb))) return rc;
-            EP_CUDA(cudaMemset(b->p, 0, 4 * vb));
-        }
+        // the (z, w) pairs, two buffers, and p, q, d; rows past n are gathered by
+        // nobody, zero all the same
+        if ((rc = h->qd.alloc(7 * vb))) return rc;
+        EP_CUDA(cudaMemset(h->qd.p, 0, 7 * vb));
     }
     // cell states (SoA) and voltage
     std::vector<double> V(h->pitch, 0.0), S((size_t)h->ns * h->pitch, 0.0);
@@ -555,7 +557,7 @@ static int reset_barriers(ep_handle *h) {
 static int plan_cg(ep_handle *h) {
     const int ws = stage_depth(h);
     int rc;
-    h->cg = CgShape{h->cg_batch, h->cg_block, 0, 0, 0, 0};
+    h->cg = CgShape{h->cg_batch, h->cg_block, 0, 0, 0, 0, 1.0f};
     if (h->cg_per_sm == 0) {
         rc = h->precision == EP_FP64
                  ? cg_auto_shape<double>(h->nslices, h->ninst, h->cg_batch, h->cg_variant, ws, &h->cg)

@@ -10,16 +10,18 @@
 // slice, one warp per slice, one lane per row) so every value/column load is
 // a coalesced 128-byte transaction.  A and B share the column array.
 //
-// One grid barrier per iteration.  Each node keeps (z, p, w, d) together, z =
-// dinv r, p the direction, w = dinv A p, d = x - V, double-buffered.  One sweep of an
-// iteration rebuilds, for every column it gathers, the neighbour's new
-//   z' = z - alpha w,  p' = z' + beta p
-// from its old triple (explicit fma, so the owner and every neighbour round
-// alike), forms q = A p' and writes the own row's (z', p', dinv q, d + alpha
-// p) to the other buffer; nothing of the old buffer changes during the sweep.
-// alpha and beta come from one reduction at the end of the sweep: besides
-// (p', q) and the residual's own (r, z), (r, r) it sums the products that
-// give the next residual's,
+// One grid barrier per iteration.  Neighbours see a node's (z, w), z = dinv r
+// and w = dinv A p, double-buffered; p, q = A p and the correction d = x - V are
+// the owner's alone.  One sweep of an iteration rebuilds, for every column it
+// gathers, the neighbour's new z' = z - alpha w (an explicit fma, so the owner
+// and every neighbour round alike), forms u = A z' and on the own row
+//   p' = z' + beta p,  q' = u + beta q  (= A p'),  w' = dinv q',  d + alpha p
+// and writes (z', w') to the other buffer; nothing of the old buffer changes
+// during the sweep.  (Gathering p as well and forming A p' directly took twice
+// the bytes a neighbour: at 16 bytes a record a sweep is bound by L1, 2600
+// cycles for 16 slices.)  alpha and beta come from one reduction at the end of
+// the sweep: besides (p', q') and the residual's own (r, z), (r, r) it sums the
+// products that give the next residual's,
 //   (r, z)_next = (r, z) - 2 alpha d(z, w) + alpha^2 d(w, w)   (d = diag A)
 // and (r, r)_next likewise.  Both start from sums of the vectors themselves
 // in every sweep, so the differences (one iteration's reduction, a factor of
@@ -42,40 +44,53 @@ namespace ep {
 __device__ __forceinline__ float ldcg(const float *p) { return __ldcg(p); }
 __device__ __forceinline__ double ldcg(const double *p) { return __ldcg(p); }
 
-// A node's vectors, (z, p, w, d), d the correction x - V so far (added to V
-// once, at the end, so V is rounded once a solve): one 16-byte (FP64: 32-byte) record, so a
-// neighbour's z, p and w come from one sector.
-template <typename R> struct Quad { R z, p, w, d; };
-__device__ __forceinline__ Quad<float> quad_load(const float *q, int i) {
-    const float4 t = reinterpret_cast<const float4 *>(q)[i];
-    return {t.x, t.y, t.z, t.w};
+// What neighbours read of a node, (z, w), in one load.
+template <typename R> struct Pair { R z, w; };
+__device__ __forceinline__ Pair<float> pair_load(const float *q, int i) {
+    const float2 t = reinterpret_cast<const float2 *>(q)[i];
+    return {t.x, t.y};
 }
-__device__ __forceinline__ Quad<double> quad_load(const double *q, int i) {
-    const double2 *t = reinterpret_cast<const double2 *>(q) + 2 * (size_t)i;
-    const double2 u = t[0], v = t[1];
-    return {u.x, u.y, v.x, v.y};
+__device__ __forceinline__ Pair<double> pair_load(const double *q, int i) {
+    const double2 t = reinterpret_cast<const double2 *>(q)[i];
+    return {t.x, t.y};
 }
-__device__ __forceinline__ void quad_store(float *q, int i, float z, float p, float w, float d) {
-    reinterpret_cast<float4 *>(q)[i] = make_float4(z, p, w, d);
+__device__ __forceinline__ void pair_store(float *q, int i, float z, float w) {
+    reinterpret_cast<float2 *>(q)[i] = make_float2(z, w);
 }
-__device__ __forceinline__ void quad_store(double *q, int i, double z, double p, double w, double d) {
-    double2 *t = reinterpret_cast<double2 *>(q) + 2 * (size_t)i;
-    t[0] = make_double2(z, p);
-    t[1] = make_double2(w, d);
+__device__ __forceinline__ void pair_store(double *q, int i, double z, double w) {
+    reinterpret_cast<double2 *>(q)[i] = make_double2(z, w);
 }
-// the new direction p' = (z - alpha w) + beta p of a gathered node
+// a gathered node's new z
 template <typename R>
-__device__ __forceinline__ R quad_dir(const R *q, int c, R alpha, R beta);
-template <>
-__device__ __forceinline__ float quad_dir(const float *q, int c, float alpha, float beta) {
-    const float4 t = reinterpret_cast<const float4 *>(q)[c];
-    return fmaf(beta, t.y, fmaf(-alpha, t.z, t.x));
+__device__ __forceinline__ R pair_z(const R *q, int c, R alpha) {
+    const Pair<R> t = pair_load(q, c);
+    return fma(-alpha, t.w, t.z);
 }
-template <>
-__device__ __forceinline__ double quad_dir(const double *q, int c, double alpha, double beta) {
-    const double2 u = reinterpret_cast<const double2 *>(q)[2 * (size_t)c];
-    const double w = q[4 * (size_t)c + 2];
-    return fma(beta, u.y, fma(-alpha, w, u.x));
+// what only the owner reads of a row: p, q = A p, d = x - V
+template <typename R> struct Own { R p, q, d; };
+template <typename R>
+__device__ __forceinline__ Own<R> own_load(const CGArgs<R> &a, int i) { return {a.po[i], a.qo[i], a.dc[i]}; }
+template <typename R>
+__device__ __forceinline__ void own_store(const CGArgs<R> &a, int i, R p, R q, R d) {
+    a.po[i] = p; a.qo[i] = q; a.dc[i] = d;
+}
+
+// One row of a sweep, with u = A z' of it: the new vectors (see the top), and
+// its terms of the seven sums.
+template <typename R>
+__device__ __forceinline__ void sweep_row(const CGArgs<R> &a, R *nxt, int row, R di, const Pair<R> &t, const Own<R> &o,
+                                          R u, R al, R be, double (&v)[7]) {
+    const R z = fma(-al, t.w, t.z), p = fma(be, o.p, z), q = fma(be, o.q, u), w = di * q;
+    pair_store(nxt, row, z, w);
+    own_store(a, row, p, q, fma(al, o.p, o.d));
+    const double d = (double)(R(1) / di), dz = d * (double)z, dw = d * (double)w;
+    v[0] += (double)p * (double)q;
+    v[1] += dz * (double)z;
+    v[2] += dz * (double)w;
+    v[3] += dw * (double)w;
+    v[4] += dz * dz;
+    v[5] += dz * dw;
+    v[6] += dw * dw;
 }
 
 // ---- grid barrier and reduction in one ----
@@ -589,14 +604,15 @@ __device__ __forceinline__ void cg_finish(const CGArgs<R> &a, const CgShare &sh,
     for (int s = sh.s0 + warp; s < sh.s1; s += nw) {
         const int row = s * kSlice + lane;
         if (row >= sh.rb && row < sh.re) {
-            const Quad<R> o = quad_load(cur, row);
+            const Pair<R> t = pair_load(cur, row);
+            const Own<R> o = own_load(a, row);
             R dn = fma(al, o.p, o.d);
             // FP32, which stops at the resolution of b: one more step for
             // free, the next iteration's direction taken with this iteration's
             // length (successive lengths differ by a few percent on these
             // mass-dominated systems, so it lowers the error 2-3 fold, as the
             // iteration itself would).  FP64 keeps the reference's iterate.
-            if (sizeof(R) == 4 && converged) dn = fma(al, fma(be, o.p, fma(-al, o.w, o.z)), dn);
+            if (sizeof(R) == 4 && converged) dn = fma(al, fma(be, o.p, fma(-al, t.w, t.z)), dn);
             a.x[row] += dn;
             if (a.delta) {
                 if (a.dext) a.dext[row] = R(2) * dn - a.delta[row];     // the next solve's start: 2 delta - delta_prev
@@ -680,8 +696,8 @@ k_cn_half(const CGArgs<R> a) {
             if (row >= rb && row < re) {
                 const R rref = bx - ax;
                 const R r = pred ? rref - ad : rref;
-                quad_store(cur, row, __ldg(a.dinv + row) * r, R(0), R(0),
-                           pred ? (lin ? a.dext[row] : a.delta[row]) : R(0));
+                pair_store(cur, row, __ldg(a.dinv + row) * r, R(0));
+                own_store(a, row, R(0), R(0), pred ? (lin ? a.dext[row] : a.delta[row]) : R(0));
                 v[0] += (double)r * (double)r;
                 v[1] += (double)bx * (double)bx;
                 v[2] += (double)rref * (double)rref;
@@ -709,25 +725,13 @@ k_cn_half(const CGArgs<R> a) {
                 prefetch_slice<R>(a.slice_ptr, a.col, a.Aval, nullptr, s + a.prefetch * nwarps, s_hi, lane);
             const int row = s * kSlice + lane;
             const int beg = __ldg(a.slice_ptr + s), w = (__ldg(a.slice_ptr + s + 1) - beg) / kSlice;
-            auto gat = [&](int c) { return quad_dir(cur, c, al, be); };
-            R q;
-            if constexpr (STAGED) q = ring_row_sum(ring, a, gwarp, nwarps, lane, w, cons, gat);
-            else if constexpr (NB == 16) q = slice_row_sum_pipe<8>(a.col, a.Aval, beg, w, lane, gat);
-            else q = slice_row_sum<NB>(a.col, a.Aval, beg, w, lane, gat);
-            if (row >= rb && row < re) {
-                const Quad<R> o = quad_load(cur, row);
-                const R di = __ldg(a.dinv + row);
-                const R z = fma(-al, o.w, o.z), p = fma(be, o.p, z), wv = di * q;
-                quad_store(nxt, row, z, p, wv, fma(al, o.p, o.d));
-                const double d = (double)(R(1) / di), dz = d * (double)z, dw = d * (double)wv;
-                v[0] += (double)p * (double)q;
-                v[1] += dz * (double)z;
-                v[2] += dz * (double)wv;
-                v[3] += dw * (double)wv;
-                v[4] += dz * dz;
-                v[5] += dz * dw;
-                v[6] += dw * dw;
-            }
+            auto gat = [&](int c) { return pair_z(cur, c, al); };
+            R u;
+            if constexpr (STAGED) u = ring_row_sum(ring, a, gwarp, nwarps, lane, w, cons, gat);
+            else if constexpr (NB == 16) u = slice_row_sum_pipe<8>(a.col, a.Aval, beg, w, lane, gat);
+            else u = slice_row_sum<NB>(a.col, a.Aval, beg, w, lane, gat);
+            if (row >= rb && row < re)
+                sweep_row(a, nxt, row, __ldg(a.dinv + row), pair_load(cur, row), own_load(a, row), u, al, be, v);
         }
         double t[7];
         if (!group_reduce(a.slots, G, ++tag, b0, nb, a.bar_extra, bar, v, t)) {
@@ -758,20 +762,21 @@ k_cn_half(const CGArgs<R> a) {
 }
 
 // ---------------------------------------------------------------------------
-// k_cn_smem: the solve of k_cn_half with the matrix in shared memory, what a
-// handle runs unless its launch shape is set.  An iteration of k_cn_half is a
-// chain of exposed memory latencies (0.5-0.6 us each under load): the slice's
-// bounds, then for every four columns their indices and values and then the
-// gathers, then the own record, some eleven a slice, so a warp took 9.5 us a
-// slice on the 765K-node shell and one 23-warp CTA 6.5 us an iteration on 715
-// nodes.  Here the gathers are the only one: the slice bounds and the matrix
-// wait in shared memory, the own record is loaded beside the gathers, and a
-// slice's gathers go out 16 (FP64: 8) at a time.
-// Where a CTA's share of the matrix fits (about 250K nodes in FP32, 165K in
-// FP64 over 148 SMs) it is copied in once and stays for the whole solve; else
-// each warp's region is a ring of units of 8 slice columns that bulk copies
-// (cp.async.bulk, one lane issuing, an mbarrier per unit) refill as units are
-// consumed, running on into the next sweep under the reduction.
+// k_cn_smem: the solve of k_cn_half with the matrix in shared memory
+// (cg_auto_shape says when).  An iteration of k_cn_half is a chain of exposed
+// memory latencies (0.5-0.6 us each under load): the slice's bounds, then for
+// every four columns their indices and values and then the gathers, then the
+// own row, some eleven a slice.  Here the gathers are the only one: the slice
+// bounds and the matrix wait in shared memory, the own row is loaded beside the
+// gathers, and a slice's gathers go out together.
+// Where a CTA's share of the matrix fits it is copied in once and stays for the
+// whole solve; else each warp's region is a ring of units of 8 slice columns
+// that bulk copies (cp.async.bulk, one lane issuing, an mbarrier per unit)
+// refill as units are consumed, running on into the next sweep under the
+// reduction.  A matrix that L2 does not hold streams through it sweep after
+// sweep, each line gone before its next use; L2 is asked to keep the first 36
+// MB of it and to pass the rest (765K nodes: 732 -> 630 us a step; 564K FP64:
+// 1275 -> 968).
 constexpr int kUnit = 8, kUnitMax = 9;        // slice columns of a unit; a single left-over column joins the last
 constexpr int kMaxUnits = 32;                 // units in a warp's ring, at most
 constexpr unsigned int kCopyPolls = 1u << 18; // tries of one unit's wait
@@ -797,11 +802,23 @@ __device__ __forceinline__ bool cg_mbar_wait(unsigned long long *b, uint32_t par
 }
 // both addresses 16-byte aligned, bytes a multiple of 16: units start on
 // 128-byte boundaries of the SELL arrays and of the region
-__device__ __forceinline__ void cg_bulk(void *dst, const void *src, uint32_t bytes, unsigned long long *bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     cg_smem_u32(dst)),
-                 "l"(src), "r"(bytes), "r"(cg_smem_u32(bar))
+__device__ __forceinline__ void cg_bulk(void *dst, const void *src, uint32_t bytes, unsigned long long *bar,
+                                        uint64_t pol) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, "
+                 "[%3], %4;" ::"r"(cg_smem_u32(dst)),
+                 "l"(src), "r"(bytes), "r"(cg_smem_u32(bar)), "l"(pol)
                  : "memory");
+}
+// L2 policies of the ring's copies: keep, pass (l2_evict_first_policy) or none
+__device__ __forceinline__ uint64_t l2_evict_last_policy() {
+    uint64_t pol;
+    asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol));
+    return pol;
+}
+__device__ __forceinline__ uint64_t l2_normal_policy() {
+    uint64_t pol;
+    asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(pol));
+    return pol;
 }
 
 // columns of the next unit of a slice with `rem` columns left
@@ -817,6 +834,8 @@ struct MatRing {
     int nw, L;                    // warps of the CTA; the warp's slices
     int slots;                    // unit slots (resident: the units of the share)
     bool resident;
+    int keep;                     // slices whose units L2 is asked to keep
+    uint64_t pol_keep, pol_pass;
     int pj, pk, pslot, pcol;      // producer (lane 0): slice, column, slot and running column of the next unit
     int slot, ccol;               // consumer: slot and running column of the next unit
     uint32_t phase;               // and its mbarrier's parity
@@ -836,8 +855,9 @@ struct MatRing {
         const R *av = vals + beg + pk * kSlice;
         if ((((uintptr_t)ci | (uintptr_t)av) & 15u) == 0) {
             cg_mbar_expect(b, (uint32_t)nc * kColBytes);
-            cg_bulk(d, ci, (uint32_t)n * 4u, b);
-            cg_bulk(d + n * 4, av, (uint32_t)n * (uint32_t)sizeof(R), b);
+            const uint64_t pol = pj < keep ? pol_keep : pol_pass;
+            cg_bulk(d, ci, (uint32_t)n * 4u, b, pol);
+            cg_bulk(d + n * 4, av, (uint32_t)n * (uint32_t)sizeof(R), b, pol);
         } else {
             // a caller's arrays that bulk copies cannot read (ep_cn_half_step_noalloc)
             for (int e = 0; e < n; e++) {
@@ -888,6 +908,9 @@ __device__ __forceinline__ void mat_start(MatRing<R> &m, const CGArgs<R> &a, con
     m.pj = m.pk = m.pslot = m.pcol = 0;
     m.slot = m.ccol = 0;
     m.phase = 0;
+    m.keep = (int)((float)m.L * a.keep);
+    m.pol_keep = a.keep >= 1.0f ? l2_normal_policy() : l2_evict_last_policy();
+    m.pol_pass = l2_evict_first_policy();
     if (lane == 0) {
         for (int k = 0; k < m.slots; k++) cg_mbar_init(m.bars + k);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -942,7 +965,7 @@ __device__ __forceinline__ void mat_slice(MatRing<R> &m, const CGArgs<R> &a, int
 
 template <typename R>
 __global__ void __launch_bounds__(512, 1) k_cn_smem(const CGArgs<R> a) {
-    constexpr int GU = sizeof(R) == 4 ? 2 : 1;
+    constexpr int GU = 2;                     // a slice's two units
     extern __shared__ __align__(128) unsigned char cg_sm[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int G = gridDim.x;
@@ -986,16 +1009,17 @@ __global__ void __launch_bounds__(512, 1) k_cn_smem(const CGArgs<R> a) {
             const R di = on ? __ldg(a.dinv + row) : R(1), d0 = on && pred ? dv0[row] : R(0);
             R ax = R(0), bx = R(0), ad = R(0);
             mat_slice<R, 1>(m, a, w, true, lane, ok, [&](int c, int k) {
-                return Quad<R>{a.x[c], __ldg(a.Bval + beg + k * kSlice + lane), pred ? dv0[c] : R(0), R(0)};
-            }, [&](R av, const Quad<R> &t) {
-                ax += av * t.z;
-                bx += t.p * t.z;
-                ad += av * t.w;
+                return Own<R>{a.x[c], __ldg(a.Bval + beg + k * kSlice + lane), pred ? dv0[c] : R(0)};
+            }, [&](R av, const Own<R> &t) {
+                ax += av * t.p;
+                bx += t.q * t.p;
+                ad += av * t.d;
             });
             if (on) {
                 const R rref = bx - ax;
                 const R r = pred ? rref - ad : rref;
-                quad_store(cur, row, di * r, R(0), R(0), d0);
+                pair_store(cur, row, di * r, R(0));
+                own_store(a, row, R(0), R(0), d0);
                 v[0] += (double)r * (double)r;
                 v[1] += (double)bx * (double)bx;
                 v[2] += (double)rref * (double)rref;
@@ -1016,24 +1040,14 @@ __global__ void __launch_bounds__(512, 1) k_cn_smem(const CGArgs<R> a) {
         for (int j = warp; j < ns; j += nw) {
             const int row = (sh.s0 + j) * kSlice + lane, w = (sp[j + 1] - sp[j]) / kSlice;
             const bool on = row >= rb && row < re;
-            Quad<R> o{R(0), R(0), R(0), R(0)};
+            Pair<R> t{R(0), R(0)};
+            Own<R> o{R(0), R(0), R(0)};
             R di = R(1);
-            if (on) { o = quad_load(cur, row); di = __ldg(a.dinv + row); }
-            R q = R(0);
-            mat_slice<R, GU>(m, a, w, false, lane, ok, [&](int c, int) { return quad_dir(cur, c, al, be); },
-                             [&](R av, R g) { q += av * g; });
-            if (on) {
-                const R z = fma(-al, o.w, o.z), p = fma(be, o.p, z), wv = di * q;
-                quad_store(nxt, row, z, p, wv, fma(al, o.p, o.d));
-                const double d = (double)(R(1) / di), dz = d * (double)z, dw = d * (double)wv;
-                v[0] += (double)p * (double)q;
-                v[1] += dz * (double)z;
-                v[2] += dz * (double)wv;
-                v[3] += dw * (double)wv;
-                v[4] += dz * dz;
-                v[5] += dz * dw;
-                v[6] += dw * dw;
-            }
+            if (on) { t = pair_load(cur, row); o = own_load(a, row); di = __ldg(a.dinv + row); }
+            R u = R(0);
+            mat_slice<R, GU>(m, a, w, false, lane, ok, [&](int c, int) { return pair_z(cur, c, al); },
+                             [&](R av, R g) { u += av * g; });
+            if (on) sweep_row(a, nxt, row, di, t, o, u, al, be, v);
         }
         double t[7];
         if (!group_reduce(a.slots, G, ++tag, b0, nb, a.bar_extra, bar, v, t, ok)) { leave(); return; }
@@ -1272,22 +1286,23 @@ int cg_max_per_sm(int block, int *per, int batch, int variant, int depth) {
 // cg_block 256, cg_batch 4 and cg_variant 0, and of ep_cn_half_step_noalloc.
 // No more CTAs than there are slices for, since every CTA takes part in each
 // iteration's reduction (measured: CG us a step, two solves, 16-30 iterations):
-//   up to 32 slices: k_cn_half on one CTA, whose reductions need no global
-//     memory (FP32, 715 nodes: 86 us against 87; FP64 takes k_cn_smem, 158
-//     against 205);
-//   up to 8 slices per SM: k_cn_smem with 256 threads, one slice per warp
-//     (28.6K nodes, FP32 / FP64: 105 / 192 us; 512 threads 111 / 223; k_cn_half
-//     149 / 257);
-//   beyond: k_cn_smem with 512 threads, one CTA per SM (143K nodes: 144 / 337
-//     us, k_cn_half 171 / 384), with 200 KB of shared memory where the matrix
-//     then stays in it, else 120 KB, which leaves the gathers more L1 (765K
-//     nodes, FP32: 735 us, 784 with 200 KB, 1131 with k_cn_half);
-//   except FP32 just past that (its matrix still in L2, up to 64 slices per
-//     SM): k_cn_half with 1024 threads, whose twice as many warps hide the
-//     latency as well (263K nodes: 270 us against 284).
-// Batches run k_cn_smem in two CTAs of 256 threads per SM (24 slabs, 446K
-// nodes: 397 us; k_cn_half 416): more CTAs split the GPU more evenly between
-// the instances, whose groups are small already.
+//   FP32 up to 32 slices: k_cn_half on one CTA, whose reductions need no global
+//     memory (715 nodes: 74 us; FP64 takes k_cn_smem, 143 against 209);
+//   k_cn_smem where a CTA's share of the matrix stays in shared memory: 256
+//     threads up to 8 slices per SM, one slice per warp (28.6K nodes, FP32 /
+//     FP64: 104 / 182 us; k_cn_half 141 / 245), 512 beyond, one CTA per SM
+//     (214K nodes FP32: 168 us against 191; 72K FP64: 204 against 258).  FP32
+//     may fill 200 KB with it, FP64 140, whose gathers need the L1 more (143K
+//     nodes: 302 us resident, 287 with k_cn_half);
+//   k_cn_half with 1024 threads per SM where the matrix no longer does but L2
+//     holds it, up to 60 MB (263K FP32: 220 us against 270 from the ring; 500K:
+//     320 against 374; 307K FP64: 578 against 618): twice the warps hide L2's
+//     latency as well, and nothing is copied;
+//   k_cn_smem's ring beyond (765K FP32: 630 us against 748; 500K FP64: 869
+//     against 1183), with 120 KB, which leaves the gathers their L1.
+// Batches the same with two CTAs per SM, which split the GPU more evenly
+// between the instances (24 slabs, 446K nodes FP32: 306 us from k_cn_half, 389
+// from the ring; FP64: 934, 854).
 // Any other launch config, and more instances than those CTAs, run k_cn_half
 // with CTAs of `block` threads, as many as fit.
 template <typename R>
@@ -1321,8 +1336,8 @@ int cg_auto_shape(int nslices, int ninst, int batch, int variant, int depth, CgS
     return EP_OK;
 }
 
-// k_cn_smem's sizes for CTAs of at most ns slices of about `cols` columns (and
-// the one range of sizes that goes back to k_cn_half)
+// The kernel for CTAs of at most ns slices of about `cols` columns, by the rule
+// above, and k_cn_smem's sizes.
 template <typename R>
 int cg_fit_smem(int ns, int cols, CgShape *out) {
     const int warps = out->block / 32, spw = div_up(ns, warps);
@@ -1330,14 +1345,17 @@ int cg_fit_smem(int ns, int cols, CgShape *out) {
         const long long budget = (long long)kb * 1024 / out->per_sm - ((long long)ns + 1) * 4;
         return (int)((budget / warps - kMaxUnits * 8) / (kSlice * (4 + (int)sizeof(R))));
     };
-    const bool stays = out->per_sm == 1 && spw * cols <= fit(200);
-    if (!stays && out->per_sm == 1 && sizeof(R) == 4 && ns <= 64) {
+    const int most = sizeof(R) == 4 ? 200 : 140;
+    const bool stays = spw * cols <= fit(most);
+    const double mb = (double)ns * out->grid * cols * kSlice * (4 + sizeof(R)) / 1e6;      // the matrix
+    if (!stays && mb <= 60.0) {
         out->batch = 4;
-        out->block = 1024;
+        out->block = 1024 / out->per_sm;
         return EP_OK;
     }
     // a share that stays gets room for slices half as wide again
-    out->ring_cols = std::min(std::max(spw * (cols + cols / 2), 2 * kUnitMax), fit(stays ? 200 : 120));
+    out->ring_cols = std::min(std::max(spw * (cols + cols / 2), 2 * kUnitMax), fit(stays ? most : 120));
+    out->keep = mb <= 60.0 ? 1.0f : (float)(36.0 / mb);
     // a slice's gathers take up to two units of the ring at once
     if (out->ring_cols < 2 * kUnitMax) { set_error("CG kernel: %d matrix columns per warp are too few", out->ring_cols); return EP_ERR_ARG; }
     out->smem = (int)smem_bytes(out->block, out->ring_cols, ns, (int)sizeof(R));

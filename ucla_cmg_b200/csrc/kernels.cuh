@@ -108,7 +108,8 @@ template <typename R> struct CGArgs {
     const int *col;
     const R *Aval, *Bval, *dinv;
     R *x;
-    R *q0, *q1;                  // two buffers of 4 * pitch: (z, p, w, d) per node (16-byte aligned)
+    R *q0, *q1;                  // two buffers of 2 * pitch: (z, w) per node (16-byte aligned)
+    R *po, *qo, *dc;             // p, A p and the correction of the own rows
     CgSlot *slots;               // 2 sets x grid x 8 reduction units (zeroed before the first launch)
     GridBarrier *bar;
     double tol;
@@ -144,6 +145,7 @@ template <typename R> struct CGArgs {
     int depth;
     // k_cn_smem: matrix columns of a warp's region and the CTA's dynamic shared memory
     int ring_cols, smem;
+    float keep;                  // share of its slices L2 is asked to keep (1: no hint)
 };
 
 // cg_batch value of the staged kernel (asynchronous copies of each warp's
@@ -163,7 +165,7 @@ template <typename R>
 int launch_cg(const CGArgs<R> &a, int grid, int block, cudaStream_t s, int batch = 4, int variant = 0);
 // a launch whose shape is left to the library: kernel (batch), threads, CTAs
 // and k_cn_smem's sizes (block: the asked size in, the launch's out)
-struct CgShape { int batch, block, grid, per_sm, ring_cols, smem; };
+struct CgShape { int batch, block, grid, per_sm, ring_cols, smem; float keep; };
 template <typename R>
 int cg_auto_shape(int nslices, int ninst, int batch, int variant, int depth, CgShape *out);
 template <typename R>

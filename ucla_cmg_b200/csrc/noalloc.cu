@@ -7,7 +7,7 @@
 // device and can fail late in a long run), or a C/Fortran caller that only
 // hands over buffers it manages.  ep_cn_half_step_noalloc gives them the
 // persistent Jacobi-PCG kernel with its working vectors (two buffers of the
-// nodes' (z, p, w, d) records), the reduction slots and the grid barrier
+// nodes' (z, w) pairs, and p, q, d), the reduction slots and the grid barrier
 // placed in one statically sized device array defined in this file, so a
 // call performs no device allocation at all.  The caller passes the matrix
 // (SELL-32 layout) and the voltage vector, both in its own device memory.
@@ -15,7 +15,7 @@
 // Limits and rules (repeated in include/ep_gpu.h):
 // * at most kNoAllocMaxRows rows; larger systems are rejected with
 //   EP_ERR_ARG;
-// * the array (about 17 MB) is part of the module: every GPU that loads the
+// * the array (about 15 MB) is part of the module: every GPU that loads the
 //   library holds it until the process exits;
 // * every call shares the one array, so calls that overlap on the GPU (two
 //   streams, two host threads) race -- serialise them;
@@ -35,7 +35,7 @@ namespace ep {
 constexpr int kNoAllocMaxRows = 262144;                 // 2^18 rows
 constexpr int kNoAllocMaxGrid = 2048;                   // >= 148 SMs x 8 blocks
 constexpr size_t kVecBytes = sizeof(double) * (size_t)kNoAllocMaxRows;   // one vector, FP64
-constexpr size_t kScratchBytes = 8 * kVecBytes                            // the (z, p, w, d) records, two buffers
+constexpr size_t kScratchBytes = 7 * kVecBytes                            // the (z, w) pairs, two buffers, and p, q, d
                                + sizeof(CgSlot) * 16 * kNoAllocMaxGrid    // reduction slots
                                + 256;                                     // barrier, stats, result
 
@@ -69,9 +69,12 @@ int run(unsigned char *base, int n, int nslices, const int *slice_ptr, const int
     a.slice_ptr = slice_ptr; a.col = col;
     a.Aval = A; a.Bval = B; a.dinv = dinv; a.x = x;
     a.q0 = (R *)(base + 0 * kVecBytes);
-    a.q1 = (R *)(base + 4 * kVecBytes);
-    a.slots = (CgSlot *)(base + 8 * kVecBytes);
-    unsigned char *tail = base + 8 * kVecBytes + sizeof(CgSlot) * 16 * kNoAllocMaxGrid;
+    a.q1 = (R *)(base + 2 * kVecBytes);
+    a.po = (R *)(base + 4 * kVecBytes);
+    a.qo = (R *)(base + 5 * kVecBytes);
+    a.dc = (R *)(base + 6 * kVecBytes);
+    a.slots = (CgSlot *)(base + 7 * kVecBytes);
+    unsigned char *tail = base + 7 * kVecBytes + sizeof(CgSlot) * 16 * kNoAllocMaxGrid;
     a.bar = (GridBarrier *)tail;                                   // 32 B
     unsigned long long *st = (unsigned long long *)(tail + 64);   // 32 B of counters
     a.iters_total = st;
@@ -83,7 +86,7 @@ int run(unsigned char *base, int n, int nslices, const int *slice_ptr, const int
     a.maxit = maxit > 0 ? maxit : 1000;
     // the barrier's tags go on from call to call (the array starts zeroed),
     // and the kernel writes the records before it reads them
-    CgShape cg{4, 256, 0, 0, 0, 0};
+    CgShape cg{4, 256, 0, 0, 0, 0, 1.0f};
     int rc = cg_auto_shape<R>(nslices, 1, 4, 0, 0, &cg);
     // the rows' widths are on the device; 16 columns are a linear-tet mesh's
     // (wider slices only make a share that would stay a ring)
@@ -91,6 +94,7 @@ int run(unsigned char *base, int n, int nslices, const int *slice_ptr, const int
     if (rc) return rc;
     a.ring_cols = cg.ring_cols;
     a.smem = cg.smem;
+    a.keep = cg.keep;
     if ((rc = launch_cg<R>(a, cg.grid, cg.block, s, cg.batch))) return rc;
     // barrier and result in one copy
     unsigned char back[160];
