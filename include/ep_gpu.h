@@ -359,10 +359,11 @@ typedef struct ep_launch_config {
                              many slices ahead (cg_variant 0; 0 = off); with
                              cg_batch 32 the units the ring holds in flight
                              (0 = 2) */
-    int32_t sg_variant;   /* learned ionic step (EP_SURROGATE): 0 two CTAs per SM,
-                             each one tile of 128 nodes at a time; 1 one CTA per SM
-                             running four tiles at once in four warpgroups (one
-                             copy of the weights); same results */
+    int32_t sg_variant;   /* learned ionic step (EP_SURROGATE): 0 the library's choice
+                             by size: one tile of 128 nodes per CTA up to one tile per
+                             SM, beyond that as 1; 1 one CTA per SM running four tiles
+                             at once in four warpgroups (one copy of the weights);
+                             same results */
 } ep_launch_config;
 /* Bounded in-kernel waits (no reference counterpart: the reference has no
  * device code; its Newton loop has no cap, Tusscher.cc:150).  Every wait of

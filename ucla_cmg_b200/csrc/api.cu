@@ -193,7 +193,8 @@ struct ep_handle {
     std::vector<int> pkind;              // kernel class started at each event
     long long launches = 0;
     // learned ionic step (EP_SURROGATE)
-    DBuf sg_wimg, sg_aux, sg_list, sg_count, sg_err, sg_pred, sg_take;
+    DBuf sg_wimg, sg_list, sg_count, sg_err, sg_pred, sg_take;
+    SurrogateAux sg_aux;
     int has_surrogate = 0, sg_vupdate = 0;
     // independent instances sharing the launches (ep_batch_create)
     int ninst = 1;
@@ -201,7 +202,7 @@ struct ep_handle {
     std::vector<int> inst_blk;           // ninst + 1 CTA offsets of the CG groups
     DBuf d_inst_row, d_inst_blk;
     // launch shape (ep_set_launch_config / ep_autotune)
-    int sg_variant = 0;                  // learned step: 0 two CTAs/SM, 1 four pipelines in one CTA/SM
+    int sg_variant = 0;                  // learned step: 0 by size, 1 four pipelines in one CTA/SM
     int cg_per_sm = 0, cg_batch = 4, cg_variant = 0, cg_predict = 0, cg_prefetch = 0, ionic_block = 128,
         ionic_min = 0, graph_steps = 0;
     cudaGraphExec_t gexec = nullptr;
@@ -647,7 +648,7 @@ static void fill_surrogate_args(ep_handle *h, const IonicArgs<float> &ia, Surrog
     sa.Cm = ia.Cm; sa.Xi = ia.Xi; sa.act_thr = ia.act_thr;
     sa.track = ia.track;
     sa.wimg = h->sg_wimg.as<unsigned short>();
-    sa.aux = h->sg_aux.as<SurrogateAux>();
+    sa.aux = h->sg_aux;
     sa.fallback_list = h->sg_list.as<int>();
     sa.fallback_count = h->sg_count.as<int>();
     sa.status = h->status.as<DevStatus>();
@@ -1657,7 +1658,6 @@ static int pack_surrogate(const ep_surrogate_desc *d, std::vector<unsigned short
     const int dims[5] = {SG_NF, SG_H, SG_H, SG_H, SG_NY};
     const int Kpad[4] = {SG_KIN, SG_H, SG_H, SG_H};
     const int base[4] = {0, SG_W1, SG_W1 + SG_W2, SG_W1 + SG_W2 + SG_W3};
-    float *bias[4] = {aux.b1, aux.b2, aux.b3, aux.b4};
     size_t off = 0;
     for (int l = 0; l < 4; l++) {
         const int nout = dims[l + 1], nin = dims[l];
@@ -1665,7 +1665,7 @@ static int pack_surrogate(const ep_surrogate_desc *d, std::vector<unsigned short
             for (int k = 0; k < nin; k++)
                 img[base[l] + core_offset(r, k, Kpad[l])] = to_bf16(p[off + (size_t)r * nin + k]);
         off += (size_t)nout * nin;
-        for (int r = 0; r < nout; r++) bias[l][r] = p[off + r];
+        for (int r = 0; r < nout; r++) aux.b[l][r] = p[off + r];
         off += nout;
     }
     for (int k = 0; k < SG_KIN; k++) {
@@ -1707,7 +1707,7 @@ int ep_set_surrogate(ep_handle *h, const ep_surrogate_desc *d) {
     if (rc) return rc;
     EP_CUDA(cudaStreamSynchronize(h->stream));
     if ((rc = upload_raw(h->sg_wimg, img.data(), img.size()))) return rc;
-    if ((rc = upload_raw(h->sg_aux, &aux, 1))) return rc;
+    h->sg_aux = aux;
     if (!h->sg_list.p) {
         if ((rc = h->sg_list.alloc(sizeof(int) * (size_t)h->pitch))) return rc;
         if ((rc = h->sg_count.alloc(sizeof(int)))) return rc;
@@ -1736,10 +1736,10 @@ int ep_surrogate_forward(const ep_surrogate_desc *d, int32_t n, const float *X, 
     SurrogateAux aux;
     int rc = pack_surrogate(d, img, aux);
     if (rc) return rc;
-    DBuf dimg, daux, dx, dy, derr, dstat;
-    if ((rc = upload_raw(dimg, img.data(), img.size())) || (rc = upload_raw(daux, &aux, 1)) ||
-        (rc = upload_raw(dx, X, (size_t)n * SG_KIN)) || (rc = dy.alloc(sizeof(float) * (size_t)n * SG_NOUT)) ||
-        (rc = derr.alloc(sizeof(unsigned int))) || (rc = dstat.alloc(sizeof(DevStatus))))
+    DBuf dimg, dx, dy, derr, dstat;
+    if ((rc = upload_raw(dimg, img.data(), img.size())) || (rc = upload_raw(dx, X, (size_t)n * SG_KIN)) ||
+        (rc = dy.alloc(sizeof(float) * (size_t)n * SG_NOUT)) || (rc = derr.alloc(sizeof(unsigned int))) ||
+        (rc = dstat.alloc(sizeof(DevStatus))))
         return rc;
     EP_CUDA(cudaMemset(derr.p, 0, sizeof(unsigned int)));
     EP_CUDA(cudaMemset(dstat.p, 0, sizeof(DevStatus)));
@@ -1747,7 +1747,7 @@ int ep_surrogate_forward(const ep_surrogate_desc *d, int32_t n, const float *X, 
     std::memset(&sa, 0, sizeof sa);
     sa.n = n;
     sa.wimg = dimg.as<unsigned short>();
-    sa.aux = daux.as<SurrogateAux>();
+    sa.aux = aux;
     sa.rawX = dx.as<float>();
     sa.rawY = dy.as<float>();
     sa.err = derr.as<unsigned int>();

@@ -1,7 +1,7 @@
 // surrogate.cu -- BF16 tensor-core (tcgen05) inference of the learned ionic
-// step, one persistent CTA per half SM.
+// step.
 //
-// Per tile of 128 nodes (one node per thread = one TMEM lane):
+// Per tile of 128 nodes (one node = one TMEM lane):
 //   1. features of the node (V, 18 states, I_stim, G_Ks, G_to, s-gate) ->
 //      normalised -> BF16 row of the A operand in shared memory;
 //   2. four layers: one elected thread issues tcgen05.mma (kind::f16, BF16 x
@@ -15,10 +15,15 @@
 //      node's state; nodes outside the training envelope (input box, fast
 //      Na-gate product m^3 h, an active stimulus) are appended to a fallback
 //      list that the plain FP32 kernel then runs.
-// The weights (80 KB) are loaded once per CTA.  Shared memory 112 KB and
-// 256 TMEM columns per CTA, so two CTAs share an SM and one's epilogue
-// overlaps the other's MMAs.  Every mbarrier wait is bounded; on timeout the
-// CTA records the error, frees its TMEM and leaves.
+// The weights (80 KB) are loaded once per CTA.  Every mbarrier wait is bounded;
+// on timeout the CTA records the error, frees its TMEM and leaves.
+//
+// What bounds it: 384 tanh a node, 16 a clock and SM (66 us for 765K nodes), and
+// the chain of a tile (row, four times barrier + MMA + commit + TMEM load, output),
+// which several tiles in flight hide.  Biases, means and ranges are kernel
+// parameters, so that they cost no load; one barrier a layer (each thread sees
+// the commit itself); a layer's descriptors step by a constant; the next rows'
+// loads go out under the output layer's MMA.  263K nodes: 92 us to 58 us.
 #include <cuda_bf16.h>
 
 #include "surrogate.cuh"
@@ -32,11 +37,8 @@ constexpr int OFF_W3 = OFF_W2 + SG_W2 * 2;
 constexpr int OFF_W4 = OFF_W3 + SG_W3 * 2;
 constexpr int OFF_A = OFF_W4 + SG_W4 * 2;                 // 128 x 128 bf16
 constexpr int OFF_MISC = OFF_A + SG_M * SG_H * 2;
-constexpr int OFF_FLAGS = OFF_MISC + 64;                 // 2 x 128 envelope flags
-constexpr int SG_SMEM = OFF_FLAGS + 2 * SG_M;
+constexpr int SG_SMEM = OFF_MISC + 64;
 constexpr uint32_t SG_TMEM_COLS = 256;
-
-size_t surrogate_smem_bytes() { return SG_SMEM; }
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
     return (uint32_t)__cvta_generic_to_shared(p);
@@ -106,7 +108,8 @@ __device__ __forceinline__ void umma_commit(uint64_t *bar) {
                  : "memory");
 }
 
-// 32 consecutive FP32 columns of this thread's TMEM lane
+// 32 consecutive FP32 columns of this thread's TMEM lane; the values are there
+// after tmem_wait
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -118,7 +121,14 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
           "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]),
           "=r"(r[30]), "=r"(r[31])
         : "r"(taddr));
+}
+
+// the loads issued so far have landed: r passes through, so that no use of it
+// moves above the wait
+__device__ __forceinline__ void tmem_wait(uint32_t (&r)[32]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int j = 0; j < 32; j++) asm volatile("" : "+r"(r[j]));
 }
 
 __device__ __forceinline__ float tanh_fast(float x) {
@@ -132,136 +142,132 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
     return *reinterpret_cast<uint32_t *>(&v);
 }
 
-// issue one layer: D[128 x N] = A[128 x K] W^T, W = [N x K]; thread 0 only
-__device__ __forceinline__ void issue_layer(uint32_t d, uint32_t sA, uint32_t sW, int K, int N, uint64_t *bar) {
-    const uint32_t sbo = (uint32_t)(K / 8) * 128u;
-    const uint32_t id = idesc_bf16(SG_M, N);
-    for (int kk = 0; kk < K / 16; kk++) {
-        const uint32_t off = (uint32_t)kk * 256u;          // two 128-byte core matrices along K
-        umma_bf16(d, umma_desc(sA + off, 128u, sbo), umma_desc(sW + off, 128u, sbo), id, kk > 0 ? 1u : 0u);
-    }
+// one layer of K inputs and N outputs: D[128 x N] = A[128 x K] W^T, W = [N x K];
+// one thread issues.  The descriptors' address fields count 16 bytes: 16 further
+// is the next two 128-byte core matrices along K.
+template <int K, int N>
+__device__ __forceinline__ void issue_layer(uint32_t d, uint32_t sA, uint32_t sW, uint64_t *bar) {
+    constexpr uint32_t sbo = (uint32_t)(K / 8) * 128u;
+    const uint64_t da = umma_desc(sA, 128u, sbo), dw = umma_desc(sW, 128u, sbo);
+#pragma unroll
+    for (int kk = 0; kk < K / 16; kk++) umma_bf16(d, da + 16u * kk, dw + 16u * kk, idesc_bf16(SG_M, N), kk > 0 ? 1u : 0u);
     umma_commit(bar);
 }
 
-// block-uniform bounded wait for the next commit of this CTA: at most
-// `polls` try-waits (0: kMbarPolls)
+// hidden layer l's MMAs; the weights' images lie one behind the other
+__device__ __forceinline__ void issue_hidden(int l, uint32_t d, uint32_t sA, uint32_t sW, uint64_t *bar) {
+    tc_fence_after();
+    if (l == 0) issue_layer<SG_KIN, SG_H>(d, sA, sW + OFF_W1, bar);
+    else issue_layer<SG_H, SG_H>(d, sA, sW + (l == 1 ? OFF_W2 : OFF_W3), bar);
+}
+
+__device__ __forceinline__ void issue_output(uint32_t d, uint32_t sA, uint32_t sW, uint64_t *bar) {
+    tc_fence_after();
+    issue_layer<SG_H, SG_NOUT>(d, sA, sW + OFF_W4, bar);
+}
+
+// Each thread's bounded wait for the next commit, at most `polls` try-waits
+// (0: kMbarPolls).  A thread that gives up sets the error, lets the MMAs in
+// flight end (again bounded) and reports false; the caller carries that to its
+// next barrier, where the whole group leaves.  A thread sees the commit itself,
+// so no barrier follows the wait.
 constexpr unsigned int kMbarPolls = 1u << 22;
 __device__ __forceinline__ bool wait_commit(uint64_t *bar, uint32_t &phase, unsigned int *err, unsigned int polls) {
     bool ok = false;
     const unsigned int lim = polls ? polls : kMbarPolls;
-    for (unsigned int it = 0; it < lim; it++)
-        if (mbar_try_wait(bar, phase)) { ok = true; break; }
+    for (unsigned int it = 0; it < lim && !ok; it++) ok = mbar_try_wait(bar, phase);
+    if (!ok) {
+        atomicExch(err, 1u);
+        for (unsigned int it = 0; it < kMbarPolls; it++)
+            if (mbar_try_wait(bar, phase)) break;
+    }
     phase ^= 1u;
-    const int bad = __syncthreads_or(ok ? 0 : 1);
-    if (bad) {
-        if (threadIdx.x == 0) atomicExch(err, 1u);
-        return false;
-    }
+    __syncwarp();
     tc_fence_after();
-    return true;
+    return __all_sync(0xffffffffu, ok);
 }
 
-// hidden-layer epilogue: TMEM -> +bias -> tanh -> BF16 A row (K = 128
-// layout).  Row r's 128 columns are split between the two warps that share
-// its TMEM lane quarter: half h takes columns [64 h, 64 h + 64).
-__device__ __forceinline__ void hidden_epilogue(uint32_t tmem_row, const float *__restrict__ bias, unsigned char *A,
-                                                int r, int half) {
-#pragma unroll 1
-    for (int qq = 0; qq < 2; qq++) {
-        const int q = 2 * half + qq;
-        uint32_t v[32];
-        tmem_ld32(tmem_row + 32u * q, v);
-        uint32_t w[16];
+// Hidden layer l's epilogue: TMEM -> +bias -> tanh -> BF16 A row (K = 128
+// layout) for columns [64 h, 64 h + 64) of row r.  Both 32-column loads go out
+// before the first is used; the biases are kernel parameters, which an add
+// reads as its constant operand.
+__device__ __forceinline__ void hidden_epilogue(const SurrogateAux &x, int l, int h, uint32_t tmem_row,
+                                                unsigned char *A, int r) {
+    uint32_t v[2][32];
+    tmem_ld32(tmem_row + 64u * h, v[0]);
+    tmem_ld32(tmem_row + 64u * h + 32u, v[1]);
+    const float *b = x.b[l] + 64 * h;
+    tmem_wait(v[0]);
+    tmem_wait(v[1]);
 #pragma unroll
-        for (int j = 0; j < 16; j++) {
-            const float a0 = tanh_fast(__uint_as_float(v[2 * j]) + __ldg(bias + 32 * q + 2 * j));
-            const float a1 = tanh_fast(__uint_as_float(v[2 * j + 1]) + __ldg(bias + 32 * q + 2 * j + 1));
-            w[j] = pack_bf16(a0, a1);
-        }
+    for (int c = 0; c < 8; c++) {
+        uint32_t w[4];
 #pragma unroll
-        for (int c = 0; c < 4; c++) {
-            const int chunk = 4 * q + c;
-            uint4 *dst = (uint4 *)(A + ((r >> 3) * (SG_H / 8) + chunk) * 128 + (r & 7) * 16);
-            *dst = make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
+        for (int j = 0; j < 4; j++) {
+            const int k = 8 * c + 2 * j;
+            w[j] = pack_bf16(tanh_fast(__uint_as_float(v[k >> 5][k & 31]) + b[k]),
+                             tanh_fast(__uint_as_float(v[k >> 5][(k & 31) + 1]) + b[k + 1]));
         }
+        uint4 *dst = (uint4 *)(A + ((r >> 3) * (SG_H / 8) + 8 * h + c) * 128 + (r & 7) * 16);
+        *dst = make_uint4(w[0], w[1], w[2], w[3]);
     }
 }
 
-// Ask L2 for the 128-byte lines that build_row will read for tile nt (V,
-// the 18 stored states, G_Ks scale, stimulus heads, node types), one line
-// per thread t of the CTA's second half, so the row build at the end of the
-// current tile finds them in L2.  A hint only; every address is below n.
-__device__ __forceinline__ void prefetch_rows(const SurrogateArgs &a, int nt, int t) {
-    const int base = nt * SG_M;
-    const void *p = nullptr;
-    if (t < 80) {
-        const int arr = t >> 2, off = base + 32 * (t & 3);
-        if (off < a.n) {
-            if (arr == 0) p = a.V + off;
-            else if (arr <= 18) p = a.S + (size_t)(arr - 1) * a.pitch + off;
-            else if (a.gks) p = a.gks + off;
-        }
-    } else if (t < 84) {
-        const int off = base + 32 * (t - 80);
-        if (a.stim_head && off < a.n) p = a.stim_head + off;
-    } else if (t == 84) {
-        if (a.type && base < a.n) p = a.type + base;
-    }
-    if (p) asm volatile("prefetch.L2 [%0];" ::"l"(p));
-}
-
-// One node's input row: features (V, 18 states, I_stim, G_Ks, G_to, s-gate),
-// logarithms of the wide-range ones, normalisation, BF16 row of A (K = 32
-// layout); returns whether the node is inside the training envelope.
-__device__ __forceinline__ bool build_row(const SurrogateArgs &a, const SurrogateAux *aux, long long step, bool raw,
-                                          int i, bool valid, int row, unsigned char *A) {
-    float xn[SG_KIN];
+// One node's input features (V, 18 states, I_stim, G_Ks, G_to, s-gate), or its
+// 32 raw inputs: the loads alone, so that they can be in flight before they
+// are used.  x[19] is the stimulus.
+__device__ __forceinline__ void load_row(const SurrogateArgs &a, long long step, bool raw, int i, bool valid,
+                                         float (&x)[SG_KIN]) {
 #pragma unroll
-    for (int k = 0; k < SG_KIN; k++) xn[k] = 0.f;
-    bool inside = false;
+    for (int k = 0; k < SG_KIN; k++) x[k] = 0.f;
     if (valid && raw) {
 #pragma unroll
-        for (int k = 0; k < SG_KIN; k++) xn[k] = a.rawX[(size_t)i * SG_KIN + k];
+        for (int k = 0; k < SG_KIN; k++) x[k] = a.rawX[(size_t)i * SG_KIN + k];
     } else if (valid) {
-        float x[SG_NF];
+        const int ty = a.type ? a.type[i] : 0;
+        int q = a.stim_head ? a.stim_head[i] : -1;
+        const float gks = a.gks ? a.gks[i] : 1.f;
         x[0] = a.V[i];
 #pragma unroll
         for (int k = 0; k < 18; k++) x[k + 1] = a.S[(size_t)k * a.pitch + i];
-        const int ty = a.type ? a.type[i] : 0;
         const float *c = a.consts + (size_t)ty * a.nconst;
-        float istim = 0.f;
-        if (a.stim_head) {
-            int k = a.stim_head[i];
-            long long best = -1;
-            while (k >= 0) {
-                const long long on = a.stim_on[k], off = a.stim_off[k];
-                if (step >= on && step < off && on > best) { best = on; istim = a.stim_amp[k]; }
-                k = a.stim_next[k];
-            }
-        }
-        x[19] = istim / (a.Cm * a.Xi);
-        x[20] = c[15] * (a.gks ? a.gks[i] : 1.f);
+        x[20] = c[15] * gks;
         x[21] = c[20];
         x[22] = c[53];
-        inside = (istim == 0.f);
+        long long best = -1;
+        while (q >= 0) {
+            const long long on = a.stim_on[q], off = a.stim_off[q];
+            if (step >= on && step < off && on > best) { best = on; x[19] = a.stim_amp[q]; }
+            q = a.stim_next[q];
+        }
+    }
+}
+
+// The row's BF16 form in A (K = 32 layout): logarithms of the wide-range
+// features, normalisation; returns whether the node is inside the training
+// envelope.
+__device__ __forceinline__ bool store_row(const SurrogateArgs &a, bool raw, bool valid, float (&x)[SG_KIN], int row,
+                                          unsigned char *A) {
+    bool inside = false;
+    if (valid && !raw) {
+        inside = (x[19] == 0.f);
+        x[19] = x[19] / (a.Cm * a.Xi);
         const float m = x[7], h = x[8];
-        inside = inside && (m * m * m * h <= aux->nah_max);
-        const unsigned int lm = aux->log_mask;
+        inside = inside && (m * m * m * h <= a.aux.nah_max);
+        const unsigned int lm = a.aux.log_mask;
 #pragma unroll
         for (int k = 0; k < SG_NF; k++) {
             // quantities spanning decades enter as logarithms
             const float xt = ((lm >> k) & 1u) ? __logf(fmaxf(x[k], 1e-30f)) : x[k];
-            inside = inside && (xt >= aux->env_lo[k]) && (xt <= aux->env_hi[k]);
-            xn[k] = (xt - aux->in_mean[k]) * aux->in_rstd[k];
+            inside = inside && (xt >= a.aux.env_lo[k]) && (xt <= a.aux.env_hi[k]);
+            x[k] = (xt - a.aux.in_mean[k]) * a.aux.in_rstd[k];
         }
     }
-    uint32_t w[16];
 #pragma unroll
-    for (int j = 0; j < 16; j++) w[j] = pack_bf16(xn[2 * j], xn[2 * j + 1]);
-#pragma unroll
-    for (int cch = 0; cch < 4; cch++) {
-        uint4 *dst = (uint4 *)(A + ((row >> 3) * (SG_KIN / 8) + cch) * 128 + (row & 7) * 16);
-        *dst = make_uint4(w[4 * cch], w[4 * cch + 1], w[4 * cch + 2], w[4 * cch + 3]);
+    for (int c = 0; c < 4; c++) {
+        uint4 *dst = (uint4 *)(A + ((row >> 3) * (SG_KIN / 8) + c) * 128 + (row & 7) * 16);
+        *dst = make_uint4(pack_bf16(x[8 * c], x[8 * c + 1]), pack_bf16(x[8 * c + 2], x[8 * c + 3]),
+                          pack_bf16(x[8 * c + 4], x[8 * c + 5]), pack_bf16(x[8 * c + 6], x[8 * c + 7]));
     }
     return inside;
 }
@@ -271,19 +277,20 @@ __device__ __forceinline__ bool build_row(const SurrogateArgs &a, const Surrogat
 // k_hybrid), and the nodes outside the envelope or with an output outside
 // its training range appended to the fallback list.  yv: the node's 32
 // output-layer accumulators (bias not yet added).
-__device__ __forceinline__ void output_node(const SurrogateArgs &a, const SurrogateAux *aux, int i, bool valid,
+__device__ __forceinline__ void output_node(const SurrogateArgs &a, int i, bool valid,
                                             bool raw, bool inside, const uint32_t (&yv)[32], double t0,
                                             unsigned int &my_fb) {
+    const SurrogateAux &x = a.aux;
     if (valid && raw) {
 #pragma unroll
-        for (int j = 0; j < SG_NOUT; j++) a.rawY[(size_t)i * SG_NOUT + j] = __uint_as_float(yv[j]) + aux->b4[j];
+        for (int j = 0; j < SG_NOUT; j++) a.rawY[(size_t)i * SG_NOUT + j] = __uint_as_float(yv[j]) + x.b[3][j];
     } else if (valid) {
         // the six concentrations the hybrid form replaces, loaded before
         // any store of this node (the stores below could alias them for
         // the compiler, which would otherwise serialise load and store)
         const int cslot[6] = {0, 1, 2, 9, 16, 17};
         float xs[6];
-        if (aux->v_update == 2) {
+        if (x.v_update == 2) {
 #pragma unroll
             for (int j = 0; j < 6; j++) xs[j] = a.S[(size_t)cslot[j] * a.pitch + i];
         }
@@ -297,20 +304,20 @@ __device__ __forceinline__ void output_node(const SurrogateArgs &a, const Surrog
             // in the hybrid form, every output otherwise) are range-checked and
             // mapped back; the others are never read
             d[j] = 0.f;
-            if ((aux->out_mask >> j) & 1u) {
-                const float u = (__uint_as_float(yv[j]) + aux->b4[j]) * aux->out_std[j] + aux->out_mean[j];
-                out_ok = out_ok && (u >= aux->out_lo[j]) && (u <= aux->out_hi[j]);
-                const float sc = aux->out_scale[j];
+            if ((x.out_mask >> j) & 1u) {
+                const float u = (__uint_as_float(yv[j]) + x.b[3][j]) * x.out_std[j] + x.out_mean[j];
+                out_ok = out_ok && (u >= x.out_lo[j]) && (u <= x.out_hi[j]);
+                const float sc = x.out_scale[j];
                 d[j] = sc > 0.f ? sc * sinhf(fminf(fmaxf(u, -80.f), 80.f)) : u;
             }
         }
-        const unsigned int lm = aux->log_mask;
-        if (aux->v_update == 2) a.take[i] = out_ok ? 1 : 0;
+        const unsigned int lm = x.log_mask;
+        if (x.v_update == 2) a.take[i] = out_ok ? 1 : 0;
         if (!out_ok) {
             const int slot = atomicAdd(a.fallback_count, 1);
             a.fallback_list[slot] = i;
             my_fb++;
-        } else if (aux->v_update == 2) {
+        } else if (x.v_update == 2) {
             // the new concentrations; k_hybrid advances gates and V
 #pragma unroll
             for (int j = 0; j < 6; j++) {
@@ -342,11 +349,18 @@ __device__ __forceinline__ void output_node(const SurrogateArgs &a, const Surrog
     }
 }
 
-// The network over tiles of 128 nodes, 256 threads per CTA.  Threads
-// 0..127 own one node each (features, the output layer, the envelope
-// decision); all eight warps share the hidden-layer epilogues (warp w reads
-// TMEM lane quarter w % 4, column half w / 4).
-__global__ void __launch_bounds__(SG_THREADS, 2) k_surrogate(const SurrogateArgs a) {
+// the weights' global image -> shared memory (already in core-matrix order)
+__device__ __forceinline__ void load_weights(const SurrogateArgs &a, unsigned char *smem) {
+    const uint4 *src = (const uint4 *)a.wimg;
+    uint4 *dst = (uint4 *)smem;
+    for (int k = threadIdx.x; k < SG_WTOT * 2 / 16; k += blockDim.x) dst[k] = __ldg(src + k);
+}
+
+// One tile of 128 nodes per CTA, for the sizes where a tile's chain is all there
+// is: its eight warps share the hidden epilogues (warp w reads TMEM lane quarter
+// w % 4, column half w / 4); threads 0..127 own one node each (features, the
+// output layer, the envelope decision).
+__global__ void __launch_bounds__(SG_THREADS, 1) k_surrogate(const __grid_constant__ SurrogateArgs a) {
     extern __shared__ __align__(1024) unsigned char smem[];
     const int tid = threadIdx.x, warp = tid >> 5;
     const int row = tid & (SG_M - 1), half = tid >> 7;
@@ -354,16 +368,18 @@ __global__ void __launch_bounds__(SG_THREADS, 2) k_surrogate(const SurrogateArgs
     uint64_t *bar = (uint64_t *)(smem + OFF_MISC);
     uint32_t *holder = (uint32_t *)(smem + OFF_MISC + 16);
     unsigned char *A = smem + OFF_A;
-    const SurrogateAux *aux = a.aux;
+    const bool raw = a.rawX != nullptr;
+    const long long step = raw ? 0 : *a.step_ptr;
+    const double t0 = (double)step * a.t_per_step;
+    const int i = (int)blockIdx.x * SG_M + row;
+    const bool valid = owner && i < a.n;
 
-    // weights: global image -> shared (already in core-matrix order)
-    {
-        const uint4 *src = (const uint4 *)a.wimg;
-        uint4 *dst = (uint4 *)smem;
-        for (int i = tid; i < SG_WTOT * 2 / 16; i += blockDim.x) dst[i] = __ldg(src + i);
-    }
+    float x[SG_KIN];
+    if (owner) load_row(a, step, raw, i, valid, x);
+    load_weights(a, smem);
     if (tid == 0) mbar_init(bar, 1);
     if (warp == 0) tmem_alloc(holder, SG_TMEM_COLS);
+    const bool inside = owner && store_row(a, raw, valid, x, row, A);
     fence_proxy_async();
     tc_fence_before();
     __syncthreads();
@@ -371,72 +387,31 @@ __global__ void __launch_bounds__(SG_THREADS, 2) k_surrogate(const SurrogateArgs
     const uint32_t tmem = *holder;
     const uint32_t lane_off = (uint32_t)(32 * (warp & 3)) << 16;
     const uint32_t d_hid = tmem, d_out = tmem + 128u;
-    const uint32_t sW1 = smem_u32(smem + OFF_W1), sW2 = smem_u32(smem + OFF_W2);
-    const uint32_t sW3 = smem_u32(smem + OFF_W3), sW4 = smem_u32(smem + OFF_W4);
-    const uint32_t sA = smem_u32(A);
+    const uint32_t sW = smem_u32(smem), sA = smem_u32(A);
     uint32_t phase = 0;
     unsigned int my_fb = 0;
-    const bool raw = a.rawX != nullptr;
-    const long long step = raw ? 0 : *a.step_ptr;
-    const double t0 = (double)step * a.t_per_step;
-    const int ntiles = (a.n + SG_M - 1) / SG_M;
-
-    // The rows of a tile are built by the owner threads for the first tile,
-    // then by the other half of the CTA while the owners finish the previous
-    // tile's output (A is free once the output layer's MMA has completed).
-    uint8_t *flags = smem + OFF_FLAGS;            // [2][SG_M]: inside the envelope
-    int buf = 0;
-    if (owner && (int)blockIdx.x < ntiles) {
-        const int i0 = (int)blockIdx.x * SG_M + row;
-        flags[row] = build_row(a, aux, step, raw, i0, i0 < a.n, row, A) ? 1 : 0;
-    }
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const int i = tile * SG_M + row;
-        const bool valid = owner && i < a.n;
-        if (!owner && !raw && tile + (int)gridDim.x < ntiles) prefetch_rows(a, tile + (int)gridDim.x, row);
-        // layer 1 (K = 32), 2, 3 (K = 128): hidden, tanh
-        const uint32_t sW[3] = {sW1, sW2, sW3};
-        const float *bias[3] = {aux->b1, aux->b2, aux->b3};
-        bool ok = true;
-#pragma unroll 1
-        for (int l = 0; l < 3 && ok; l++) {
-            fence_proxy_async();
-            tc_fence_before();
-            __syncthreads();
-            if (tid == 0) {
-                tc_fence_after();
-                issue_layer(d_hid, sA, sW[l], l == 0 ? SG_KIN : SG_H, SG_H, bar);
-            }
-            ok = wait_commit(bar, phase, a.err, a.mbar_polls);
-            if (ok) hidden_epilogue(d_hid + lane_off, bias[l], A, row, half);
-        }
-        if (!ok) break;
-        // output layer (K = 128, N = 32)
+    bool ok = true;
+    // A is complete: the next layer's MMAs may go out (false: a wait gave up)
+    auto ready = [&]() -> bool {
         fence_proxy_async();
         tc_fence_before();
-        __syncthreads();
-        if (tid == 0) {
-            tc_fence_after();
-            issue_layer(d_out, sA, sW4, SG_H, SG_NOUT, bar);
+        return !__syncthreads_or(!ok);
+    };
+#pragma unroll 1
+    for (int l = 0; l < 3 && ready(); l++) {
+        if (tid == 0) issue_hidden(l, d_hid, sA, sW, bar);
+        ok = wait_commit(bar, phase, a.err, a.mbar_polls);
+        if (ok) hidden_epilogue(a.aux, l, half, d_hid + lane_off, A, row);
+    }
+    if (ready()) {
+        if (tid == 0) issue_output(d_out, sA, sW, bar);
+        ok = wait_commit(bar, phase, a.err, a.mbar_polls);
+        if (ok && owner) {
+            uint32_t yv[32];
+            tmem_ld32(d_out + lane_off, yv);
+            tmem_wait(yv);
+            output_node(a, i, valid, raw, inside, yv, t0, my_fb);
         }
-        if (!wait_commit(bar, phase, a.err, a.mbar_polls)) break;
-        if (!owner) {
-            // the next tile's rows (its layer-1 MMA waits for the barrier at
-            // the top of the next iteration)
-            const int nt = tile + (int)gridDim.x;
-            if (nt < ntiles) {
-                const int i1 = nt * SG_M + row;
-                flags[(buf ^ 1) * SG_M + row] = build_row(a, aux, step, raw, i1, i1 < a.n, row, A) ? 1 : 0;
-            }
-            buf ^= 1;
-            continue;
-        }
-        const bool inside = flags[buf * SG_M + row] != 0;
-        buf ^= 1;
-        uint32_t yv[32];
-        tmem_ld32(d_out + lane_off, yv);
-        tc_fence_before();
-        output_node(a, aux, i, valid, raw, inside, yv, t0, my_fb);
     }
     // count fallback node-steps
     for (int o = 16; o > 0; o >>= 1) my_fb += __shfl_xor_sync(0xffffffffu, my_fb, o);
@@ -453,9 +428,8 @@ __global__ void __launch_bounds__(SG_THREADS, 2) k_surrogate(const SurrogateArgs
 // columns [128 g, 128 g + 128) (the output layer reuses the first 32 once the
 // last hidden epilogue has read them), an mbarrier and a named barrier; it
 // runs its tiles start to end -- row build, four MMA layers, output --
-// while the other three do the same, so four tiles are in flight per SM
-// against two with k_surrogate, with one copy of the weights (80 KB) instead
-// of two.  Each thread owns one node of its slot's tile and its whole row in
+// while the other three do the same, so four tiles' chains are in flight per
+// SM with one copy of the weights (80 KB).  Each thread owns one node of its slot's tile and its whole row in
 // the hidden epilogues.  Same instructions per tile, same results.
 constexpr int SG4_SLOTS = 4;
 constexpr int SG4_THREADS = SG4_SLOTS * SG_M;
@@ -464,8 +438,7 @@ constexpr int OFF4_MISC = OFF4_A + SG4_SLOTS * SG_M * SG_H * 2;
 constexpr int SG4_SMEM = OFF4_MISC + 128;
 constexpr uint32_t SG4_TMEM_COLS = 512;
 
-// named barrier `id` over the 128 threads of one warpgroup
-__device__ __forceinline__ void wg_sync(int id) { asm volatile("bar.sync %0, 128;" ::"r"(id) : "memory"); }
+// whether any of a warpgroup's 128 threads says so: a barrier (named `id`) too
 __device__ __forceinline__ bool wg_any(bool pred, int id) {
     uint32_t r;
     asm volatile(
@@ -479,23 +452,7 @@ __device__ __forceinline__ bool wg_any(bool pred, int id) {
     return r != 0;
 }
 
-// wait_commit for one warpgroup (bounded, warpgroup-uniform)
-__device__ __forceinline__ bool wait_commit_wg(uint64_t *bar, uint32_t &phase, unsigned int *err, unsigned int polls,
-                                               int id) {
-    bool ok = false;
-    const unsigned int lim = polls ? polls : kMbarPolls;
-    for (unsigned int it = 0; it < lim; it++)
-        if (mbar_try_wait(bar, phase)) { ok = true; break; }
-    phase ^= 1u;
-    if (wg_any(!ok, id)) {
-        if ((threadIdx.x & (SG_M - 1)) == 0) atomicExch(err, 1u);
-        return false;
-    }
-    tc_fence_after();
-    return true;
-}
-
-__global__ void __launch_bounds__(SG4_THREADS, 1) k_surrogate4(const SurrogateArgs a) {
+__global__ void __launch_bounds__(SG4_THREADS, 1) k_surrogate4(const __grid_constant__ SurrogateArgs a) {
     extern __shared__ __align__(1024) unsigned char smem[];
     const int tid = threadIdx.x, warp = tid >> 5;
     const int g = tid >> 7, row = tid & (SG_M - 1);
@@ -503,15 +460,21 @@ __global__ void __launch_bounds__(SG4_THREADS, 1) k_surrogate4(const SurrogateAr
     uint64_t *bars = (uint64_t *)(smem + OFF4_MISC);
     uint32_t *holder = (uint32_t *)(smem + OFF4_MISC + 64);
     unsigned char *A = smem + OFF4_A + (size_t)g * SG_M * SG_H * 2;
-    const SurrogateAux *aux = a.aux;
-    {
-        const uint4 *src = (const uint4 *)a.wimg;
-        uint4 *dst = (uint4 *)smem;
-        for (int k = tid; k < SG_WTOT * 2 / 16; k += blockDim.x) dst[k] = __ldg(src + k);
-    }
+    const bool raw = a.rawX != nullptr;
+    const long long step = raw ? 0 : *a.step_ptr;
+    const double t0 = (double)step * a.t_per_step;
+    const int ntiles = (a.n + SG_M - 1) / SG_M;
+    // a CTA's slots take tiles a grid apart, so that the last tiles spread over
+    // the SMs instead of filling the slots of a few
+    const int first = (int)blockIdx.x + (int)gridDim.x * g, stride = (int)gridDim.x * SG4_SLOTS;
+    float x[SG_KIN];
+    bool inside = false;
+    load_row(a, step, raw, first * SG_M + row, first * SG_M + row < a.n, x);
+    load_weights(a, smem);
     if (tid == 0)
         for (int k = 0; k < SG4_SLOTS; k++) mbar_init(bars + k, 1);
     if (warp == 0) tmem_alloc(holder, SG4_TMEM_COLS);
+    inside = store_row(a, raw, first * SG_M + row < a.n, x, row, A);
     fence_proxy_async();
     tc_fence_before();
     __syncthreads();
@@ -519,45 +482,40 @@ __global__ void __launch_bounds__(SG4_THREADS, 1) k_surrogate4(const SurrogateAr
     const uint32_t tmem = *holder;
     const uint32_t lane_off = (uint32_t)(32 * (warp & 3)) << 16;
     const uint32_t d_acc = tmem + 128u * (uint32_t)g;
-    const uint32_t sW[4] = {smem_u32(smem + OFF_W1), smem_u32(smem + OFF_W2), smem_u32(smem + OFF_W3),
-                            smem_u32(smem + OFF_W4)};
-    const float *bias[3] = {aux->b1, aux->b2, aux->b3};
+    const uint32_t sW = smem_u32(smem);
     const uint32_t sA = smem_u32(A);
     uint64_t *bar = bars + g;
     uint32_t phase = 0;
     unsigned int my_fb = 0;
-    const bool raw = a.rawX != nullptr;
-    const long long step = raw ? 0 : *a.step_ptr;
-    const double t0 = (double)step * a.t_per_step;
-    const int ntiles = (a.n + SG_M - 1) / SG_M;
-    for (int tile = (int)blockIdx.x * SG4_SLOTS + g; tile < ntiles; tile += (int)gridDim.x * SG4_SLOTS) {
-        const int i = tile * SG_M + row;
-        const bool valid = i < a.n;
-        const bool inside = build_row(a, aux, step, raw, i, valid, row, A);
-        bool ok = true;
+    bool ok = true;
+    auto ready = [&]() -> bool {
+        fence_proxy_async();
+        tc_fence_before();
+        return !wg_any(!ok, bid);
+    };
+    for (int tile = first; tile < ntiles; tile += stride) {
+        const int i = tile * SG_M + row, i1 = (tile + stride) * SG_M + row;
 #pragma unroll 1
-        for (int l = 0; l < 4 && ok; l++) {
-            fence_proxy_async();
-            tc_fence_before();
-            wg_sync(bid);
-            if (row == 0) {
-                tc_fence_after();
-                issue_layer(d_acc, sA, sW[l], l == 0 ? SG_KIN : SG_H, l == 3 ? SG_NOUT : SG_H, bar);
-            }
-            ok = wait_commit_wg(bar, phase, a.err, a.mbar_polls, bid);
-            if (ok && l < 3) {
-                hidden_epilogue(d_acc + lane_off, bias[l], A, row, 0);
-                hidden_epilogue(d_acc + lane_off, bias[l], A, row, 1);
-            }
+        for (int l = 0; l < 3 && ready(); l++) {
+            if (row == 0) issue_hidden(l, d_acc, sA, sW, bar);
+            ok = wait_commit(bar, phase, a.err, a.mbar_polls);
+#pragma unroll 1
+            for (int h = 0; h < 2 && ok; h++) hidden_epilogue(a.aux, l, h, d_acc + lane_off, A, row);
         }
-        if (!ok) break;
+        if (!ready()) break;
+        if (row == 0) issue_output(d_acc, sA, sW, bar);
+        // the next tile's rows are loaded under the output layer's MMA
+        load_row(a, step, raw, i1, i1 < a.n, x);
+        ok = wait_commit(bar, phase, a.err, a.mbar_polls);
+        if (!ok) continue;
         uint32_t yv[32];
         tmem_ld32(d_acc + lane_off, yv);
+        tmem_wait(yv);
         tc_fence_before();
-        output_node(a, aux, i, valid, raw, inside, yv, t0, my_fb);
-        // the next tile's row build overwrites A: every thread of the slot
-        // is past its last read of this tile's TMEM and A above
-        wg_sync(bid);
+        output_node(a, i, i < a.n, raw, inside, yv, t0, my_fb);
+        // the output layer's MMA has read A; the next MMA overwrites the
+        // accumulator after the barrier in front of it
+        inside = store_row(a, raw, i1 < a.n, x, row, A);
     }
     for (int o = 16; o > 0; o >>= 1) my_fb += __shfl_xor_sync(0xffffffffu, my_fb, o);
     if ((tid & 31) == 0 && my_fb && a.status) atomicAdd(&a.status->fallback, (unsigned long long)my_fb);
@@ -571,11 +529,11 @@ __global__ void __launch_bounds__(SG4_THREADS, 1) k_surrogate4(const SurrogateAr
 // gate update and current balance over the sub-steps, with the six
 // concentrations moving from their start to the network's end values
 // (geometrically for the log-scaled Cai and Cass).  One thread per node.
-__global__ void __launch_bounds__(128, 4) k_hybrid(const SurrogateArgs a) {
-    const SurrogateAux *aux = a.aux;
+__global__ void __launch_bounds__(128, 4) k_hybrid(const __grid_constant__ SurrogateArgs a) {
+    const SurrogateAux &x = a.aux;
     const long long step = *a.step_ptr;
     const double t0 = (double)step * a.t_per_step;
-    const unsigned int lm = aux->log_mask;
+    const unsigned int lm = x.log_mask;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x) {
         if (!a.take[i]) continue;
         float s[18], c0[6], c1[6];
@@ -594,13 +552,13 @@ __global__ void __launch_bounds__(128, 4) k_hybrid(const SurrogateArgs a) {
         bool dirty = false;
         const bool trk = a.track != nullptr;
         if (trk) tr = a.track[i];
-        const int ns = aux->hyb_sub > 0 ? aux->hyb_sub : a.nsub;
+        const int ns = x.hyb_sub > 0 ? x.hyb_sub : a.nsub;
         const float hu = (float)a.t_per_step / (float)ns;
         const float rdt = 1.f / (float)a.t_per_step;
         float V = a.V[i], tsum = 0.f;
         double tsub = t0;
         for (int k = 0; k < ns; k++) {
-            const float h = aux->hyb_sub > 0 ? hu : a.sub_dt[k];
+            const float h = x.hyb_sub > 0 ? hu : a.sub_dt[k];
             tts::tt_gate_step(s, V, h, c);
             tsum += h;
             const float w = fminf(tsum * rdt, 1.f);
@@ -621,25 +579,26 @@ __global__ void __launch_bounds__(128, 4) k_hybrid(const SurrogateArgs a) {
     }
 }
 
-// variant 0: k_surrogate, two CTAs of one tile pipeline per SM; 1:
-// k_surrogate4, one CTA of four tile pipelines per SM
+// variant 0: the faster kernel for the size.  Up to one tile an SM a tile's
+// chain is all there is, and it is shorter in k_surrogate, where eight warps
+// share an epilogue (1.5 us of 40 a step at 1.5K-10K nodes, equal at 19K);
+// beyond, chains in flight count: against two CTAs an SM of one chain each, four
+// chains took the ionic phase of 46K nodes from 51.8 to 47.6 us, of 263K from
+// 106 to 91, of 765K from 222 to 193.  1: k_surrogate4 at every size.
 int launch_surrogate(const SurrogateArgs &a, cudaStream_t s, int variant) {
-    // the shared-memory limit is per kernel and per device; setting it again
-    // is cheap and keeps a second device right
-    if (variant == 1)
-        EP_CUDA(cudaFuncSetAttribute(k_surrogate4, cudaFuncAttributeMaxDynamicSharedMemorySize, SG4_SMEM));
-    else
-        EP_CUDA(cudaFuncSetAttribute(k_surrogate, cudaFuncAttributeMaxDynamicSharedMemorySize, SG_SMEM));
     int dev = 0, nsm = 148;
     EP_CUDA(cudaGetDevice(&dev));
     EP_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     const int ntiles = (a.n + SG_M - 1) / SG_M;
     if (ntiles <= 0) return EP_OK;
-    if (variant == 1) {
-        const int want = (ntiles + SG4_SLOTS - 1) / SG4_SLOTS;
-        k_surrogate4<<<want < nsm ? want : nsm, SG4_THREADS, SG4_SMEM, s>>>(a);
+    // the shared-memory limit is per kernel and per device; setting it again
+    // is cheap and keeps a second device right
+    if (variant == 1 || ntiles > nsm) {
+        EP_CUDA(cudaFuncSetAttribute(k_surrogate4, cudaFuncAttributeMaxDynamicSharedMemorySize, SG4_SMEM));
+        k_surrogate4<<<ntiles < nsm ? ntiles : nsm, SG4_THREADS, SG4_SMEM, s>>>(a);
     } else {
-        k_surrogate<<<ntiles < 2 * nsm ? ntiles : 2 * nsm, SG_THREADS, SG_SMEM, s>>>(a);
+        EP_CUDA(cudaFuncSetAttribute(k_surrogate, cudaFuncAttributeMaxDynamicSharedMemorySize, SG_SMEM));
+        k_surrogate<<<ntiles, SG_THREADS, SG_SMEM, s>>>(a);
     }
     EP_CUDA(cudaGetLastError());
     return EP_OK;

@@ -19,9 +19,9 @@ constexpr int SG_W3 = SG_H * SG_H;
 constexpr int SG_W4 = SG_NOUT * SG_H;
 constexpr int SG_WTOT = SG_W1 + SG_W2 + SG_W3 + SG_W4;   // 40960 bf16 = 80 KB
 
-// FP32 side parameters (device, global memory)
+// FP32 side parameters, passed with the launch: constant operands in the kernels
 struct SurrogateAux {
-    float b1[SG_H], b2[SG_H], b3[SG_H], b4[SG_NOUT];
+    float b[4][SG_H];           // biases (the output layer's first SG_NOUT)
     float in_mean[SG_KIN], in_rstd[SG_KIN];
     float out_mean[SG_NOUT], out_std[SG_NOUT];
     float out_scale[SG_NOUT];   // > 0: output j is asinh(delta / out_scale[j])
@@ -59,7 +59,7 @@ struct SurrogateArgs {
     float Cm, Xi, act_thr;
     Track *track;
     const unsigned short *wimg;         // SG_WTOT bf16 (core-matrix images W1|W2|W3|W4)
-    const SurrogateAux *aux;
+    SurrogateAux aux;
     int *fallback_list, *fallback_count;
     DevStatus *status;
     unsigned int *err;                  // set when an in-kernel wait gave up
@@ -73,8 +73,9 @@ struct SurrogateArgs {
     uint8_t *take;
 };
 
+static_assert(sizeof(SurrogateArgs) <= 4096, "a kernel's parameters");
+
 int launch_surrogate(const SurrogateArgs &a, cudaStream_t s, int variant = 0);
 int launch_hybrid(const SurrogateArgs &a, cudaStream_t s);
-size_t surrogate_smem_bytes();
 
 }  // namespace ep
