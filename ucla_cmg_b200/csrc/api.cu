@@ -559,10 +559,11 @@ static int plan_cg(ep_handle *h) {
     const int ws = stage_depth(h);
     int rc;
     h->cg = CgShape{h->cg_batch, h->cg_block, 0, 0, 0, 0, 1.0f};
+    const long long all_cols = (long long)(h->col.bytes / sizeof(int)) / kSlice;      // of the matrix's slices
     if (h->cg_per_sm == 0) {
         rc = h->precision == EP_FP64
-                 ? cg_auto_shape<double>(h->nslices, h->ninst, h->cg_batch, h->cg_variant, ws, &h->cg)
-                 : cg_auto_shape<float>(h->nslices, h->ninst, h->cg_batch, h->cg_variant, ws, &h->cg);
+                 ? cg_auto_shape<double>(h->nslices, all_cols, h->ninst, h->cg_batch, h->cg_variant, ws, &h->cg)
+                 : cg_auto_shape<float>(h->nslices, all_cols, h->ninst, h->cg_batch, h->cg_variant, ws, &h->cg);
         h->cg_grid = h->cg.grid;
     } else {
         rc = h->precision == EP_FP64
@@ -592,7 +593,7 @@ static int plan_cg(ep_handle *h) {
             const int all = div_up(h->inst_row[k + 1], kSlice) - h->inst_row[k] / kSlice;
             ns = std::max(ns, div_up(all, h->inst_blk[k + 1] - h->inst_blk[k]));
         }
-        const int cols = div_up((long long)(h->col.bytes / sizeof(int)), (long long)kSlice * h->nslices);
+        const int cols = (int)div_up(all_cols, (long long)h->nslices);
         rc = h->precision == EP_FP64 ? cg_fit_smem<double>(ns, cols, &h->cg) : cg_fit_smem<float>(ns, cols, &h->cg);
         if (rc) return rc;
     }

@@ -75,15 +75,10 @@ __device__ __forceinline__ void own_store(const CGArgs<R> &a, int i, R p, R q, R
     a.po[i] = p; a.qo[i] = q; a.dc[i] = d;
 }
 
-// One row of a sweep, with u = A z' of it: the new vectors (see the top), and
-// its terms of the seven sums.
+// A row's terms of the seven sums (see the top).
 template <typename R>
-__device__ __forceinline__ void sweep_row(const CGArgs<R> &a, R *nxt, int row, R di, const Pair<R> &t, const Own<R> &o,
-                                          R u, R al, R be, double (&v)[7]) {
-    const R z = fma(-al, t.w, t.z), p = fma(be, o.p, z), q = fma(be, o.q, u), w = di * q;
-    pair_store(nxt, row, z, w);
-    own_store(a, row, p, q, fma(al, o.p, o.d));
-    const double d = (double)(R(1) / di), dz = d * (double)z, dw = d * (double)w;
+__device__ __forceinline__ void row_sums(double d, R z, R w, R p, R q, double (&v)[7]) {
+    const double dz = d * (double)z, dw = d * (double)w;
     v[0] += (double)p * (double)q;
     v[1] += dz * (double)z;
     v[2] += dz * (double)w;
@@ -91,6 +86,16 @@ __device__ __forceinline__ void sweep_row(const CGArgs<R> &a, R *nxt, int row, R
     v[4] += dz * dz;
     v[5] += dz * dw;
     v[6] += dw * dw;
+}
+
+// One row of a sweep, with u = A z' of it: the new vectors and the sums.
+template <typename R>
+__device__ __forceinline__ void sweep_row(const CGArgs<R> &a, R *nxt, int row, R di, const Pair<R> &t, const Own<R> &o,
+                                          R u, R al, R be, double (&v)[7]) {
+    const R z = fma(-al, t.w, t.z), p = fma(be, o.p, z), q = fma(be, o.q, u), w = di * q;
+    pair_store(nxt, row, z, w);
+    own_store(a, row, p, q, fma(al, o.p, o.d));
+    row_sums((double)(R(1) / di), z, w, p, q, v);
 }
 
 // ---- grid barrier and reduction in one ----
@@ -121,18 +126,11 @@ __device__ __forceinline__ void slot_load(const CgSlot *p, double &v, unsigned l
 }
 __device__ __forceinline__ void fence_acq_rel_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 
-// NV <= 8 sums over the CTAs [b0, b0 + nb) of a group, the same bits in every
-// thread of every CTA, and a barrier between what the group wrote before and
-// what it reads after.  false: a wait gave up, here or (ok false) before.
+// A warp's sums of NV <= 8 values: each step halves the values a lane carries, so
+// lane l ends with value l / 4 (18 shuffles for 8 FP64 sums instead of 80).
 template <int NV>
-__device__ __forceinline__ bool group_reduce(CgSlot *slots, int G, unsigned long long tag, int b0, int nb,
-                                             unsigned int hold, GridBarrier *bar, const double (&vin)[NV],
-                                             double (&tot)[NV], bool ok = true) {
-    static_assert(NV <= kRedMax, "too many values");
-    __shared__ double sh_a[32][kRedMax], sh_b[32][kRedMax];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
-    // a warp's sums: each step halves the values a lane carries, so lane l
-    // ends with value l / 4 (18 shuffles for 8 FP64 sums instead of 80)
+__device__ __forceinline__ double warp_sums(const double (&vin)[NV]) {
+    const int lane = threadIdx.x & 31;
     double v[kRedMax];
 #pragma unroll
     for (int k = 0; k < kRedMax; k++) v[k] = k < NV ? vin[k < NV ? k : 0] : 0.0;
@@ -148,16 +146,31 @@ __device__ __forceinline__ bool group_reduce(CgSlot *slots, int G, unsigned long
     }
     v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
     v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
-    if ((lane & 3) == 0) sh_a[warp][lane >> 2] = v[0];
+    return v[0];
+}
+// value lane & 7 summed over the rows of a [rows][8] array, on every lane
+__device__ __forceinline__ double column_sum(const double (*sh)[kRedMax], int rows) {
+    const int lane = threadIdx.x & 31;
+    double t = 0.0;
+    for (int r = lane >> 3; r < rows; r += 4) t += sh[r][lane & 7];
+    t += __shfl_xor_sync(0xffffffffu, t, 8);
+    t += __shfl_xor_sync(0xffffffffu, t, 16);
+    return t;
+}
+
+// NV <= 8 sums over the CTAs [b0, b0 + nb) of a group, the same bits in every
+// thread of every CTA, and a barrier between what the group wrote before and
+// what it reads after.  false: a wait gave up, here or (ok false) before.
+template <int NV>
+__device__ __forceinline__ bool group_reduce(CgSlot *slots, int G, unsigned long long tag, int b0, int nb,
+                                             unsigned int hold, GridBarrier *bar, const double (&vin)[NV],
+                                             double (&tot)[NV], bool ok = true) {
+    static_assert(NV <= kRedMax, "too many values");
+    __shared__ double sh_a[32][kRedMax], sh_b[32][kRedMax];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+    const double own = warp_sums(vin);
+    if ((lane & 3) == 0) sh_a[warp][lane >> 2] = own;
     __syncthreads();
-    // value lane & 7 summed over the rows of a [rows][8] array, on every lane
-    auto column_sum = [&](const double (*sh)[kRedMax], int rows) {
-        double t = 0.0;
-        for (int r = lane >> 3; r < rows; r += 4) t += sh[r][lane & 7];
-        t += __shfl_xor_sync(0xffffffffu, t, 8);
-        t += __shfl_xor_sync(0xffffffffu, t, 16);
-        return t;
-    };
     double t;
     if (nb == 1 && !hold) {
         t = column_sum(sh_a, nw);
@@ -598,28 +611,24 @@ __device__ __forceinline__ CgShare cg_share(const CGArgs<R> &a) {
 // The end of a solve: V + its correction (alpha p of the last step added),
 // which is also the next solve's predictor (own rows), and the statistics.
 template <typename R>
-__device__ __forceinline__ void cg_finish(const CGArgs<R> &a, const CgShare &sh, int warp, int nw, int lane,
-                                          const R *cur, R al, R be, bool converged, unsigned long long tag, int it,
-                                          double rr, double rr0) {
-    for (int s = sh.s0 + warp; s < sh.s1; s += nw) {
-        const int row = s * kSlice + lane;
-        if (row >= sh.rb && row < sh.re) {
-            const Pair<R> t = pair_load(cur, row);
-            const Own<R> o = own_load(a, row);
-            R dn = fma(al, o.p, o.d);
-            // FP32, which stops at the resolution of b: one more step for
-            // free, the next iteration's direction taken with this iteration's
-            // length (successive lengths differ by a few percent on these
-            // mass-dominated systems, so it lowers the error 2-3 fold, as the
-            // iteration itself would).  FP64 keeps the reference's iterate.
-            if (sizeof(R) == 4 && converged) dn = fma(al, fma(be, o.p, fma(-al, t.w, t.z)), dn);
-            a.x[row] += dn;
-            if (a.delta) {
-                if (a.dext) a.dext[row] = R(2) * dn - a.delta[row];     // the next solve's start: 2 delta - delta_prev
-                a.delta[row] = dn;
-            }
-        }
+__device__ __forceinline__ void finish_row(const CGArgs<R> &a, int row, const Pair<R> &t, const Own<R> &o, R al, R be,
+                                           bool converged) {
+    R dn = fma(al, o.p, o.d);
+    // FP32, which stops at the resolution of b: one more step for
+    // free, the next iteration's direction taken with this iteration's
+    // length (successive lengths differ by a few percent on these
+    // mass-dominated systems, so it lowers the error 2-3 fold, as the
+    // iteration itself would).  FP64 keeps the reference's iterate.
+    if (sizeof(R) == 4 && converged) dn = fma(al, fma(be, o.p, fma(-al, t.w, t.z)), dn);
+    a.x[row] += dn;
+    if (a.delta) {
+        if (a.dext) a.dext[row] = R(2) * dn - a.delta[row];     // the next solve's start: 2 delta - delta_prev
+        a.delta[row] = dn;
     }
+}
+template <typename R>
+__device__ __forceinline__ void finish_statistics(const CGArgs<R> &a, const CgShare &sh, bool converged,
+                                                  unsigned long long tag, int it, double rr, double rr0) {
     if ((int)blockIdx.x == sh.b0 && threadIdx.x == 0) {
         a.bar[sh.inst].seq = tag;             // every CTA of the group has read the old one
         atomicAdd(a.iters_total, (unsigned long long)it);
@@ -630,6 +639,16 @@ __device__ __forceinline__ void cg_finish(const CGArgs<R> &a, const CgShare &sh,
             a.last[2 * sh.inst + 1] = rr0 > 0.0 ? sqrt(fmax(rr, 0.0) / rr0) : 0.0;
         }
     }
+}
+template <typename R>
+__device__ __forceinline__ void cg_finish(const CGArgs<R> &a, const CgShare &sh, int warp, int nw, int lane,
+                                          const R *cur, R al, R be, bool converged, unsigned long long tag, int it,
+                                          double rr, double rr0) {
+    for (int s = sh.s0 + warp; s < sh.s1; s += nw) {
+        const int row = s * kSlice + lane;
+        if (row >= sh.rb && row < sh.re) finish_row(a, row, pair_load(cur, row), own_load(a, row), al, be, converged);
+    }
+    finish_statistics(a, sh, converged, tag, it, rr, rr0);
 }
 
 // The solve.  NB: slice columns gathered together (4, 8; 16: 8 with the next
@@ -1068,6 +1087,222 @@ __global__ void __launch_bounds__(512, 1) k_cn_smem(const CGArgs<R> a) {
 }
 
 // ---------------------------------------------------------------------------
+// k_cn_one: the solve on one CTA, for meshes whose matrix fits one SM's shared
+// memory.  There an iteration needs no other memory: the matrix, the gathered z'
+// and the reductions are in shared memory, and a thread keeps the vectors of its
+// NR rows in registers: 715 nodes, 4.3 us an iteration to 2.2 in FP64, 3.3 to 2.1
+// in FP32.  Two CTA barriers stand in for the grid reduction's
+// store, fence and polls.  What is left is a chain of instructions with few warps
+// to hide it, so the matrix lies four columns to a lane's load (values, and byte
+// offsets into z in 16 bits), its slices padded with zeros to whole groups.
+// Same iterates as the other kernels.
+__host__ __device__ constexpr int one_cols(long long cols, int ns) {
+    return (int)((cols + 3 * (long long)ns + 3) / 4 * 4);       // with the padding, at most
+}
+template <typename R> __host__ __device__ constexpr long long one_bytes(long long cols, int ns) {
+    return kSlice * (ns * (long long)sizeof(R) + one_cols(cols, ns) * (2 + (long long)sizeof(R)));
+}
+// the four values of a group, from lane's place in it
+__device__ __forceinline__ void one_values(const float *g, int lane, float (&v)[4]) {
+    const float4 t = reinterpret_cast<const float4 *>(g)[lane];
+    v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+}
+__device__ __forceinline__ void one_values(const double *g, int lane, double (&v)[4]) {
+    const double2 t = reinterpret_cast<const double2 *>(g)[lane], u = reinterpret_cast<const double2 *>(g)[32 + lane];
+    v[0] = t.x; v[1] = t.y; v[2] = u.x; v[3] = u.y;
+}
+__device__ __forceinline__ void one_store(float *g, int lane, const float (&v)[4]) {
+    reinterpret_cast<float4 *>(g)[lane] = make_float4(v[0], v[1], v[2], v[3]);
+}
+__device__ __forceinline__ void one_store(double *g, int lane, const double (&v)[4]) {
+    reinterpret_cast<double2 *>(g)[lane] = make_double2(v[0], v[1]);
+    reinterpret_cast<double2 *>(g)[32 + lane] = make_double2(v[2], v[3]);
+}
+
+// The sums of the CTA's warps, the same bits in every thread, as group_reduce
+// forms them, with one barrier: the partials of two calls in turn have their own
+// places (buf), so a call's are read while the next one's are written.
+template <int NV>
+__device__ __forceinline__ void one_reduce(int buf, const double (&vin)[NV], double (&tot)[NV]) {
+    __shared__ double sh[2][32][kRedMax], sum[32][kRedMax];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const double own = warp_sums(vin);
+    if ((lane & 3) == 0) sh[buf][warp][lane >> 2] = own;
+    __syncthreads();
+    const double t = column_sum(sh[buf], nw);
+    if (lane < kRedMax) sum[warp][lane] = t;
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < NV; k++) tot[k] = sum[warp][k];
+    __syncwarp();
+}
+
+template <typename R, int NR>
+__global__ void __launch_bounds__(512, 1) k_cn_one(const CGArgs<R> a) {
+    extern __shared__ __align__(128) unsigned char cg_sm[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, ns = a.nslices;
+    const CgShare sh = cg_share(a);
+    unsigned long long tag = *(volatile unsigned long long *)&a.bar->seq;
+    const int first = __ldg(a.slice_ptr), cols = (__ldg(a.slice_ptr + ns) - first) / kSlice;
+    // a caller's matrix may be wider than the launch assumed: then it is read
+    // from L2 in every sweep
+    const bool fits = one_bytes<R>(cols, ns) <= a.smem;
+    R *vs = reinterpret_cast<R *>(cg_sm), *zs = vs + (fits ? one_cols(cols, ns) : 0) * kSlice;
+    uint2 *is = reinterpret_cast<uint2 *>(zs + ns * kSlice);     // a lane's four offsets
+    int beg[NR], grp[NR], w[NR], row[NR];     // entries before the slice, its first group, columns
+    bool on[NR];
+    R z[NR], q[NR], wv[NR], p[NR], d[NR], di[NR];
+#pragma unroll
+    for (int k = 0; k < NR; k++) {
+        const int s = warp + k * nw;
+        row[k] = s * kSlice + lane;
+        on[k] = s < ns && row[k] < a.n;
+        beg[k] = grp[k] = w[k] = 0;
+        if (s < ns) {
+            beg[k] = __ldg(a.slice_ptr + s);
+            w[k] = (__ldg(a.slice_ptr + s + 1) - beg[k]) / kSlice;
+            grp[k] = ((beg[k] - first) / kSlice + 3 * s + 3) / 4;
+            zs[row[k]] = on[k] ? a.x[row[k]] : R(0);
+        }
+        di[k] = on[k] ? __ldg(a.dinv + row[k]) : R(1);
+        z[k] = q[k] = wv[k] = p[k] = d[k] = R(0);
+    }
+    __syncthreads();
+    // the row sum of row k, columns in order
+    auto row_sum = [&](int k) {
+        R u = R(0);
+        if (fits) {
+            const R *vp = vs + grp[k] * 4 * kSlice;
+            const uint2 *ip = is + grp[k] * kSlice + lane;
+            const unsigned char *zb = reinterpret_cast<const unsigned char *>(zs);
+#pragma unroll (sizeof(R) == 4 ? 4 : 2)
+            for (int g = 0; 4 * g < w[k]; g++) {
+                const uint2 o = ip[g * kSlice];
+                R v[4];
+                one_values(vp + g * 4 * kSlice, lane, v);
+                const R z0 = *reinterpret_cast<const R *>(zb + (o.x & 0xffffu)), z1 = *reinterpret_cast<const R *>(zb + (o.x >> 16));
+                const R z2 = *reinterpret_cast<const R *>(zb + (o.y & 0xffffu)), z3 = *reinterpret_cast<const R *>(zb + (o.y >> 16));
+                u += v[0] * z0;
+                u += v[1] * z1;
+                u += v[2] * z2;
+                u += v[3] * z3;
+            }
+        } else {
+            for (int c = 0; c < w[k]; c++) {
+                const int e = beg[k] + c * kSlice + lane;
+                u += __ldg(a.Aval + e) * zs[__ldg(a.col + e)];
+            }
+        }
+        return u;
+    };
+    // ---- prologue, as k_cn_half's; the matrix comes in with it ----
+    const bool pred = a.delta != nullptr;
+    double rr0, stop2, rr_last;
+    bool converged;
+    {
+        double v[3] = {0.0, 0.0, 0.0};
+        R ax[NR], bx[NR];
+#pragma unroll
+        for (int k = 0; k < NR; k++) {
+            ax[k] = bx[k] = R(0);
+#pragma unroll 2
+            for (int c = 0; c < w[k]; c += 4) {
+                R av[4], bv[4];
+                int ci[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const int e = beg[k] + (c + j) * kSlice + lane;
+                    const bool in = c + j < w[k];
+                    ci[j] = in ? __ldg(a.col + e) : 0;
+                    av[j] = in ? __ldg(a.Aval + e) : R(0);
+                    bv[j] = in ? __ldg(a.Bval + e) : R(0);
+                }
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const R t = zs[ci[j]];
+                    if (c + j < w[k]) {
+                        ax[k] += av[j] * t;
+                        bx[k] += bv[j] * t;
+                    }
+                }
+                if (fits) {
+                    const int g = grp[k] + c / 4;
+                    constexpr unsigned int S = sizeof(R);
+                    one_store(vs + g * 4 * kSlice, lane, av);
+                    is[g * kSlice + lane] = make_uint2(S * ci[0] | S * ci[1] << 16, S * ci[2] | S * ci[3] << 16);
+                }
+            }
+        }
+        if (pred) {
+            const R *dv0 = a.dext ? a.dext : a.delta;
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < NR; k++)
+                if (on[k]) zs[row[k]] = d[k] = dv0[row[k]];
+            __syncthreads();
+        }
+#pragma unroll
+        for (int k = 0; k < NR; k++) {
+            const R ad = pred ? row_sum(k) : R(0);
+            if (on[k]) {
+                const R rref = bx[k] - ax[k], r = pred ? rref - ad : rref;
+                z[k] = di[k] * r;
+                v[0] += (double)r * (double)r;
+                v[1] += (double)bx[k] * (double)bx[k];
+                v[2] += (double)rref * (double)rref;
+            }
+        }
+        double t[3];
+        if (a.bar_extra) {                    // arrivals that never come (ep_test_hold_barrier)
+            if (!group_reduce(a.slots, 1, ++tag, 0, 1, a.bar_extra, a.bar, v, t)) return;
+        }
+        one_reduce(0, v, t);
+        rr0 = t[2];
+        stop2 = fmax(a.tol * a.tol * rr0, a.floor_rel * a.floor_rel * t[1]);
+        rr_last = t[0];
+        converged = t[0] <= stop2;
+    }
+    int it = 0;
+    R al = R(0), be = R(0), diag[NR];
+#pragma unroll
+    for (int k = 0; k < NR; k++) diag[k] = R(1) / di[k];
+    while (!converged && it < a.maxit) {
+        double v[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+        for (int k = 0; k < NR; k++)
+            if (on[k]) zs[row[k]] = z[k] = fma(-al, wv[k], z[k]);
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < NR; k++) {
+            const R u = row_sum(k);
+            if (on[k]) {
+                d[k] = fma(al, p[k], d[k]);
+                p[k] = fma(be, p[k], z[k]);
+                q[k] = fma(be, q[k], u);
+                wv[k] = di[k] * q[k];
+                row_sums((double)diag[k], z[k], wv[k], p[k], q[k], v);
+            }
+        }
+        double t[7];
+        one_reduce((it & 1) ^ 1, v, t);
+        // the scalars and tests of k_cn_half
+        if (t[4] <= stop2) { rr_last = t[4]; converged = true; al = R(0); break; }
+        const double alpha = t[1] / t[0], irz = 1.0 / t[1];
+        const double rz = t[1] - 2.0 * alpha * t[2] + alpha * alpha * t[3];
+        rr_last = t[4] - 2.0 * alpha * t[5] + alpha * alpha * t[6];
+        it++;
+        al = (R)alpha;
+        be = (R)(rz * irz);
+        if (!isfinite(rr_last)) break;
+        converged = rr_last <= stop2 && stop2 >= 1e-12 * t[4];
+    }
+#pragma unroll
+    for (int k = 0; k < NR; k++)
+        if (on[k]) finish_row(a, row[k], Pair<R>{z[k], wv[k]}, Own<R>{p[k], q[k], d[k]}, al, be, converged);
+    finish_statistics(a, sh, converged, tag, it, rr_last, rr0);
+}
+
+// ---------------------------------------------------------------------------
 // The same solve by the Chronopoulos-Gear recurrences: one grid barrier per
 // iteration instead of two.  With z = dinv r and w = A z,
 //   gamma = (r, z), delta = (z, w)                 (one reduction)
@@ -1286,8 +1521,10 @@ int cg_max_per_sm(int block, int *per, int batch, int variant, int depth) {
 // cg_block 256, cg_batch 4 and cg_variant 0, and of ep_cn_half_step_noalloc.
 // No more CTAs than there are slices for, since every CTA takes part in each
 // iteration's reduction (measured: CG us a step, two solves, 16-30 iterations):
-//   FP32 up to 32 slices: k_cn_half on one CTA, whose reductions need no global
-//     memory (715 nodes: 74 us; FP64 takes k_cn_smem, 143 against 209);
+//   up to 64 slices, where the matrix fits one SM: k_cn_one, whose iterations
+//     need no global memory (FP32 / FP64: 280 nodes 33 / 49 us, with the other
+//     kernels 49 / 143; 715 nodes 48 / 76 against 74 / 145; 1200 nodes 58 / 101
+//     against 92 / 149; 1900 nodes FP32 77 against 92);
 //   k_cn_smem where a CTA's share of the matrix stays in shared memory: 256
 //     threads up to 8 slices per SM, one slice per warp (28.6K nodes, FP32 /
 //     FP64: 104 / 182 us; k_cn_half 141 / 245), 512 beyond, one CTA per SM
@@ -1305,17 +1542,35 @@ int cg_max_per_sm(int block, int *per, int batch, int variant, int depth) {
 // from the ring; FP64: 934, 854).
 // Any other launch config, and more instances than those CTAs, run k_cn_half
 // with CTAs of `block` threads, as many as fit.
+// slices a warp of k_cn_one takes (measured for each, FP32 / FP64, CG us a step:
+// 9 slices 33 / 49 with one, 36 / 54 with two; 23 slices 54 / 86, 48 / 76 with
+// two, 50 / 82 with three; 38 slices, three 58 / 101, four 66 / 116: fewer warps
+// shuffle less in the reductions, up to where the rows' own chains add up)
+static int one_rows(int nslices) { return nslices <= 12 ? 1 : nslices <= 32 ? 2 : nslices <= 48 ? 3 : 4; }
 template <typename R>
-int cg_auto_shape(int nslices, int ninst, int batch, int variant, int depth, CgShape *out) {
+static const void *one_kernel(int nslices) {
+    switch (one_rows(nslices)) {
+    case 1: return (const void *)k_cn_one<R, 1>;
+    case 2: return (const void *)k_cn_one<R, 2>;
+    case 3: return (const void *)k_cn_one<R, 3>;
+    default: return (const void *)k_cn_one<R, 4>;
+    }
+}
+
+template <typename R>
+int cg_auto_shape(int nslices, long long cols, int ninst, int batch, int variant, int depth, CgShape *out) {
     int dev = 0, nsm = 0, per = 0;
     EP_CUDA(cudaGetDevice(&dev));
     EP_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     out->batch = batch;
     out->ring_cols = out->smem = 0;
     if (variant == 0 && batch == 4 && out->block == 256 && ninst <= 2 * nsm) {
-        if (ninst == 1 && sizeof(R) == 4 && nslices <= 32) {
-            out->block = std::max(256, nslices * 32);
-            out->grid = 1;
+        if (ninst == 1 && nslices <= 64 && one_bytes<R>(cols, nslices) <= kOneMax) {
+            out->batch = kOneBatch;
+            out->block = 32 * div_up(nslices, one_rows(nslices));
+            out->grid = out->per_sm = 1;
+            out->smem = kOneMax;
+            EP_CUDA(cudaFuncSetAttribute(one_kernel<R>(nslices), cudaFuncAttributeMaxDynamicSharedMemorySize, kOneMax));
             return EP_OK;
         }
         out->batch = kSmemBatch;
@@ -1389,7 +1644,11 @@ int launch_cg(const CGArgs<R> &a, int grid, int block, cudaStream_t s, int batch
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (batch == kSmemBatch) {
+    if (batch == kOneBatch) {
+        cfg.dynamicSmemBytes = a.smem;
+        void *args[] = {const_cast<CGArgs<R> *>(&a)};
+        EP_CUDA(cudaLaunchKernelExC(&cfg, one_kernel<R>(a.nslices), args));
+    } else if (batch == kSmemBatch) {
         cfg.dynamicSmemBytes = a.smem;
         EP_CUDA(cudaLaunchKernelEx(&cfg, k_cn_smem<R>, a));
     } else if (batch == kStagedBatch) {
@@ -1415,8 +1674,8 @@ int launch_cg(const CGArgs<R> &a, int grid, int block, cudaStream_t s, int batch
 
 template int launch_cg<float>(const CGArgs<float> &, int, int, cudaStream_t, int, int);
 template int launch_cg<double>(const CGArgs<double> &, int, int, cudaStream_t, int, int);
-template int cg_auto_shape<float>(int, int, int, int, int, CgShape *);
-template int cg_auto_shape<double>(int, int, int, int, int, CgShape *);
+template int cg_auto_shape<float>(int, long long, int, int, int, int, CgShape *);
+template int cg_auto_shape<double>(int, long long, int, int, int, int, CgShape *);
 template int cg_fit_smem<float>(int, int, CgShape *);
 template int cg_fit_smem<double>(int, int, CgShape *);
 template int cg_grid_size<float>(int, int *, int, int, int, int);

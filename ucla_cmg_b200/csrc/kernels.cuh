@@ -154,6 +154,9 @@ template <typename R> struct CGArgs {
 constexpr int kStagedBatch = 32;
 // the library's own choice (k_cn_smem; not a cg_batch value) and its shared memory at most
 constexpr int kSmemBatch = 64;
+// and of k_cn_one, the solve on one CTA
+constexpr int kOneBatch = 65;
+constexpr int kOneMax = 208 * 1024;
 constexpr int kSmemMax = 216 * 1024;
 constexpr int kStageMaxDepth = 4;
 constexpr int kStageDepthDefault = 2;
@@ -167,7 +170,7 @@ int launch_cg(const CGArgs<R> &a, int grid, int block, cudaStream_t s, int batch
 // and k_cn_smem's sizes (block: the asked size in, the launch's out)
 struct CgShape { int batch, block, grid, per_sm, ring_cols, smem; float keep; };
 template <typename R>
-int cg_auto_shape(int nslices, int ninst, int batch, int variant, int depth, CgShape *out);
+int cg_auto_shape(int nslices, long long cols, int ninst, int batch, int variant, int depth, CgShape *out);
 template <typename R>
 int cg_fit_smem(int ns, int cols, CgShape *out);
 // CTAs of the persistent launch: per_sm (0 = as many as fit) x SM count

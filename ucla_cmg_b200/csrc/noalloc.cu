@@ -87,7 +87,7 @@ int run(unsigned char *base, int n, int nslices, const int *slice_ptr, const int
     // the barrier's tags go on from call to call (the array starts zeroed),
     // and the kernel writes the records before it reads them
     CgShape cg{4, 256, 0, 0, 0, 0, 1.0f};
-    int rc = cg_auto_shape<R>(nslices, 1, 4, 0, 0, &cg);
+    int rc = cg_auto_shape<R>(nslices, 16ll * nslices, 1, 4, 0, 0, &cg);
     // the rows' widths are on the device; 16 columns are a linear-tet mesh's
     // (wider slices only make a share that would stay a ring)
     if (!rc && cg.batch == kSmemBatch) rc = cg_fit_smem<R>(div_up(nslices, cg.grid), 16, &cg);
