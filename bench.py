@@ -237,6 +237,7 @@ def algorithmic_bytes(kernel, n, nnz, cg_iters_per_solve, rbytes, nstate=19, ne=
       prologue  nnz*(A + B + col) + n*(x + dinv read + r, z, p write)
       iteration nnz*(A + col) + n*(z, p_old read + p_new, q write)         [phase A]
                 + n*(p_new, x, r, q, dinv read + x, r, z write)             [phase B]
+        (the textbook schedule's two passes; the kernels' one-pass sweep moves 11 vectors)
       predictor (cg_predict k = 1, 2): n*(the start correction read + V saved)
                 in the prologue (k = 2: the extrapolation the previous solve
                 stored), n*(x, V, k corrections read + x, k corrections

@@ -1464,7 +1464,7 @@ static size_t smem_bytes(int block, int cols, int ns, int rsize) {
 }
 
 // the kernel of a (gather width, variant) choice and its dynamic shared
-// memory; cg_batch kStagedBatch selects k_cn_half_staged with `depth` units
+// memory; cg_batch kStagedBatch selects k_cn_half's staged form with `depth` units
 // in flight per warp (1 .. kStageMaxDepth)
 // (set_attr: allow the staged kernel the largest ring any handle can ask
 // for -- 256 threads, kStageMaxDepth units -- once, from the planning path,
