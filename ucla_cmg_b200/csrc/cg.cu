@@ -982,8 +982,8 @@ __device__ __forceinline__ void mat_slice(MatRing<R> &m, const CGArgs<R> &a, int
     }
 }
 
-template <typename R>
-__global__ void __launch_bounds__(512, 1) k_cn_smem(const CGArgs<R> a) {
+template <typename R, int MAXT>
+__global__ void __launch_bounds__(MAXT, 1) k_cn_smem(const CGArgs<R> a) {
     constexpr int GU = 2;                     // a slice's two units
     extern __shared__ __align__(128) unsigned char cg_sm[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -1471,7 +1471,7 @@ static size_t smem_bytes(int block, int cols, int ns, int rsize) {
 // never during a stream capture; the attribute only caps the request)
 template <typename R>
 static int cg_kernel(int block, int batch, int variant, int depth, const void **fn, size_t *smem,
-                     bool set_attr) {
+                     bool set_attr, int per_sm = 1) {
     *smem = 0;                 // (k_cn_smem: `depth` is its bytes)
     if (batch == kStagedBatch) {
         if (variant != 0) { set_error("the staged CG runs the two-reduction recurrences only"); return EP_ERR_ARG; }
@@ -1487,8 +1487,13 @@ static int cg_kernel(int block, int batch, int variant, int depth, const void **
         return EP_OK;
     }
     if (batch == kSmemBatch) {
-        *fn = (const void *)k_cn_smem<R>;
+        *fn = (const void *)k_cn_smem<R, 512>;
         *smem = (size_t)depth;
+        if constexpr (sizeof(R) == 8) {
+            // alone on its SM with fewer threads FP64 has the registers it needs
+            // (128 spill); a batch's two CTAs share them
+            if (per_sm == 1) *fn = block <= 256 ? (const void *)k_cn_smem<R, 256> : (const void *)k_cn_smem<R, 384>;
+        }
         if (set_attr)
             EP_CUDA(cudaFuncSetAttribute(*fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
         return EP_OK;
@@ -1501,10 +1506,10 @@ static int cg_kernel(int block, int batch, int variant, int depth, const void **
 }
 
 template <typename R>
-int cg_max_per_sm(int block, int *per, int batch, int variant, int depth) {
+int cg_max_per_sm(int block, int *per, int batch, int variant, int depth, int per_sm) {
     const void *fn = nullptr;
     size_t smem = 0;
-    int rc = cg_kernel<R>(block, batch, variant, depth, &fn, &smem, true);
+    int rc = cg_kernel<R>(block, batch, variant, depth, &fn, &smem, true, per_sm);
     if (rc) return rc;
     cudaFuncAttributes fa;
     EP_CUDA(cudaFuncGetAttributes(&fa, fn));
@@ -1525,18 +1530,22 @@ int cg_max_per_sm(int block, int *per, int batch, int variant, int depth) {
 //     need no global memory (FP32 / FP64: 280 nodes 33 / 49 us, with the other
 //     kernels 49 / 143; 715 nodes 48 / 76 against 74 / 145; 1200 nodes 58 / 101
 //     against 92 / 149; 1900 nodes FP32 77 against 92);
-//   k_cn_smem where a CTA's share of the matrix stays in shared memory: 256
-//     threads up to 8 slices per SM, one slice per warp (28.6K nodes, FP32 /
-//     FP64: 104 / 182 us; k_cn_half 141 / 245), 512 beyond, one CTA per SM
-//     (214K nodes FP32: 168 us against 191; 72K FP64: 204 against 258).  FP32
-//     may fill 200 KB with it, FP64 140, whose gathers need the L1 more (143K
-//     nodes: 302 us resident, 287 with k_cn_half);
+//   k_cn_smem where a CTA's share of the matrix stays in shared memory, one CTA
+//     per SM: 256 threads up to 8 slices per SM in FP32 and 6 in FP64 (28.6K
+//     nodes, FP32: 103 us, 109 with 512 threads, 141 with k_cn_half; 14K FP64:
+//     150, 160 with 384, 178 with 256 of 128 registers), beyond it 512 in FP32
+//     (214K nodes: 162 us against 195 with 384 and 191 with k_cn_half) and 384
+//     in FP64, whose 168 registers hold a slice's gathers without spills (34K:
+//     158 us against 199 with 512; 91K: 210 against 260).  FP32 may fill 200 KB
+//     with it, FP64 140, whose gathers need the L1 more;
 //   k_cn_half with 1024 threads per SM where the matrix no longer does but L2
-//     holds it, up to 60 MB (263K FP32: 220 us against 270 from the ring; 500K:
-//     320 against 374; 307K FP64: 578 against 618): twice the warps hide L2's
-//     latency as well, and nothing is copied;
-//   k_cn_smem's ring beyond (765K FP32: 630 us against 748; 500K FP64: 869
-//     against 1183), with 120 KB, which leaves the gathers their L1.
+//     holds it, up to 60 MB in FP32 (263K: 220 us against 270 from the ring;
+//     500K: 320 against 374): twice the warps hide L2's latency as well, and
+//     nothing is copied; in FP64 up to 27 MB (133K: 281 against 310; 153K 370
+//     against 317);
+//   k_cn_smem's ring beyond (765K FP32: 630 us against 748; 306K FP64: 540
+//     against 710; 562K: 869, 973 with 512 threads), with 120 KB, which leaves
+//     the gathers their L1.
 // Batches the same with two CTAs per SM, which split the GPU more evenly
 // between the instances (24 slabs, 446K nodes FP32: 306 us from k_cn_half, 389
 // from the ring; FP64: 934, 854).
@@ -1575,7 +1584,7 @@ int cg_auto_shape(int nslices, long long cols, int ninst, int batch, int variant
         }
         out->batch = kSmemBatch;
         out->per_sm = ninst > 1 ? 2 : 1;
-        out->block = ninst > 1 || nslices <= 8 * nsm ? 256 : 512;
+        out->block = ninst > 1 || nslices <= (sizeof(R) == 4 ? 8 : 6) * nsm ? 256 : sizeof(R) == 4 ? 512 : 384;
         out->grid = std::min(out->per_sm * nsm, div_up(nslices, out->block / 32) + (ninst > 1 ? ninst : 0));
         return EP_OK;
     }
@@ -1603,7 +1612,7 @@ int cg_fit_smem(int ns, int cols, CgShape *out) {
     const int most = sizeof(R) == 4 ? 200 : 140;
     const bool stays = spw * cols <= fit(most);
     const double mb = (double)ns * out->grid * cols * kSlice * (4 + sizeof(R)) / 1e6;      // the matrix
-    if (!stays && mb <= 60.0) {
+    if (!stays && mb <= (sizeof(R) == 8 && out->per_sm == 1 ? 27.0 : 60.0)) {
         out->batch = 4;
         out->block = 1024 / out->per_sm;
         return EP_OK;
@@ -1615,7 +1624,7 @@ int cg_fit_smem(int ns, int cols, CgShape *out) {
     if (out->ring_cols < 2 * kUnitMax) { set_error("CG kernel: %d matrix columns per warp are too few", out->ring_cols); return EP_ERR_ARG; }
     out->smem = (int)smem_bytes(out->block, out->ring_cols, ns, (int)sizeof(R));
     int per = 0;
-    int rc = cg_max_per_sm<R>(out->block, &per, kSmemBatch, 0, out->smem);
+    int rc = cg_max_per_sm<R>(out->block, &per, kSmemBatch, 0, out->smem, out->per_sm);
     if (!rc && per < out->per_sm) { set_error("CG kernel: %d CTAs per SM instead of %d", per, out->per_sm); rc = EP_ERR_CUDA; }
     return rc;
 }
@@ -1650,7 +1659,12 @@ int launch_cg(const CGArgs<R> &a, int grid, int block, cudaStream_t s, int batch
         EP_CUDA(cudaLaunchKernelExC(&cfg, one_kernel<R>(a.nslices), args));
     } else if (batch == kSmemBatch) {
         cfg.dynamicSmemBytes = a.smem;
-        EP_CUDA(cudaLaunchKernelEx(&cfg, k_cn_smem<R>, a));
+        const void *fn = nullptr;
+        size_t smem = 0;
+        int rc = cg_kernel<R>(block, batch, variant, a.smem, &fn, &smem, false, a.ninst > 1 ? 2 : 1);
+        if (rc) return rc;
+        void *args[] = {const_cast<CGArgs<R> *>(&a)};
+        EP_CUDA(cudaLaunchKernelExC(&cfg, fn, args));
     } else if (batch == kStagedBatch) {
         const void *fn = nullptr;
         size_t smem = 0;
@@ -1680,8 +1694,8 @@ template int cg_fit_smem<float>(int, int, CgShape *);
 template int cg_fit_smem<double>(int, int, CgShape *);
 template int cg_grid_size<float>(int, int *, int, int, int, int);
 template int cg_grid_size<double>(int, int *, int, int, int, int);
-template int cg_max_per_sm<float>(int, int *, int, int, int);
-template int cg_max_per_sm<double>(int, int *, int, int, int);
+template int cg_max_per_sm<float>(int, int *, int, int, int, int);
+template int cg_max_per_sm<double>(int, int *, int, int, int, int);
 
 // ---------------------------------------------------------------------------
 // One forward-Euler diffusion sub-step of the explicit scheme

@@ -177,7 +177,7 @@ int cg_fit_smem(int ns, int cols, CgShape *out);
 template <typename R>
 int cg_grid_size(int block, int *grid, int per_sm = 0, int batch = 4, int variant = 0, int depth = 0);
 template <typename R>
-int cg_max_per_sm(int block, int *per, int batch = 4, int variant = 0, int depth = 0);
+int cg_max_per_sm(int block, int *per, int batch = 4, int variant = 0, int depth = 0, int per_sm = 1);
 
 // ECG_k = sum_i W[k n + i] V[i] (ComputeECG.h:172-189 in per-node form) of
 // `frames` voltage fields, n apart, deterministic two-level reduction, written
