@@ -7,7 +7,7 @@ import pytest
 import torch
 
 from ucla_cmg_b200 import capi, mesh as M
-from ucla_cmg_b200.simulation import Monodomain
+from ucla_cmg_b200.simulation import Batch, Monodomain
 
 pytestmark = pytest.mark.gpu
 D = M.sigma_to_D(1.2, 0.2)
@@ -71,3 +71,27 @@ def test_wide_rows(gpu, prec, ty, n, wide):
     # number, below 10 for these three, and FP32's rounding of the same size
     tol = 1e-10 if prec == capi.FP64 else 1e-5
     assert np.linalg.norm(arrays[-1].cpu().numpy() - ref) <= tol * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("prec", [capi.FP64, capi.FP32])
+@pytest.mark.parametrize("count", [2, 37, 38])
+def test_batches_of_few_and_many_instances(gpu, prec, count):
+    """Batches at the edge between one and two CTAs per SM (a quarter as many
+    instances as 148 SMs), uneven instances: each as on its own."""
+    dims = [(5 + k % 7, 4 + k % 5, 4) for k in range(count)]
+    dims[0] = (41, 31, 9)
+    meshes = [M.slab(*d, *(0.02 * (k - 1) for k in d)) for d in dims]
+    rng = np.random.default_rng(count)
+    V = [-85.0 + 120.0 * (m.xyz[:, 0] < m.xyz[:, 0].mean()) + rng.normal(0, 1.0, m.n) for m in meshes]
+    b = Batch([dict(mesh=m, D=D) for m in meshes], capi.TUSSCHER, prec, dt=0.1, ionic_dt=0.02)
+    b.set_voltage(np.concatenate(V))
+    b.diffusion_half_step()
+    got = b.split(b.voltage())
+    b.close()
+    for k in (0, 1, count - 1):
+        g = Monodomain(meshes[k], capi.TUSSCHER, prec, dt=0.1, ionic_dt=0.02, D=D)
+        g.set_launch_config(cg_per_sm=1)
+        g.set_voltage(V[k])
+        g.diffusion_half_step()
+        assert np.max(np.abs(g.voltage() - got[k])) <= TOL[prec] * np.max(np.abs(V[k]))
+        g.close()

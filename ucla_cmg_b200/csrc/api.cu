@@ -350,6 +350,7 @@ void fill_cg_args(ep_handle *h, CGArgs<R> &a) {
     a.depth = stage_depth(h);
     a.ring_cols = h->cg.ring_cols;
     a.smem = h->cg.smem;
+    a.per_sm = h->cg.per_sm;
     a.keep = h->cg.keep;
 }
 

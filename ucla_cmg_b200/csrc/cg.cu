@@ -1548,7 +1548,9 @@ int cg_max_per_sm(int block, int *per, int batch, int variant, int depth, int pe
 //     the gathers their L1.
 // Batches the same with two CTAs per SM, which split the GPU more evenly
 // between the instances (24 slabs, 446K nodes FP32: 306 us from k_cn_half, 389
-// from the ring; FP64: 934, 854).
+// from the ring); in FP64, whose CTAs want the registers, with one up to a
+// quarter as many instances as SMs (24 slabs: 757 us, 849 with two; 8 slabs,
+// 155K nodes: 316, 372; 2 slabs, 15K: 149, 175).
 // Any other launch config, and more instances than those CTAs, run k_cn_half
 // with CTAs of `block` threads, as many as fit.
 // slices a warp of k_cn_one takes (measured for each, FP32 / FP64, CG us a step:
@@ -1583,8 +1585,9 @@ int cg_auto_shape(int nslices, long long cols, int ninst, int batch, int variant
             return EP_OK;
         }
         out->batch = kSmemBatch;
-        out->per_sm = ninst > 1 ? 2 : 1;
-        out->block = ninst > 1 || nslices <= (sizeof(R) == 4 ? 8 : 6) * nsm ? 256 : sizeof(R) == 4 ? 512 : 384;
+        // (FP64 batches keep one CTA per SM while an instance has four SMs or more)
+        out->per_sm = ninst > 1 && (sizeof(R) == 4 || 4 * ninst > nsm) ? 2 : 1;
+        out->block = out->per_sm == 2 || nslices <= (sizeof(R) == 4 ? 8 : 6) * nsm ? 256 : sizeof(R) == 4 ? 512 : 384;
         out->grid = std::min(out->per_sm * nsm, div_up(nslices, out->block / 32) + (ninst > 1 ? ninst : 0));
         return EP_OK;
     }
@@ -1661,7 +1664,7 @@ int launch_cg(const CGArgs<R> &a, int grid, int block, cudaStream_t s, int batch
         cfg.dynamicSmemBytes = a.smem;
         const void *fn = nullptr;
         size_t smem = 0;
-        int rc = cg_kernel<R>(block, batch, variant, a.smem, &fn, &smem, false, a.ninst > 1 ? 2 : 1);
+        int rc = cg_kernel<R>(block, batch, variant, a.smem, &fn, &smem, false, a.per_sm);
         if (rc) return rc;
         void *args[] = {const_cast<CGArgs<R> *>(&a)};
         EP_CUDA(cudaLaunchKernelExC(&cfg, fn, args));

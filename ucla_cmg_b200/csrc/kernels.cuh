@@ -143,8 +143,9 @@ template <typename R> struct CGArgs {
     // staged variant (cg_batch kStagedBatch): units of 8 slice columns each
     // warp keeps in flight in its shared-memory ring (1 .. kStageMaxDepth)
     int depth;
-    // k_cn_smem: matrix columns of a warp's region and the CTA's dynamic shared memory
-    int ring_cols, smem;
+    // k_cn_smem: matrix columns of a warp's region, the CTA's dynamic shared memory
+    // and CTAs per SM
+    int ring_cols, smem, per_sm;
     float keep;                  // share of its slices L2 is asked to keep (1: no hint)
 };
 

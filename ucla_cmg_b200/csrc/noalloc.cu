@@ -94,6 +94,7 @@ int run(unsigned char *base, int n, int nslices, const int *slice_ptr, const int
     if (rc) return rc;
     a.ring_cols = cg.ring_cols;
     a.smem = cg.smem;
+    a.per_sm = cg.per_sm;
     a.keep = cg.keep;
     if ((rc = launch_cg<R>(a, cg.grid, cg.block, s, cg.batch))) return rc;
     // barrier and result in one copy
