@@ -601,7 +601,7 @@ static int plan_cg(ep_handle *h) {
     if ((rc = upload_raw(h->d_inst_row, h->inst_row.data(), h->inst_row.size()))) return rc;
     if ((rc = upload_raw(h->d_inst_blk, h->inst_blk.data(), h->inst_blk.size()))) return rc;
     if (h->cg_variant == 1 && (rc = h->partial.alloc(sizeof(double) * 12 * (size_t)h->cg_grid))) return rc;
-    if ((rc = h->slots.alloc(sizeof(CgSlot) * 16 * (size_t)h->cg_grid))) return rc;
+    if ((rc = h->slots.alloc(sizeof(CgSlot) * 32 * (size_t)h->cg_grid))) return rc;
     EP_CUDA(cudaMemsetAsync(h->slots.p, 0, h->slots.bytes, h->stream));
     if (h->bar.bytes != sizeof(GridBarrier) * (size_t)h->ninst) {
         if ((rc = h->bar.alloc(sizeof(GridBarrier) * (size_t)h->ninst))) return rc;

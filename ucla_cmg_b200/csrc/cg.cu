@@ -158,10 +158,49 @@ __device__ __forceinline__ double column_sum(const double (*sh)[kRedMax], int ro
     return t;
 }
 
+// A group of many CTAs (a launch shape set by the caller): every CTA reading
+// every line is nb^2 reads (1184 CTAs of 128 threads, 28.6K nodes FP32: 670 us
+// of CG a step), so every 32nd CTA adds its 32 lines first and the others read
+// those sums, one more round trip (205 us; 592 of 256 threads 255 -> 183).
+// `lines` lines from `line` on, their sum to `sum`.  Not inlined: its registers
+// are not the sweep's (and the gather width 4 has an instance without it, WIDE
+// false, which 781K nodes run 10 % faster at 148 CTAs).
+constexpr int kRedFlat = 296, kRedGroup = 32;
+__device__ __noinline__ bool add_lines(const CgSlot *line, CgSlot *sum, int lines, int nv, unsigned long long tag,
+                                       GridBarrier *bar, unsigned int lim) {
+    __shared__ double sh[32][kRedMax];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned int polls = 0;
+    int bad = 0;
+    double acc = 0.0;
+    for (int u = threadIdx.x; u < lines * kRedMax && (u & (kRedMax - 1)) < nv && !bad; u += blockDim.x) {
+        double x;
+        unsigned long long t;
+        for (slot_load(line + u, x, t); t != tag; slot_load(line + u, x, t)) {
+            if (++polls > lim) { atomicExch(&bar->err, 1u); bad = 1; break; }
+            if ((polls & 15u) == 0) {
+                if (*(volatile unsigned int *)&bar->err) { bad = 1; break; }
+                __nanosleep(64);
+            }
+        }
+        acc += x;
+    }
+    acc += __shfl_xor_sync(0xffffffffu, acc, 8);
+    acc += __shfl_xor_sync(0xffffffffu, acc, 16);
+    if (lane < kRedMax) sh[warp][lane] = acc;
+    if (__syncthreads_or(bad)) return false;
+    if (warp == 0) {
+        const double t = column_sum(sh, blockDim.x >> 5);
+        fence_acq_rel_gpu();                  // what the CTAs released before their sum's tag
+        if (lane < nv) slot_store(sum + lane, t, tag);
+    }
+    return true;
+}
+
 // NV <= 8 sums over the CTAs [b0, b0 + nb) of a group, the same bits in every
 // thread of every CTA, and a barrier between what the group wrote before and
 // what it reads after.  false: a wait gave up, here or (ok false) before.
-template <int NV>
+template <int NV, bool WIDE = false>
 __device__ __forceinline__ bool group_reduce(CgSlot *slots, int G, unsigned long long tag, int b0, int nb,
                                              unsigned int hold, GridBarrier *bar, const double (&vin)[NV],
                                              double (&tot)[NV], bool ok = true) {
@@ -187,7 +226,18 @@ __device__ __forceinline__ bool group_reduce(CgSlot *slots, int G, unsigned long
         }
         const unsigned int lim = bar->limit ? bar->limit : kGridPolls;
         const CgSlot *grp = set + (size_t)b0 * kRedMax;
-        const int units = nb * kRedMax;
+        int units = nb * kRedMax, every = 1;  // the lines to read, `every` lines apart
+        if (WIDE && nb > kRedFlat) {
+            const int k = (int)blockIdx.x - b0;
+            CgSlot *sums = set + (size_t)2 * G * kRedMax;
+            if (k % kRedGroup == 0 && !add_lines(grp + (size_t)k * kRedMax, sums + (size_t)blockIdx.x * kRedMax,
+                                                 min(kRedGroup, nb - k), NV, tag, bar, lim))
+                return false;
+            grp = sums + (size_t)b0 * kRedMax;
+            units = (nb + kRedGroup - 1) / kRedGroup * kRedMax;
+            every = kRedGroup;
+        }
+        auto unit = [&](int u) { return grp + (WIDE ? u + (u / kRedMax) * (every - 1) * kRedMax : u); };
         const bool mine = (tid & (kRedMax - 1)) < NV;
         unsigned int polls = 0;
         int bad = ok ? 0 : 1;
@@ -207,7 +257,7 @@ __device__ __forceinline__ bool group_reduce(CgSlot *slots, int G, unsigned long
                 double xv[4];
 #pragma unroll
                 for (int i = 0; i < 4; i++)
-                    if (pend >> i & 1u) slot_load(grp + u0 + i * (int)blockDim.x, xv[i], tg[i]);
+                    if (pend >> i & 1u) slot_load(unit(u0 + i * (int)blockDim.x), xv[i], tg[i]);
 #pragma unroll
                 for (int i = 0; i < 4; i++)
                     if ((pend >> i & 1u) && tg[i] == tag) { x[i] = xv[i]; pend &= ~(1u << i); }
@@ -669,7 +719,7 @@ __device__ __forceinline__ void cg_finish(const CGArgs<R> &a, const CgShare &sh,
 // reduction.  No wait on it spins: cp.async.wait_group is the hardware's wait
 // for the thread's own copies, and every exit path waits for all of them.
 // Same order of additions in every form, so the same bits on the same grid.
-template <typename R, int NB>
+template <typename R, int NB, bool WIDE = NB != 4>
 __global__ void __launch_bounds__(NB == 4 ? 1024 : 256, NB == 4 ? 1 : (NB == kStagedBatch && sizeof(R) == 8) ? 3 : 4)
 k_cn_half(const CGArgs<R> a) {
     constexpr bool STAGED = NB == kStagedBatch;
@@ -723,7 +773,7 @@ k_cn_half(const CGArgs<R> a) {
             }
         }
         double t[3];
-        if (!group_reduce(a.slots, G, ++tag, b0, nb, a.bar_extra, bar, v, t)) {
+        if (!group_reduce<3, WIDE>(a.slots, G, ++tag, b0, nb, a.bar_extra, bar, v, t)) {
             if constexpr (STAGED) cp_wait_all();
             return;
         }
@@ -753,7 +803,7 @@ k_cn_half(const CGArgs<R> a) {
                 sweep_row(a, nxt, row, __ldg(a.dinv + row), pair_load(cur, row), own_load(a, row), u, al, be, v);
         }
         double t[7];
-        if (!group_reduce(a.slots, G, ++tag, b0, nb, a.bar_extra, bar, v, t)) {
+        if (!group_reduce<7, WIDE>(a.slots, G, ++tag, b0, nb, a.bar_extra, bar, v, t)) {
             if constexpr (STAGED) cp_wait_all();
             return;
         }
@@ -1501,7 +1551,7 @@ static int cg_kernel(int block, int batch, int variant, int depth, const void **
     *fn = variant == 1 ? (batch >= 8 ? (const void *)k_cn_half_cg1<R, 8> : (const void *)k_cn_half_cg1<R, 4>)
           : batch == 8 ? (const void *)k_cn_half<R, 8>
           : batch == 16 ? (const void *)k_cn_half<R, 16>
-                        : (const void *)k_cn_half<R, 4>;
+                        : (const void *)k_cn_half<R, 4, true>;
     return EP_OK;
 }
 
@@ -1683,8 +1733,10 @@ int launch_cg(const CGArgs<R> &a, int grid, int block, cudaStream_t s, int batch
         EP_CUDA(cudaLaunchKernelEx(&cfg, k_cn_half<R, 8>, a));
     } else if (batch == 16) {
         EP_CUDA(cudaLaunchKernelEx(&cfg, k_cn_half<R, 16>, a));
+    } else if (grid > kRedFlat) {
+        EP_CUDA(cudaLaunchKernelEx(&cfg, k_cn_half<R, 4, true>, a));
     } else {
-        EP_CUDA(cudaLaunchKernelEx(&cfg, k_cn_half<R, 4>, a));
+        EP_CUDA(cudaLaunchKernelEx(&cfg, k_cn_half<R, 4, false>, a));
     }
     return EP_OK;
 }

@@ -110,7 +110,8 @@ template <typename R> struct CGArgs {
     R *x;
     R *q0, *q1;                  // two buffers of 2 * pitch: (z, w) per node (16-byte aligned)
     R *po, *qo, *dc;             // p, A p and the correction of the own rows
-    CgSlot *slots;               // 2 sets x grid x 8 reduction units (zeroed before the first launch)
+    CgSlot *slots;               // 2 sets x grid x 8 reduction units, and as many of groups of CTAs (zeroed
+                                 // before the first launch)
     GridBarrier *bar;
     double tol;
     double floor_rel;            // stop also when ||r|| <= floor_rel ||B x||
