@@ -330,7 +330,10 @@ int  ep_assemble_operators(const ep_mesh_desc *mesh, const ep_cables_desc *cable
  * per CTA of the persistent CG launch (128, 256, 512 or 768); cg_per_sm: its CTAs per
  * SM (0 = by the size of the mesh: no more CTAs than it has slices for, and for
  * cg_block 256 with cg_batch 4 one CTA of up to 1024 threads per SM on large
- * meshes, since every CTA takes part in each iteration's reduction); ionic_block: threads per CTA of the
+ * meshes, since every CTA takes part in each iteration's reduction; otherwise
+ * at most as many as the kernel's registers let reside, e.g. with cg_batch 8,
+ * 16 or 32 and cg_block 256 three in FP32 and two in FP64); ionic_block:
+ * threads per CTA of the
  * ionic kernel (64 or 128); graph_steps: 0 launches every kernel from the
  * host, k > 0 replays the steps from an instantiated CUDA graph of k steps
  * (rounded up to a multiple of the ECG interval); ionic_min_ctas: FP32

@@ -703,8 +703,12 @@ __device__ __forceinline__ void cg_finish(const CGArgs<R> &a, const CgShare &sh,
 
 // The solve.  NB: slice columns gathered together (4, 8; 16: 8 with the next
 // group's indices and values loaded ahead; kStagedBatch: 8 out of a shared-
-// memory ring, below).  64 registers in all of them, so one CTA of up to 1024
-// threads (NB = 4) or four of 256 per SM.
+// memory ring, below).  NB = 4 has 64 registers, so one CTA of up to 1024
+// threads per SM; the others, whose gathered values spill in 64, three of 256
+// threads in FP32 (80 registers) and two in FP64 (128).  CG us a step of width
+// 8 / 16 / staged, with four CTAs (64 registers; FP64 staged three) and now:
+// FP32 214K nodes 248 / 307 / 314 -> 206 / 239 / 266, 781K 766 / 820 / 796 ->
+// 760 / 792 / 694; FP64 214K 590 / 833 / 607 -> 361 / 385 / 389.
 //
 // The staged form takes the matrix stream of the sweeps off the warps'
 // critical path.  A warp's slices are cut into units of kUnitCols slice
@@ -720,7 +724,7 @@ __device__ __forceinline__ void cg_finish(const CGArgs<R> &a, const CgShare &sh,
 // for the thread's own copies, and every exit path waits for all of them.
 // Same order of additions in every form, so the same bits on the same grid.
 template <typename R, int NB, bool WIDE = NB != 4>
-__global__ void __launch_bounds__(NB == 4 ? 1024 : 256, NB == 4 ? 1 : (NB == kStagedBatch && sizeof(R) == 8) ? 3 : 4)
+__global__ void __launch_bounds__(NB == 4 ? 1024 : 256, NB == 4 ? 1 : sizeof(R) == 8 ? 2 : 3)
 k_cn_half(const CGArgs<R> a) {
     constexpr bool STAGED = NB == kStagedBatch;
     extern __shared__ __align__(128) unsigned char cg_sm[];
