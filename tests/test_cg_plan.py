@@ -1,0 +1,60 @@
+"""Which CG kernel a launch of the library's choice runs (csrc/cg_plan.cuh), on the
+host: every size gets one, also where a CTA's slice bounds leave no ring."""
+import ctypes as C
+import os
+import shutil
+import subprocess
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+ROOT = os.path.dirname(HERE)
+SRC = os.path.join(HERE, "native", "cg_plan_host.cu")
+OUT = os.path.join(HERE, "native", "_build", "libcg_plan_host.so")
+DEPS = [SRC] + [os.path.join(ROOT, "ucla_cmg_b200", "csrc", f) for f in ("cg_plan.cuh", "common.cuh")]
+SMS = 148
+# (FP32, threads, CTAs per SM) of the launches left to the library
+SHAPES = [(1, 256, 1), (1, 512, 1), (1, 256, 2), (0, 256, 1), (0, 384, 1), (0, 256, 2)]
+
+
+@pytest.fixture(scope="module")
+def plan():
+    nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
+    nvcc = nvcc if os.path.exists(nvcc) else shutil.which("nvcc")
+    if nvcc is None:
+        pytest.skip("nvcc not available to build the host harness")
+    if not os.path.exists(OUT) or os.path.getmtime(OUT) < max(os.path.getmtime(d) for d in DEPS):
+        os.makedirs(os.path.dirname(OUT), exist_ok=True)
+        subprocess.run([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-O2", "-std=c++17", "-Xcompiler", "-fPIC",
+                        "-shared", "-I", os.path.join(ROOT, "include"), "-o", OUT, SRC], check=True, capture_output=True)
+    lib = C.CDLL(OUT)
+
+    def f(fp32, block, per_sm, ns, cols, nslices, grid=None):
+        o = [C.c_int(0), C.c_int(0), C.c_int(0), C.c_double(0)]
+        k = lib.cg_plan(fp32, ns, C.c_longlong(cols), nslices, block, grid or SMS * per_sm, per_sm, *map(C.byref, o))
+        return (k,) + tuple(v.value for v in o)
+    return f
+
+
+@pytest.mark.parametrize("fp32,block,per_sm", SHAPES)
+def test_every_size_gets_a_launch(plan, fp32, block, per_sm):
+    seen = set()
+    for wide in (1, 8, 9, 15, 16, 17, 40, 300):
+        for ns in (1, 2, 7, 31, 64, 500, 1023, 1024, 1563, 5631, 5632, 9215, 9216, 11263, 11264, 20000, 60000):
+            nslices = min(ns * SMS * per_sm, (1 << 31) // (32 * wide))
+            k, threads, ring, smem, keep = plan(fp32, block, per_sm, ns, nslices * wide, nslices)
+            seen.add(k)
+            if k == 1:
+                # two units of nine columns, 227 KB of shared memory an SM (1 KB of it a CTA's own)
+                assert threads == block and ring >= 18 and per_sm * (smem + 6144) <= 227 * 1024
+                assert 0 < keep <= 1
+            else:
+                assert k == 0 and threads == 1024 // per_sm and ring == 0
+    assert seen == {0, 1}
+
+
+@pytest.mark.parametrize("fp32,block,per_sm,ns", [(1, 512, 1, 11264), (0, 384, 1, 9216), (0, 256, 2, 1024),
+                                                  (0, 256, 2, 1563), (1, 256, 2, 5632)])
+def test_shares_whose_bounds_leave_no_ring_run_without(plan, fp32, block, per_sm, ns):
+    nslices = ns * SMS * per_sm
+    assert plan(fp32, block, per_sm, ns, 15 * nslices, nslices)[0] == 0

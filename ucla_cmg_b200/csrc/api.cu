@@ -594,8 +594,8 @@ static int plan_cg(ep_handle *h) {
             const int all = div_up(h->inst_row[k + 1], kSlice) - h->inst_row[k] / kSlice;
             ns = std::max(ns, div_up(all, h->inst_blk[k + 1] - h->inst_blk[k]));
         }
-        const int cols = (int)div_up(all_cols, (long long)h->nslices);
-        rc = h->precision == EP_FP64 ? cg_fit_smem<double>(ns, cols, &h->cg) : cg_fit_smem<float>(ns, cols, &h->cg);
+        rc = h->precision == EP_FP64 ? cg_fit_smem<double>(ns, all_cols, h->nslices, &h->cg)
+                                     : cg_fit_smem<float>(ns, all_cols, h->nslices, &h->cg);
         if (rc) return rc;
     }
     if ((rc = upload_raw(h->d_inst_row, h->inst_row.data(), h->inst_row.size()))) return rc;

@@ -850,8 +850,6 @@ k_cn_half(const CGArgs<R> a) {
 // sweep, each line gone before its next use; L2 is asked to keep the first 36
 // MB of it and to pass the rest (765K nodes: 732 -> 630 us a step; 564K FP64:
 // 1275 -> 968).
-constexpr int kUnit = 8, kUnitMax = 9;        // slice columns of a unit; a single left-over column joins the last
-constexpr int kMaxUnits = 32;                 // units in a warp's ring, at most
 constexpr unsigned int kCopyPolls = 1u << 18; // tries of one unit's wait
 
 __device__ __forceinline__ void cg_mbar_init(unsigned long long *b) {
@@ -1511,12 +1509,6 @@ __global__ void __launch_bounds__(NB == 4 ? 768 : 256, NB == 4 ? 2 : 4) k_cn_hal
     }
 }
 
-// k_cn_smem: shared memory of a CTA with `cols` matrix columns per warp and ns
-// slices at most
-static size_t smem_bytes(int block, int cols, int ns, int rsize) {
-    return (size_t)(block / 32) * ((size_t)cols * kSlice * (4 + rsize) + kMaxUnits * 8) + ((size_t)ns + 1) * 4;
-}
-
 // the kernel of a (gather width, variant) choice and its dynamic shared
 // memory; cg_batch kStagedBatch selects k_cn_half's staged form with `depth` units
 // in flight per warp (1 .. kStageMaxDepth)
@@ -1657,29 +1649,9 @@ int cg_auto_shape(int nslices, long long cols, int ninst, int batch, int variant
     return EP_OK;
 }
 
-// The kernel for CTAs of at most ns slices of about `cols` columns, by the rule
-// above, and k_cn_smem's sizes.
 template <typename R>
-int cg_fit_smem(int ns, int cols, CgShape *out) {
-    const int warps = out->block / 32, spw = div_up(ns, warps);
-    auto fit = [&](int kb) {
-        const long long budget = (long long)kb * 1024 / out->per_sm - ((long long)ns + 1) * 4;
-        return (int)((budget / warps - kMaxUnits * 8) / (kSlice * (4 + (int)sizeof(R))));
-    };
-    const int most = sizeof(R) == 4 ? 200 : 140;
-    const bool stays = spw * cols <= fit(most);
-    const double mb = (double)ns * out->grid * cols * kSlice * (4 + sizeof(R)) / 1e6;      // the matrix
-    if (!stays && mb <= (sizeof(R) == 8 && out->per_sm == 1 ? 27.0 : 60.0)) {
-        out->batch = 4;
-        out->block = 1024 / out->per_sm;
-        return EP_OK;
-    }
-    // a share that stays gets room for slices half as wide again
-    out->ring_cols = std::min(std::max(spw * (cols + cols / 2), 2 * kUnitMax), fit(stays ? most : 120));
-    out->keep = mb <= 60.0 ? 1.0f : (float)(36.0 / mb);
-    // a slice's gathers take up to two units of the ring at once
-    if (out->ring_cols < 2 * kUnitMax) { set_error("CG kernel: %d matrix columns per warp are too few", out->ring_cols); return EP_ERR_ARG; }
-    out->smem = (int)smem_bytes(out->block, out->ring_cols, ns, (int)sizeof(R));
+int cg_fit_smem(int ns, long long cols, int nslices, CgShape *out) {
+    if (!cg_fit<R>(ns, cols, nslices, out)) return EP_OK;        // k_cn_half
     int per = 0;
     int rc = cg_max_per_sm<R>(out->block, &per, kSmemBatch, 0, out->smem, out->per_sm);
     if (!rc && per < out->per_sm) { set_error("CG kernel: %d CTAs per SM instead of %d", per, out->per_sm); rc = EP_ERR_CUDA; }
@@ -1749,8 +1721,8 @@ template int launch_cg<float>(const CGArgs<float> &, int, int, cudaStream_t, int
 template int launch_cg<double>(const CGArgs<double> &, int, int, cudaStream_t, int, int);
 template int cg_auto_shape<float>(int, long long, int, int, int, int, CgShape *);
 template int cg_auto_shape<double>(int, long long, int, int, int, int, CgShape *);
-template int cg_fit_smem<float>(int, int, CgShape *);
-template int cg_fit_smem<double>(int, int, CgShape *);
+template int cg_fit_smem<float>(int, long long, int, CgShape *);
+template int cg_fit_smem<double>(int, long long, int, CgShape *);
 template int cg_grid_size<float>(int, int *, int, int, int, int);
 template int cg_grid_size<double>(int, int *, int, int, int, int);
 template int cg_max_per_sm<float>(int, int *, int, int, int, int);

@@ -1,6 +1,7 @@
 // kernels.cuh -- launch interfaces of the device kernels (host side).
 #pragma once
 #include "common.cuh"
+#include "cg_plan.cuh"
 #include "tt.cuh"
 #include "tt_step.cuh"
 #include "mahajan.cuh"
@@ -150,16 +151,7 @@ template <typename R> struct CGArgs {
     float keep;                  // share of its slices L2 is asked to keep (1: no hint)
 };
 
-// cg_batch value of the staged kernel (asynchronous copies of each warp's
-// next units of SELL columns into shared memory), its deepest ring and the
-// depth it runs at when none is asked for
-constexpr int kStagedBatch = 32;
-// the library's own choice (k_cn_smem; not a cg_batch value) and its shared memory at most
-constexpr int kSmemBatch = 64;
-// and of k_cn_one, the solve on one CTA
-constexpr int kOneBatch = 65;
-constexpr int kOneMax = 208 * 1024;
-constexpr int kSmemMax = 216 * 1024;
+// the staged kernel's deepest ring and the depth it runs at when none is asked for
 constexpr int kStageMaxDepth = 4;
 constexpr int kStageDepthDefault = 2;
 
@@ -168,13 +160,10 @@ constexpr int kStageDepthDefault = 2;
 // (needs r, r1, w0, w1, s0, s1, p0)
 template <typename R>
 int launch_cg(const CGArgs<R> &a, int grid, int block, cudaStream_t s, int batch = 4, int variant = 0);
-// a launch whose shape is left to the library: kernel (batch), threads, CTAs
-// and k_cn_smem's sizes (block: the asked size in, the launch's out)
-struct CgShape { int batch, block, grid, per_sm, ring_cols, smem; float keep; };
 template <typename R>
 int cg_auto_shape(int nslices, long long cols, int ninst, int batch, int variant, int depth, CgShape *out);
 template <typename R>
-int cg_fit_smem(int ns, int cols, CgShape *out);
+int cg_fit_smem(int ns, long long cols, int nslices, CgShape *out);
 // CTAs of the persistent launch: per_sm (0 = as many as fit) x SM count
 template <typename R>
 int cg_grid_size(int block, int *grid, int per_sm = 0, int batch = 4, int variant = 0, int depth = 0);
