@@ -58,3 +58,17 @@ def test_every_size_gets_a_launch(plan, fp32, block, per_sm):
 def test_shares_whose_bounds_leave_no_ring_run_without(plan, fp32, block, per_sm, ns):
     nslices = ns * SMS * per_sm
     assert plan(fp32, block, per_sm, ns, 15 * nslices, nslices)[0] == 0
+
+
+@pytest.mark.parametrize("fp32,per_sm,ns,mb,choice", [
+    (1, 2, 70, 27.0, 0),      # one large instance among 250 small ones: its CTAs' shares are 5 times the average,
+    (1, 2, 360, 50.0, 0),     # the whole matrix is what L2 holds or does not
+    (1, 2, 360, 70.0, 1),
+    (0, 1, 200, 20.0, 0),
+    (0, 1, 200, 40.0, 1)])
+def test_uneven_shares_are_judged_by_the_whole_matrix(plan, fp32, per_sm, ns, mb, choice):
+    cols = int(mb * 1e6 / (32 * (8 if fp32 else 12)))
+    k, threads, ring, smem, keep = plan(fp32, 256, per_sm, ns, cols, cols // 15)
+    assert k == choice
+    if k:
+        assert keep == pytest.approx(36.0 / mb if mb > 60 else 1.0, rel=1e-3)

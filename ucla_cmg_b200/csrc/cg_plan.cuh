@@ -44,7 +44,7 @@ bool cg_fit(int ns, long long cols, int nslices, CgShape *out) {
     };
     const int most = sizeof(R) == 4 ? 200 : 140;
     const bool stays = (long long)spw * wide <= fit(most);
-    const double mb = (double)ns * out->grid * wide * kSlice * (4 + sizeof(R)) / 1e6;      // the matrix
+    const double mb = (double)cols * kSlice * (4 + sizeof(R)) / 1e6;      // the matrix
     // a share that stays gets room for slices half as wide again
     out->ring_cols = (int)std::min<long long>(std::max<long long>((long long)spw * (wide + wide / 2), 2 * kUnitMax),
                                               fit(stays ? most : 120));
