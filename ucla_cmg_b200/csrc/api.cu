@@ -556,20 +556,33 @@ static int reset_barriers(ep_handle *h) {
     return EP_OK;
 }
 
+// the columns of the matrix's slices, and the kernel (gather width, two passes or
+// one) of a launch shape with per_sm CTAs per SM (0: as many as fit)
+static long long matrix_cols(const ep_handle *h) { return (long long)(h->col.bytes / sizeof(int)) / kSlice; }
+static int shape_batch(const ep_handle *h, int block, int per_sm, int batch, int variant) {
+    const double mb = (double)matrix_cols(h) * kSlice * (4 + h->rsize) / 1e6;
+    const int warps = per_sm ? per_sm * block / 32 : 64;
+    const bool two = variant == 0 && (h->precision == EP_FP64 ? cg_named_two<double>(batch, block, warps, h->ninst, mb)
+                                                              : cg_named_two<float>(batch, block, warps, h->ninst, mb));
+    return batch + (two ? kTwo : 0);
+}
+
 static int plan_cg(ep_handle *h) {
     const int ws = stage_depth(h);
     int rc;
     h->cg = CgShape{h->cg_batch, h->cg_block, 0, 0, 0, 0, 1.0f};
-    const long long all_cols = (long long)(h->col.bytes / sizeof(int)) / kSlice;      // of the matrix's slices
+    const long long all_cols = matrix_cols(h);
+    const int batch = shape_batch(h, h->cg_block, h->cg_per_sm, h->cg_batch, h->cg_variant);
     if (h->cg_per_sm == 0) {
         rc = h->precision == EP_FP64
-                 ? cg_auto_shape<double>(h->nslices, all_cols, h->ninst, h->cg_batch, h->cg_variant, ws, &h->cg)
-                 : cg_auto_shape<float>(h->nslices, all_cols, h->ninst, h->cg_batch, h->cg_variant, ws, &h->cg);
+                 ? cg_auto_shape<double>(h->nslices, all_cols, h->ninst, batch, h->cg_variant, ws, &h->cg)
+                 : cg_auto_shape<float>(h->nslices, all_cols, h->ninst, batch, h->cg_variant, ws, &h->cg);
         h->cg_grid = h->cg.grid;
     } else {
+        h->cg.batch = batch;
         rc = h->precision == EP_FP64
-                 ? cg_grid_size<double>(h->cg_block, &h->cg_grid, h->cg_per_sm, h->cg_batch, h->cg_variant, ws)
-                 : cg_grid_size<float>(h->cg_block, &h->cg_grid, h->cg_per_sm, h->cg_batch, h->cg_variant, ws);
+                 ? cg_grid_size<double>(h->cg_block, &h->cg_grid, h->cg_per_sm, batch, h->cg_variant, ws)
+                 : cg_grid_size<float>(h->cg_block, &h->cg_grid, h->cg_per_sm, batch, h->cg_variant, ws);
     }
     if (rc) return rc;
     if (h->cg_variant == 1 && !h->w0.p) {
@@ -579,28 +592,36 @@ static int plan_cg(ep_handle *h) {
             EP_CUDA(cudaMemset(b->p, 0, vb));
         }
     }
-    if (h->ninst > h->cg_grid) {
-        set_error("%d instances but only %d CTAs in the persistent launch", h->ninst, h->cg_grid);
-        return EP_ERR_ARG;
-    }
-    h->inst_blk.assign(h->ninst + 1, 0);
-    if ((rc = ep_batch_plan(h->ninst, h->inst_row.data(), h->cg_grid, h->inst_blk.data()))) {
-        set_error("bad instance layout");
-        return rc;
-    }
+    auto groups = [&]() {
+        if (h->ninst > h->cg_grid) {
+            set_error("%d instances but only %d CTAs in the persistent launch", h->ninst, h->cg_grid);
+            return (int)EP_ERR_ARG;
+        }
+        h->inst_blk.assign(h->ninst + 1, 0);
+        const int bad = ep_batch_plan(h->ninst, h->inst_row.data(), h->cg_grid, h->inst_blk.data());
+        if (bad) set_error("bad instance layout");
+        return bad;
+    };
+    if ((rc = groups())) return rc;
     if (h->cg.batch == kSmemBatch) {
-        int ns = 0;                       // slices of a CTA, at most
+        int ns = 0, largest = 0;          // slices of a CTA and of an instance, at most
         for (int k = 0; k < h->ninst; k++) {
             const int all = div_up(h->inst_row[k + 1], kSlice) - h->inst_row[k] / kSlice;
             ns = std::max(ns, div_up(all, h->inst_blk[k + 1] - h->inst_blk[k]));
+            largest = std::max(largest, all);
         }
-        rc = h->precision == EP_FP64 ? cg_fit_smem<double>(ns, all_cols, h->nslices, &h->cg)
-                                     : cg_fit_smem<float>(ns, all_cols, h->nslices, &h->cg);
+        rc = h->precision == EP_FP64 ? cg_fit_smem<double>(ns, all_cols, h->nslices, h->ninst, largest, &h->cg)
+                                     : cg_fit_smem<float>(ns, all_cols, h->nslices, h->ninst, largest, &h->cg);
         if (rc) return rc;
+        if (h->cg.grid != h->cg_grid) {
+            h->cg_grid = h->cg.grid;
+            if ((rc = groups())) return rc;
+        }
     }
     if ((rc = upload_raw(h->d_inst_row, h->inst_row.data(), h->inst_row.size()))) return rc;
     if ((rc = upload_raw(h->d_inst_blk, h->inst_blk.data(), h->inst_blk.size()))) return rc;
-    if (h->cg_variant == 1 && (rc = h->partial.alloc(sizeof(double) * 12 * (size_t)h->cg_grid))) return rc;
+    if ((h->cg_variant == 1 || (h->cg.batch & kTwo)) &&
+        (rc = h->partial.alloc(sizeof(double) * 12 * (size_t)h->cg_grid))) return rc;
     if ((rc = h->slots.alloc(sizeof(CgSlot) * 32 * (size_t)h->cg_grid))) return rc;
     EP_CUDA(cudaMemsetAsync(h->slots.p, 0, h->slots.bytes, h->stream));
     if (h->bar.bytes != sizeof(GridBarrier) * (size_t)h->ninst) {
@@ -1966,8 +1987,9 @@ int ep_autotune(ep_handle *h, int32_t trial_steps, ep_launch_config *best, doubl
                 if (nb == kStagedBatch && (blk != 256 || cg0.cg_variant != 0)) break;
                 const int pf = nb == kStagedBatch ? dp : cg0.cg_prefetch;
                 int maxper = 0;
-                if ((h->precision == EP_FP64 ? cg_max_per_sm<double>(blk, &maxper, nb, cg0.cg_variant, dp)
-                                             : cg_max_per_sm<float>(blk, &maxper, nb, cg0.cg_variant, dp)))
+                const int batch = shape_batch(h, blk, 0, nb, cg0.cg_variant);
+                if ((h->precision == EP_FP64 ? cg_max_per_sm<double>(blk, &maxper, batch, cg0.cg_variant, dp)
+                                             : cg_max_per_sm<float>(blk, &maxper, batch, cg0.cg_variant, dp)))
                     continue;
                 maxper = std::min(maxper, 8);
                 for (int per : {maxper, maxper / 2}) {

@@ -658,8 +658,17 @@ __device__ __forceinline__ CgShare cg_share(const CGArgs<R> &a) {
     return h;
 }
 
-// The end of a solve: V + its correction (alpha p of the last step added),
-// which is also the next solve's predictor (own rows), and the statistics.
+// The end of a solve: V + its correction, which is also the next solve's
+// predictor (own rows), and the statistics.
+template <typename R>
+__device__ __forceinline__ void finish_correction(const CGArgs<R> &a, int row, R dn) {
+    a.x[row] += dn;
+    if (a.delta) {
+        if (a.dext) a.dext[row] = R(2) * dn - a.delta[row];     // the next solve's start: 2 delta - delta_prev
+        a.delta[row] = dn;
+    }
+}
+// (the last step's alpha p is still to be added)
 template <typename R>
 __device__ __forceinline__ void finish_row(const CGArgs<R> &a, int row, const Pair<R> &t, const Own<R> &o, R al, R be,
                                            bool converged) {
@@ -670,11 +679,7 @@ __device__ __forceinline__ void finish_row(const CGArgs<R> &a, int row, const Pa
     // mass-dominated systems, so it lowers the error 2-3 fold, as the
     // iteration itself would).  FP64 keeps the reference's iterate.
     if (sizeof(R) == 4 && converged) dn = fma(al, fma(be, o.p, fma(-al, t.w, t.z)), dn);
-    a.x[row] += dn;
-    if (a.delta) {
-        if (a.dext) a.dext[row] = R(2) * dn - a.delta[row];     // the next solve's start: 2 delta - delta_prev
-        a.delta[row] = dn;
-    }
+    finish_correction(a, row, dn);
 }
 template <typename R>
 __device__ __forceinline__ void finish_statistics(const CGArgs<R> &a, const CgShare &sh, bool converged,
@@ -832,6 +837,162 @@ k_cn_half(const CGArgs<R> a) {
     }
     if constexpr (STAGED) cp_wait_all();      // the units that ran ahead into the next sweep
     cg_finish(a, sh, (int)(threadIdx.x >> 5), nwarps, lane, cur, al, be, converged, tag, it, rr_last, rr0);
+}
+
+// ---------------------------------------------------------------------------
+// k_cn_two: the solve in two passes an iteration, for a matrix that streams from
+// DRAM.  There the reductions hardly count and what counts is how many loads are
+// in flight, that is warps: a pass over the matrix with one sum (q = A p, (p, q))
+// and a pass over the own rows with two ((r, z), (r, r)) run in 40 registers (gather
+// width 4), 48 warps an SM, where the one-pass sweep's seven sums allow 32 at best.
+// Neighbours gather (z, p) pairs; r, p', q and the correction are the owner's.  The
+// group's warps take its slices in turns, so that all CTAs work on one stretch of
+// the mesh at a time and L2 holds what they gather of it.  NB as in k_cn_half.
+// When it runs: cg_fit and cg_named_two, with the times.
+
+// The sums of a phase through a.partial and the counter barrier (consecutive
+// phases use disjoint places, from `at` on): the tagged lines' polls would take
+// the registers.
+template <int NV, typename R>
+__device__ __forceinline__ bool group_sums(const CGArgs<R> &a, int at, const CgShare &sh, double (&v)[NV]) {
+    const int G = (int)gridDim.x;
+    block_reduce_store<NV>(v, a.partial + at * G, G);
+    if (!grid_sync(a.bar + sh.inst, sh.nb + a.bar_extra)) return false;
+    grid_total<NV>(a.partial + at * G, G, sh.b0, sh.nb, v);
+    return true;
+}
+
+template <typename R, int NB>
+__global__ void __launch_bounds__(NB == 4 ? 768 : 256, NB == 4 ? 2 : (NB == kStagedBatch && sizeof(R) == 8) ? 3 : 4)
+k_cn_two(const CGArgs<R> a) {
+    constexpr bool STAGED = NB == kStagedBatch;
+    extern __shared__ __align__(128) unsigned char cg_sm[];
+    const int lane = threadIdx.x & 31;
+    const CgShare sh = cg_share(a);
+    // the group's warps take its slices in turns
+    const int rb = sh.rb, re = sh.re, s_hi = (re + kSlice - 1) / kSlice, step = sh.nb * ((int)blockDim.x >> 5);
+    const int gwarp = rb / kSlice + (((int)blockIdx.x - sh.b0) * (int)blockDim.x + (int)threadIdx.x) / 32;
+    R *zp = a.q0, *rv = a.q1;
+
+    UnitRing<R> ring;                         // this warp's ring (staged form)
+    if constexpr (STAGED) {
+        ring_start(ring, a, cg_sm, gwarp, step, s_hi);
+        for (int d = 0; d < ring.depth; d++) unit_issue(ring, a, gwarp, step, lane);
+    }
+
+    // ---- prologue, as k_cn_half's ----
+    const bool pred = a.delta != nullptr;
+    double rz, rr0, stop2, rr_last;
+    {
+        const R *dv0 = a.dext ? a.dext : a.delta;
+        double v[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int s = gwarp; s < s_hi; s += step) {
+            if (!STAGED && a.prefetch)
+                prefetch_slice(a.slice_ptr, a.col, a.Aval, a.Bval, s + a.prefetch * step, s_hi, lane);
+            const int row = s * kSlice + lane;
+            const int beg = a.slice_ptr[s], w = (a.slice_ptr[s + 1] - beg) / kSlice;
+            R ax = R(0), bx = R(0), ad = R(0);
+            slice_ab_sums<NB == 4 ? 2 : 4>(a.col, a.Aval, a.Bval, a.x, beg, w, lane, pred, [&](int c) {
+                return a.dext ? a.dext[c] : a.delta[c];
+            }, ax, bx, ad);
+            if (row >= rb && row < re) {
+                const R rref = bx - ax, r = pred ? rref - ad : rref, z = __ldg(a.dinv + row) * r;
+                pair_store(zp, row, z, R(0));
+                rv[row] = r;
+                a.dc[row] = pred ? dv0[row] : R(0);
+                v[0] += (double)r * (double)r;
+                v[1] += (double)bx * (double)bx;
+                v[2] += (double)rref * (double)rref;
+                v[3] += (double)r * (double)z;
+            }
+        }
+        if (!group_sums(a, 6, sh, v)) {
+            if constexpr (STAGED) cp_wait_all();
+            return;
+        }
+        rr_last = v[0];
+        rr0 = v[2];
+        stop2 = fmax(a.tol * a.tol * v[2], a.floor_rel * a.floor_rel * v[1]);
+        rz = v[3];
+    }
+    bool converged = rr_last <= stop2;
+    int it = 0, cons = 0;                     // cons: ring units consumed so far
+    R al = R(0), be = R(0);
+    while (!converged && it < a.maxit) {
+        {   // p' = z + beta p, q = A p'
+            double v[1] = {0.0};
+            for (int s = gwarp; s < s_hi; s += step) {
+                if (!STAGED && a.prefetch)
+                    prefetch_slice<R>(a.slice_ptr, a.col, a.Aval, nullptr, s + a.prefetch * step, s_hi, lane);
+                const int row = s * kSlice + lane;
+                const int beg = __ldg(a.slice_ptr + s), w = (__ldg(a.slice_ptr + s + 1) - beg) / kSlice;
+                auto gat = [&](int c) {
+                    const Pair<R> t = pair_load(zp, c);
+                    return fma(be, t.w, t.z);
+                };
+                R q;
+                if constexpr (STAGED) q = ring_row_sum(ring, a, gwarp, step, lane, w, cons, gat);
+                else if constexpr (NB == 16) q = slice_row_sum_pipe<8>(a.col, a.Aval, beg, w, lane, gat);
+                else q = slice_row_sum<NB>(a.col, a.Aval, beg, w, lane, gat);
+                if (row >= rb && row < re) {
+                    const Pair<R> t = pair_load(zp, row);
+                    const R p = fma(be, t.w, t.z);
+                    a.po[row] = p;
+                    a.qo[row] = q;
+                    v[0] += (double)p * (double)q;
+                }
+            }
+            if (!group_sums(a, 3, sh, v)) {
+                if constexpr (STAGED) cp_wait_all();
+                return;
+            }
+            al = (R)(rz / v[0]);
+        }
+        double v[2] = {0.0, 0.0};
+        // two of the warp's slices at a time: both slices' loads go out before
+        // either is updated
+        for (int s = gwarp; s < s_hi; s += 2 * step) {
+            const int row = s * kSlice + lane, row2 = row + step * kSlice;
+            const bool on = row >= rb && row < re, on2 = s + step < s_hi && row2 >= rb && row2 < re;
+            R pi = R(0), xi = R(0), ri = R(0), qi = R(0), di = R(0);
+            R pi2 = R(0), xi2 = R(0), ri2 = R(0), qi2 = R(0), di2 = R(0);
+            if (on) { pi = a.po[row]; xi = a.dc[row]; ri = rv[row]; qi = a.qo[row]; di = __ldg(a.dinv + row); }
+            if (on2) { pi2 = a.po[row2]; xi2 = a.dc[row2]; ri2 = rv[row2]; qi2 = a.qo[row2]; di2 = __ldg(a.dinv + row2); }
+            auto one = [&](int i, R p, R x, R r0, R q, R d) {
+                a.dc[i] = x + al * p;
+                const R r = r0 - al * q, z = d * r;
+                rv[i] = r;
+                pair_store(zp, i, z, p);
+                v[0] += (double)r * (double)z;
+                v[1] += (double)r * (double)r;
+            };
+            if (on) one(row, pi, xi, ri, qi, di);
+            if (on2) one(row2, pi2, xi2, ri2, qi2, di2);
+        }
+        if (!group_sums(a, 0, sh, v)) {
+            if constexpr (STAGED) cp_wait_all();
+            return;
+        }
+        it++;
+        be = (R)(v[0] / rz);
+        rr_last = v[1];
+        rz = v[0];
+        if (!isfinite(rr_last)) break;        // as in k_cn_half
+        converged = rr_last <= stop2;
+    }
+    if constexpr (STAGED) cp_wait_all();      // the units that ran ahead into the next pass
+    for (int s = gwarp; s < s_hi; s += step) {
+        const int row = s * kSlice + lane;
+        if (row >= rb && row < re) {
+            R dn = a.dc[row];
+            if (sizeof(R) == 4 && converged) {
+                const Pair<R> t = pair_load(zp, row);
+                dn = fma(al, fma(be, t.w, t.z), dn);
+            }
+            finish_correction(a, row, dn);
+        }
+    }
+    finish_statistics(a, sh, converged, a.bar[sh.inst].seq, it, rr_last, rr0);
 }
 
 // ---------------------------------------------------------------------------
@@ -1519,17 +1680,24 @@ template <typename R>
 static int cg_kernel(int block, int batch, int variant, int depth, const void **fn, size_t *smem,
                      bool set_attr, int per_sm = 1) {
     *smem = 0;                 // (k_cn_smem: `depth` is its bytes)
-    if (batch == kStagedBatch) {
-        if (variant != 0) { set_error("the staged CG runs the two-reduction recurrences only"); return EP_ERR_ARG; }
+    const bool two = (batch & kTwo) != 0;
+    if ((batch & ~kTwo) == kStagedBatch) {
+        if (variant != 0) { set_error("the staged CG runs the reference's recurrences only (cg_variant 0)"); return EP_ERR_ARG; }
         if (depth < 1 || depth > kStageMaxDepth) {
             set_error("staged CG: %d units in flight, not 1..%d", depth, kStageMaxDepth);
             return EP_ERR_ARG;
         }
-        *fn = (const void *)k_cn_half<R, kStagedBatch>;
+        *fn = two ? (const void *)k_cn_two<R, kStagedBatch> : (const void *)k_cn_half<R, kStagedBatch>;
         *smem = stage_smem_bytes(block, depth, (int)sizeof(R));
         if (set_attr)
             EP_CUDA(cudaFuncSetAttribute(*fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)stage_smem_bytes(256, kStageMaxDepth, (int)sizeof(R))));
+        return EP_OK;
+    }
+    if (two) {
+        *fn = batch == kTwo + 8 ? (const void *)k_cn_two<R, 8>
+              : batch == kTwo + 16 ? (const void *)k_cn_two<R, 16>
+                                   : (const void *)k_cn_two<R, 4>;
         return EP_OK;
     }
     if (batch == kSmemBatch) {
@@ -1591,14 +1759,14 @@ int cg_max_per_sm(int block, int *per, int batch, int variant, int depth, int pe
 //     against 317);
 //   k_cn_smem's ring beyond (765K FP32: 630 us against 748; 306K FP64: 540
 //     against 710; 562K: 869, 973 with 512 threads), with 120 KB, which leaves
-//     the gathers their L1.
+//     the gathers their L1; and k_cn_two for the largest (cg_fit).
 // Batches the same with two CTAs per SM, which split the GPU more evenly
 // between the instances (24 slabs, 446K nodes FP32: 306 us from k_cn_half, 389
 // from the ring); in FP64, whose CTAs want the registers, with one up to a
 // quarter as many instances as SMs (24 slabs: 757 us, 849 with two; 8 slabs,
 // 155K nodes: 316, 372; 2 slabs, 15K: 149, 175).
-// Any other launch config, and more instances than those CTAs, run k_cn_half
-// with CTAs of `block` threads, as many as fit.
+// Any other launch config, and more instances than those CTAs, run k_cn_half, or
+// k_cn_two (cg_named_two), with CTAs of `block` threads, as many as fit.
 // slices a warp of k_cn_one takes (measured for each, FP32 / FP64, CG us a step:
 // 9 slices 33 / 49 with one, 36 / 54 with two; 23 slices 54 / 86, 48 / 76 with
 // two, 50 / 82 with three; 38 slices, three 58 / 101, four 66 / 116: fewer warps
@@ -1621,7 +1789,7 @@ int cg_auto_shape(int nslices, long long cols, int ninst, int batch, int variant
     EP_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     out->batch = batch;
     out->ring_cols = out->smem = 0;
-    if (variant == 0 && batch == 4 && out->block == 256 && ninst <= 2 * nsm) {
+    if (variant == 0 && (batch & ~kTwo) == 4 && out->block == 256 && ninst <= 2 * nsm) {
         if (ninst == 1 && nslices <= 64 && one_bytes<R>(cols, nslices) <= kOneMax) {
             out->batch = kOneBatch;
             out->block = 32 * div_up(nslices, one_rows(nslices));
@@ -1650,9 +1818,17 @@ int cg_auto_shape(int nslices, long long cols, int ninst, int batch, int variant
 }
 
 template <typename R>
-int cg_fit_smem(int ns, long long cols, int nslices, CgShape *out) {
-    if (!cg_fit<R>(ns, cols, nslices, out)) return EP_OK;        // k_cn_half
+int cg_fit_smem(int ns, long long cols, int nslices, int ninst, int largest, CgShape *out) {
     int per = 0;
+    if (!cg_fit<R>(ns, cols, nslices, ninst, largest, out)) {
+        if (out->grid) return EP_OK;
+        int dev = 0, nsm = 0;
+        EP_CUDA(cudaGetDevice(&dev));
+        EP_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+        const int rc = cg_max_per_sm<R>(out->block, &per, out->batch);
+        out->grid = std::min(std::min(per, out->per_sm) * nsm, div_up(nslices, out->block / 32) + (ninst > 1 ? ninst : 0));
+        return rc;
+    }
     int rc = cg_max_per_sm<R>(out->block, &per, kSmemBatch, 0, out->smem, out->per_sm);
     if (!rc && per < out->per_sm) { set_error("CG kernel: %d CTAs per SM instead of %d", per, out->per_sm); rc = EP_ERR_CUDA; }
     return rc;
@@ -1694,13 +1870,15 @@ int launch_cg(const CGArgs<R> &a, int grid, int block, cudaStream_t s, int batch
         if (rc) return rc;
         void *args[] = {const_cast<CGArgs<R> *>(&a)};
         EP_CUDA(cudaLaunchKernelExC(&cfg, fn, args));
-    } else if (batch == kStagedBatch) {
+    } else if ((batch & kTwo) || batch == kStagedBatch) {
+        if ((batch & kTwo) && !a.partial) { set_error("the two-pass CG needs its partial sums"); return EP_ERR_ARG; }
         const void *fn = nullptr;
         size_t smem = 0;
         int rc = cg_kernel<R>(block, batch, variant, a.depth, &fn, &smem, false);
         if (rc) return rc;
         cfg.dynamicSmemBytes = smem;
-        EP_CUDA(cudaLaunchKernelEx(&cfg, k_cn_half<R, kStagedBatch>, a));
+        void *args[] = {const_cast<CGArgs<R> *>(&a)};
+        EP_CUDA(cudaLaunchKernelExC(&cfg, fn, args));
     } else if (variant == 1) {
         if (!a.r1 || !a.w0 || !a.w1 || !a.s0 || !a.s1) { set_error("single-reduction CG needs its vectors"); return EP_ERR_ARG; }
         if (batch >= 8) EP_CUDA(cudaLaunchKernelEx(&cfg, k_cn_half_cg1<R, 8>, a));
@@ -1721,8 +1899,8 @@ template int launch_cg<float>(const CGArgs<float> &, int, int, cudaStream_t, int
 template int launch_cg<double>(const CGArgs<double> &, int, int, cudaStream_t, int, int);
 template int cg_auto_shape<float>(int, long long, int, int, int, int, CgShape *);
 template int cg_auto_shape<double>(int, long long, int, int, int, int, CgShape *);
-template int cg_fit_smem<float>(int, long long, int, CgShape *);
-template int cg_fit_smem<double>(int, long long, int, CgShape *);
+template int cg_fit_smem<float>(int, long long, int, int, int, CgShape *);
+template int cg_fit_smem<double>(int, long long, int, int, int, CgShape *);
 template int cg_grid_size<float>(int, int *, int, int, int, int);
 template int cg_grid_size<double>(int, int *, int, int, int, int);
 template int cg_max_per_sm<float>(int, int *, int, int, int, int);

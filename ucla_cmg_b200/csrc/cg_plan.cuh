@@ -14,6 +14,8 @@ constexpr int kStagedBatch = 32;
 constexpr int kSmemBatch = 64;
 // and of k_cn_one, the solve on one CTA
 constexpr int kOneBatch = 65;
+// added to a gather width: k_cn_two, two passes an iteration
+constexpr int kTwo = 128;
 constexpr int kOneMax = 208 * 1024;
 constexpr int kSmemMax = 216 * 1024;
 constexpr int kUnit = 8, kUnitMax = 9;        // slice columns of a unit; a single left-over column joins the last
@@ -29,14 +31,38 @@ inline size_t smem_bytes(int block, int cols, int ns, int rsize) {
     return (size_t)(block / 32) * ((size_t)cols * kSlice * (4 + rsize) + kMaxUnits * 8) + ((size_t)ns + 1) * 4;
 }
 
-// The kernel for a matrix of `cols` columns in nslices slices, at most ns of them
-// a CTA's, by the rule above cg_auto_shape: true with k_cn_smem's sizes, or
-// k_cn_half in *out.  A CTA's slice bounds take shared memory too: where they
-// leave a warp no ring of two units (from some 11000 slices a CTA in FP32, 1000
-// in an FP64 batch's, whose large instance got few CTAs), k_cn_half, which needs
-// none of it.
+// Whether a launch shape that the caller set (gather width `batch`, threads a
+// CTA, warps an SM) runs k_cn_two: a matrix of `mb` MB that streams from DRAM, and a
+// shape that had more warps or wider gathers in flight before the one-pass sweep
+// (CG us a step, k_cn_two / k_cn_half: FP32 2.2M nodes width 8 1917 / 2459, staged
+// 1832 / 2445, 768 threads 2162 / 2672, but 0.8M 940 / 934 and width 4 with 32
+// warps 2979 / 2357; FP64 2.2M width 8 3994 / 4627, staged 3545 / 4144, 768 threads
+// 3640 / 4564, width 16 5158 / 4530; 100 instances of 1.8M nodes, width 4, 32 warps
+// 2.0 / 2.0 ms in FP32, 3.0 / 3.2 in FP64).
 template <typename R>
-bool cg_fit(int ns, long long cols, int nslices, CgShape *out) {
+bool cg_named_two(int batch, int block, int warps, int ninst, double mb) {
+    const bool one = ninst == 1;
+    if (sizeof(R) == 4) return mb > (batch != 4 || block == 768 ? 85.0 : warps > 32 ? (one ? 300.0 : 200.0) : 1e30);
+    if (batch != 4) return mb > (batch == 8 ? 140.0 : batch == kStagedBatch ? 180.0 : one ? 1e30 : 140.0);
+    return mb > (block == 768 ? 130.0 : warps > 32 ? (one ? 150.0 : 130.0) : one ? 450.0 : 300.0);
+}
+
+// The kernel for a matrix of `cols` columns in nslices slices, `largest` of them
+// the largest of ninst instances', at most ns a CTA's, by the rule above
+// cg_auto_shape: true with k_cn_smem's sizes, or another kernel in *out (grid 0:
+// as many CTAs as its per_sm, another plan).
+//   A matrix that streams from DRAM on every sweep runs k_cn_two, with two CTAs of
+// 768 threads an SM, or six of 256 where instances are many: CG us a step, one
+// tissue FP32 2.2M nodes 2162 against 2018 from the ring, 3.2M 2979 / 3077, 5.5M
+// 4910 / 5564; FP64 1.25M 2340 / 2006, 2.2M 3640 / 3763, 5.5M 8900 / 10020.  In
+// batches sooner (4 slabs, 1.6M FP64 2455 / 2608; 10, 2.1M 3189 / 3725; 64, 1.2M
+// 1702 / 1980, FP32 1195 / 1096; 100, 1.8M 2542 / 3410, FP32 1710 / 1826): the
+// instances' CTAs are few then and their shares uneven, so with two CTAs per SM the
+// size counts by the largest share.
+//   A CTA's slice bounds take shared memory too: where they leave a warp no ring of
+// two units (from some 11000 slices a CTA in FP32), k_cn_half, which needs none.
+template <typename R>
+bool cg_fit(int ns, long long cols, int nslices, int ninst, int largest, CgShape *out) {
     const int warps = out->block / 32, spw = (ns + warps - 1) / warps, wide = (int)((cols + nslices - 1) / nslices);
     auto fit = [&](int kb) {
         const long long budget = (long long)kb * 1024 / out->per_sm - ((long long)ns + 1) * 4;
@@ -45,6 +71,16 @@ bool cg_fit(int ns, long long cols, int nslices, CgShape *out) {
     const int most = sizeof(R) == 4 ? 200 : 140;
     const bool stays = (long long)spw * wide <= fit(most);
     const double mb = (double)cols * kSlice * (4 + sizeof(R)) / 1e6;      // the matrix
+    const double even = out->per_sm == 1 ? 1.0 : (double)ns * out->grid / nslices;         // 1: all shares alike
+    const double stream = sizeof(R) == 4 ? (out->per_sm == 1 ? 390.0 : 260.0)
+                                         : (ninst == 1 ? 350.0 : out->per_sm == 1 ? 250.0 : 150.0);
+    if (mb * even > stream) {
+        out->batch = kTwo + 4;
+        out->per_sm = ninst <= 36 ? 2 : 6;
+        out->block = 1536 / out->per_sm;
+        out->grid = 0;
+        return false;
+    }
     // a share that stays gets room for slices half as wide again
     out->ring_cols = (int)std::min<long long>(std::max<long long>((long long)spw * (wide + wide / 2), 2 * kUnitMax),
                                               fit(stays ? most : 120));

@@ -163,7 +163,7 @@ int launch_cg(const CGArgs<R> &a, int grid, int block, cudaStream_t s, int batch
 template <typename R>
 int cg_auto_shape(int nslices, long long cols, int ninst, int batch, int variant, int depth, CgShape *out);
 template <typename R>
-int cg_fit_smem(int ns, long long cols, int nslices, CgShape *out);
+int cg_fit_smem(int ns, long long cols, int nslices, int ninst, int largest, CgShape *out);
 // CTAs of the persistent launch: per_sm (0 = as many as fit) x SM count
 template <typename R>
 int cg_grid_size(int block, int *grid, int per_sm = 0, int batch = 4, int variant = 0, int depth = 0);

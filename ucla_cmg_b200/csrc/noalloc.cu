@@ -90,7 +90,7 @@ int run(unsigned char *base, int n, int nslices, const int *slice_ptr, const int
     int rc = cg_auto_shape<R>(nslices, 16ll * nslices, 1, 4, 0, 0, &cg);
     // the rows' widths are on the device; 16 columns are a linear-tet mesh's
     // (wider slices only make a share that would stay a ring)
-    if (!rc && cg.batch == kSmemBatch) rc = cg_fit_smem<R>(div_up(nslices, cg.grid), 16ll * nslices, nslices, &cg);
+    if (!rc && cg.batch == kSmemBatch) rc = cg_fit_smem<R>(div_up(nslices, cg.grid), 16ll * nslices, nslices, 1, nslices, &cg);
     if (rc) return rc;
     a.ring_cols = cg.ring_cols;
     a.smem = cg.smem;
