@@ -96,6 +96,13 @@ def test_large_matrices_take_two_passes(plan):
     assert plan(1, 256, 2, -(-2 * cols // 15 // (2 * SMS)), cols, cols // 15, ninst=64, largest=cols // 600)[0] == 2
 
 
+def test_one_large_among_many_small_instances_gets_more_ctas(plan):
+    nslices = 250 * 16 + 600
+    k, threads, _, _, _, grid, per = plan(1, 256, 2, 16, 15 * nslices, nslices, ninst=251, largest=600)
+    assert (k, threads, grid, per) == (0, 256, 0, 4)
+    assert plan(1, 256, 2, 16, 15 * 4000, 4000, ninst=250, largest=16)[5] != 0
+
+
 def test_named_shapes_of_large_matrices(plan):
     assert not plan.named(1, 8, 256, 32, 1, 60.0) and plan.named(1, 8, 256, 32, 1, 200.0)
     assert not plan.named(1, 4, 256, 32, 1, 5000.0) and plan.named(1, 4, 768, 48, 1, 200.0)

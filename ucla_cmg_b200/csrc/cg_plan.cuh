@@ -59,6 +59,9 @@ bool cg_named_two(int batch, int block, int warps, int ninst, double mb) {
 // 1702 / 1980, FP32 1195 / 1096; 100, 1.8M 2542 / 3410, FP32 1710 / 1826): the
 // instances' CTAs are few then and their shares uneven, so with two CTAs per SM the
 // size counts by the largest share.
+//   A batch whose CTAs are fewer than four an instance, with an instance twice the
+// mean, gets twice the CTAs of k_cn_half (250 slabs of 500 nodes and one of 98K,
+// FP32 / FP64: 277 / 440 us against 577 / 984; and one of 5K: 189 / 287, 278 / 438).
 //   A CTA's slice bounds take shared memory too: where they leave a warp no ring of
 // two units (from some 11000 slices a CTA in FP32), k_cn_half, which needs none.
 template <typename R>
@@ -71,6 +74,13 @@ bool cg_fit(int ns, long long cols, int nslices, int ninst, int largest, CgShape
     const int most = sizeof(R) == 4 ? 200 : 140;
     const bool stays = (long long)spw * wide <= fit(most);
     const double mb = (double)cols * kSlice * (4 + sizeof(R)) / 1e6;      // the matrix
+    if (mb <= 60.0 && out->grid < 4 * ninst && (long long)largest * ninst > 2ll * nslices) {
+        out->batch = 4;
+        out->block = 256;
+        out->per_sm = 4;
+        out->grid = 0;
+        return false;
+    }
     const double even = out->per_sm == 1 ? 1.0 : (double)ns * out->grid / nslices;         // 1: all shares alike
     const double stream = sizeof(R) == 4 ? (out->per_sm == 1 ? 390.0 : 260.0)
                                          : (ninst == 1 ? 350.0 : out->per_sm == 1 ? 250.0 : 150.0);
