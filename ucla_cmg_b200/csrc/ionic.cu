@@ -377,6 +377,15 @@ int launch_ionic(int model, const IonicArgs<R> &a, cudaStream_t st, int block, i
         // registers; 24-slab batch 58 us a step against 62 with three and 77
         // unbounded), three for the others (Mahajan, 214K nodes: 41 us against
         // 43; four spill)
+        // unbounded, without spills, for the reference's order of operations where
+        // two CTAs an SM take all nodes at once (28.6K nodes: 42.6 us against 44.9
+        // with four; 214K, two waves of two: 241 against 139)
+        const bool wave = model == EP_TUSSCHER && (!a.tt.jac_true || a.ref_order) && a.n <= 2 * 128 * nsm;
+        if (min_ctas == 0 && wave) {
+            k_ionic<R, kTusscherRef, TT_NS, 1><<<grid, block, 0, st>>>(a);
+            EP_CUDA(cudaGetLastError());
+            return EP_OK;
+        }
         if (min_ctas == 0) min_ctas = model == EP_TUSSCHER ? 4 : 3;
         if (min_ctas == 3) dispatch_ionic<R, 3>(model, a, grid, block, nsm, st);
         else dispatch_ionic<R, 4>(model, a, grid, block, nsm, st);
