@@ -35,10 +35,25 @@ template <typename R> struct TTRev {            // concentration-dependent terms
 // The 12 gates of one Compute_Ion call (kinetics Tusscher.cc:5-55): the
 // semi-implicit (s + dt inf/tau) / (1 + dt/tau) at voltage V
 // (UpdateStateVariables, Tusscher.cc:116-195).  With inf = I / A and tau = N /
-// D the new value is (s N A + dt D I) / ((N + dt D) A): one division a gate in
-// place of four to nine.
+// D the step is dt D (I - s A) / ((N + dt D) A): one division a gate in place of
+// four to nine, and added to s its own rounding counts only as much as the gate
+// moves (as one quotient, s N A + dt D I over the same, the new value's error was
+// a quarter larger than the reference's order of operations gives; it is half of
+// that: RMS over a wave's states 0.35-0.5 of 1e-16 in FP64, 0.8-0.95 there).
 template <typename R>
-EP_HD R tt_gate(R s, R dt, R N, R D, R A) { return dv(s * N * A + dt * D, (N + dt * D) * A); }
+EP_HD R tt_gate(R s, R dt, R N, R D, R A) {
+    const R e = dt * D;
+    return s + dv(e * (R(1) - s * A), (N + e) * A);
+}
+// the same for m, whose time constant may be far below dt: then the quotient,
+// which keeps the digits of a small new value
+template <typename R>
+EP_HD R tt_gate_fast(R s, R dt, R N, R D, R A) {
+    const R e = dt * D;
+    const bool slow = e < N;
+    const R q = dv(slow ? e * (R(1) - s * A) : s * N * A + e, (N + e) * A);
+    return slow ? s + q : q;
+}
 
 template <typename R>
 EP_HD void tt_gate_step(R s[TT_NS], R V, R dt, const R *__restrict__ c) {
@@ -55,7 +70,7 @@ EP_HD void tt_gate_step(R s[TT_NS], R V, R dt, const R *__restrict__ c) {
     {   // m
         const R t = one + cexp(over(R(-56.86) - V, 9.03));
         const R b1 = one + cexp(over(V + R(35), 5)), b2 = one + cexp(over(V - R(50), 200));
-        s[6] = tt_gate(s[6], dt, R(0.1) * (b1 + b2), (one + cexp(over(R(-60) - V, 5))) * b1 * b2, t * t);
+        s[6] = tt_gate_fast(s[6], dt, R(0.1) * (b1 + b2), (one + cexp(over(R(-60) - V, 5))) * b1 * b2, t * t);
     }
     {   // h, j
         const R t = one + cexp(over(V + R(71.55), 7.43));
@@ -90,11 +105,12 @@ EP_HD void tt_gate_step(R s[TT_NS], R V, R dt, const R *__restrict__ c) {
     {   // f2: inf = 0.67 / A + 0.33
         const R b1 = one + cexp(over(R(25) - V, 10)), A = one + cexp(over(V + R(35), 7));
         const R N = R(562) * exp(over(-v27, 240)) * b1 * b30 + R(31) * b30 + R(80) * b1, D = b1 * b30;
-        s[12] = dv(s[12] * N * A + dt * D * (R(0.67) + R(0.33) * A), (N + dt * D) * A);
+        const R e = dt * D;
+        s[12] += dv(e * (R(0.67) + (R(0.33) - s[12]) * A), (N + e) * A);
     }
     {   // fCass: inf = 0.6 / q + 0.4, tau = 80 / q + 2
         const R t = R(20) * s[9], q = one + t * t, N = R(80) + R(2) * q;
-        s[13] = dv(s[13] * N + dt * (R(0.6) + R(0.4) * q), N + dt * q);
+        s[13] += dv(dt * (R(0.6) + (R(0.4) - s[13]) * q), N + dt * q);
     }
     if (c[53] == R(0)) {   // s
         const R b = one + cexp(over(V - R(20), 5));
