@@ -125,13 +125,24 @@ template <typename R> EP_HD R over(R x, double d) {
     const R lo = sizeof(R) == 4 ? (R)(1.0 / d - (double)hi) : (R)(fma(-(double)hi, d, 1.0) / d);
     return fma(x, hi, x * lo);
 }
+// the smaller of x and a number; NaN stays NaN
+EP_HD float cap(float x, float most) {
+#ifdef __CUDA_ARCH__
+    float y;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(x), "f"(most));
+    return y;
+#else
+    return x > most ? most : x;
+#endif
+}
+EP_HD double cap(double x, double most) { return x > most ? most : x; }
 // exp(x), the argument capped where 1 + exp(x) is exp(x) to every digit and
 // products of three such factors still fit the type
-EP_HD float cexp(float x) { return expf(fminf(x, 28.f)); }
-EP_HD double cexp(double x) { return exp(fmin(x, 200.0)); }
+EP_HD float cexp(float x) { return expf(cap(x, 28.f)); }
+EP_HD double cexp(double x) { return exp(cap(x, 200.0)); }
 // exp(x) - 1, the argument capped as the reach of the type asks
-EP_HD float cexpm1(float x) { return expm1f(fminf(x, 80.f)); }
-EP_HD double cexpm1(double x) { return expm1(fmin(x, 600.0)); }
+EP_HD float cexpm1(float x) { return expm1f(cap(x, 80.f)); }
+EP_HD double cexpm1(double x) { return expm1(cap(x, 600.0)); }
 
 template <typename T> struct RealName;
 template <> struct RealName<float> { static constexpr const char *s = "f32"; };
