@@ -168,6 +168,7 @@ struct ep_handle {
     double act_thr = -40.0;
     TTOpts tt{};
     int mh_abs = 0;
+    int odd_consts = 0;                  // ten Tusscher constants that only tt.cuh takes
     long long step = 0;
     int nslices = 0;
     // device memory
@@ -285,6 +286,18 @@ int substeps(double dt, double idt, double *out) {
     return k;
 }
 
+// Constants that the time steps' ten Tusscher source (tt_step.cuh) is not made for:
+// it forms products of up to four of them and of the exponentials, where FP32
+// overflows, and an infinite one (a flux switched off) gives infinity times zero.
+// Beyond 1e6, ten times the largest ordinary constant, the reference's order of
+// operations runs (tt.cuh), which forms quotients one by one.
+static bool odd_consts(int model, const std::vector<double> &c) {
+    if (model != EP_TUSSCHER) return false;
+    for (double v : c)
+        if (!(std::fabs(v) <= 1e6)) return true;
+    return false;
+}
+
 template <typename R>
 void fill_ionic_args(ep_handle *h, IonicArgs<R> &a) {
     std::memset(&a, 0, sizeof a);
@@ -310,6 +323,7 @@ void fill_ionic_args(ep_handle *h, IonicArgs<R> &a) {
     a.dvdt_out = nullptr;
     a.tt = h->tt;
     a.mh_abs = h->mh_abs;
+    a.ref_order = h->odd_consts;
     a.lr_table = h->lr_table.as<R>();
     a.stride = h->scheme != EP_SCHEME_CN ? 1 : 0;
     a.stride_dt = (R)h->ionic_dt;
@@ -406,6 +420,7 @@ int create_typed(ep_handle *h, const HostCSR &csr, const std::vector<double> &st
     }
     if ((rc = upload<R>(h->V, V))) return rc;
     if ((rc = upload<R>(h->S, S))) return rc;
+    h->odd_consts = odd_consts(h->model, consts);
     if ((rc = upload<R>(h->consts, consts))) return rc;
     if (!gks.empty()) {
         if ((rc = upload<R>(h->gks, gks))) return rc;
@@ -2406,7 +2421,7 @@ static int ionic_batch(const ep_model_desc *md, int32_t precision, int32_t n, do
             a.step_ptr = (const long long *)(status + 1);
             a.track = nullptr;
             a.dvdt_out = dvdt ? Dv : nullptr;
-            a.ref_order = sizeof(R) == 4;        // FP32 plugin results keep their bits
+            a.ref_order = sizeof(R) == 4 || odd_consts(md->model, consts);       // FP32 plugin results keep their bits
             const int first = is_lr(md->model) ? 0 : 1, vslot = is_lr(md->model) ? 7 : 0;
             auto cells = [&](bool back) {
                 k_cells<R><<<div_up(m, 256), 256, 0, s>>>(m, (int)pitch, nst, h.ns, first, vslot, back, (double *)db,

@@ -106,7 +106,10 @@ __device__ __forceinline__ bool grid_sync(GridBarrier *b, unsigned int nblocks) 
 // of the / operator, which the models' wide-ranging denominators take often
 // enough to cost more than the arithmetic around them (Mahajan's FP32 kernel
 // ran with 9 of 32 lanes active).  Within 0.51 ulp where b and the quotient
-// are normal and |b| < 2^126; the callers keep their denominators there.
+// are normal and |b| < 2^126; the callers keep their denominators there (a zero
+// or infinite one gives NaN).  dvc: for denominators a caller's constants decide,
+// zero and infinity as with / (a test and a select more: everywhere, they cost
+// 5 to 13 % of the ionic phase).
 EP_HD double dv(double a, double b) { return a / b; }
 EP_HD float dv(float a, float b) {
 #ifdef __CUDA_ARCH__
@@ -114,6 +117,17 @@ EP_HD float dv(float a, float b) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
     const float q = a * r;
     return fmaf(fmaf(-b, q, a), r, q);
+#else
+    return a / b;
+#endif
+}
+EP_HD double dvc(double a, double b) { return a / b; }
+EP_HD float dvc(float a, float b) {
+#ifdef __CUDA_ARCH__
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
+    const float q = a * r, rem = fmaf(-b, q, a);
+    return fabsf(rem) < INFINITY ? fmaf(rem, r, q) : q;
 #else
     return a / b;
 #endif

@@ -73,7 +73,7 @@ EP_HD void mh_part(const R s[26], const R *__restrict__ c, R h, R r[26], MhExcha
             ex.xina = c[15] * gh * gj * (gm * gm * gm) * (V - rtf * log(dv(c[0], s[19])));
             r[2] = relax(dv(ah, ah + bh), s[2], h * (ah + bh));
             const R ij = dv(one, aj + bj);
-            r[3] = relax(aj * (c[34] * ij), s[3], dv(h * (aj + bj), c[34]));
+            r[3] = relax(aj * (c[34] * ij), s[3], dvc(h * (aj + bj), c[34]));
             r[1] = relax(dv(am, am + bm), s[1], h * (am + bm));
         }
     }
@@ -117,7 +117,7 @@ EP_HD void mh_part(const R s[26], const R *__restrict__ c, R h, R r[26], MhExcha
         // driving force of I_Ca
         {
             const R za = R(2) * vf;
-            const R factor1 = dv(R(4) * R(0.00054) * c[23] * c[23], c[22] * c[20]);
+            const R factor1 = dvc(R(4) * R(0.00054) * c[23] * c[23], c[22] * c[20]);
             const R em = cexpm1(za);
             const R num = factor1 * (csm * (em + one) - R(0.341) * c[3]);
             if (fabs(za) < R(0.001)) ex.rxa = dv(num, R(2) * frt);
@@ -188,7 +188,7 @@ EP_HD void mh_part(const R s[26], const R *__restrict__ c, R h, R r[26], MhExcha
             ex.jnaca = dv(c[8] * c3 * zw3, (c3 + R(0.027)) * (one + R(0.2) * ez) * yz);
         }
         // Ca cycling
-        const R jd = own.jd = dv(c[28] * (s[8] - s[9]), c[14]);
+        const R jd = own.jd = dvc(c[28] * (s[8] - s[9]), c[14]);
         r[24] = c[29] * (R(0.0327) * s[9] * (R(70) - s[24]) - R(0.0196) * s[24]);
         r[25] = R(0.0327) * s[8] * (R(70) - s[25]) - R(0.0196) * s[25];
         const R jup = dv(c[30] * c[13] * (s[9] * s[9]), s[9] * s[9] + R(0.25));
@@ -203,19 +203,19 @@ EP_HD void mh_part(const R s[26], const R *__restrict__ c, R h, R r[26], MhExcha
         own.buf8 = buf(s[8]);
         r[9] = buf(s[9]) * (jd - jup + jleak - r[24]);
         r[10] = -s[12] + jup - jleak;
-        r[11] = dv(s[10] - s[11], c[17]);
+        r[11] = dvc(s[10] - s[11], c[17]);
         {
             const R bv = (c[19] - c[26]) - c[18] * c[19];
             R q = R(0);
             if (s[11] > c[26] && s[11] < c[19]) q = s[11] - c[26];
             else if (s[11] >= c[19]) q = c[18] * s[11] + bv;
             if (q >= c[25]) q = c[25];
-            own.Qr = dv(s[10] * q, c[19]);
+            own.Qr = dvc(s[10] * q, c[19]);
         }
         const R e12 = cexp(R(-0.05) * (V + R(30))), e7 = cexp(R(-0.3576) * (V + R(30)));
         own.frac12 = dv(e12, one + e12);
         own.frac7 = dv(e7, one + e7);
-        r[12] = s[12] * (dv(one, c[16]) - dv(r[10], s[10]));
+        r[12] = s[12] * (dvc(one, c[16]) - dv(r[10], s[10]));
     }
 }
 
