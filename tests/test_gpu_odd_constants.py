@@ -107,3 +107,25 @@ def test_device_quotients(gpu, quotients):
     with np.errstate(all="ignore"):
         want = a / b
     assert np.array_equal(quotients(a, b)[1], want, equal_nan=True)
+
+
+@pytest.mark.parametrize("k", [23, 31])
+def test_learned_step_with_a_flux_switched_off(gpu, k):
+    """The nodes the network takes advance V by the current balance, which an infinite
+    constant leaves finite."""
+    from ucla_cmg_b200.surrogate import Surrogate
+    m = M.slab(5, 5, 3, 0.04, 0.04, 0.02)
+    out = []
+    for v in (np.inf, 9e5):
+        c = np.array([capi.default_consts(capi.TUSSCHER, 0)])
+        c[0, k] = v
+        g = Monodomain(m, capi.TUSSCHER, capi.SURROGATE, dt=0.1, ionic_dt=0.02, D=(1e-3,) * 3, type_consts=c,
+                       tt_jacobian=capi.TT_JAC_TRUE)
+        Surrogate.load().deploy(g)
+        g.set_voltage(-85.2)
+        st = g.step(1)
+        out.append(g.voltage())
+        assert st["fallback_nodes"] < m.n
+        g.close()
+    # a current of at most 1 uA/uF, 1e-4 of it, over 0.1 ms, and FP32's digits of V
+    assert np.all(np.isfinite(out[0])) and np.max(np.abs(out[0] - out[1])) < 1e-4

@@ -132,12 +132,12 @@ EP_HD TTFixed<R> tt_fixed(R V, const R *s, const R *__restrict__ c, R ist, R gks
     f.V = V; f.ist = ist;
     f.rtf = dv(RT, F);
     f.rtf_half = R(0.5) * f.rtf;
-    f.nak = dv(c[21] * c[10],
+    f.nak = dvc(c[21] * c[10],
                (c[10] + c[22]) * (R(1) + R(0.1245) * cexp(R(-0.1) * u) + R(0.0353) * cexp(-u)));
     f.g_na = c[16] * (s[6] * s[6] * s[6]) * s[7] * s[8];
     const R e_g = exp(c[27] * u), e_g1 = exp((c[27] - R(1)) * u);
     const R nao3 = c[11] * c[11] * c[11];
-    const R naca = dv(c[24], ((c[29] * c[29] * c[29]) + nao3) * (c[28] + c[12]) * (R(1) + c[25] * e_g1));
+    const R naca = dvc(c[24], ((c[29] * c[29] * c[29]) + nao3) * (c[28] + c[12]) * (R(1) + c[25] * e_g1));
     f.naca_n = naca * e_g * c[12];
     f.naca_c = naca * e_g1 * nao3 * c[26];
     const R sq_ko = sqrt(over(c[10], 5.4));
@@ -206,7 +206,7 @@ EP_HD void tt_nr_rates(const R x[6], const TTRev<R> &e, const TTFixed<R> &f,
                                             const R *c, R r[6], R &dvdt) {
     const R V = f.V;
     const R Nai = x[1], Cai = x[2], Cass = x[3], Casr = x[4], Rp = x[5];
-    const R i_nak = f.nak * dv(Nai, Nai + c[23]);
+    const R i_nak = f.nak * dvc(Nai, Nai + c[23]);
     const R i_na = f.g_na * (V - e.ENa);
     const R i_bna = c[17] * (V - e.ENa);
     const R i_naca = f.naca_n * (Nai * Nai * Nai) - f.naca_c * Cai;
@@ -218,7 +218,7 @@ EP_HD void tt_nr_rates(const R x[6], const TTRev<R> &e, const TTFixed<R> &f,
     const R i_cal = f.cal_s * Cass - f.cal_0;
     const R i_bca = c[19] * (V - e.ECa);
     const R i_pk = f.g_pk * vk;
-    const R i_pca = dv(c[30] * Cai, Cai + c[31]);
+    const R i_pca = dvc(c[30] * Cai, Cai + c[31]);
     dvdt = -(i_k1 + i_to + i_kr + i_ks + i_cal + i_nak + i_na + i_bna + i_naca + i_bca + i_pk + i_pca + f.ist);
     r[0] = -((i_k1 + i_to + i_kr + i_ks + i_pk + f.ist) - R(2) * i_nak) * f.cap;
     r[1] = -(i_na + i_bna + R(3) * i_nak + R(3) * i_naca) * f.cap;
