@@ -2193,8 +2193,9 @@ static int upload_pieces(void *dst, const void *src, size_t bytes, cudaStream_t 
 int ep_ecg_eval(ep_ecg *e, int32_t n_frames, const double *V, double *out) {
     EP_CHECK_ARG(e && n_frames >= 0 && (n_frames == 0 || (V && out)), "bad arguments");
     EP_CUDA(cudaSetDevice(e->device));
-    // frames go up in chunks of at most ~256 MB
-    const int chunk = std::max(1, (int)std::min<long long>(n_frames, (256ll << 20) / (8ll * e->n)));
+    // frames go up in chunks of at most ~256 MB, and of a launch's 65535 groups
+    const int chunk = std::max(1, (int)std::min({(long long)n_frames, (256ll << 20) / (8ll * e->n),
+                                                 65535ll * ecg_frames(e->ne)}));
     int rc;
     const int nodes = ecg_chunks(e->n, e->ne, chunk), groups = div_up(std::max(1, chunk), ecg_frames(e->ne));
     if (chunk > e->cap_frames) {
