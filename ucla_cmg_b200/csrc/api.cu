@@ -47,6 +47,26 @@ struct DBuf {
     template <typename T> T *as() const { return (T *)p; }
 };
 
+// Which context the calling thread works in: a number no other context of the
+// process ever has, also not one that cudaDeviceReset puts in its place (0 where
+// the driver cannot tell).
+static unsigned long long context_id() {
+    using Fn = int (*)(void *, unsigned long long *);
+    static const Fn fn = [] {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult st{};
+        if (cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &st) != cudaSuccess ||
+            st != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            p = nullptr;
+        }
+        return (Fn)p;
+    }();
+    unsigned long long id = 0;
+    if (!fn || fn(nullptr, &id) != 0) return 0;
+    return id;
+}
+
 // What the calls without a handle of their own (the plugin-level cells) and the
 // offline ECG's uploads work in: a stream, two events, one device block and one
 // pinned block per host thread, so that concurrent calls share nothing.  Kept
@@ -57,6 +77,7 @@ struct DBuf {
 struct CallBuffers {
     static constexpr size_t kKeep = 64u << 20;
     int device = -1;
+    unsigned long long context = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev[2] = {};
     void *dev = nullptr, *pin = nullptr;
@@ -67,13 +88,15 @@ struct CallBuffers {
         int cur = 0;
         EP_CUDA(cudaGetDevice(&cur));
         if (stream && cur != device) drop();
-        // a cudaDeviceReset since the last call took everything with it
-        cudaPointerAttributes at{};
-        if ((dev || pin) && (cudaPointerGetAttributes(&at, dev ? dev : pin) != cudaSuccess ||
-                             at.type != (dev ? cudaMemoryTypeDevice : cudaMemoryTypeHost))) {
-            cudaGetLastError();
-            forget();
+        // a cudaDeviceReset since the last call took everything with it, and its
+        // addresses may be another's by now
+        unsigned long long id = context_id();
+        if (!id) {                                  // the thread's first call, or after a reset
+            EP_CUDA(cudaFree(nullptr));
+            id = context_id();
         }
+        if (id != context) forget();
+        context = id;
         device = cur;
         if (!stream) {
             EP_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
@@ -112,11 +135,13 @@ struct CallBuffers {
         int cur = 0;
         if (cudaGetDevice(&cur) == cudaSuccess) {
             if (device >= 0) cudaSetDevice(device);
-            if (dev) cudaFree(dev);
-            if (pin) cudaFreeHost(pin);
-            for (cudaEvent_t e : ev)
-                if (e) cudaEventDestroy(e);
-            if (stream) cudaStreamDestroy(stream);
+            if (context_id() == context) {
+                if (dev) cudaFree(dev);
+                if (pin) cudaFreeHost(pin);
+                for (cudaEvent_t e : ev)
+                    if (e) cudaEventDestroy(e);
+                if (stream) cudaStreamDestroy(stream);
+            }
             cudaSetDevice(cur);
         }
         cudaGetLastError();
