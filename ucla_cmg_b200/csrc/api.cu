@@ -3,6 +3,7 @@
 #include <cstdarg>
 #include <cstring>
 #include <cmath>
+#include <new>
 #include <vector>
 #include <string>
 #include <memory>
@@ -69,22 +70,30 @@ static unsigned long long context_id() {
 
 // What the calls without a handle of their own (the plugin-level cells) and the
 // offline ECG's uploads work in: a stream, two events, one device block and one
-// pinned block per host thread, so that concurrent calls share nothing.  Kept
+// host block per host thread, so that concurrent calls share nothing.  Kept
 // from call to call up to kKeep bytes each (a dozen cudaMalloc / cudaFree pairs
-// a call took most of its time), a larger block goes back when its call
-// returns, all of it when the thread ends.  Every call has waited for its work
-// when it returns, so nothing here is in use between calls.
+// a call took most of its time), a larger block goes back when its call returns, all of it when the
+// thread ends.  Every call has waited for its work when it returns, so nothing
+// here is in use between calls.
+// The host block is ordinary memory at first: pinning takes 2 ms for a page and
+// 6.5 for 8 MB, as long as several whole calls (first call of a thread, 100 cells
+// 3.6 ms with it and 0.95 without, a dozen cudaMallocs took 1.1; 64 ECG frames of
+// 28.6K nodes 9 and 1.8, 2.0), and is paid when the calls that went without
+// have saved about as much (64 MB of frames, five calls of cells).
 struct CallBuffers {
     static constexpr size_t kKeep = 64u << 20;
+    static constexpr size_t kPin = 64u << 20;       // bytes through ordinary memory before pinning
+    static constexpr size_t kCall = kPin / 5;       // what a call of the cells counts at least
     int device = -1;
     unsigned long long context = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev[2] = {};
     void *dev = nullptr, *pin = nullptr;
-    size_t dev_bytes = 0, pin_bytes = 0;
+    size_t dev_bytes = 0, pin_bytes = 0, plain_bytes = 0, moved = 0;
+    std::unique_ptr<char[]> plain;
 
-    // blocks of at least d (device) and p (pinned) bytes on the current device
-    int reserve(size_t d, size_t p) {
+    // the stream, and a block of at least d bytes on the current device
+    int reserve(size_t d) {
         int cur = 0;
         EP_CUDA(cudaGetDevice(&cur));
         if (stream && cur != device) drop();
@@ -113,22 +122,42 @@ struct CallBuffers {
             }
             dev_bytes = d;
         }
-        if (p > pin_bytes) {
-            if (pin) cudaFreeHost(pin);
-            pin = nullptr;
-            pin_bytes = 0;
-            if (cudaMallocHost(&pin, p) != cudaSuccess) {
-                cudaGetLastError();
-                set_error("cudaMallocHost(%zu) failed", p);
-                return EP_ERR_NOMEM;
-            }
-            pin_bytes = p;
-        }
         return EP_OK;
+    }
+    // whether a pinned block of p bytes is there for a call that moves `bytes`
+    // (after reserve)
+    bool pinned(size_t p, size_t bytes) {
+        if (p <= pin_bytes) return true;
+        if ((moved += bytes) < kPin) return false;
+        moved = 0;
+        p = std::max(p, (size_t)1 << 20);
+        if (pin) cudaFreeHost(pin);
+        pin = nullptr;
+        pin_bytes = 0;
+        if (cudaMallocHost(&pin, p) != cudaSuccess) {
+            cudaGetLastError();
+            pin = nullptr;
+            return false;
+        }
+        pin_bytes = p;
+        return true;
+    }
+    // a host block of p bytes, pinned or not
+    char *host(size_t p, size_t bytes) {
+        if (pinned(p, bytes)) return (char *)pin;
+        if (p > plain_bytes) {
+            plain.reset();
+            plain_bytes = 0;
+            plain.reset(new (std::nothrow) char[p]);
+            if (!plain) { set_error("%zu bytes of host memory are not there", p); return nullptr; }
+            plain_bytes = p;
+        }
+        return plain.get();
     }
     void trim() {
         if (dev_bytes > kKeep) { cudaFree(dev); dev = nullptr; dev_bytes = 0; }
         if (pin_bytes > kKeep) { cudaFreeHost(pin); pin = nullptr; pin_bytes = 0; }
+        if (plain_bytes > kKeep) { plain.reset(); plain_bytes = 0; }
     }
     void forget() { stream = nullptr; ev[0] = ev[1] = nullptr; dev = pin = nullptr; dev_bytes = pin_bytes = 0; }
     void drop() {
@@ -2154,8 +2183,7 @@ int ep_compute_ecg(ep_handle *h, double *out) {
 struct ep_ecg {
     int device = 0, n = 0, ne = 0;
     cudaStream_t stream = nullptr;
-    DBuf W, V, out, partial, counter;
-    int cap_frames = 0;
+    DBuf W, work;                        // work: frames, leads, counters and partial sums of a chunk
     ~ep_ecg() { if (stream) cudaStreamDestroy(stream); }
 };
 
@@ -2195,15 +2223,18 @@ int ep_ecg_create(const ep_mesh_desc *mesh, const ep_cables_desc *cables, int32_
 }
 
 // host data to the device through two pinned pieces, the copy into one under
-// the transfer of the other (the driver stages pageable memory with one thread)
+// the transfer of the other (the driver stages pageable memory with one thread),
+// where the thread has them (CallBuffers)
 static int upload_pieces(void *dst, const void *src, size_t bytes, cudaStream_t s) {
-    constexpr size_t piece = 4u << 20;
-    if (bytes < (1u << 20)) {
+    constexpr size_t piece = 2u << 20;
+    if (bytes >= piece) {
+        int rc = t_buf.reserve(0);
+        if (rc) return rc;
+    }
+    if (bytes < piece || !t_buf.pinned(2 * piece, bytes)) {
         EP_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s));
         return EP_OK;
     }
-    int rc = t_buf.reserve(0, 2 * piece);
-    if (rc) return rc;
     for (size_t at = 0, k = 0; at < bytes; at += piece, k++) {
         const size_t b = std::min(piece, bytes - at);
         char *p = (char *)t_buf.pin + (k & 1) * piece;
@@ -2222,24 +2253,21 @@ int ep_ecg_eval(ep_ecg *e, int32_t n_frames, const double *V, double *out) {
     const int chunk = std::max(1, (int)std::min({(long long)n_frames, (256ll << 20) / (8ll * e->n),
                                                  65535ll * ecg_frames(e->ne)}));
     int rc;
-    const int nodes = ecg_chunks(e->n, e->ne, chunk), groups = div_up(std::max(1, chunk), ecg_frames(e->ne));
-    if (chunk > e->cap_frames) {
-        if ((rc = e->V.alloc(sizeof(double) * (size_t)chunk * e->n))) return rc;
-        if ((rc = e->out.alloc(sizeof(double) * (size_t)chunk * e->ne))) return rc;
-        if ((rc = e->counter.alloc(sizeof(unsigned int) * (size_t)groups))) return rc;
-        EP_CUDA(cudaMemsetAsync(e->counter.p, 0, e->counter.bytes, e->stream));
-        e->cap_frames = chunk;
-    }
-    if (e->partial.bytes < sizeof(double) * (size_t)chunk * e->ne * nodes &&
-        (rc = e->partial.alloc(sizeof(double) * (size_t)chunk * e->ne * nodes)))
+    const int nodes = ecg_chunks(e->n, e->ne, chunk), groups = div_up(chunk, ecg_frames(e->ne));
+    const size_t bV = sizeof(double) * (size_t)chunk * e->n, bO = sizeof(double) * (size_t)chunk * e->ne;
+    const size_t bC = (sizeof(unsigned int) * (size_t)groups + 15) / 16 * 16;
+    if (e->work.bytes < bV + bO * (1 + (size_t)nodes) + bC &&
+        (rc = e->work.alloc(bV + bO * (1 + (size_t)nodes) + bC)))
         return rc;
+    double *dV = e->work.as<double>(), *dO = dV + (size_t)chunk * e->n, *partial = dO + (size_t)chunk * e->ne;
+    unsigned int *counter = (unsigned int *)(partial + (size_t)chunk * e->ne * nodes);
+    EP_CUDA(cudaMemsetAsync(counter, 0, bC, e->stream));
     for (int f0 = 0; f0 < n_frames; f0 += chunk) {
         const int nf = std::min(chunk, n_frames - f0);
-        if ((rc = upload_pieces(e->V.p, V + (size_t)f0 * e->n, sizeof(double) * (size_t)nf * e->n, e->stream))) return rc;
-        rc = launch_ecg<double>(e->n, e->ne, e->W.as<double>(), e->n, e->V.as<double>(), nf, e->partial.as<double>(),
-                                e->counter.as<unsigned int>(), e->out.as<double>(), nodes, e->stream);
+        if ((rc = upload_pieces(dV, V + (size_t)f0 * e->n, sizeof(double) * (size_t)nf * e->n, e->stream))) return rc;
+        rc = launch_ecg<double>(e->n, e->ne, e->W.as<double>(), e->n, dV, nf, partial, counter, dO, nodes, e->stream);
         if (rc) return rc;
-        EP_CUDA(cudaMemcpyAsync(out + (size_t)f0 * e->ne, e->out.p, sizeof(double) * (size_t)nf * e->ne,
+        EP_CUDA(cudaMemcpyAsync(out + (size_t)f0 * e->ne, dO, sizeof(double) * (size_t)nf * e->ne,
                                 cudaMemcpyDeviceToHost, e->stream));
         EP_CUDA(cudaStreamSynchronize(e->stream));
     }
@@ -2416,9 +2444,11 @@ static int ionic_batch(const ep_model_desc *md, int32_t precision, int32_t n, do
         };
         const size_t in_cap = (in_bytes(most) + 255) / 256 * 256;
         const size_t dev = in_cap + sizeof(R) * pitch * (h.ns + 4) + 256;
-        if ((r2 = t_buf.reserve(dev, in_cap))) return r2;
+        if ((r2 = t_buf.reserve(dev))) return r2;
+        char *hb = t_buf.host(in_cap, std::max(2 * in_cap, CallBuffers::kCall));
+        if (!hb) return EP_ERR_NOMEM;
         cudaStream_t s = t_buf.stream;
-        char *db = (char *)t_buf.dev, *hb = (char *)t_buf.pin;
+        char *db = (char *)t_buf.dev;
         R *S = (R *)(db + in_cap), *Vr = S + pitch * h.ns, *Ist = Vr + pitch, *Gks = Ist + pitch, *Dv = Gks + pitch;
         DevStatus *status = (DevStatus *)(db + dev - 256);
         for (int i0 = 0; i0 < n; i0 += most) {
