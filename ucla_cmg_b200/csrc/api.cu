@@ -72,7 +72,8 @@ static unsigned long long context_id() {
 // offline ECG's uploads work in: a stream, two events, one device block and one
 // host block per host thread, so that concurrent calls share nothing.  Kept
 // from call to call up to kKeep bytes each (a dozen cudaMalloc / cudaFree pairs
-// a call took most of its time), a larger block goes back when its call returns, all of it when the
+// a call took most of its time; of the device four times that, which holds 1.2M
+// cells), a larger block goes back when its call returns, all of it when the
 // thread ends.  Every call has waited for its work when it returns, so nothing
 // here is in use between calls.
 // The host block is ordinary memory at first: pinning takes 2 ms for a page and
@@ -155,7 +156,7 @@ struct CallBuffers {
         return plain.get();
     }
     void trim() {
-        if (dev_bytes > kKeep) { cudaFree(dev); dev = nullptr; dev_bytes = 0; }
+        if (dev_bytes > 4 * kKeep) { cudaFree(dev); dev = nullptr; dev_bytes = 0; }
         if (pin_bytes > kKeep) { cudaFreeHost(pin); pin = nullptr; pin_bytes = 0; }
         if (plain_bytes > kKeep) { plain.reset(); plain_bytes = 0; }
     }
@@ -2397,7 +2398,7 @@ extern "C" {
 // Independent cells through the ionic kernel: one Compute_Ion call per cell
 // returning dV/dt (dvdt != NULL, V unchanged), or a whole ionic phase of
 // sub-steps with the V update (dvdt == NULL, V advanced in place).  In chunks
-// that bound the buffers; a chunk is one copy each way.
+// that bound the host block; a chunk is one copy each way.
 static int ionic_batch(const ep_model_desc *md, int32_t precision, int32_t n, double dt,
                        double ionic_dt, double Cm, double *V, const double *istim, double *states,
                        double *dvdt) {
@@ -2443,15 +2444,19 @@ static int ionic_batch(const ep_model_desc *md, int32_t precision, int32_t n, do
             return sizeof(double) * (m * (nst + 2 + (gks ? 1 : 0)) + consts.size()) + (types ? m : 0);
         };
         const size_t in_cap = (in_bytes(most) + 255) / 256 * 256;
-        const size_t dev = in_cap + sizeof(R) * pitch * (h.ns + 4) + 256;
+        // on the device one for each chunk: no result goes to the caller before every
+        // chunk has run
+        const size_t all_in = in_cap * (size_t)div_up(n, std::max(most, 1));
+        const size_t dev = all_in + sizeof(R) * pitch * (h.ns + 4) + 256;
         if ((r2 = t_buf.reserve(dev))) return r2;
         char *hb = t_buf.host(in_cap, std::max(2 * in_cap, CallBuffers::kCall));
         if (!hb) return EP_ERR_NOMEM;
         cudaStream_t s = t_buf.stream;
         char *db = (char *)t_buf.dev;
-        R *S = (R *)(db + in_cap), *Vr = S + pitch * h.ns, *Ist = Vr + pitch, *Gks = Ist + pitch, *Dv = Gks + pitch;
+        R *S = (R *)(db + all_in), *Vr = S + pitch * h.ns, *Ist = Vr + pitch, *Gks = Ist + pitch, *Dv = Gks + pitch;
         DevStatus *status = (DevStatus *)(db + dev - 256);
-        for (int i0 = 0; i0 < n; i0 += most) {
+        for (int i0 = 0; i0 < n; i0 += most, db += in_cap) {
+            if (i0) EP_CUDA(cudaEventSynchronize(t_buf.ev[0]));      // the host block is free again
             const int m = std::min(most, n - i0);
             const size_t oV = sizeof(double) * (size_t)m * nst, oI = oV + sizeof(double) * m, oG = oI + sizeof(double) * m;
             const size_t oC = oG + (gks ? sizeof(double) * m : 0), oT = oC + sizeof(double) * consts.size();
@@ -2463,6 +2468,7 @@ static int ionic_batch(const ep_model_desc *md, int32_t precision, int32_t n, do
             for (size_t k = 0; k < consts.size(); k++) ((R *)(hb + oC))[k] = (R)consts[k];
             if (types) host_copy(hb + oT, md->node_type + i0, m);
             EP_CUDA(cudaMemcpyAsync(db, hb, in_bytes(m), cudaMemcpyHostToDevice, s));
+            EP_CUDA(cudaEventRecord(t_buf.ev[0], s));
             EP_CUDA(cudaMemsetAsync(status, 0, 256, s));           // the status and, behind it, step 0
             h.n = m;
             h.pitch = (int)pitch;
@@ -2489,8 +2495,13 @@ static int ionic_batch(const ep_model_desc *md, int32_t precision, int32_t n, do
             EP_CUDA(cells(false));
             if ((r2 = launch_ionic<R>(h.model, a, s))) return r2;
             EP_CUDA(cells(true));
-            EP_CUDA(cudaMemcpyAsync(hb, db, oI, cudaMemcpyDeviceToHost, s));
-            EP_CUDA(cudaStreamSynchronize(s));
+        }
+        db = (char *)t_buf.dev;
+        for (int i0 = 0; i0 < n; i0 += most, db += in_cap) {
+            const int m = std::min(most, n - i0);
+            const size_t oV = sizeof(double) * (size_t)m * nst;
+            EP_CUDA(cudaMemcpyAsync(hb, db, oV + sizeof(double) * m, cudaMemcpyDeviceToHost, s));
+            EP_CUDA(cudaStreamSynchronize(s));        // the first: of every chunk's kernels
             host_copy(states + (size_t)i0 * nst, hb, oV);
             host_copy((dvdt ? dvdt : V) + i0, hb + oV, sizeof(double) * m);
         }
