@@ -202,7 +202,10 @@ int  ep_step(ep_handle *h, int32_t n_steps, ep_step_stats *stats);
 int  ep_set_profiling(ep_handle *h, int on);
 /* One Crank-Nicolson half diffusion step on the current voltage, nothing
  * else: V <- A^-1 (B V) (EP_CrankNicholson.cc:99-104).  *iters receives the
- * CG iteration count, *relres the final ||r||/||r0||. */
+ * CG iteration count, *relres the ||r||/||r0|| that ended it.  An FP32 handle
+ * then adds one more step of the last length in the next direction, which costs
+ * nothing and lowers the error two- to threefold: the returned V is past the
+ * iterate of *iters and *relres.  An FP64 handle returns that iterate. */
 int  ep_diffusion_half_step(ep_handle *h, int32_t *iters, double *relres);
 /* Allocation-free Crank-Nicolson half diffusion step.  No counterpart in
  * the reference: it exists for callers that own all device memory and may
@@ -332,13 +335,13 @@ int  ep_assemble_operators(const ep_mesh_desc *mesh, const ep_cables_desc *cable
  * cg_block 256 with cg_batch 4 one CTA of up to 1024 threads per SM on large
  * meshes, since every CTA takes part in each iteration's reduction; otherwise
  * at most as many as the kernel's registers let reside, e.g. with cg_batch 8,
- * 16 or 32 and cg_block 256 three in FP32 and two in FP64); ionic_block:
- * threads per CTA of the
- * ionic kernel (64 or 128); graph_steps: 0 launches every kernel from the
- * host, k > 0 replays the steps from an instantiated CUDA graph of k steps
+ * 16 or 32 and cg_block 256 three in FP32 and two in FP64; matrices that stream
+ * from DRAM run two passes an iteration there, with CTAs of fewer registers);
+ * ionic_block: threads per CTA of the ionic kernel (64 or 128; Mahajan's always
+ * has 128); graph_steps: 0 launches every kernel from the host, k > 0 replays the steps from an instantiated CUDA graph of k steps
  * (rounded up to a multiple of the ECG interval); ionic_min_ctas: FP32
  * ionic kernel compiled for at least 3 or 4 resident 128-thread CTAs per SM
- * (fewer registers per thread), 0 = the library's choice by cell model;
+ * (fewer registers per thread), 0 = the library's choice by cell model and size;
  * cg_batch: SELL columns whose gathers the CG kernel issues together (4 or
  * 8; 8 keeps more loads in flight at a larger register budget; 16: groups of
  * 8 with the next group's index loads issued before the current gathers;
@@ -359,7 +362,9 @@ typedef struct ep_launch_config {
                              to B V - A V */
     int32_t cg_prefetch;  /* 0..4: each warp of the CG launch asks L2 for the
                              SELL indices and values of the slice it reads that
-                             many slices ahead (cg_variant 0; 0 = off); with
+                             many slices ahead (cg_variant 0; 0 = off; without
+                             effect where the library's own launch keeps or
+                             streams the matrix through shared memory); with
                              cg_batch 32 the units the ring holds in flight
                              (0 = 2) */
     int32_t sg_variant;   /* learned ionic step (EP_SURROGATE): 0 the library's choice
@@ -409,7 +414,13 @@ int  ep_read_restart(ep_handle *h, double t, const char *dir);
 /* Plugin-level entry: IonicModel::Compute_Ion for a batch of independent
  * cells (IonicModel/IonicModel.h:34-35, Body/CardiacBody.cc:405-435).
  * states: n * nstate node-major, updated in place; dvdt[i] receives the
- * return value.  Host buffers; runs on the current CUDA device. */
+ * return value.  Host buffers; runs on the current CUDA device.  On an error
+ * the arrays are as they were.
+ *   This call, ep_ionic_phase and ep_ecg_eval keep what they work in for the
+ * calling host thread's next call: a stream, up to 256 MB of device memory, up
+ * to 64 MB of pinned host memory (pinned only after a few calls) and as much
+ * ordinary memory.  Larger blocks go back when the call returns, all of it when
+ * the thread ends or works on another device. */
 int  ep_ionic_step(const ep_model_desc *model, int32_t precision, int32_t n,
                    double dt, double Cm, const double *V, const double *istim,
                    double *states, double *dvdt);

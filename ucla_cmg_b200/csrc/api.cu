@@ -2093,8 +2093,11 @@ int ep_autotune(ep_handle *h, int32_t trial_steps, ep_launch_config *best, doubl
             if (t >= 0 && t < t_best) { t_best = t; b = c; }
         }
         const ep_launch_config b1 = b;
+        // (the staged kernel's depth is tuned above; a matrix in shared memory is not prefetched)
+        bool prefetch = b1.cg_batch != kStagedBatch && ep_set_launch_config(h, &b1) == EP_OK;
+        prefetch = prefetch && h->cg.batch != kSmemBatch && h->cg.batch != kOneBatch;
         for (int pf : {0, 2}) {
-            if (pf == b1.cg_prefetch || b1.cg_batch == kStagedBatch) continue;   // the staged kernel's depth is tuned above
+            if (pf == b1.cg_prefetch || !prefetch) continue;
             ep_launch_config c = b1;
             c.cg_prefetch = pf;
             const double t = trial(c);
@@ -2108,7 +2111,7 @@ int ep_autotune(ep_handle *h, int32_t trial_steps, ep_launch_config *best, doubl
         if (t >= 0 && t < t_best) { t_best = t; b = c; }
     }
     for (int ib : {64, 128}) {
-        if (ib == b.ionic_block) continue;
+        if (ib == b.ionic_block || h->model == EP_MAHAJAN || h->model == EP_MAHAJAN_FAIL) continue;   // always 128
         ep_launch_config c = b;
         c.ionic_block = ib;
         const double t = trial(c);

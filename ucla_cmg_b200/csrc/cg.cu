@@ -1516,8 +1516,9 @@ __global__ void __launch_bounds__(512, 1) k_cn_one(const CGArgs<R> a) {
 }
 
 // ---------------------------------------------------------------------------
-// The same solve by the Chronopoulos-Gear recurrences: one grid barrier per
-// iteration instead of two.  With z = dinv r and w = A z,
+// The same solve by the Chronopoulos-Gear recurrences, whose one reduction an
+// iteration gives both scalars as sums of the vectors themselves (k_cn_half's
+// next residual is a difference).  With z = dinv r and w = A z,
 //   gamma = (r, z), delta = (z, w)                 (one reduction)
 //   beta = gamma / gamma_old, alpha = gamma / (delta - beta gamma / alpha_old)
 //   p = z + beta p, s = w + beta s, x += alpha p, r -= alpha s
