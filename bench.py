@@ -205,8 +205,8 @@ def _traffic(kernel, form, cg_iters, cg_predict=0, cg_batch=8):
     summary (profiles/traffic.json); the CG launch's bytes grow with its
     iteration count, so they are stored as prologue + per iteration, plus the
     predictor's own passes when one is on (None if that was not captured).
-    The staged CG kernel (cg_batch 32) has its own entry: its evict-first
-    matrix stream leaves the vectors in L2."""
+    The staged CG kernel (cg_batch 32: k_cn_two at this size) has its own
+    entry: its evict-first matrix stream leaves the vectors in L2."""
     try:
         with open(os.path.join(ROOT, "profiles", "traffic.json")) as f:
             t = json.load(f)
@@ -237,7 +237,9 @@ def algorithmic_bytes(kernel, n, nnz, cg_iters_per_solve, rbytes, nstate=19, ne=
       prologue  nnz*(A + B + col) + n*(x + dinv read + r, z, p write)
       iteration nnz*(A + col) + n*(z, p_old read + p_new, q write)         [phase A]
                 + n*(p_new, x, r, q, dinv read + x, r, z write)             [phase B]
-        (the textbook schedule's two passes; the kernels' one-pass sweep moves 11 vectors)
+        (the two passes of the recurrences, as k_cn_two runs them on meshes of
+        this size, which writes p beside z again in phase B; the one-pass sweep
+        of the other kernels moves 11 vectors instead of 12)
       predictor (cg_predict k = 1, 2): n*(the start correction read + V saved)
                 in the prologue (k = 2: the extrapolation the previous solve
                 stored), n*(x, V, k corrections read + x, k corrections

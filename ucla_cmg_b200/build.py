@@ -22,7 +22,8 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-fopenmp,-O3",
           "-I" + os.path.join(ROOT, "include"), "--expt-relaxed-constexpr"]
 # the learned step's per-node physics (gate update and current balance of the
 # hybrid form) stands beside a network whose own error is ~1e-3: fast
-# intrinsics there; every other file keeps IEEE expf/logf/division
+# intrinsics there; every other file keeps IEEE expf/logf and division, but for
+# the cell models' own FP32 quotient (csrc/common.cuh, dv)
 PER_FILE = {"surrogate.cu": ["--use_fast_math"]}
 
 

@@ -1764,8 +1764,10 @@ int cg_max_per_sm(int block, int *per, int batch, int variant, int depth, int pe
 // Batches the same with two CTAs per SM, which split the GPU more evenly
 // between the instances (24 slabs, 446K nodes FP32: 306 us from k_cn_half, 389
 // from the ring); in FP64, whose CTAs want the registers, with one up to a
-// quarter as many instances as SMs (24 slabs: 757 us, 849 with two; 8 slabs,
-// 155K nodes: 316, 372; 2 slabs, 15K: 149, 175).
+// quarter as many instances as SMs (CG us a step with one / two: 8 slabs, 155K
+// nodes 315 / 309; 24, 446K 625 / 723; 36, 667K 999 / 1031 and 111K 216 / 205;
+// beyond, 40 slabs of 123K 287 / 216, 72 of 222K 351 / 304 and of 1.3M 2592 /
+// 1901, though small ones still gain: 72 of 36K 119 / 151).
 // Any other launch config, and more instances than those CTAs, run k_cn_half, or
 // k_cn_two (cg_named_two), with CTAs of `block` threads, as many as fit.
 // slices a warp of k_cn_one takes (measured for each, FP32 / FP64, CG us a step:
