@@ -640,20 +640,26 @@ static int shape_batch(const ep_handle *h, int block, int per_sm, int batch, int
 static int plan_cg(ep_handle *h) {
     const int ws = stage_depth(h);
     int rc;
-    h->cg = CgShape{h->cg_batch, h->cg_block, 0, 0, 0, 0, 1.0f};
     const long long all_cols = matrix_cols(h);
-    const int batch = shape_batch(h, h->cg_block, h->cg_per_sm, h->cg_batch, h->cg_variant);
-    if (h->cg_per_sm == 0) {
-        rc = h->precision == EP_FP64
-                 ? cg_auto_shape<double>(h->nslices, all_cols, h->ninst, batch, h->cg_variant, ws, &h->cg)
-                 : cg_auto_shape<float>(h->nslices, all_cols, h->ninst, batch, h->cg_variant, ws, &h->cg);
-        h->cg_grid = h->cg.grid;
-    } else {
+    auto shape = [&](int batch) {
+        h->cg = CgShape{h->cg_batch, h->cg_block, 0, 0, 0, 0, 1.0f};
+        if (h->cg_per_sm == 0) {
+            const int r = h->precision == EP_FP64
+                     ? cg_auto_shape<double>(h->nslices, all_cols, h->ninst, batch, h->cg_variant, ws, &h->cg)
+                     : cg_auto_shape<float>(h->nslices, all_cols, h->ninst, batch, h->cg_variant, ws, &h->cg);
+            h->cg_grid = h->cg.grid;
+            return r;
+        }
         h->cg.batch = batch;
-        rc = h->precision == EP_FP64
+        return h->precision == EP_FP64
                  ? cg_grid_size<double>(h->cg_block, &h->cg_grid, h->cg_per_sm, batch, h->cg_variant, ws)
                  : cg_grid_size<float>(h->cg_block, &h->cg_grid, h->cg_per_sm, batch, h->cg_variant, ws);
-    }
+    };
+    const int batch = shape_batch(h, h->cg_block, h->cg_per_sm, h->cg_batch, h->cg_variant);
+    rc = shape(batch);
+    // an instance needs a CTA of its own: where the one-pass sweep's registers leave
+    // too few (768 threads, one an SM), the two-pass kernel's CTAs (two)
+    if (!rc && h->ninst > h->cg_grid && h->cg_variant == 0) rc = shape(batch | kTwo);
     if (rc) return rc;
     if (h->cg_variant == 1 && !h->w0.p) {
         const size_t vb = (size_t)h->pitch * h->rsize;
