@@ -84,9 +84,9 @@ template <typename R> struct SubSteps {
 };
 
 // one node's ionic phase (all sub-steps), counters accumulated by the caller.
-// False (Mahajan only): a sub-step wants to be redone in ten, which is left to
-// mh_group; nothing of the node is changed.
-template <typename R, int MODEL, int NS>
+// False (Mahajan without TEN only): a sub-step wants to be redone in ten, which is
+// left to a second pass; nothing of the node is changed.
+template <typename R, int MODEL, int NS, bool TEN = false>
 __device__ __forceinline__ bool ionic_node(const IonicArgs<R> &a, const int i, unsigned int &my_newton,
                                            unsigned int &my_caps, unsigned int &my_bad) {
     const long long step = *a.step_ptr;
@@ -121,11 +121,26 @@ __device__ __forceinline__ bool ionic_node(const IonicArgs<R> &a, const int i, u
             const R *__restrict__ c = a.consts + (size_t)ty * a.nconst;
             R r[26];
             s[0] = V;
-            mh_rhs(s, c, h, istim / (a.Cm * a.Xi), r);
-            dvdt = r[0];
-            if (mh_wants_substeps(dvdt, a.mh_abs)) return false;
+            // TEN: one call site for all evaluations; a single sub-step is known to
+            // want ten, its first one is skipped
+            bool ten = TEN && !a.stride && a.nsub == 1;
+            R he = ten ? h / R(10) : h;
+            if (ten) my_newton++;
+#pragma unroll 1
+            for (int e = ten ? 1 : 0; e <= (TEN ? 10 : 0); e++) {
+                mh_rhs(s, c, he, istim / (a.Cm * a.Xi), r);
+                dvdt = r[0];
+                if (e == 0 && mh_wants_substeps(dvdt, a.mh_abs)) {
+                    if (!TEN) return false;
+                    my_newton++;
+                    ten = true;
+                    he = h / R(10);
+                    continue;
+                }
 #pragma unroll
-            for (int j = 0; j < 26; j++) s[j] += r[j] * h;
+                for (int j = 0; j < 26; j++) s[j] += r[j] * he;
+                if (!ten) break;
+            }
         } else if constexpr (MODEL == EP_PURKINJE) {
             // the stimulus in uA/cm^3 and the model's (or the user's) Xi;
             // C_m does not enter (Purkinje.cc:183-213)
@@ -181,7 +196,15 @@ __device__ __forceinline__ void ionic_status(DevStatus *status, unsigned int my_
 // lane a node and each of the four warps one part of the rates (mh_part).
 // 214K nodes: 123 us a step to 41.  Bound by the latency of one evaluation's chain
 // for every chunk of the CTA, then ten parts' chains (some 20 us).
+// FP64 takes a list of more than two groups one thread a node: 128 nodes cost 105 us
+// (140 with two CTAs an SM), a group 45 (87), since its four parts are uneven and each
+// forms the logarithms and reciprocals that they share.  (A front along the node order,
+// 2 / 25 % of 67K nodes: 197 / 341 us a step in groups, 137 / 139 so; of 529K: 511 /
+// 1465, 338 / 745; in FP32 groups are never the slower ones: 128 nodes 55 us either way.)
+// The whole list by its length, so that a run repeats to the bit; the two ways differ
+// in the rounding of the compiler's fused products.
 constexpr int kMhChunks = 8;                     // chunks put aside together, at most
+constexpr int kMhMany = 65;
 template <typename R> struct MhShared {
     int list[kMhChunks * 128], count;
     R s[26][32];                                 // the group's states ([0] and [19] are registers)
@@ -300,9 +323,15 @@ __global__ void __launch_bounds__(128, MINB) k_mahajan(const IonicArgs<R> a, int
     }
     __syncthreads();
     const int count = sh.count;
-    for (int g = 0; g < count; g += 32) {
-        const int k = g + (threadIdx.x & 31);
-        mh_group(a, sh, sh.list[k < count ? k : g], k < count, my_newton, my_bad);
+    if (sizeof(R) == 8 && count >= kMhMany) {
+        unsigned int none = 0;
+        for (int k = threadIdx.x; k < count; k += 128)
+            ionic_node<R, EP_MAHAJAN, MH_NS, sizeof(R) == 8>(a, sh.list[k], my_newton, none, my_bad);
+    } else {
+        for (int g = 0; g < count; g += 32) {
+            const int k = g + (threadIdx.x & 31);
+            mh_group(a, sh, sh.list[k < count ? k : g], k < count, my_newton, my_bad);
+        }
     }
     ionic_status(a.status, my_newton, 0, my_bad, s_newton, s_caps, s_bad);
 }
