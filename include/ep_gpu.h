@@ -336,7 +336,8 @@ int  ep_assemble_operators(const ep_mesh_desc *mesh, const ep_cables_desc *cable
  * meshes, since every CTA takes part in each iteration's reduction; otherwise
  * at most as many as the kernel's registers let reside, e.g. with cg_batch 8,
  * 16 or 32 and cg_block 256 three in FP32 and two in FP64; matrices that stream
- * from DRAM run two passes an iteration there, with CTAs of fewer registers);
+ * from DRAM, and batches of more instances than those CTAs, run two passes an
+ * iteration there, with CTAs of fewer registers);
  * ionic_block: threads per CTA of the ionic kernel (64 or 128; Mahajan's always
  * has 128); graph_steps: 0 launches every kernel from the host, k > 0 replays the steps from an instantiated CUDA graph of k steps
  * (rounded up to a multiple of the ECG interval); ionic_min_ctas: FP32

@@ -10,7 +10,8 @@
 // slice, one warp per slice, one lane per row) so every value/column load is
 // a coalesced 128-byte transaction.  A and B share the column array.
 //
-// One grid barrier per iteration.  Neighbours see a node's (z, w), z = dinv r
+// One grid barrier per iteration (k_cn_two, for matrices that stream from DRAM,
+// has two).  Neighbours see a node's (z, w), z = dinv r
 // and w = dinv A p, double-buffered; p, q = A p and the correction d = x - V are
 // the owner's alone.  One sweep of an iteration rebuilds, for every column it
 // gathers, the neighbour's new z' = z - alpha w (an explicit fma, so the owner
