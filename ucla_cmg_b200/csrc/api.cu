@@ -1358,7 +1358,7 @@ static int put_voltage(ep_handle *h, const double *V) {
         int b, e;
         io_range(h->n, k, K, b, e);
         if (e <= b) continue;
-#pragma omp parallel for schedule(static) if (e - b >= (1 << 14))
+#pragma omp parallel for schedule(static) if (h->n >= (1 << 14))
         for (int i = b; i < e; i++) st[i] = (R)V[i];
         EP_CUDA(cudaMemcpyAsync(h->V.as<R>() + b, st + b, sizeof(R) * (e - b), cudaMemcpyHostToDevice, h->stream));
     }
